@@ -3,6 +3,7 @@ storm-nucleotide / storm-color command-line binaries linked against it.  Outputs
 source tree (storm_b200/lib, storm_b200/bin) so that they travel with the repository."""
 from __future__ import annotations
 
+import concurrent.futures
 import os
 import shutil
 import subprocess
@@ -13,7 +14,7 @@ LIB_DIR = os.path.join(PKG, "lib")
 BIN_DIR = os.path.join(PKG, "bin")
 LIB = os.path.join(LIB_DIR, "libstormgpu.so")
 HOST_LIB = os.path.join(LIB_DIR, "libstormhost.so")
-CU_SOURCES = ["stormgpu.cu", "index_build.cu", "map_kernels.cu", "sw_filter.cu", "gather.cu", "intpeak.cu", "align_noalloc.cu", "server.cu", "genome_map.cu", "genome_map_ctx.cu", "autotune.cu"]
+CU_SOURCES = ["stormgpu.cu", "index_build.cu", "map_kernels.cu", "sw_filter.cu", "score_bound.cu", "gather.cu", "intpeak.cu", "align_noalloc.cu", "server.cu", "genome_map.cu", "genome_map_ctx.cu", "autotune.cu"]
 HOST_SOURCES = ["host/storm_host.c", "host/storm_cli.c", "host/storm_gpu_main.c"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
@@ -54,12 +55,15 @@ def build(verbose: bool = False, force: bool = False) -> str:
     objdir = os.path.join(PKG, "_build")
     os.makedirs(objdir, exist_ok=True)
     if force or _stale(LIB, deps):
-        objs = []
+        objs, jobs = [], []
         for src in CU_SOURCES:
             obj = os.path.join(objdir, src.replace(".cu", ".o"))
             if force or _stale(obj, deps):
-                _run([nvcc()] + NVCC_FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj], verbose)
+                jobs.append([nvcc()] + NVCC_FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj])
             objs.append(obj)
+        with concurrent.futures.ThreadPoolExecutor(min(8, os.cpu_count() or 1)) as pool:
+            for f in [pool.submit(_run, j, verbose) for j in jobs]:
+                f.result()
         _run([nvcc(), "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", LIB] + objs + ["-cudart", "static"], verbose)
     if force or _stale(HOST_LIB, deps):
         _run(["gcc", "-O2", "-std=gnu11", "-fopenmp", "-fPIC", "-shared", "-o", HOST_LIB,

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "band_core.cuh"
 #include "common.cuh"
 #include "index_build.cuh"
 
@@ -92,12 +93,21 @@ struct stormgpu_ctx {
   sg::DevBuf<uint8_t> flag;       // pass byte per candidate
   sg::DevBuf<uint32_t> flagw;     // pass bits, one word per 32 candidates
   sg::DevBuf<uint8_t> rexp;
+  // score bound: passing candidates before it (p_read / p_diag hold those it keeps), read streams,
+  // its constants (bound_set: computed for this context's scores)
+  sg::DevBuf<int32_t> q_read, q_diag;
+  sg::DevBuf<int16_t> q_ub, p_ub;  // the bounds of both lists
+  sg::DevBuf<uint32_t> bstream, wstream;
+  sg::BandConst bound_c;
+  bool bound_set = false;
   sg::DevBuf<int32_t> a_score, a_bound, a_tblen, big_tmp;
   sg::DevBuf<int16_t> a_pos;
   sg::DevBuf<uint8_t> a_tb;
   sg::DevBuf<uint32_t> scratch;
-  sg::DevBuf<int32_t> thr, round_slots;  // alignment rounds: per-read threshold, per-round slot lists
-  sg::DevBuf<int64_t> rounds;           // [0, 8): slots per round, [8, 16): the lists' fill cursors
+  // replay: two lists of reads with candidates left; alignment rounds: per-read threshold and range of
+  // the last selection, the round's slots; per round the counts of both lists
+  sg::DevBuf<int32_t> active, thr, round_cur, round_slots;
+  sg::DevBuf<unsigned long long> rounds;
   sg::DevBuf<unsigned long long> counters;
   sg::DevBuf<uint32_t> ord, ord_tmp;  // length order of a mixed-length batch: sort keys and values, sort scratch
   cudaEvent_t ev[8];
@@ -109,10 +119,10 @@ struct stormgpu_ctx {
   // call: a batch that would exceed a pass's bounds at that density is cut up front instead of
   // after its gather
   double dens_cand = 0, dens_pass = 0;
-  // the same densities for the list sizes of a graph call: the larger of the last call's and
-  // 0.9 x the value before it, so that calls of different densities in turn (one read length
-  // after another) do not outgrow their lists each time
-  double gdens_cand = 0, gdens_pass = 0;
+  // the same densities, and that of the aligned candidates, for the list sizes of a graph call: the
+  // larger of the last call's and 0.9 x the value before it, so that calls of different densities
+  // in turn (one read length after another) do not outgrow their lists each time
+  double gdens_cand = 0, gdens_pass = 0, gdens_kept = 0;
   // CUDA graph of the strand passes: on unless turned off (stormgpu_set_graphs, STORMGPU_GRAPHS=0)
   // or broken (a capture or instantiation that failed turns it off for the context); the
   // executable graph of the last call, updated in place by the next call of the same shape; its

@@ -502,20 +502,22 @@ __device__ __forceinline__ int align_one_nuc(const ReadsDev& rd, const ScorePara
 // pb.cursor a persistent grid whose warps take the next 32 slots from the cursor (the slot
 // count read from pb.npass_dev when it is given; scratch column = the thread's index in the
 // grid, so the scratch holds align_workers() columns).
+// Resident blocks of 128 threads per SM the registers are bounded for: the packed form holds about
+// BWT registers of cells, the general one (scores and states apart) twice that.
+constexpr int align_blocks(int bw, int cm) {
+  return bw <= 0 ? 1 : cm == 2 ? (bw <= 15 ? 7 : bw <= 23 ? 6 : bw <= 31 ? 5 : 4) : (bw <= 15 ? 5 : bw <= 31 ? 4 : 3);
+}
+
 template <int BWT, int CM>
-__global__ void __launch_bounds__(128, CM == 2 ? (BWT > 0 && BWT <= 15 ? 7 : BWT == 31 ? 5 : BWT == 41 ? 4 : 1)
-                                              : (BWT > 0 && BWT <= 15 ? 5 : BWT == 31 ? 4 : BWT == 41 ? 3 : 1)) align_kernel(ReadsDev rd, ScoreParams sp, const uint8_t* __restrict__ genome,
+__global__ void __launch_bounds__(128, align_blocks(BWT, CM)) align_kernel(ReadsDev rd, ScoreParams sp,
+                                                    const uint8_t* __restrict__ genome,
                                                     const uint8_t* __restrict__ mask, int64_t slot0, int64_t nslots,
                                                     PassBuffers pb) {
   // one call site of align_one (its band code is large and fully unrolled)
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool steal = pb.cursor != nullptr;
   int64_t n = steal && pb.npass_dev ? *pb.npass_dev : nslots;
-  int64_t list0 = 0;  // with rounds: this round's slots are round_slots[list0 .. list0 + n)
-  if (pb.round_slots) {
-    n = pb.round_count[pb.round];
-    for (int k = 0; k < pb.round; ++k) list0 += pb.round_count[k];
-  }
+  if (pb.round_slots) n = (int64_t)*pb.round_count;  // with rounds: round_slots[0 .. n)
   const int64_t ns = steal ? (int64_t)gridDim.x * blockDim.x : nslots;
   const int lane = threadIdx.x & 31;
   const int take = pb.steal >= 32 ? pb.steal & ~31 : 32;
@@ -531,7 +533,7 @@ __global__ void __launch_bounds__(128, CM == 2 ? (BWT > 0 && BWT <= 15 ? 7 : BWT
       s += lane;
     }
     if (s < n) {
-      const int64_t slot = pb.round_slots ? (int64_t)pb.round_slots[list0 + s] : slot0 + s;
+      const int64_t slot = pb.round_slots ? (int64_t)pb.round_slots[s] : slot0 + s;
       if constexpr (CM == 2)
         rows += (unsigned long long)align_one_nuc<BWT>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb);
       else
@@ -546,10 +548,21 @@ __global__ void __launch_bounds__(128, CM == 2 ? (BWT > 0 && BWT <= 15 ? 7 : BWT
   }
 }
 
+// The packed nucleotide form has every band width up to 41 as a constant (the general form in local
+// memory ran -i 5 at 50 GCUPS, a twentieth of the packed form's rate); the others the widths of the
+// filter's own limits and of -i 20.
 static const void* align_kernel_of(const ScoreParams& sp) {
+  if (sp.packed) {
+#define SG_ALIGN(BW) case BW: return (const void*)align_kernel<BW, 2>;
+    switch (2 * sp.I + 1) {
+      SG_ALIGN(3) SG_ALIGN(5) SG_ALIGN(7) SG_ALIGN(9) SG_ALIGN(11) SG_ALIGN(13) SG_ALIGN(15) SG_ALIGN(17)
+      SG_ALIGN(19) SG_ALIGN(21) SG_ALIGN(23) SG_ALIGN(25) SG_ALIGN(27) SG_ALIGN(29) SG_ALIGN(31) SG_ALIGN(33)
+      SG_ALIGN(35) SG_ALIGN(37) SG_ALIGN(39) SG_ALIGN(41)
+    }
+#undef SG_ALIGN
+  }
 #define SG_ALIGN(BW) \
-  case BW: return sp.colour ? (const void*)align_kernel<BW, 1> \
-                  : sp.packed ? (const void*)align_kernel<BW, 2> : (const void*)align_kernel<BW, 0>;
+  case BW: return sp.colour ? (const void*)align_kernel<BW, 1> : (const void*)align_kernel<BW, 0>;
   switch (2 * sp.I + 1) {
     SG_ALIGN(7)
     SG_ALIGN(15)
@@ -583,149 +596,230 @@ __device__ __forceinline__ int tbget(const uint8_t* t, int i) { return (t[i >> 1
 // threshold starting at -t for every (sequence, strand, read): aborted iff the bound is
 // below the running threshold; accepted iff not aborted and score > threshold; then
 // hit_map__update (hit_map.c:50-144) and threshold = max(threshold, 4th score).
-// With rounds, the ranks [lo, hi) of each read, starting from the threshold the ranks before
-// left in pb.thr (the first round starts from -t), which it updates.
-__global__ void replay_kernel(int64_t n, ScoreParams sp, int ref_id, int sense, PassBuffers pb, int lo, int hi,
-                              stormgpu_hit* __restrict__ hits, uint8_t* __restrict__ tbo, int64_t tbs,
-                              uint8_t* __restrict__ mapped) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  const int P = pb.pcount[r];
-  if (P <= lo) return;
-  const int64_t s0 = pb.pstart[r];
-  int T = (pb.thr && lo > 0) ? pb.thr[r] : sp.min_score;
-  stormgpu_hit* h = hits + r * 4;
-  const int kend = P < hi ? P : hi;
-  for (int k = lo; k < kend; ++k) {
-    const int64_t slot = s0 + k;
-    const int score = pb.a_score[slot];
-    if (!(pb.a_bound[slot] >= T && score > T)) continue;
-    const int win = max(pb.p_diag[slot] - sp.I, -sp.Is);
-    const int bi = pb.a_pos[slot * 4 + 0], bj = pb.a_pos[slot * 4 + 1];
-    const int i0 = pb.a_pos[slot * 4 + 2], j0 = pb.a_pos[slot * 4 + 3];
-    mapped[r] = 1;
-    int q;
-    bool dup_worse = false;
-    for (q = 0; q < 4 && h[q].ref_id != -1; ++q) {
-      if (h[q].ref_id == ref_id &&
-          ((h[q].ref_start == win + j0 && h[q].read_start == i0) ||
-           (h[q].ref_end == win + bj && h[q].read_end == bi))) {
-        if (score > h[q].score) break;
-        dup_worse = true;
-        break;
-      }
+//
+// One warp per read: the lanes test 32 candidates at once against the threshold (few of a read's
+// hundreds exceed it), lane 0 runs the update for those that do, on the read's four hits in shared
+// memory, and the threshold it leaves is tested again.  Tracebacks are written once, at the end, from
+// where each surviving hit came from.
+//
+// The warps go over a list of reads, those with candidates left (pb.active): slot_lists_kernel fills
+// the first one, each round's replay the next, so that a round in which few reads have work costs a
+// launch and no more.
+//
+// With rounds (pb.round_slots) the kernel replays the ranks its read's last selection covered and
+// then selects the next ones: the ranks from there on whose score bound exceeds the threshold (all,
+// without bounds), up to `take` of them (0: none left to select), appended to the next round's list;
+// ranks passed over are marked as below every threshold.  Each round quadruples or so the ranks a
+// read has behind it, and of those after them only about 4 per (ranks seen) can still enter the
+// four hits, so nearly every later candidate is dropped by its bound alone.
+constexpr int kReplayWarps = 4;
+
+// hit_map__update for one accepted candidate on h[4] (src: where each hit's traceback is, -1 - row
+// for a row already in place, else the slot).
+__device__ __forceinline__ void hit_update(stormgpu_hit* h, int64_t* src, const PassBuffers& pb, const ScoreParams& sp,
+                                           int64_t slot, int score, int ref_id, int sense) {
+  const int win = max(pb.p_diag[slot] - sp.I, -sp.Is);
+  const int bi = pb.a_pos[slot * 4 + 0], bj = pb.a_pos[slot * 4 + 1];
+  const int i0 = pb.a_pos[slot * 4 + 2], j0 = pb.a_pos[slot * 4 + 3];
+  int q;
+  for (q = 0; q < 4 && h[q].ref_id != -1; ++q) {
+    if (h[q].ref_id == ref_id && ((h[q].ref_start == win + j0 && h[q].read_start == i0) ||
+                                  (h[q].ref_end == win + bj && h[q].read_end == bi))) {
+      if (score > h[q].score) break;
+      return;  // the same place with a score at least as high
     }
-    if (!dup_worse) {
-      if (q == 4) q--;
-      int i = q;
-      while (i >= 0 && score > h[i].score) i--;
-      if (i != 3) {
-        for (int j = q; j > i + 1; --j) {
-          h[j] = h[j - 1];
-          for (int64_t b = 0; b < tbs; ++b) tbo[(r * 4 + j) * tbs + b] = tbo[(r * 4 + j - 1) * tbs + b];
-        }
-        stormgpu_hit nh;
-        nh.score = score;
-        nh.ref_id = ref_id;
-        nh.ref_start = win + j0;
-        nh.ref_end = win + bj;
-        nh.read_start = (int16_t)i0;
-        nh.read_end = (int16_t)bi;
-        nh.sense = sense;
-        const int tl = pb.a_tblen[slot];
-        nh.tb_len = tl;
-        h[i + 1] = nh;
-        uint8_t* dst = tbo + (r * 4 + i + 1) * tbs;
-        const uint8_t* srcb = pb.a_tb + slot * pb.tbs;
-        for (int64_t b = 0; b < tbs; ++b) dst[b] = 0;
-        for (int p = 0; p < tl; ++p) {
-          int v = tbget(srcb, tl - 1 - p);
-          if (p & 1) dst[p >> 1] |= (uint8_t)v;
-          else dst[p >> 1] |= (uint8_t)(v << 4);
-        }
-      }
-    }
-    if (h[3].score > T) T = h[3].score;
   }
-  if (pb.thr) pb.thr[r] = T;
+  if (q == 4) q--;
+  int i = q;
+  while (i >= 0 && score > h[i].score) i--;
+  if (i == 3) return;
+  for (int j = q; j > i + 1; --j) {
+    h[j] = h[j - 1];
+    src[j] = src[j - 1];
+  }
+  stormgpu_hit nh;
+  nh.score = score;
+  nh.ref_id = ref_id;
+  nh.ref_start = win + j0;
+  nh.ref_end = win + bj;
+  nh.read_start = (int16_t)i0;
+  nh.read_end = (int16_t)bi;
+  nh.sense = sense;
+  nh.tb_len = pb.a_tblen[slot];
+  h[i + 1] = nh;
+  src[i + 1] = slot;
 }
 
-void launch_replay(int64_t n, const ScoreParams& sp, int ref_id, int sense, PassBuffers& pb,
+__device__ __forceinline__ void replay_read(int64_t r, const ScoreParams& sp, int ref_id, int sense, const PassBuffers& pb,
+                                            int take, stormgpu_hit* __restrict__ hits, uint8_t* __restrict__ tbo,
+                                            int64_t tbs, uint8_t* __restrict__ mapped, stormgpu_hit* h, int64_t* src) {
+  const int lane = threadIdx.x & 31;
+  const int P = pb.pcount[r];
+  const int64_t s0 = pb.pstart[r];
+  const bool rounds = pb.round_slots != nullptr;
+  int lo = 0, hi = P, T = sp.min_score;
+  if (rounds) {
+    lo = pb.round_cur[2 * r];
+    hi = pb.round_cur[2 * r + 1];
+    if (pb.round > 0) T = pb.thr[r];
+  }
+  {
+    bool loaded = false;
+    for (int base = lo; base < hi; base += 32) {
+      const int k = base + lane;
+      const bool in = k < hi;
+      const int score = in ? pb.a_score[s0 + k] : kMinScore;
+      const int bound = in && score > T ? pb.a_bound[s0 + k] : kMinScore;
+      unsigned m = __ballot_sync(0xffffffffu, in && score > T && bound >= T);
+      if (m && !loaded) {
+        loaded = true;
+        const int32_t* g = reinterpret_cast<const int32_t*>(hits + r * 4);
+        if (lane < 28) reinterpret_cast<int32_t*>(h)[lane] = g[lane];
+        if (lane < 4) src[lane] = -1 - lane;
+        __syncwarp();
+      }
+      while (m) {
+        const int l = __ffs(m) - 1;
+        const int sc = __shfl_sync(0xffffffffu, score, l);
+        if (lane == 0) {
+          hit_update(h, src, pb, sp, s0 + base + l, sc, ref_id, sense);
+          if (h[3].score > T) T = h[3].score;
+        }
+        T = __shfl_sync(0xffffffffu, T, 0);
+        m = __ballot_sync(0xffffffffu, in && lane > l && score > T && bound >= T);
+      }
+    }
+    if (loaded) {
+      __syncwarp();
+      if (lane == 0) mapped[r] = 1;
+      int32_t* g = reinterpret_cast<int32_t*>(hits + r * 4);
+      if (lane < 28) g[lane] = reinterpret_cast<const int32_t*>(h)[lane];
+      // rows in place only move to higher ranks: the highest rank first, every source is intact
+      for (int q = 3; q >= 0; --q) {
+        const int64_t f = src[q];
+        if (f == -1 - q) continue;
+        uint8_t* dst = tbo + (r * 4 + q) * tbs;
+        if (f < 0) {
+          const uint8_t* from = tbo + (r * 4 + (-1 - f)) * tbs;
+          for (int64_t b = lane; b < tbs; b += 32) dst[b] = from[b];
+        } else {
+          const uint8_t* from = pb.a_tb + f * pb.tbs;
+          const int tl = h[q].tb_len;
+          for (int64_t b = lane; b < tbs; b += 32) {
+            const int p = (int)(2 * b);
+            int v = 0;
+            if (p < tl) v = tbget(from, tl - 1 - p) << 4;
+            if (p + 1 < tl) v |= tbget(from, tl - 2 - p);
+            dst[b] = (uint8_t)v;
+          }
+        }
+        __syncwarp();
+      }
+    }
+  }
+  if (!rounds) return;
+  // the next round's candidates
+  int end = hi, left = take;
+  bool any = false;
+  while (left > 0 && end < P) {
+    const int k = end + lane;
+    const bool in = k < P;
+    const bool may = in && (!pb.ub || pb.ub[s0 + k] > T);
+    unsigned m = __ballot_sync(0xffffffffu, may);
+    int stop = min(32, P - end);
+    if (__popc(m) >= left) {  // ends at the last one taken
+      for (int over = __popc(m) - left; over > 0; --over) m &= ~(1u << (31 - __clz(m)));
+      stop = 32 - __clz(m);
+    }
+    left -= __popc(m);
+    any |= m != 0;
+    unsigned long long b = 0;
+    if (lane == 0 && m) b = atomicAdd(pb.round_count + 1, (unsigned long long)__popc(m));
+    b = __shfl_sync(0xffffffffu, b, 0);
+    if ((m >> lane) & 1u) pb.round_slots[b + __popc(m & ((1u << lane) - 1u))] = (int32_t)(s0 + k);
+    else if (lane < stop) pb.a_score[s0 + k] = kMinScore;
+    end += stop;
+  }
+  if (lane == 0 && any) {  // a read with no candidate left to select is done
+    pb.round_cur[2 * r] = hi;
+    pb.round_cur[2 * r + 1] = end;
+    pb.thr[r] = T;
+    pb.active_next[atomicAdd(pb.active_count + 1, 1)] = (int32_t)r;
+  }
+}
+
+__global__ void __launch_bounds__(kReplayWarps * 32) replay_kernel(ScoreParams sp, int ref_id, int sense, PassBuffers pb,
+                                                                   int take, stormgpu_hit* __restrict__ hits,
+                                                                   uint8_t* __restrict__ tbo, int64_t tbs,
+                                                                   uint8_t* __restrict__ mapped) {
+  __shared__ stormgpu_hit sh_hits[kReplayWarps][4];
+  __shared__ int64_t sh_src[kReplayWarps][4];
+  const int w = threadIdx.x >> 5;
+  const int n = *pb.active_count;
+  for (int k = blockIdx.x * kReplayWarps + w; k < n; k += gridDim.x * kReplayWarps) {
+    replay_read(pb.active[k], sp, ref_id, sense, pb, take, hits, tbo, tbs, mapped, sh_hits[w], sh_src[w]);
+    __syncwarp();
+  }
+}
+
+void launch_replay(int64_t n, const ScoreParams& sp, int ref_id, int sense, PassBuffers& pb, int take,
                    stormgpu_hit* hits, uint8_t* tb, int64_t tbs, uint8_t* mapped, cudaStream_t st) {
   if (n <= 0) return;
-  replay_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(n, sp, ref_id, sense, pb, 0, 0x7fffffff, hits, tb, tbs,
-                                                             mapped);
+  const int64_t blocks = std::min<int64_t>((n + kReplayWarps - 1) / kReplayWarps,
+                                           resident_grid(replay_kernel, kReplayWarps * 32));
+  replay_kernel<<<(unsigned)blocks, kReplayWarps * 32, 0, st>>>(sp, ref_id, sense, pb, take, hits, tb, tbs, mapped);
 }
 
-void launch_replay_round(int64_t n, const ScoreParams& sp, int ref_id, int sense, PassBuffers& pb, int rounds,
-                         stormgpu_hit* hits, uint8_t* tb, int64_t tbs, uint8_t* mapped, cudaStream_t st) {
-  if (n <= 0) return;
-  const int lo = align_round_bound(pb.round, rounds), hi = align_round_bound(pb.round + 1, rounds);
-  replay_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(n, sp, ref_id, sense, pb, lo, hi, hits, tb, tbs, mapped);
+// ------------------------------------------------------------------------------ slots of a read
+
+__global__ void slot_starts_kernel(int64_t npass, const int64_t* __restrict__ npass_dev,
+                                   const int32_t* __restrict__ p_read, int32_t* __restrict__ pstart) {
+  if (npass_dev) npass = *npass_dev;
+  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < npass; s += (int64_t)gridDim.x * blockDim.x) {
+    const int r = p_read[s];
+    if (s == 0 || p_read[s - 1] != r) pstart[r] = (int32_t)s;
+  }
 }
 
-// ------------------------------------------------------------------------------ rounds
-
-__device__ __forceinline__ int round_of_rank(int rank, int rounds) {
-  int k = 0;
-  while (k + 1 < rounds && rank >= align_round_bound(k + 1, rounds)) ++k;
-  return k;
-}
-
-// per round: slots whose rank falls in it (one atomic per warp and round)
-__global__ void round_count_kernel(int64_t npass, const int64_t* __restrict__ npass_dev, int rounds,
-                                   const int32_t* __restrict__ p_read, const int32_t* __restrict__ pstart,
-                                   int64_t* __restrict__ count) {
+// Per read its number of slots, the list of reads with slots, and with rounds the first round's
+// slots: the first `take` of each read (their bounds exceed -t, the threshold it starts from).
+__global__ void slot_lists_kernel(int64_t npass, const int64_t* __restrict__ npass_dev, PassBuffers pb, int take) {
   if (npass_dev) npass = *npass_dev;
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < npass; base += stride) {
     const int64_t s = base + lane;
-    const int k = s < npass ? round_of_rank((int)(s - pstart[p_read[s]]), rounds) : -1;
-    for (int j = 0; j < rounds; ++j) {
-      const unsigned m = __ballot_sync(0xffffffffu, k == j);
-      if (m && lane == 0) atomicAdd(reinterpret_cast<unsigned long long*>(&count[j]), (unsigned long long)__popc(m));
-    }
-  }
-}
-
-// the lists: a warp's slots of one round go out together, in slot order
-__global__ void round_scatter_kernel(int64_t npass, const int64_t* __restrict__ npass_dev, int rounds,
-                                     const int32_t* __restrict__ p_read, const int32_t* __restrict__ pstart,
-                                     const int64_t* __restrict__ count, unsigned long long* __restrict__ cursors,
-                                     int32_t* __restrict__ slots) {
-  if (npass_dev) npass = *npass_dev;
-  const int lane = threadIdx.x & 31;
-  int64_t start[kMaxAlignRounds];
-  int64_t acc = 0;
-  for (int j = 0; j < kMaxAlignRounds; ++j) {
-    start[j] = acc;
-    if (j < rounds) acc += count[j];
-  }
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < npass; base += stride) {
-    const int64_t s = base + lane;
-    const int k = s < npass ? round_of_rank((int)(s - pstart[p_read[s]]), rounds) : -1;
-    for (int j = 0; j < rounds; ++j) {
-      const unsigned m = __ballot_sync(0xffffffffu, k == j);
-      if (!m) continue;
-      unsigned long long b = 0;
-      if (lane == 0) b = atomicAdd(&cursors[j], (unsigned long long)__popc(m));
+    const bool in = s < npass;
+    const int r = in ? pb.p_read[s] : -1;
+    const int rank = in ? (int)(s - pb.pstart[r]) : -1;
+    const bool last = in && (s == npass - 1 || pb.p_read[s + 1] != r);
+    if (last) pb.pcount[r] = rank + 1;
+    const unsigned mf = __ballot_sync(0xffffffffu, rank == 0);
+    if (mf) {
+      int b = 0;
+      if (lane == 0) b = atomicAdd(pb.active_count, __popc(mf));
       b = __shfl_sync(0xffffffffu, b, 0);
-      if (k == j) slots[start[j] + (int64_t)b + __popc(m & ((1u << lane) - 1u))] = (int32_t)s;
+      if (rank == 0) pb.active[b + __popc(mf & ((1u << lane) - 1u))] = r;
+    }
+    if (!pb.round_slots) continue;
+    const bool sel = in && rank < take;
+    if (rank == 0) pb.round_cur[2 * r] = 0;
+    if (sel && (last || rank == take - 1)) pb.round_cur[2 * r + 1] = rank + 1;
+    const unsigned m = __ballot_sync(0xffffffffu, sel);
+    if (m) {
+      unsigned long long b = 0;
+      if (lane == 0) b = atomicAdd(pb.round_count, (unsigned long long)__popc(m));
+      b = __shfl_sync(0xffffffffu, b, 0);
+      if (sel) pb.round_slots[b + __popc(m & ((1u << lane) - 1u))] = (int32_t)s;
     }
   }
 }
 
-void launch_round_lists(int64_t npass, const int64_t* npass_dev, int rounds, const int32_t* p_read,
-                        const int32_t* pstart, int64_t* round_count, unsigned long long* cursors, int32_t* round_slots,
-                        cudaStream_t st) {
+void launch_slot_lists(int64_t npass, const int64_t* npass_dev, PassBuffers& pb, int take, cudaStream_t st) {
   if (npass <= 0) return;
-  int64_t blocks = (npass + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  round_count_kernel<<<(unsigned)blocks, 256, 0, st>>>(npass, npass_dev, rounds, p_read, pstart, round_count);
-  round_scatter_kernel<<<(unsigned)blocks, 256, 0, st>>>(npass, npass_dev, rounds, p_read, pstart, round_count,
-                                                         cursors, round_slots);
+  const int64_t blocks = std::min<int64_t>((npass + 255) / 256, 148 * 32);
+  slot_starts_kernel<<<(unsigned)blocks, 256, 0, st>>>(npass, npass_dev, pb.p_read, pb.pstart);
+  slot_lists_kernel<<<(unsigned)blocks, 256, 0, st>>>(npass, npass_dev, pb, take);
 }
 
 }  // namespace sg

@@ -49,8 +49,13 @@ struct IndexView {
 
 struct PassBuffers {
   // filter -> flat list of passing candidates
-  int32_t* pstart;      // per read: first slot
-  int32_t* pcount;      // per read: number of passing candidates
+  int32_t* pstart;      // per read with candidates: first slot
+  int32_t* pcount;      // and their number
+  // reads with candidates left: the list of this replay (count at active_count[0]) and of the next
+  // (active_count[1])
+  int32_t* active;
+  int32_t* active_next;
+  int32_t* active_count;
   int32_t* p_read;      // per slot
   int32_t* p_diag;
   int64_t p_cap;
@@ -69,23 +74,24 @@ struct PassBuffers {
   unsigned long long* cursor;
   const int64_t* npass_dev;  // may be null; else the slot count is read from here
   int steal;                 // with a cursor: slots a warp takes at a time, a multiple of 32 (0 = 32)
-  // Rounds (all null for one round over every slot).  The passing candidates of a read are
-  // aligned in rounds of increasing rank (rank = slot - pstart[read]): round k takes the ranks
-  // [align_round_bound(k), align_round_bound(k + 1)), listed in round_slots after the lists of
-  // the rounds before it (round_count[k] slots); thr[read] holds the replay's running threshold
-  // after the rounds before, below which a candidate can no longer be accepted, so that its
-  // alignment may stop there.
-  const int32_t* round_slots;
-  const int64_t* round_count;  // [kMaxAlignRounds]
+  // Rounds (all null for one round over every slot).  The candidates of a read are aligned in rounds:
+  // each takes its next candidates that may still exceed the read's running threshold (see
+  // replay_kernel), listed in round_slots, round_count[0] of them (round_count[1]: of the next round); thr[read] holds the replay's running
+  // threshold after the rounds before, below which a candidate can no longer be accepted, so that its
+  // alignment may stop there; round_cur[2 read], [2 read + 1] the ranks the last selection covered.
+  const int16_t* ub;           // may be null; per slot, an upper bound of its score
+  int32_t* round_slots;
+  unsigned long long* round_count;
   int round;                   // the round of this launch
+  int32_t* round_cur;
   int32_t* thr;                // per read; written by the replay of each round
   unsigned long long* cells;   // may be null; += band cells the alignment computed
 };
 
 constexpr int kMaxAlignRounds = 6;
-// first rank of each round: 0, 8, 32, 128, 512, 2048, then every rank left
-__host__ __device__ __forceinline__ int align_round_bound(int k, int rounds) {
-  return k <= 0 ? 0 : k >= rounds ? 0x7fffffff : 8 << (2 * (k - 1));
+// candidates of a read in round k: 8, 16, 32, ...; in the last round all that are left
+__host__ __device__ __forceinline__ int align_round_take(int k, int rounds) {
+  return k >= rounds ? 0 : k == rounds - 1 ? 0x7fffffff : 8 << k;
 }
 
 void launch_reverse_reads(const ReadsDev& in, const uint8_t* first_levels, int colour,
@@ -97,18 +103,13 @@ void launch_align(const ReadsDev& r, const ScoreParams& sp, const uint8_t* genom
                   cudaStream_t st);
 // scratch columns of a launch_align with a cursor (the threads of its persistent grid)
 int64_t align_workers(int64_t nslots, const ScoreParams& sp);
-void launch_replay(int64_t n, const ScoreParams& sp, int ref_id, int sense, PassBuffers& pb,
+// pstart / pcount and the first active list of the pass's slots (npass of them, or with npass_dev (may
+// be null) an upper bound for the grid and the count is read from there); with rounds the first
+// round's slots, `take` per read.  The counts are zeroed by the caller.
+void launch_slot_lists(int64_t npass, const int64_t* npass_dev, PassBuffers& pb, int take, cudaStream_t st);
+// Replay of the active reads (at most n): the whole read (no rounds), or the ranks selected last and
+// then the selection of up to `take` candidates for the next round.
+void launch_replay(int64_t n, const ScoreParams& sp, int ref_id, int sense, PassBuffers& pb, int take,
                    stormgpu_hit* hits, uint8_t* tb, int64_t tbs, uint8_t* mapped, cudaStream_t st);
-// The slots of every round of a pass, in slot order within a warp's run: counts into
-// round_count (zeroed by the caller), then the lists into round_slots.  `cursors` holds
-// `rounds` zeroed counters.  With npass_dev (may be null) npass is an upper bound for the grid
-// and the slot count is read from there.
-void launch_round_lists(int64_t npass, const int64_t* npass_dev, int rounds, const int32_t* p_read,
-                        const int32_t* pstart, int64_t* round_count, unsigned long long* cursors, int32_t* round_slots,
-                        cudaStream_t st);
-// Replay of round pb.round (the ranks of that round), continuing from pb.thr.
-void launch_replay_round(int64_t n, const ScoreParams& sp, int ref_id, int sense, PassBuffers& pb, int rounds,
-                         stormgpu_hit* hits, uint8_t* tb, int64_t tbs, uint8_t* mapped, cudaStream_t st);
-
 
 }  // namespace sg

@@ -14,6 +14,7 @@
 #include "map_kernels.cuh"
 #include "scan.cuh"
 #include "sw_filter.cuh"
+#include "score_bound.cuh"
 #include "gather.cuh"
 #include "radix.cuh"
 #include "context.cuh"
@@ -204,10 +205,11 @@ extern "C" void stormgpu_close(stormgpu_ctx* c) {
   c->a_pos.release(); c->a_tb.release(); c->scratch.release(); c->counters.release();
   c->foff.release(); c->fr.release(); c->fd.release(); c->flag.release(); c->flagw.release();
   c->rexp.release();
+  c->q_read.release(); c->q_diag.release(); c->q_ub.release(); c->p_ub.release(); c->bstream.release(); c->wstream.release();
   c->gm_k0.release(); c->gm_v0.release(); c->gm_k1.release(); c->gm_v1.release(); c->gm_tmp.release();
   c->gm_base.release();
   c->ord.release(); c->ord_tmp.release();
-  c->thr.release(); c->round_slots.release(); c->rounds.release();
+  c->thr.release(); c->active.release(); c->round_cur.release(); c->round_slots.release(); c->rounds.release();
   for (auto& e : c->ev) cudaEventDestroy(e);
   for (auto& e : c->rev) cudaEventDestroy(e);
   cudaStreamDestroy(c->st);
@@ -314,7 +316,7 @@ constexpr int kGraphRetry = 2;
 // words of the graph's device state (c->gstate)
 enum : int {
   kGsCand = 0,    // candidates the filter of the current pass takes (0: skipped)
-  kGsPass,        // passing candidates the alignment of the current pass takes (0: skipped)
+  kGsPass,        // passing candidates the score bound of the current pass takes (0: skipped)
   kGsStatus,      // 1: a list outgrew its capacity, 2: the batch must be cut, 4: too many passing
   kGsLookups,     // sums over the passes of the stage counters
   kGsPositions,
@@ -325,6 +327,9 @@ enum : int {
   kGsPassed,
   kGsMaxCand,     // densest pass
   kGsMaxPass,
+  kGsKept,        // candidates the alignment of the current pass takes (0: skipped)
+  kGsAligned,     // their sum over the passes
+  kGsMaxKept,
   kGsWords = 16
 };
 
@@ -355,6 +360,18 @@ static __global__ void gate_filter_kernel(const int64_t* __restrict__ total, int
   if ((unsigned long long)p > gs[kGsMaxPass]) gs[kGsMaxPass] = (unsigned long long)p;
 }
 
+// total: candidates the score bound kept
+static __global__ void gate_bound_kernel(const int64_t* __restrict__ total, int64_t kept_cap,
+                                         unsigned long long* __restrict__ gs) {
+  const int64_t p = *total;
+  unsigned long long s = gs[kGsStatus];
+  if (p > kept_cap) s |= 4;
+  gs[kGsStatus] = s;
+  gs[kGsKept] = s ? 0 : (unsigned long long)p;
+  if (!s) gs[kGsAligned] += (unsigned long long)p;
+  if ((unsigned long long)p > gs[kGsMaxKept]) gs[kGsMaxKept] = (unsigned long long)p;
+}
+
 static __global__ void pass_sums_kernel(const unsigned long long* __restrict__ counters,
                                         unsigned long long* __restrict__ gs) {
   gs[kGsCandidates] += counters[5];
@@ -363,14 +380,17 @@ static __global__ void pass_sums_kernel(const unsigned long long* __restrict__ c
   gs[kGsAlignCells] += counters[13];
 }
 
-static void set_densities(stormgpu_ctx* c, double cand, double pass) {
+static void set_densities(stormgpu_ctx* c, double cand, double pass, double kept) {
   c->dens_cand = cand;
   c->dens_pass = pass;
   c->gdens_cand = std::max(cand, 0.9 * c->gdens_cand);
   c->gdens_pass = std::max(pass, 0.9 * c->gdens_pass);
+  c->gdens_kept = std::max(kept, 0.9 * c->gdens_kept);
 }
 
 // What the passes of one call share (set up by map_device_once before them).
+constexpr int kRoundCounts = kMaxAlignRounds + 1;
+
 struct PassSetup {
   ScoreParams sp;
   ReadsDev fwd, rev;
@@ -378,48 +398,106 @@ struct PassSetup {
   int maxL, minL;
   double wsum;
   int wpr;          // scratch words per row of an alignment
-  int64_t tbs;      // traceback bytes per passing candidate
+  int64_t tbs;      // traceback bytes per aligned candidate
+  int rounds;       // alignment rounds
+  int bound_H;      // band registers of the score bound, 0: every passing candidate is aligned
   stormgpu_results* out;
+};
+
+// The score bound of one pass: streams of its reads, then the flags of the passing candidates
+// (q_read, q_diag), read from n_dev when given.
+static void launch_bound_pass(stormgpu_ctx* c, const PassSetup& P, const ReadsDev& rd, const RefSeq& R, int64_t n,
+                              const int64_t* n_dev, cudaStream_t st) {
+  const int64_t words = band_stream_words(P.maxL, P.bound_H);
+  launch_band_streams(rd, P.bound_H, words, c->bstream.p, rd.levels ? c->wstream.p : nullptr, c->bound_c, st);
+  BoundJob job;
+  memset(&job, 0, sizeof(job));
+  job.n = n; job.n_dev = n_dev; job.read = c->q_read.p; job.diag = c->q_diag.p; job.lengths = rd.lengths;
+  job.gexp = R.d_gexp; job.rs = c->bstream.p; job.ws = rd.levels ? c->wstream.p : nullptr; job.words = words;
+  job.H = P.bound_H; job.I = P.sp.I; job.Is = P.sp.Is; job.min_score = P.sp.min_score;
+  job.match = P.sp.pair[0][3]; job.mismatch = -P.sp.pair[1][3];
+  job.flag = c->flag.p; job.ub = c->q_ub.p;
+  launch_score_bound(job, c->bound_c, st);
+}
+
+// Buffers of the replay's lists: two lists of active reads, and with rounds the round's slots.
+static int round_lists_grow(stormgpu_ctx* c, int64_t n, int64_t kept, int rounds) {
+  if (c->active.grow(2 * n) || c->rounds.grow(2 * kRoundCounts)) return STORMGPU_ENOMEM;
+  if (rounds > 1 && (c->thr.grow(n) || c->round_cur.grow(2 * n) || c->round_slots.grow(kept))) return STORMGPU_ENOMEM;
+  return 0;
+}
+
+// Their pointers for round k.
+static void round_buffers(stormgpu_ctx* c, int k, PassBuffers& pb) {
+  const int64_t half = c->active.cap / 2;
+  pb.round = k;
+  pb.round_count = c->rounds.p + k;
+  pb.active = c->active.p + (k & 1 ? half : 0);
+  pb.active_next = c->active.p + (k & 1 ? 0 : half);
+  pb.active_count = reinterpret_cast<int32_t*>(c->rounds.p + kRoundCounts) + k;
+  pb.cursor = c->counters.p + 16 + k;  // zeroed with the counters of the pass
+}
+
+static int setup_rounds(stormgpu_ctx* c, int rounds, PassBuffers& pb, cudaStream_t st) {
+  SG_CUDA(cudaMemsetAsync(c->rounds.p, 0, sizeof(unsigned long long) * 2 * kRoundCounts, st));
+  round_buffers(c, 0, pb);
+  if (rounds > 1) {
+    pb.round_slots = c->round_slots.p;
+    pb.round_cur = c->round_cur.p;
+    pb.thr = c->thr.p;
+  }
+  return 0;
+}
+
+// List capacities of a graph call.
+struct GraphCaps {
+  int64_t cand, pass, kept;
+  int64_t grid_h;  // blocks of the gather for the reads with the most positions
 };
 
 // The lists a graph call needs (false: they could not be allocated, and the call runs without a
 // graph).
-static bool graph_buffers(stormgpu_ctx* c, const PassSetup& P, int64_t* cand_cap, int64_t* pass_cap,
-                          int64_t* grid_h) {
+static bool graph_buffers(stormgpu_ctx* c, const PassSetup& P, GraphCaps* caps) {
   const int64_t n = P.n;
-  const int64_t want_cand = (int64_t)(c->gdens_cand * P.wsum * 1.25) + 65536;
+  const int64_t want_cand = (int64_t)(c->gdens_cand * P.wsum * 1.25) + 61440;  // small calls: one scan block
   const int64_t want_pass = (int64_t)(c->gdens_pass * P.wsum * 1.25) + 4096;
+  const int64_t want_kept = P.bound_H ? (int64_t)(c->gdens_kept * P.wsum * 1.25) + 4096 : want_pass;
   const int64_t grid_b = gather_block_grid(false);
-  *grid_h = std::max<int64_t>(1, std::min<int64_t>(grid_b, ((int64_t)1 << 25) / c->huge_cap));
-  const int rounds = std::max(1, std::min<int>(c->tune.align_rounds, kMaxAlignRounds));
+  caps->grid_h = std::max<int64_t>(1, std::min<int64_t>(grid_b, ((int64_t)1 << 25) / c->huge_cap));
   if (c->fr.grow(want_cand) || c->fd.grow(want_cand) || c->big_count.grow(4) || c->gstate.grow(kGsWords) ||
-      c->big_tmp.grow(std::max(grid_b * 2 * (int64_t)kBlockGatherCap, *grid_h * 2 * c->huge_cap)) ||
+      c->big_tmp.grow(std::max(grid_b * 2 * (int64_t)kBlockGatherCap, caps->grid_h * 2 * c->huge_cap)) ||
       c->rexp.grow(n * rexp_stride(P.maxL)))
     return false;
-  *cand_cap = std::min(c->fr.cap, c->fd.cap);
-  const int64_t nw = (*cand_cap + 31) / 32;
-  if (c->flag.grow(nw * 32) || c->flagw.grow(nw) || c->foff.grow(nw + 1) ||
-      c->scan_tmp64.grow(scan_tmp_elems(std::max<int64_t>(nw, n)) + 8) || c->p_read.grow(want_pass) ||
-      c->p_diag.grow(want_pass) || c->a_score.grow(want_pass) || c->a_bound.grow(want_pass) ||
-      c->a_tblen.grow(want_pass) || c->a_pos.grow(want_pass * 4) || c->a_tb.grow(want_pass * P.tbs))
+  if (P.bound_H && (c->q_read.grow(want_pass) || c->q_diag.grow(want_pass) || c->q_ub.grow(want_pass) ||
+                    c->p_ub.grow(want_kept)))
     return false;
-  *pass_cap = std::min({c->p_read.cap, c->p_diag.cap, c->a_score.cap, c->a_bound.cap, c->a_tblen.cap,
-                        c->a_pos.cap / 4, c->a_tb.cap / P.tbs});
-  if (c->scratch.grow(align_workers(*pass_cap, P.sp) * (int64_t)P.maxL * P.wpr)) return false;
-  if (rounds > 1 && (c->thr.grow(n) || c->round_slots.grow(*pass_cap) || c->rounds.grow(16))) return false;
-  return true;
+  if (c->p_read.grow(want_kept) || c->p_diag.grow(want_kept) || c->a_score.grow(want_kept) ||
+      c->a_bound.grow(want_kept) || c->a_tblen.grow(want_kept) || c->a_pos.grow(want_kept * 4) ||
+      c->a_tb.grow(want_kept * P.tbs))
+    return false;
+  // what was asked for, not what a buffer has grown to: the grids are sized by it
+  caps->cand = want_cand;
+  caps->kept = want_kept;
+  caps->pass = P.bound_H ? want_pass : caps->kept;
+  const int64_t nw = (std::max(caps->cand, caps->pass) + 31) / 32;
+  if (c->flag.grow(nw * 32) || c->flagw.grow(nw) || c->foff.grow(nw + 1) ||
+      c->scan_tmp64.grow(scan_tmp_elems(std::max<int64_t>(nw, n)) + 8) ||
+      c->scratch.grow(align_workers(caps->kept, P.sp) * (int64_t)P.maxL * P.wpr))
+    return false;
+  return round_lists_grow(c, n, caps->kept, P.rounds) == 0;
 }
 
 // The launches of every pass on c's stream, each list size read from the device (captured into
 // the graph; nothing here waits for the device).  E: the stage events, per_pass per pass.
-static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, int64_t cand_cap, int64_t pass_cap,
-                                int64_t grid_h, int per_pass, int64_t& launches) {
+static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const GraphCaps& caps, int per_pass,
+                                int64_t& launches) {
   cudaStream_t st = c->st;
+  const int64_t cand_cap = caps.cand, pass_cap = caps.pass, kept_cap = caps.kept, grid_h = caps.grid_h;
   const ScoreParams& sp = P.sp;
   const int64_t n = P.n;
   unsigned long long* gs = c->gstate.p;
-  const int64_t nw = (cand_cap + 31) / 32;
-  const int rounds = std::max(1, std::min<int>(c->tune.align_rounds, kMaxAlignRounds));
+  const int64_t nw = (cand_cap + 31) / 32, nwq = (pass_cap + 31) / 32;
+  const int rounds = P.rounds;
   const int64_t rstride = rexp_stride(P.maxL);
   const int64_t grid_s = gather_block_grid(true), grid_b = gather_block_grid(false);
   auto rec = [&](cudaEvent_t e) { return cudaEventRecordWithFlags(e, st, cudaEventRecordExternal); };
@@ -482,46 +560,54 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, int64_t can
                                         c->scan_tmp64.p, st);
       gate_filter_kernel<<<1, 1, 0, st>>>(c->foff.p + nw, pass_cap, kMaxPassingPerPass, n, gs);
       launches += 2 + scan_launches(nw);
-      const int64_t* np = reinterpret_cast<const int64_t*>(gs + kGsPass);
       PassBuffers pb;
       memset(&pb, 0, sizeof(pb));
       pb.pstart = c->pstart.p; pb.pcount = c->pcount.p;
       pb.counters = c->counters.p;
-      SG_CUDA(cudaMemsetAsync(c->pcount.p, 0, sizeof(int32_t) * n, st));
-      pb.p_read = c->p_read.p; pb.p_diag = c->p_diag.p; pb.p_cap = pass_cap;
-      launch_compact(nw, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->p_diag.p, pass_cap, st);
-      launch_slot_bounds(pass_cap, np, c->p_read.p, c->pstart.p, c->pcount.p, st);
-      launches += 3;
+      pb.p_read = c->p_read.p; pb.p_diag = c->p_diag.p; pb.p_cap = kept_cap;
+      if (P.bound_H) {
+        // the candidates whose score can exceed -t, in order
+        launch_compact(nw, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->q_read.p, c->q_diag.p, pass_cap, nullptr, nullptr, st);
+        launch_bound_pass(c, P, rd, R, pass_cap, reinterpret_cast<const int64_t*>(gs + kGsPass), st);
+        launch_pack_flags(pass_cap, gs + kGsPass, c->flag.p, c->flagw.p, st);
+        exclusive_scan<PassWord, int64_t>(reinterpret_cast<const PassWord*>(c->flagw.p), c->foff.p, nwq,
+                                          c->foff.p + nwq, c->scan_tmp64.p, st);
+        gate_bound_kernel<<<1, 1, 0, st>>>(c->foff.p + nwq, kept_cap, gs);
+        launch_compact(nwq, c->flagw.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->p_diag.p, kept_cap,
+                       c->q_ub.p, c->p_ub.p, st);
+        pb.ub = c->p_ub.p;
+        launches += 6 + scan_launches(nwq);
+      } else {
+        gate_bound_kernel<<<1, 1, 0, st>>>(c->foff.p + nw, kept_cap, gs);
+        launch_compact(nw, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->p_diag.p, kept_cap, nullptr, nullptr,
+                       st);
+        launches += 2;
+      }
+      const int64_t* np = reinterpret_cast<const int64_t*>(gs + kGsKept);
+      setup_rounds(c, rounds, pb, st);
+      launch_slot_lists(kept_cap, np, pb, align_round_take(0, rounds), st);
+      launches += 2;
       pb.a_score = c->a_score.p; pb.a_bound = c->a_bound.p; pb.a_tblen = c->a_tblen.p;
       pb.a_pos = c->a_pos.p; pb.a_tb = c->a_tb.p; pb.tbs = P.tbs;
-      pb.cursor = c->counters.p + 11;
       pb.npass_dev = np;
       pb.steal = c->tune.align_steal;
       pb.a_scratch = c->scratch.p;
       pb.cells = c->counters.p + 13;
       if (rounds == 1) {
-        launch_align(rd, sp, R.d_codes, R.d_mask, 0, pass_cap, pb, st);
+        launch_align(rd, sp, R.d_codes, R.d_mask, 0, kept_cap, pb, st);
         launches++;
         SG_CUDA(rec(E[3]));
-        launch_replay(n, sp, (int)ref_id, strand ? -1 : 1, pb, P.out->hits, P.out->tb, P.out->tb_stride,
+        launch_replay(n, sp, (int)ref_id, strand ? -1 : 1, pb, 0, P.out->hits, P.out->tb, P.out->tb_stride,
                       P.out->mapped, st);
         launches++;
       } else {
-        SG_CUDA(cudaMemsetAsync(c->rounds.p, 0, sizeof(int64_t) * 16, st));
-        launch_round_lists(pass_cap, np, rounds, c->p_read.p, c->pstart.p, c->rounds.p,
-                           reinterpret_cast<unsigned long long*>(c->rounds.p + 8), c->round_slots.p, st);
-        launches += 2;
-        pb.round_slots = c->round_slots.p;
-        pb.round_count = c->rounds.p;
-        pb.thr = c->thr.p;
         SG_CUDA(rec(E[5]));
         for (int k = 0; k < rounds; ++k) {
-          pb.round = k;
-          pb.cursor = c->counters.p + 16 + k;
-          launch_align(rd, sp, R.d_codes, R.d_mask, 0, pass_cap, pb, st);
+          round_buffers(c, k, pb);
+          launch_align(rd, sp, R.d_codes, R.d_mask, 0, kept_cap, pb, st);
           SG_CUDA(rec(E[6 + 2 * k]));
-          launch_replay_round(n, sp, (int)ref_id, strand ? -1 : 1, pb, rounds, P.out->hits, P.out->tb,
-                              P.out->tb_stride, P.out->mapped, st);
+          launch_replay(n, sp, (int)ref_id, strand ? -1 : 1, pb, align_round_take(k + 1, rounds), P.out->hits,
+                        P.out->tb, P.out->tb_stride, P.out->mapped, st);
           SG_CUDA(rec(E[7 + 2 * k]));
           launches += 2;
         }
@@ -540,13 +626,13 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, int64_t can
 // the call must run the host-synced passes; else an error code.
 static int map_passes_graph(stormgpu_ctx* c, const PassSetup& P, int64_t launches) {
   cudaStream_t st = c->st;
-  int64_t cand_cap = 0, pass_cap = 0, grid_h = 0;
-  if (!graph_buffers(c, P, &cand_cap, &pass_cap, &grid_h)) {
+  GraphCaps caps;
+  if (!graph_buffers(c, P, &caps)) {
     cudaGetLastError();
     c->work.over = false;  // the host-synced passes allocate what they need, no more
     return kGraphRetry;
   }
-  const int rounds = std::max(1, std::min<int>(c->tune.align_rounds, kMaxAlignRounds));
+  const int rounds = P.rounds;
   const int per_pass = 5 + (rounds > 1 ? 1 + 2 * rounds : 0);
   int npasses = 0;
   for (size_t r = 0; r < c->refs.size(); ++r)
@@ -566,7 +652,7 @@ static int map_passes_graph(stormgpu_ctx* c, const PassSetup& P, int64_t launche
     return kGraphRetry;
   };
   if (cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed) != cudaSuccess) return broken();
-  const int erc = enqueue_graph_passes(c, P, cand_cap, pass_cap, grid_h, per_pass, launches);
+  const int erc = enqueue_graph_passes(c, P, caps, per_pass, launches);
   const cudaError_t ece = cudaStreamEndCapture(st, &g);
   if (erc || ece != cudaSuccess || !g) return broken();
   bool ready = false;
@@ -600,7 +686,7 @@ static int map_passes_graph(stormgpu_ctx* c, const PassSetup& P, int64_t launche
   S.seed_lookups = (int64_t)h[kGsLookups];
   S.hit_positions = (int64_t)h[kGsPositions];
   S.filter_passed = (int64_t)h[kGsPassed];
-  S.aligned = (int64_t)h[kGsPassed];
+  S.aligned = (int64_t)h[kGsAligned];
   S.align_cells = (int64_t)h[kGsAlignCells];
   S.passes = npasses;
   S.graph_passes = npasses;
@@ -613,7 +699,7 @@ static int map_passes_graph(stormgpu_ctx* c, const PassSetup& P, int64_t launche
     cudaEventElapsedTime(&b, E[1], E[2]);
     cudaEventElapsedTime(&d, E[2], E[3]);
     cudaEventElapsedTime(&e, E[3], E[4]);
-    for (int k = 0; rounds > 1 && k < rounds; ++k) {
+    for (int k = 0; rounds > 1 && k < rounds; ++k) {  // the rounds' replays count as replay time
       float x = 0;
       cudaEventElapsedTime(&x, E[6 + 2 * k], E[7 + 2 * k]);
       d -= x;
@@ -625,7 +711,7 @@ static int map_passes_graph(stormgpu_ctx* c, const PassSetup& P, int64_t launche
   cudaGetLastError();
   S.ms_gather = tg; S.ms_filter = tf; S.ms_align = ta; S.ms_replay = tr; S.ms_total = tt;
   S.kernels = launches;
-  if (P.wsum > 0) set_densities(c, (double)h[kGsMaxCand] / P.wsum, (double)h[kGsMaxPass] / P.wsum);
+  if (P.wsum > 0) set_densities(c, (double)h[kGsMaxCand] / P.wsum, (double)h[kGsMaxPass] / P.wsum, (double)h[kGsMaxKept] / P.wsum);
   return 0;
 }
 
@@ -688,8 +774,21 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
   const int BW = 2 * sp.I + 1;
   const int wpr = (2 * BW + 31) / 32 + (sp.colour ? (BW + 31) / 32 : 0);
   const int64_t tbs = ((maxL + sp.I + 1) / 2 + 7) & ~7LL;
+  // score bound: nucleotide space, scores it has constants for, a band it is instantiated for
+  if (!c->bound_set) {
+    memset(&c->bound_c, 0, sizeof(c->bound_c));
+    if (!sp.colour && sp.I <= kMaxBoundIndels) c->bound_c = band_bound_consts(sp.pair, sp.gap_open, sp.gap_ext);
+    c->bound_set = true;
+  }
+  const int bound_H = c->bound_c.ok ? bound_registers(sp.I) : 0;
+  if (bound_H) {
+    const int64_t words = n * band_stream_words(maxL, bound_H);
+    if (c->bstream.grow(words) || (reads->levels && c->wstream.grow(words))) return STORMGPU_ENOMEM;
+  }
+  // a call of a few reads is all launch latency: one round
+  const int rounds = n <= 256 ? 1 : std::max(1, std::min<int>(c->tune.align_rounds, kMaxAlignRounds));
+  const PassSetup P{sp, fwd, rev, n, maxL, minL, wsum, wpr, tbs, rounds, bound_H, out};
   if (c->graphs && !c->graph_broken && c->gdens_cand > 0 && c->huge_cap <= ((int64_t)1 << 22)) {
-    const PassSetup P{sp, fwd, rev, n, maxL, minL, wsum, wpr, tbs, out};
     const int g = map_passes_graph(c, P, launches);
     if (g != kGraphRetry) return g;
     // a list outgrew its capacity: the passes again, each sized by the host (the graph's
@@ -698,7 +797,7 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
     launches++;
   }
   float tg = 0, tf = 0, ta = 0, tr = 0;
-  int64_t max_cand = 0, max_pass = 0;  // densest strand pass of this call
+  int64_t max_cand = 0, max_pass = 0, max_kept = 0;  // densest strand pass of this call
   SG_CUDA(cudaEventRecord(c->ev[6], st));
   for (size_t ref_id = 0; ref_id < c->refs.size(); ++ref_id) {
     RefSeq& R = c->refs[ref_id];
@@ -815,56 +914,68 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
       memset(&pb, 0, sizeof(pb));
       pb.pstart = c->pstart.p; pb.pcount = c->pcount.p;
       pb.counters = c->counters.p;
-      SG_CUDA(cudaMemsetAsync(c->pcount.p, 0, sizeof(int32_t) * n, st));
-      const int rounds = std::max(1, std::min<int>(c->tune.align_rounds, kMaxAlignRounds));
-      if (npass > 0) {
-        if (c->p_read.grow(npass) || c->p_diag.grow(npass) || c->a_score.grow(npass) || c->a_bound.grow(npass) ||
-            c->a_tblen.grow(npass) || c->a_pos.grow(npass * 4) || c->a_tb.grow(npass * tbs))
+      int64_t nkept = npass;  // candidates that are aligned
+      if (npass > 0 && bound_H) {
+        // those whose score can exceed -t, in order
+        const int64_t nwq = (npass + 31) / 32;
+        if (c->q_read.grow(npass) || c->q_diag.grow(npass) || c->q_ub.grow(npass)) return STORMGPU_ENOMEM;
+        launch_compact(nwords, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->q_read.p, c->q_diag.p, c->q_read.cap,
+                       nullptr, nullptr, st);
+        launch_bound_pass(c, P, rd, R, npass, nullptr, st);
+        launch_pack_flags(npass, nullptr, c->flag.p, c->flagw.p, st);
+        exclusive_scan<PassWord, int64_t>(reinterpret_cast<const PassWord*>(c->flagw.p), c->foff.p, nwq,
+                                          c->foff.p + nwq, c->scan_tmp64.p, st);
+        launches += 4 + scan_launches(nwq);
+        SG_CUDA(cudaMemcpyAsync(&nkept, c->foff.p + nwq, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        SG_CUDA(cudaStreamSynchronize(st));
+      }
+      max_kept = std::max(max_kept, nkept);
+      if (nkept > 0) {
+        if (c->p_read.grow(nkept) || c->p_diag.grow(nkept) || c->a_score.grow(nkept) || c->a_bound.grow(nkept) ||
+            c->a_tblen.grow(nkept) || c->a_pos.grow(nkept * 4) || c->a_tb.grow(nkept * tbs) ||
+            (bound_H && c->p_ub.grow(nkept)))
           return STORMGPU_ENOMEM;
         pb.p_read = c->p_read.p; pb.p_diag = c->p_diag.p; pb.p_cap = c->p_read.cap;
-        launch_compact(nwords, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->p_diag.p, c->p_read.cap, st);
-        launch_slot_bounds(npass, nullptr, c->p_read.p, c->pstart.p, c->pcount.p, st);
+        if (bound_H) {
+          launch_compact((npass + 31) / 32, c->flagw.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->p_diag.p,
+                         c->p_read.cap, c->q_ub.p, c->p_ub.p, st);
+          pb.ub = c->p_ub.p;
+        } else {
+          launch_compact(nwords, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->p_diag.p, c->p_read.cap,
+                         nullptr, nullptr, st);
+        }
+        if (round_lists_grow(c, n, nkept, rounds) || setup_rounds(c, rounds, pb, st)) return STORMGPU_ENOMEM;
+        launch_slot_lists(nkept, nullptr, pb, align_round_take(0, rounds), st);
         launches += 3;
         pb.a_score = c->a_score.p; pb.a_bound = c->a_bound.p; pb.a_tblen = c->a_tblen.p;
         pb.a_pos = c->a_pos.p; pb.a_tb = c->a_tb.p; pb.tbs = tbs;
-        // one persistent launch over all passing candidates; scratch for its threads only
-        pb.cursor = c->counters.p + 11;  // zeroed with the counters at the start of the pass
+        // one persistent launch over all kept candidates; scratch for its threads only
         pb.steal = c->tune.align_steal;
         const int64_t per_slot = (int64_t)maxL * wpr;
-        if (c->scratch.grow(align_workers(npass, sp) * per_slot)) return STORMGPU_ENOMEM;
+        if (c->scratch.grow(align_workers(nkept, sp) * per_slot)) return STORMGPU_ENOMEM;
         pb.a_scratch = c->scratch.p;
         pb.cells = c->counters.p + 13;
         if (rounds == 1) {
-          launch_align(rd, sp, R.d_codes, R.d_mask, 0, npass, pb, st);
+          launch_align(rd, sp, R.d_codes, R.d_mask, 0, nkept, pb, st);
           launches++;
         } else {
-          // rounds of increasing rank, each aligned with the thresholds the replay of the rounds
-          // before left, then replayed
-          if (c->thr.grow(n) || c->round_slots.grow(npass) || c->rounds.grow(16)) return STORMGPU_ENOMEM;
-          SG_CUDA(cudaMemsetAsync(c->rounds.p, 0, sizeof(int64_t) * 16, st));
-          launch_round_lists(npass, nullptr, rounds, c->p_read.p, c->pstart.p, c->rounds.p,
-                             reinterpret_cast<unsigned long long*>(c->rounds.p + 8), c->round_slots.p, st);
-          launches += 2;
-          pb.round_slots = c->round_slots.p;
-          pb.round_count = c->rounds.p;
-          pb.thr = c->thr.p;
+          // rounds, each of the candidates the replay of the round before selected
           SG_CUDA(cudaEventRecord(c->rev[0], st));
           for (int k = 0; k < rounds; ++k) {
-            pb.round = k;
-            pb.cursor = c->counters.p + 16 + k;  // zeroed with the counters of the pass
-            launch_align(rd, sp, R.d_codes, R.d_mask, 0, npass, pb, st);
+            round_buffers(c, k, pb);
+            launch_align(rd, sp, R.d_codes, R.d_mask, 0, nkept, pb, st);
             SG_CUDA(cudaEventRecord(c->rev[2 * k + 1], st));
-            launch_replay_round(n, sp, (int)ref_id, strand ? -1 : 1, pb, rounds, out->hits, out->tb, out->tb_stride,
-                                out->mapped, st);
+            launch_replay(n, sp, (int)ref_id, strand ? -1 : 1, pb, align_round_take(k + 1, rounds), out->hits,
+                          out->tb, out->tb_stride, out->mapped, st);
             SG_CUDA(cudaEventRecord(c->rev[2 * k + 2], st));
             launches += 2;
           }
         }
-        S.aligned += npass;
+        S.aligned += nkept;
       }
       SG_CUDA(cudaEventRecord(c->ev[3], st));
-      if (npass > 0 && rounds == 1) {
-        launch_replay(n, sp, (int)ref_id, strand ? -1 : 1, pb, out->hits, out->tb, out->tb_stride, out->mapped, st);
+      if (nkept > 0 && rounds == 1) {
+        launch_replay(n, sp, (int)ref_id, strand ? -1 : 1, pb, 0, out->hits, out->tb, out->tb_stride, out->mapped, st);
         launches++;
       }
       SG_CUDA(cudaEventRecord(c->ev[4], st));
@@ -874,7 +985,7 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
       cudaEventElapsedTime(&b, c->ev[1], c->ev[2]);
       cudaEventElapsedTime(&d, c->ev[2], c->ev[3]);
       cudaEventElapsedTime(&e, c->ev[3], c->ev[4]);
-      if (npass > 0 && rounds > 1) {  // the rounds' replays count as replay time
+      if (nkept > 0 && rounds > 1) {  // the rounds' replays count as replay time
         for (int k = 0; k < rounds; ++k) {
           float x = 0;
           cudaEventElapsedTime(&x, c->rev[2 * k + 1], c->rev[2 * k + 2]);
@@ -883,7 +994,7 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
         }
       }
       tg += a; tf += b; ta += d; tr += e;
-      if (npass > 0) {
+      if (nkept > 0) {
         unsigned long long cells = 0;
         SG_CUDA(cudaMemcpyAsync(&cells, c->counters.p + 13, sizeof(cells), cudaMemcpyDeviceToHost, st));
         SG_CUDA(cudaStreamSynchronize(st));
@@ -898,7 +1009,7 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
   cudaEventElapsedTime(&tt, c->ev[6], c->ev[7]);
   S.ms_gather = tg; S.ms_filter = tf; S.ms_align = ta; S.ms_replay = tr; S.ms_total = tt;
   S.kernels = launches;
-  if (n > 0 && wsum > 0) set_densities(c, (double)max_cand / wsum, (double)max_pass / wsum);
+  if (n > 0 && wsum > 0) set_densities(c, (double)max_cand / wsum, (double)max_pass / wsum, (double)max_kept / wsum);
   return 0;
 }
 

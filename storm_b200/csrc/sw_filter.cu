@@ -269,7 +269,8 @@ void launch_pack_flags(int64_t ncap, const unsigned long long* n_dev, const uint
 // (slots from pcap on are not written)
 __global__ void compact_kernel(int64_t nwords, const uint32_t* __restrict__ flag, const int64_t* __restrict__ woff,
                                const int32_t* __restrict__ fr, const int32_t* __restrict__ fd,
-                               int32_t* __restrict__ p_read, int32_t* __restrict__ p_diag, int64_t pcap) {
+                               int32_t* __restrict__ p_read, int32_t* __restrict__ p_diag, int64_t pcap,
+                               const int16_t* __restrict__ ub, int16_t* __restrict__ p_ub) {
   for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += (int64_t)gridDim.x * blockDim.x) {
     uint32_t m = flag[w];
     if (!m) continue;
@@ -278,47 +279,19 @@ __global__ void compact_kernel(int64_t nwords, const uint32_t* __restrict__ flag
       const int64_t t = w * 32 + (__ffs(m) - 1);
       p_read[o] = fr[t];
       p_diag[o] = fd[t];
+      if (p_ub) p_ub[o] = ub[t];
       ++o;
       m &= m - 1;
     }
   }
 }
 
-__global__ void slot_bounds_kernel(int64_t npass, const int64_t* __restrict__ npass_dev,
-                                   const int32_t* __restrict__ p_read, int32_t* __restrict__ pstart,
-                                   int32_t* __restrict__ pcount) {
-  if (npass_dev) npass = *npass_dev;
-  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < npass; s += (int64_t)gridDim.x * blockDim.x) {
-    const int r = p_read[s];
-    if (s == 0 || p_read[s - 1] != r) pstart[r] = (int32_t)s;
-  }
-}
-
-__global__ void slot_count_kernel(int64_t npass, const int64_t* __restrict__ npass_dev,
-                                  const int32_t* __restrict__ p_read, const int32_t* __restrict__ pstart,
-                                  int32_t* __restrict__ pcount) {
-  if (npass_dev) npass = *npass_dev;
-  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < npass; s += (int64_t)gridDim.x * blockDim.x) {
-    const int r = p_read[s];
-    if (s == npass - 1 || p_read[s + 1] != r) pcount[r] = (int32_t)(s - pstart[r] + 1);
-  }
-}
-
 void launch_compact(int64_t nwords, const uint32_t* flag, const int64_t* woff, const int32_t* fr, const int32_t* fd,
-                    int32_t* p_read, int32_t* p_diag, int64_t pcap, cudaStream_t st) {
+                    int32_t* p_read, int32_t* p_diag, int64_t pcap, const int16_t* ub, int16_t* p_ub, cudaStream_t st) {
   if (nwords <= 0) return;
   int64_t blocks = (nwords + 255) / 256;
   if (blocks > 148 * 32) blocks = 148 * 32;
-  compact_kernel<<<(unsigned)blocks, 256, 0, st>>>(nwords, flag, woff, fr, fd, p_read, p_diag, pcap);
-}
-
-void launch_slot_bounds(int64_t npass, const int64_t* npass_dev, const int32_t* p_read, int32_t* pstart,
-                        int32_t* pcount, cudaStream_t st) {
-  if (npass <= 0) return;
-  int64_t blocks = (npass + 255) / 256;
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  slot_bounds_kernel<<<(unsigned)blocks, 256, 0, st>>>(npass, npass_dev, p_read, pstart, pcount);
-  slot_count_kernel<<<(unsigned)blocks, 256, 0, st>>>(npass, npass_dev, p_read, pstart, pcount);
+  compact_kernel<<<(unsigned)blocks, 256, 0, st>>>(nwords, flag, woff, fr, fd, p_read, p_diag, pcap, ub, p_ub);
 }
 
 }  // namespace sg

@@ -53,12 +53,7 @@ struct PassWord {
   }
 };
 // passing candidates, in order: word w's set bits go to woff[w], woff[w] + 1, ... (those below
-// pcap: the capacity of p_read / p_diag)
+// pcap: the capacity of p_read / p_diag); with p_ub (may be null) their score bounds too
 void launch_compact(int64_t nwords, const uint32_t* flag, const int64_t* woff, const int32_t* fr, const int32_t* fd,
-                    int32_t* p_read, int32_t* p_diag, int64_t pcap, cudaStream_t st);
-// pstart / pcount of every read with passing candidates; npass is the slot count, or with
-// npass_dev (may be null) an upper bound for the grid and the count is read from there
-void launch_slot_bounds(int64_t npass, const int64_t* npass_dev, const int32_t* p_read, int32_t* pstart,
-                        int32_t* pcount, cudaStream_t st);
-
+                    int32_t* p_read, int32_t* p_diag, int64_t pcap, const int16_t* ub, int16_t* p_ub, cudaStream_t st);
 }  // namespace sg

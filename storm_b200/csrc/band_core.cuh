@@ -18,7 +18,7 @@
 //   * filter: zero at pattern 0x7C00 - (threshold + 1).  The cell value threshold + 1 is then 65536,
 //     which rounds to infinity, and infinity plus any score is infinity: a cell that passes the
 //     threshold marks its diagonal to the end of the read, and no running maximum is kept; the
-//     cells of the last read row are looked at instead.  Exact for any threshold up to 254.
+//     cells are looked at once, after the last row.  Exact for any threshold up to 254.
 //   * bound: zero at 1280.0 (unit 1): values -248 .. 767 exact, see score_bound.cu.
 // The score: nibbles 4 + c (read) and g (genome) differ by 1..7, 4 where the codes are equal, and
 // one prmt turns the differences of four cells into four bytes (match or mismatch byte).  A byte
@@ -28,11 +28,15 @@
 // factor, and scores that have none (above 7 or so) take the kernels of filter_core.cuh.
 // The match byte is negative and the mismatch byte positive (the factor is negative): read nibble 11
 // then picks, whatever the genome code, the sign of a mismatch byte, a score of zero.  The read is
-// padded with it to a whole number of blocks: a row of zero scores hands every cell down its
-// diagonal unchanged (gaps cannot raise the maximum), so the largest cell of the padded last row is
-// that of the read's, and the blocks need no remainder.
+// padded with it on both sides: a row of zero scores hands every cell down its diagonal unchanged and
+// gaps cannot raise the maximum, so the cells before the read stay zero, those after it keep their
+// last row's value, and one loop of whole blocks without masks runs the candidate, reads shorter
+// than the band included.  (Masks on the first and last W pairs save 4 % of the cells, 97.5 against
+// 102.4 ms before the immediates below, for code five times as long and a case apart for short reads.)
 // So a register of two cells costs 3 add-max / max and half a prmt on the ALU pipe, where
-// filter_core.cuh's form costs 4.5 (three maxima, a prmt, half a running-maximum fold).
+// filter_core.cuh's form costs 4.5 (three maxima, a prmt, half a running-maximum fold): 8.5 against
+// 6.1 T cell updates/s on the mixed workload's reads, ALU pipe at 81 % of its peak before the
+// immediates (the rest: operand reads of three-register instructions).
 #pragma once
 
 #include <cmath>
@@ -92,10 +96,11 @@ SG_HD void ldg128(const uint32_t* p, uint32_t (&v)[4]) {
 __host__ __device__ constexpr int band_block(int H) { return H == 2 ? 4 : H; }  // pairs of a main block: a multiple of 4 and of H
 
 // Read stream of a band of H registers: word p (the codes entering at pair p) holds the nibbles of
-// positions p - H - 1, p - H, p - 1 and p: 4 + code inside the read, 4 before it, 11 after it.
+// positions p - H - 1, p - H, p - 1 and p: 4 + code inside the read, 11 outside it.
 constexpr uint32_t kBandPad = 11;
 __host__ __device__ inline int64_t band_stream_words(int max_len, int H) {
-  return ((int64_t)max_len + band_block(H) + 2 * H + 3) & ~3LL;
+  const int bp = band_block(H);
+  return ((int64_t)max_len + 2 * H - 1 + bp - 1) / bp * bp;
 }
 SG_HD uint32_t band_stream_word(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   return a | (b << 4) | (c << 8) | (d << 12);
@@ -112,59 +117,41 @@ struct Band {
   uint32_t wt[H];         // factors of cells (j, j + H), weighted form only
 };
 
-// Cells computed at pair K of a phase.  MODE 0 main: all; 1 prologue: cells k >= W - 1 - K are inside
-// the read, the others keep zero; 2 epilogue (pair L + K): cells k <= W - 2 - K are.
-template <int H, int MODE, int K>
-__host__ __device__ constexpr bool band_in(int k) {
-  return MODE == 0 ? true : MODE == 1 ? k >= 2 * H - 1 - K : k <= 2 * H - 2 - K;
-}
-
 // One step; Q = pair mod H.
-template <int H, bool ODD, int Q, int MODE, int K, bool WTD>
-SG_HD void band_step(Band<H>& b, const BandConst& c) {
-  // a register is computed when one of its cells is inside (the prologue's low cells enter last,
-  // the epilogue's high cells leave first)
-  auto active = [](int j) constexpr { return MODE == 1 ? band_in<H, MODE, K>(j + H) : band_in<H, MODE, K>(j); };
+template <int H, bool ODD, int Q, bool WTD, class C>
+SG_HD void band_step(Band<H>& b, const C& c) {
   uint32_t sc[H], J[H];
 #pragma unroll
   for (int q = 0; q < H / 2; ++q) {
-    if (active(2 * q) || active(2 * q + 1)) {
-      const uint32_t sel = b.ra[(Q + 1 + 2 * q) % H] - b.gb[((ODD ? Q : Q - 1) - 2 * q + 2 * H) % H];
-      const uint32_t x = prmt(c.t0, c.t1, sel);
-      sc[2 * q + 1] = x;
-      sc[2 * q] = x << 8;
-    }
+    const uint32_t sel = b.ra[(Q + 1 + 2 * q) % H] - b.gb[((ODD ? Q : Q - 1) - 2 * q + 2 * H) % H];
+    const uint32_t x = prmt(c.t0, c.t1, sel);
+    sc[2 * q + 1] = x;
+    sc[2 * q] = x << 8;
   }
 #pragma unroll
   for (int j = 0; j < H; ++j) {
-    if (active(j)) {
-      uint32_t nb;
-      if (ODD) nb = j > 0 ? b.G[j - 1] : prmt(c.fl, b.G[H - 1], 0x5410);
-      else     nb = j < H - 1 ? b.G[j + 1] : prmt(b.G[0], c.fl, 0x5432);
-      J[j] = __vimax3_s16x2(b.G[j], nb, c.fl);
-    }
+    uint32_t nb;
+    if (ODD) nb = j > 0 ? b.G[j - 1] : prmt(c.fl, b.G[H - 1], 0x5410);
+    else     nb = j < H - 1 ? b.G[j + 1] : prmt(b.G[0], c.fl, 0x5432);
+    J[j] = __vimax3_s16x2(b.G[j], nb, c.fl);
   }
 #pragma unroll
   for (int j = 0; j < H; ++j) {
-    if (active(j)) {
-      const uint32_t w = WTD ? b.wt[(Q + 1 + j) % H] : c.k;
-      uint32_t D = band_fma(sc[j], w, b.M2[j]);
-      if (MODE == 1 && !band_in<H, MODE, K>(j)) D = (D & 0xFFFF0000u) | (c.z & 0x0000FFFFu);
-      const uint32_t mn = __viaddmax_s16x2(J[j], c.no, D);
-      b.G[j] = __viaddmax_s16x2(J[j], c.ne, D);
-      b.M2[j] = b.M1[j];
-      b.M1[j] = mn;
-    }
+    const uint32_t w = WTD ? b.wt[(Q + 1 + j) % H] : c.k;
+    const uint32_t D = band_fma(sc[j], w, b.M2[j]);
+    b.G[j] = __viaddmax_s16x2(J[j], c.ne, D);
+    b.M2[j] = b.M1[j];
+    b.M1[j] = __viaddmax_s16x2(J[j], c.no, D);
   }
 }
 
-template <int H, int Q, int MODE, int K, bool WTD>
-SG_HD void band_pair(Band<H>& b, const BandConst& c, uint32_t rs, uint32_t ws, uint32_t gg) {
+template <int H, int Q, bool WTD, class C>
+SG_HD void band_pair(Band<H>& b, const C& c, uint32_t rs, uint32_t ws, uint32_t gg) {
   b.ra[(Q + H - 1) % H] = rs;
   if (WTD) b.wt[Q % H] = ws;
-  band_step<H, false, Q % H, MODE, K, WTD>(b, c);
+  band_step<H, false, Q % H, WTD>(b, c);
   b.gb[Q % H] = gg;
-  band_step<H, true, Q % H, MODE, K, WTD>(b, c);
+  band_step<H, true, Q % H, WTD>(b, c);
 }
 
 // Genome words from code x0 on: byte-expanded codes (c * 0x11) regrouped so that byte x holds the
@@ -198,29 +185,22 @@ SG_HD uint32_t band_entry(const uint32_t (&t)[NW]) {
   return prmt(t[X / 4], t[Y / 4], (uint32_t)(X % 4) | ((uint32_t)(4 + Y % 4) << 4));
 }
 
-// Pairs K .. NP - 1 of a group whose pair 0 is QB mod H; t holds the group's genome words after NH
-// words of history; rs / ws the entering read and factor words.
-template <int H, int MODE, int QB, int K, int NP, bool WTD, int NW, int NR, int NS>
-SG_HD void band_run(Band<H>& b, const BandConst& c, const uint32_t (&t)[NW], const uint32_t (&rs)[NR],
+// Pairs K .. NP - 1 of a block; t holds the block's genome words after NH words of history; rs / ws
+// the entering read and factor words.
+template <int H, int K, int NP, bool WTD, int NW, int NR, int NS, class C>
+SG_HD void band_run(Band<H>& b, const C& c, const uint32_t (&t)[NW], const uint32_t (&rs)[NR],
                     const uint32_t (&ws)[NS]) {
   if constexpr (K < NP) {
-    band_pair<H, QB + K, MODE, K, WTD>(b, c, rs[K], WTD ? ws[WTD ? K : 0] : 0u, band_entry<H, 4 * Band<H>::NH + K, NW>(t));
-    band_run<H, MODE, QB, K + 1, NP, WTD, NW, NR, NS>(b, c, t, rs, ws);
+    band_pair<H, K, WTD>(b, c, rs[K], WTD ? ws[WTD ? K : 0] : 0u, band_entry<H, 4 * Band<H>::NH + K, NW>(t));
+    band_run<H, K + 1, NP, WTD, NW, NR, NS>(b, c, t, rs, ws);
   }
 }
 
-// Epilogue pairs K..: after pair L' + K (L' the padded length) cell W - 2 - K is on the last row, in
-// the even step's M (now M2) and the odd step's (M1).  hi / lo: their maxima, in the high halves for cells >= H, in the low
-// halves for the others.
-template <int H, int K, bool WTD, int NW, int NR, int NS>
-SG_HD void band_tail(Band<H>& b, const BandConst& c, const uint32_t (&t)[NW], const uint32_t (&rs)[NR],
-                     const uint32_t (&ws)[NS], uint32_t& hi, uint32_t& lo) {
-  if constexpr (K < 2 * H - 1) {
-    constexpr int k = 2 * H - 2 - K;
-    band_pair<H, K, 2, K, WTD>(b, c, rs[K], WTD ? ws[WTD ? K : 0] : 0u, band_entry<H, 4 * Band<H>::NH + K, NW>(t));
-    if constexpr (k >= H) hi = __vimax3_s16x2(hi, b.M1[k - H], b.M2[k - H]);
-    else lo = __vimax3_s16x2(lo, b.M1[k], b.M2[k]);
-    band_tail<H, K + 1, WTD, NW, NR, NS>(b, c, t, rs, ws, hi, lo);
+template <int H, int X, int NW>
+SG_HD void band_fill(Band<H>& b, const uint32_t (&t)[NW]) {  // genome entries X .. W - 1 (code 0: the window's first)
+  if constexpr (X < 2 * H) {
+    b.gb[X % H] = band_entry<H, X, NW>(t);
+    band_fill<H, X + 1, NW>(b, t);
   }
 }
 
@@ -236,49 +216,36 @@ SG_HD void band_load(const uint32_t* p, uint32_t (&v)[M]) {
   }
 }
 
-template <int H, int X, int NW>
-SG_HD void band_fill(Band<H>& b, const uint32_t (&t)[NW]) {  // genome entries X .. W - 1 (code 0: the window's first)
-  if constexpr (X < 2 * H) {
-    b.gb[X % H] = band_entry<H, X, NW>(t);
-    band_fill<H, X + 1, NW>(b, t);
-  }
-}
-
 // One candidate: the largest cell of the last read row, as a pattern (see the two placements).
-// gexp: byte-expanded genome (code c -> c * 0x11) at code 0, 4-byte aligned, readable from pos - 4 to
+// gexp: byte-expanded genome (code c -> c * 0x11) at code 0, 4-byte aligned, readable from pos to
 // pos + L + 3W + 8; rs: the read's stream, 16-byte aligned, band_stream_words(L, H) words; ws: its
-// factor stream (weighted form): word p the factors of positions p - H and p.  Requires L >= W.
-template <int H, bool WTD>
+// factor stream (weighted form): word p the factors of positions p - H and p.
+template <int H, bool WTD, class C>
 SG_HD int band_last_row(const uint8_t* __restrict__ gexp, int64_t pos, const uint32_t* __restrict__ rs,
-                        const uint32_t* __restrict__ ws, int L, const BandConst& c) {
+                        const uint32_t* __restrict__ ws, int L, const C& c) {
   constexpr int W = 2 * H, NH = Band<H>::NH, BP = Band<H>::BP, NB = BP / 4, NP4 = W / 4;
   Band<H> b;
 #pragma unroll
   for (int j = 0; j < H; ++j) {
     b.M1[j] = c.z; b.M2[j] = c.z; b.G[j] = c.z;
-    b.ra[j] = 0x4444u;
+    b.ra[j] = kBandPad * 0x1111u;
     b.gb[j] = 0;
     b.wt[j] = c.k;
   }
   BandGenome gs;
   gs.init(gexp, pos);
   uint32_t hist[NH];
-  {  // prologue: pairs 0 .. W - 1 over codes pos .. pos + 2W - 1
-    uint32_t t[2 * NP4], r[W], w[WTD ? W : 4];
+  {  // codes pos .. pos + W - 1
+    uint32_t t[NP4];
 #pragma unroll
-    for (int m = 0; m < 2 * NP4; ++m) t[m] = gs.next();
-    band_fill<H, H + 1, 2 * NP4>(b, t);
-    band_load<W>(rs, r);
-    if (WTD) band_load<WTD ? W : 4>(ws, w);
-    uint32_t u[NH + NP4];  // the same words, from NH words before the first entering code
+    for (int m = 0; m < NP4; ++m) t[m] = gs.next();
+    band_fill<H, H + 1, NP4>(b, t);
 #pragma unroll
-    for (int m = 0; m < NH + NP4; ++m) u[m] = t[NP4 - NH + m];
-    band_run<H, 1, 0, 0, W, WTD, NH + NP4, W, (WTD ? W : 4)>(b, c, u, r, w);
-#pragma unroll
-    for (int m = 0; m < NH; ++m) hist[m] = u[NP4 + m];
+    for (int m = 0; m < NH; ++m) hist[m] = t[NP4 - NH + m];
   }
-  int p = W;
-  for (; p < L; p += BP) {  // main: pairs W .. L' - 1, L' = L padded to a whole number of blocks
+  const int n = L + W - 1;  // after that many pairs every cell is on the last row or below it
+#pragma unroll 1
+  for (int p = 0; p < n; p += BP) {
     uint32_t t[NH + NB], r[BP], w[WTD ? BP : 4];
 #pragma unroll
     for (int m = 0; m < NH; ++m) t[m] = hist[m];
@@ -286,23 +253,15 @@ SG_HD int band_last_row(const uint8_t* __restrict__ gexp, int64_t pos, const uin
     for (int m = 0; m < NB; ++m) t[NH + m] = gs.next();
     band_load<BP>(rs + p, r);
     if (WTD) band_load<WTD ? BP : 4>(ws + p, w);
-    band_run<H, 0, 0, 0, BP, WTD, NH + NB, BP, (WTD ? BP : 4)>(b, c, t, r, w);
+    band_run<H, 0, BP, WTD, NH + NB, BP, (WTD ? BP : 4)>(b, c, t, r, w);
 #pragma unroll
     for (int m = 0; m < NH; ++m) hist[m] = t[NB + m];
   }
-  uint32_t hi = __vimax3_s16x2(b.M1[H - 1], b.M2[H - 1], 0x80008000u), lo = 0x80008000u;  // pair L' - 1: cell W - 1
-  {  // epilogue: pairs L' .. L' + W - 2
-    uint32_t t[NH + NP4], r[W], w[WTD ? W : 4];
+  uint32_t mx = 0x80008000u;
 #pragma unroll
-    for (int m = 0; m < NH; ++m) t[m] = hist[m];
-#pragma unroll
-    for (int m = 0; m < NP4; ++m) t[NH + m] = gs.next();
-    band_load<W>(rs + p, r);
-    if (WTD) band_load<WTD ? W : 4>(ws + p, w);
-    band_tail<H, 0, WTD, NH + NP4, W, (WTD ? W : 4)>(b, c, t, r, w, hi, lo);
-  }
-  const int a = (int)(int16_t)(hi >> 16), d = (int)(int16_t)(lo & 0xFFFFu);
-  return a > d ? a : d;
+  for (int j = 0; j < H; ++j) mx = __vimax3_s16x2(mx, b.M1[j], b.M2[j]);
+  const int hi = (int)(int16_t)(mx >> 16), lo = (int)(int16_t)(mx & 0xFFFFu);
+  return hi > lo ? hi : lo;
 }
 
 // ------------------------------------------------------------------------------ constants (host)
@@ -367,6 +326,31 @@ inline BandConst band_filter_consts(int fm, int fx, int fo, int fe, int fthr) {
   c.no = (uint32_t)(uint16_t)(-fo) * 0x10001u;
   c.ne = (uint32_t)(uint16_t)(-(fe < fo ? fe : fo)) * 0x10001u;
   return c;
+}
+
+// The constants of the default scores (5, -4, -9, -4; alignment.h:24-28) as immediates: a cell's four
+// instructions then read two or three registers each instead of up to three and a constant, and
+// the register file, not only the ALU pipe, limits them (4,000 mixed reads at -i 15: filter 99.6 ms
+// with run-time constants, 88.2-91.8 ms with these).  Other scores run the same kernels on a
+// BandConst; band_is_default compares, so that these follow band_consts' choice.
+struct BandFilterDefault {
+  static constexpr uint32_t t0 = 0x18181800u, t1 = 0x18181899u, k = 0xfb84fb84u, no = 0xfff7fff7u, ne = 0xfffcfffcu;
+  uint32_t z, fl;  // by the threshold
+  SG_HD BandFilterDefault(const BandConst& c) : z(c.z), fl(c.fl) {}
+};
+struct BandBoundDefault {
+  static constexpr uint32_t t0 = 0x10101000u, t1 = 0x10101091u, k = 0xef8bef8bu, no = 0xfff7fff7u, ne = 0xfffcfffcu;
+  static constexpr uint32_t z = 0x65006500u, fl = 0x64116411u;
+  SG_HD BandBoundDefault(const BandConst&) {}
+};
+inline bool band_is_default_filter(const BandConst& c) {
+  using D = BandFilterDefault;
+  return c.ok && c.t0 == D::t0 && c.t1 == D::t1 && c.k == D::k && c.no == D::no && c.ne == D::ne;
+}
+inline bool band_is_default_bound(const BandConst& c) {
+  using D = BandBoundDefault;
+  return c.ok && c.t0 == D::t0 && c.t1 == D::t1 && c.k == D::k && c.no == D::no && c.ne == D::ne && c.z == D::z &&
+         c.fl == D::fl;
 }
 
 // The bound's constants: pair scores per quality level (pair[0] match, pair[1] mismatch), gap scores

@@ -93,13 +93,14 @@ struct stormgpu_ctx {
   sg::DevBuf<uint8_t> flag;       // pass byte per candidate
   sg::DevBuf<uint32_t> flagw;     // pass bits, one word per 32 candidates
   sg::DevBuf<uint8_t> rexp;
-  // score bound: passing candidates before it (p_read / p_diag hold those it keeps), read streams,
-  // its constants (bound_set: computed for this context's scores)
+  // score bound: passing candidates before it (p_read / p_diag hold those it keeps); read streams of
+  // the banded core, its constants for the filter and the bound (band_set: computed for this
+  // context's scores)
   sg::DevBuf<int32_t> q_read, q_diag;
   sg::DevBuf<int16_t> q_ub, p_ub;  // the bounds of both lists
   sg::DevBuf<uint32_t> bstream, wstream;
-  sg::BandConst bound_c;
-  bool bound_set = false;
+  sg::BandConst filter_c, bound_c;
+  bool band_set = false;
   sg::DevBuf<int32_t> a_score, a_bound, a_tblen, big_tmp;
   sg::DevBuf<int16_t> a_pos;
   sg::DevBuf<uint8_t> a_tb;

@@ -11,8 +11,7 @@
 //   * Every quality level's pair scores come from one factor per read position (band_bound_consts:
 //     the rounded products are at least the level's scores, equal at level 3).
 //   * Values -248 .. 767 are exact.  Lower ones are raised to -248, which only raises the bound; a read
-//     long enough to exceed 767 has a bound only below band_bound_limit; one shorter than the band has
-//     none.
+//     long enough to exceed 767 has a bound only below band_bound_limit.
 // The bound also orders the work among the candidates kept: the replay's threshold rises to a
 // read's fourth best score, and each round of the alignment takes only candidates whose bound is
 // above the threshold the rounds before left (replay_kernel).
@@ -32,7 +31,7 @@ __global__ void band_streams_kernel(ReadsDev rd, int H, int64_t words, uint32_t*
     const int L = rd.lengths[r];
     const uint8_t* cd = rd.codes + r * rd.cstride;
     const uint8_t* lv = ws && rd.levels ? rd.levels + r * rd.lstride : nullptr;
-    auto nib = [&](int i) { return i >= L ? kBandPad : 4u + (uint32_t)(i >= 0 ? code_at(cd, i) : 0); };
+    auto nib = [&](int i) { return i < 0 || i >= L ? kBandPad : 4u + (uint32_t)code_at(cd, i); };
     auto fac = [&](int i) { return (uint32_t)c.wl[lv && i >= 0 && i < L ? code_at(lv, i) : 3]; };
     for (int64_t p = lane; p < words; p += 32) {
       const int i = (int)p;
@@ -51,9 +50,11 @@ void launch_band_streams(const ReadsDev& rd, int H, int64_t words, uint32_t* rs,
 
 // One candidate per thread, blocks in list order (neighbouring candidates are of one read, or of
 // reads of one length).
-template <int H, bool WTD>
+// C: the constants, BandBoundDefault for the default scores.
+template <int H, bool WTD, class C>
 __global__ void __launch_bounds__(128, H <= 4 ? 8 : H <= 8 ? 4 : 3)
-    score_bound_kernel(BoundJob job, const __grid_constant__ BandConst c) {
+    score_bound_kernel(BoundJob job, const __grid_constant__ BandConst bc) {
+  const C c(bc);
   const int64_t n = job.n_dev ? *job.n_dev : job.n;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
@@ -61,7 +62,7 @@ __global__ void __launch_bounds__(128, H <= 4 ? 8 : H <= 8 ? 4 : 3)
   const int L = job.lengths[r];
   int ub = 32767;
   const int lim = band_bound_limit(job.match, job.mismatch, L);
-  if (L >= 2 * H && lim > kBoundFloor - kBoundZero) {
+  if (lim > kBoundFloor - kBoundZero) {
     const int64_t win = max(job.diag[t] - job.I, -job.Is);  // run.c:667
     const int v = band_last_row<H, WTD>(job.gexp, win, job.rs + (int64_t)r * job.words,
                                         WTD ? job.ws + (int64_t)r * job.words : nullptr, L, c);
@@ -74,18 +75,21 @@ __global__ void __launch_bounds__(128, H <= 4 ? 8 : H <= 8 ? 4 : 3)
 void launch_score_bound(const BoundJob& job, const BandConst& c, cudaStream_t st) {
   if (job.n <= 0) return;
   const unsigned blocks = (unsigned)((job.n + 127) / 128);
-#define SG_BOUND(H)                                                                     \
+#define SG_BOUND(H, C)                                                                  \
   case H:                                                                               \
-    if (job.ws) score_bound_kernel<H, true><<<blocks, 128, 0, st>>>(job, c);            \
-    else score_bound_kernel<H, false><<<blocks, 128, 0, st>>>(job, c);                  \
+    if (job.ws) score_bound_kernel<H, true, C><<<blocks, 128, 0, st>>>(job, c);         \
+    else score_bound_kernel<H, false, C><<<blocks, 128, 0, st>>>(job, c);               \
     break;
-  switch (job.H) {
-    SG_BOUND(2)
-    SG_BOUND(4)
-    SG_BOUND(8)
-    SG_BOUND(12)
-  default: break;
+#define SG_BOUNDS(C) \
+  switch (job.H) {   \
+    SG_BOUND(2, C)   \
+    SG_BOUND(4, C)   \
+    SG_BOUND(8, C)   \
+    SG_BOUND(12, C)  \
+  default: break;    \
   }
+  if (band_is_default_bound(c)) { SG_BOUNDS(BandBoundDefault) } else { SG_BOUNDS(BandConst) }
+#undef SG_BOUNDS
 #undef SG_BOUND
 }
 

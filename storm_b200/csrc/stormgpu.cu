@@ -400,16 +400,41 @@ struct PassSetup {
   int wpr;          // scratch words per row of an alignment
   int64_t tbs;      // traceback bytes per aligned candidate
   int rounds;       // alignment rounds
+  int filter_H;     // band registers of the filter's core, 0: the core of filter_core.cuh
   int bound_H;      // band registers of the score bound, 0: every passing candidate is aligned
   stormgpu_results* out;
 };
 
-// The score bound of one pass: streams of its reads, then the flags of the passing candidates
-// (q_read, q_diag), read from n_dev when given.
+// Read streams of one pass for the filter, and for the score bound too when its band is the same.
+static void launch_filter_streams(stormgpu_ctx* c, const PassSetup& P, const ReadsDev& rd, cudaStream_t st) {
+  if (!P.filter_H) {
+    launch_expand_reads(rd, c->rexp.p, rexp_stride(P.maxL), st);
+    return;
+  }
+  const bool both = P.filter_H == P.bound_H;
+  launch_band_streams(rd, P.filter_H, band_stream_words(P.maxL, P.filter_H), c->bstream.p,
+                      both && rd.levels ? c->wstream.p : nullptr, c->bound_c, st);
+}
+
+static void set_filter_job(stormgpu_ctx* c, const PassSetup& P, const ReadsDev& rd, const RefSeq& R, FilterJob& job) {
+  const ScoreParams& sp = P.sp;
+  job.rows = c->tune.filter_rows;
+  job.fr = c->fr.p; job.fd = c->fd.p; job.flag = c->flag.p; job.codes = rd.codes;
+  job.cstride = rd.cstride; job.lengths = rd.lengths; job.genome = R.d_codes; job.W = sp.W; job.Is = sp.Is;
+  job.fm = sp.fm; job.fx = sp.fx; job.fo = sp.fo; job.fe = sp.fe; job.fthr = sp.fthr;
+  job.counters = c->counters.p;
+  job.gexp = R.d_gexp; job.rexp = c->rexp.p; job.rstride = rexp_stride(P.maxL); job.min_len = P.minL;
+  job.band_H = P.filter_H; job.band = c->filter_c; job.bs = c->bstream.p;
+  job.bwords = P.filter_H ? band_stream_words(P.maxL, P.filter_H) : 0;
+}
+
+// The score bound of one pass: streams of its reads (unless the filter's serve), then the flags of the
+// passing candidates (q_read, q_diag), their number read from n_dev when given.
 static void launch_bound_pass(stormgpu_ctx* c, const PassSetup& P, const ReadsDev& rd, const RefSeq& R, int64_t n,
                               const int64_t* n_dev, cudaStream_t st) {
   const int64_t words = band_stream_words(P.maxL, P.bound_H);
-  launch_band_streams(rd, P.bound_H, words, c->bstream.p, rd.levels ? c->wstream.p : nullptr, c->bound_c, st);
+  if (P.filter_H != P.bound_H)
+    launch_band_streams(rd, P.bound_H, words, c->bstream.p, rd.levels ? c->wstream.p : nullptr, c->bound_c, st);
   BoundJob job;
   memset(&job, 0, sizeof(job));
   job.n = n; job.n_dev = n_dev; job.read = c->q_read.p; job.diag = c->q_diag.p; job.lengths = rd.lengths;
@@ -465,8 +490,7 @@ static bool graph_buffers(stormgpu_ctx* c, const PassSetup& P, GraphCaps* caps) 
   const int64_t grid_b = gather_block_grid(false);
   caps->grid_h = std::max<int64_t>(1, std::min<int64_t>(grid_b, ((int64_t)1 << 25) / c->huge_cap));
   if (c->fr.grow(want_cand) || c->fd.grow(want_cand) || c->big_count.grow(4) || c->gstate.grow(kGsWords) ||
-      c->big_tmp.grow(std::max(grid_b * 2 * (int64_t)kBlockGatherCap, caps->grid_h * 2 * c->huge_cap)) ||
-      c->rexp.grow(n * rexp_stride(P.maxL)))
+      c->big_tmp.grow(std::max(grid_b * 2 * (int64_t)kBlockGatherCap, caps->grid_h * 2 * c->huge_cap)))
     return false;
   if (P.bound_H && (c->q_read.grow(want_pass) || c->q_diag.grow(want_pass) || c->q_ub.grow(want_pass) ||
                     c->p_ub.grow(want_kept)))
@@ -498,7 +522,6 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const Graph
   unsigned long long* gs = c->gstate.p;
   const int64_t nw = (cand_cap + 31) / 32, nwq = (pass_cap + 31) / 32;
   const int rounds = P.rounds;
-  const int64_t rstride = rexp_stride(P.maxL);
   const int64_t grid_s = gather_block_grid(true), grid_b = gather_block_grid(false);
   auto rec = [&](cudaEvent_t e) { return cudaEventRecordWithFlags(e, st, cudaEventRecordExternal); };
   SG_CUDA(cudaMemsetAsync(gs, 0, sizeof(unsigned long long) * kGsWords, st));
@@ -543,14 +566,9 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const Graph
       FilterJob job;
       memset(&job, 0, sizeof(job));
       if (c->tune.filter_cursor) job.cursor = c->counters.p + 10;
-      job.rows = c->tune.filter_rows;
       job.n = cand_cap; job.n_dev = gs + kGsCand;
-      job.fr = c->fr.p; job.fd = c->fd.p; job.flag = c->flag.p; job.codes = rd.codes;
-      job.cstride = rd.cstride; job.lengths = rd.lengths; job.genome = R.d_codes; job.W = sp.W; job.Is = sp.Is;
-      job.fm = sp.fm; job.fx = sp.fx; job.fo = sp.fo; job.fe = sp.fe; job.fthr = sp.fthr;
-      job.counters = c->counters.p;
-      launch_expand_reads(rd, c->rexp.p, rstride, st);
-      job.gexp = R.d_gexp; job.rexp = c->rexp.p; job.rstride = rstride; job.min_len = P.minL;
+      set_filter_job(c, P, rd, R, job);
+      launch_filter_streams(c, P, rd, st);
       launch_filter_flat_job(job, sp, filter_dpx_ok(sp, P.maxL), st);
       launches += 2;
       SG_CUDA(rec(E[2]));
@@ -774,20 +792,27 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
   const int BW = 2 * sp.I + 1;
   const int wpr = (2 * BW + 31) / 32 + (sp.colour ? (BW + 31) / 32 : 0);
   const int64_t tbs = ((maxL + sp.I + 1) / 2 + 7) & ~7LL;
-  // score bound: nucleotide space, scores it has constants for, a band it is instantiated for
-  if (!c->bound_set) {
+  // the banded core's constants; score bound: nucleotide space, a band it is instantiated for
+  if (!c->band_set) {
+    c->filter_c = band_filter_consts(sp.fm, sp.fx, sp.fo, sp.fe, sp.fthr);
     memset(&c->bound_c, 0, sizeof(c->bound_c));
     if (!sp.colour && sp.I <= kMaxBoundIndels) c->bound_c = band_bound_consts(sp.pair, sp.gap_open, sp.gap_ext);
-    c->bound_set = true;
+    c->band_set = true;
   }
+  const int filter_H = filter_band_registers(sp.W, c->filter_c);
   const int bound_H = c->bound_c.ok ? bound_registers(sp.I) : 0;
-  if (bound_H) {
-    const int64_t words = n * band_stream_words(maxL, bound_H);
-    if (c->bstream.grow(words) || (reads->levels && c->wstream.grow(words))) return STORMGPU_ENOMEM;
+  {
+    const int64_t words = n * std::max(filter_H ? band_stream_words(maxL, filter_H) : 0,
+                                       bound_H ? band_stream_words(maxL, bound_H) : 0);
+    if (c->bstream.grow(words) || (bound_H && reads->levels && c->wstream.grow(words)) ||
+        (!filter_H && c->rexp.grow(n * rexp_stride(maxL))))
+      return STORMGPU_ENOMEM;
   }
-  // a call of a few reads is all launch latency: one round
-  const int rounds = n <= 256 ? 1 : std::max(1, std::min<int>(c->tune.align_rounds, kMaxAlignRounds));
-  const PassSetup P{sp, fwd, rev, n, maxL, minL, wsum, wpr, tbs, rounds, bound_H, out};
+  // Rounds pay where the bound lets each round drop most of what is left (mixed reads at -i 15: 45 % of
+  // the cells of one round); without it they only shorten alignments that stop early (3 %) and cost
+  // an alignment's latency each (300 colour reads: alignment and replay 0.70 -> 0.60 ms), as they do in a call of a few reads.
+  const int rounds = !bound_H || n <= 256 ? 1 : std::max(1, std::min<int>(c->tune.align_rounds, kMaxAlignRounds));
+  const PassSetup P{sp, fwd, rev, n, maxL, minL, wsum, wpr, tbs, rounds, filter_H, bound_H, out};
   if (c->graphs && !c->graph_broken && c->gdens_cand > 0 && c->huge_cap <= ((int64_t)1 << 22)) {
     const int g = map_passes_graph(c, P, launches);
     if (g != kGraphRetry) return g;
@@ -879,15 +904,9 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
       FilterJob job;
       memset(&job, 0, sizeof(job));
       if (c->tune.filter_cursor) job.cursor = c->counters.p + 10;  // zeroed with the counters of the pass
-      job.rows = c->tune.filter_rows;
-      job.n = utot; job.fr = c->fr.p; job.fd = c->fd.p; job.flag = c->flag.p; job.codes = rd.codes;
-      job.cstride = rd.cstride; job.lengths = rd.lengths; job.genome = R.d_codes; job.W = sp.W; job.Is = sp.Is;
-      job.fm = sp.fm; job.fx = sp.fx; job.fo = sp.fo; job.fe = sp.fe; job.fthr = sp.fthr;
-      job.counters = c->counters.p;
-      const int64_t rstride = rexp_stride(maxL);
-      if (c->rexp.grow(n * rstride)) return STORMGPU_ENOMEM;
-      launch_expand_reads(rd, c->rexp.p, rstride, st);
-      job.gexp = R.d_gexp; job.rexp = c->rexp.p; job.rstride = rstride; job.min_len = minL;
+      job.n = utot;
+      set_filter_job(c, P, rd, R, job);
+      launch_filter_streams(c, P, rd, st);
       launch_filter_flat_job(job, sp, filter_dpx_ok(sp, maxL), st);
       launches += 2;
       S.passes++;
@@ -1246,6 +1265,15 @@ extern "C" int stormgpu_sw_filter(int W, int read_len, uint32_t match, uint32_t 
     job.lengths = dl; job.genome = gb; job.W = W; job.Is = 0;
     job.gexp = gx + kGexpPad; job.rexp = rx; job.rstride = rstride; job.min_len = read_len;
     job.fm = sp.fm; job.fx = sp.fx; job.fo = sp.fo; job.fe = sp.fe; job.fthr = sp.fthr;
+    job.band = band_filter_consts(sp.fm, sp.fx, sp.fo, sp.fe, sp.fthr);
+    job.band_H = filter_band_registers(W, job.band);
+    uint32_t* bs = nullptr;
+    if (job.band_H) {
+      job.bwords = band_stream_words(read_len, job.band_H);
+      SG_CUDA(cudaMalloc(&bs, job.bwords * sizeof(uint32_t)));
+      launch_band_streams(one, job.band_H, job.bwords, bs, nullptr, job.band, 0);
+      job.bs = bs;
+    }
     launch_filter_flat_job(job, sp, filter_dpx_ok(sp, read_len), 0);
     SG_CUDA(cudaGetLastError());
     SG_CUDA(cudaDeviceSynchronize());
@@ -1253,6 +1281,7 @@ extern "C" int stormgpu_sw_filter(int W, int read_len, uint32_t match, uint32_t 
     cudaFree(dzero);
     cudaFree(gx);
     cudaFree(rx);
+    if (bs) cudaFree(bs);
   }
   SG_CUDA(cudaGetLastError());
   SG_CUDA(cudaDeviceSynchronize());

@@ -136,6 +136,29 @@ __global__ void __launch_bounds__(256, (W <= 8 ? 4 : 2)) filter_flat_dpx_kernel(
   if (job.counters) add_filter_counters(job.counters, cells, cands, band);
 }
 
+// The same over band_core.cuh's core: a candidate passes when a cell of the last row is infinite.
+// C: the constants, BandFilterDefault for the default scores.  Three blocks per SM for W = 8 (72
+// registers) and two for 16 measured best: 24.6 -> 24.0 ms and 102.4 -> 99.6 ms against four and
+// three (colour workload's candidates, mixed ones).
+template <int H, bool CURSOR, class C>
+__global__ void __launch_bounds__(256, (H <= 2 ? 4 : H <= 4 ? 3 : 2)) filter_band_kernel(const __grid_constant__ FilterJob job) {
+  constexpr int W = 2 * H;
+  const C c(job.band);
+  unsigned long long cells = 0, cands = 0, band = 0;
+  const int64_t n = job.n_dev ? (int64_t)*job.n_dev : job.n;
+  for_filter_tiles<CURSOR>(job, n, job.rows > 0 ? job.rows : kFilterTile, [&](int64_t t) {
+    const int r = job.fr[t];
+    const int64_t pos = (int64_t)job.fd[t] - job.Is;
+    const int L = job.lengths[r];
+    const int mx = band_last_row<H, false>(job.gexp, pos, job.bs + (int64_t)r * job.bwords, nullptr, L, c);
+    job.flag[t] = mx >= kBandInf ? 1 : 0;
+    cells += (unsigned long long)(2 * W) * (unsigned long long)(L + W - 1);
+    band += (unsigned long long)L * (2 * job.Is + 1);
+    cands++;
+  });
+  if (job.counters) add_filter_counters(job.counters, cells, cands, band);
+}
+
 __global__ void expand_genome_kernel(const uint8_t* __restrict__ codes, int64_t n_codes, uint8_t* __restrict__ gexp) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_codes; i += (int64_t)gridDim.x * blockDim.x)
     gexp[i] = (uint8_t)(code_at(codes, i) * 0x11);
@@ -215,7 +238,19 @@ void launch_filter_flat_job(const FilterJob& job, const ScoreParams& sp, bool dp
   default: SG_FILTER((filter_flat_dpx_kernel<16, S, C>), job); break;    \
   }
   const bool cur = job.cursor != nullptr, shrt = job.min_len < job.W;
-  if (!dpx) {
+#define SG_FILTER_B(CUR, C)                                           \
+  switch (job.band_H) {                                               \
+  case 2: SG_FILTER((filter_band_kernel<2, CUR, C>), job); break;     \
+  case 4: SG_FILTER((filter_band_kernel<4, CUR, C>), job); break;     \
+  default: SG_FILTER((filter_band_kernel<8, CUR, C>), job); break;    \
+  }
+  if (job.band_H) {
+    if (band_is_default_filter(job.band)) {
+      if (cur) { SG_FILTER_B(true, BandFilterDefault) } else { SG_FILTER_B(false, BandFilterDefault) }
+    } else {
+      if (cur) { SG_FILTER_B(true, BandConst) } else { SG_FILTER_B(false, BandConst) }
+    }
+  } else if (!dpx) {
     if (cur) SG_FILTER(filter_flat_scalar_kernel<true>, job, sp);
     else SG_FILTER(filter_flat_scalar_kernel<false>, job, sp);
   } else if (!shrt) {
@@ -223,6 +258,7 @@ void launch_filter_flat_job(const FilterJob& job, const ScoreParams& sp, bool dp
   } else {
     if (cur) { SG_FILTER_W(true, true) } else { SG_FILTER_W(true, false) }
   }
+#undef SG_FILTER_B
 #undef SG_FILTER_W
 #undef SG_FILTER
 }

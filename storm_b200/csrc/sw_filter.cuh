@@ -1,9 +1,15 @@
 // sw_filter.cuh -- packed 16-bit banded filter over a flat candidate list (sw_filter.cu).
 #pragma once
 
+#include "band_core.cuh"
 #include "map_kernels.cuh"
 
 namespace sg {
+
+// The banded core of band_core.cuh takes bands of 4, 8 and 16 cells and scores it has bytes for;
+// everything else takes filter_core.cuh's.  Both sides at the line, mixed reads at -i 15: 125.6 ms
+// with filter_core.cuh, 89.9 ms with band_core.cuh (colour at -i 7: 27.4 and 21.3 ms).
+inline int filter_band_registers(int W, const BandConst& c) { return W >= 4 && c.ok ? W / 2 : 0; }
 
 struct FilterJob {
   int64_t n;                    // candidates
@@ -27,6 +33,11 @@ struct FilterJob {
   // may be null; else a zeroed work cursor: the grid is the resident set, and every block takes
   // the next tile of 256 * kFilterTile candidates from it, in list order, until none is left
   unsigned long long* cursor;
+  // band registers of the core of band_core.cuh (0: not used), its constants and read streams
+  int band_H;
+  BandConst band;
+  const uint32_t* bs;
+  int64_t bwords;  // of a row of bs
   int rows;  // with a cursor: rows of 256 candidates in a block's tile (0 = 8); without: 8
 };
 

@@ -21,16 +21,20 @@ static void pack(const std::vector<int>& c, uint8_t* out) {
 
 template <int H, bool WTD>
 static int core(const uint8_t* gexp, int64_t pos, const std::vector<int>& read, const std::vector<int>& lev,
-                const sg::BandConst& c) {
+                const sg::BandConst& c) {  // the default scores through their immediates, as the kernels
   const int L = (int)read.size();
   const int64_t nw = sg::band_stream_words(L, H);
   std::vector<uint32_t> rs(nw), ws(nw);
-  auto nib = [&](int i) { return i >= L ? sg::kBandPad : 4u + (uint32_t)(i >= 0 ? read[i] : 0); };
+  auto nib = [&](int i) { return i < 0 || i >= L ? sg::kBandPad : 4u + (uint32_t)read[i]; };
   auto fac = [&](int i) { return (uint32_t)c.wl[i >= 0 && i < L ? lev[i] : 3]; };
   for (int64_t p = 0; p < nw; ++p) {
     rs[p] = sg::band_stream_word(nib((int)p - H - 1), nib((int)p - H), nib((int)p - 1), nib((int)p));
     ws[p] = fac((int)p - H) | fac((int)p) << 16;
   }
+  if (sg::band_is_default_filter(c))
+    return sg::band_last_row<H, WTD>(gexp, pos, rs.data(), ws.data(), L, sg::BandFilterDefault(c));
+  if (sg::band_is_default_bound(c))
+    return sg::band_last_row<H, WTD>(gexp, pos, rs.data(), ws.data(), L, sg::BandBoundDefault(c));
   return sg::band_last_row<H, WTD>(gexp, pos, rs.data(), ws.data(), L, c);
 }
 
@@ -85,8 +89,8 @@ int main(int argc, char** argv) {
   for (int i = 0; i < G; ++i) gexp[i] = (uint8_t)(g[i] * 0x11);
   int nfilter = 0, nequal = 0, nbound = 0, passed = 0, kept = 0;
   for (int t = 0; t < cases; ++t) {
-    const int Ls[16] = {4, 7, 8, 15, 16, 17, 24, 31, 33, 35, 49, 50, 76, 100, 150, 251};
-    const int L = Ls[rng() % 16];
+    const int Ls[18] = {1, 2, 4, 7, 8, 15, 16, 17, 24, 31, 33, 35, 49, 50, 76, 100, 150, 251};
+    const int L = Ls[rng() % 18];
     const int src = (int)(rng() % (G - L - 80));
     std::vector<int> read(L), lev(L), three(L, 3);
     const double rate = (rng() % 5) * 0.1;
@@ -107,10 +111,10 @@ int main(int argc, char** argv) {
     const int Ws[3] = {4, 8, 16};
     const int W = Ws[rng() % 3];
     const int64_t pos = (rng() % 3 == 0) ? (int64_t)(rng() % (G + 2 * L)) - L : src - (int64_t)(rng() % (2 * W));
-    if (L >= W) {
+    {
       const int thr = (int)(rng() % 4 ? 5 + rng() % 200 : rng() % 260);
       const sg::BandConst c = sg::band_filter_consts(match, mism, go, ge, thr >= 255 ? 254 : thr);
-      if (def && !c.ok) { printf("default scores have no score bytes\n"); return 1; }
+      if (def && !sg::band_is_default_filter(c)) { printf("default scores have other score bytes\n"); return 1; }
       if (c.ok) {
         const int got = core_h<false>(W / 2, gexp, pos, read, three, c) >= sg::kBandInf;
         const int exp = or_sw_filter(W, L, match, mism, go, ge, thr, gen, pos, rb.data());
@@ -126,11 +130,11 @@ int main(int argc, char** argv) {
     const int Is[8] = {1, 3, 5, 7, 10, 15, 20, 23};
     const int I = Is[rng() % 8];
     const int H = I <= 3 ? 2 : I <= 7 ? 4 : I <= 15 ? 8 : 12;
-    if (L >= 2 * H) {
+    {
       int pair[2][4];
       for (int l = 0; l < 4; ++l) { pair[0][l] = match * (l + 1) / 4; pair[1][l] = -(mism * (l + 1) / 4); }
       const sg::BandConst c = sg::band_bound_consts(pair, -go, -ge);
-      if (def && !c.ok) { printf("default scores have no score bytes (bound)\n"); return 1; }
+      if (def && !sg::band_is_default_bound(c)) { printf("default scores have other score bytes (bound)\n"); return 1; }
       const int tm = 100;
       if (!c.ok) continue;
       const int lim = sg::band_bound_limit(match, mism, L);  // bounds below it are exact

@@ -97,7 +97,9 @@ struct stormgpu_ctx {
   // the banded core, its constants for the filter and the bound (band_set: computed for this
   // context's scores)
   sg::DevBuf<int32_t> q_read, q_diag;
-  sg::DevBuf<int16_t> q_ub, p_ub;  // the bounds of both lists
+  sg::DevBuf<int16_t> q_ub, k_ub, p_ub;  // the bounds of the lists
+  // the kept candidates' diagonals before they are put in order, the reads with many of them
+  sg::DevBuf<int32_t> k_diag, long_list;
   sg::DevBuf<uint32_t> bstream, wstream;
   sg::BandConst filter_c, bound_c;
   bool band_set = false;

@@ -4,16 +4,15 @@
 // strictly greater than the previous one in sorted order, the previous of the first being -I
 // (run.c:617, :648, :697).
 //
-// One warp per read: keys computed from the packed read, CSR offsets read from the
-// (L2-resident) key table, positions gathered straight into the warp's shared memory, bitonic
-// sort there, de-duplication by ballot, and the surviving diagonals appended to the flat
-// candidate list (reads contiguous, diagonals ascending within a read).  Every lane looks up
-// several (seed, position) keys before any result is used, so that a read costs two memory
-// latencies (key table, positions) rather than two per seed.  Up to 32 positions are sorted in
-// registers; more are first reduced to distinct values (warp_dedupe), then bucket-sorted
-// (bucket_sort_emit).  Reads with more index positions than a warp can hold go to a
-// block-per-read kernel (shared memory up to 32768 positions) and, beyond that, to a
-// global-memory variant run one read at a time.
+// One warp per read: keys computed from the packed read, CSR offsets read from the (L2-resident) key
+// table, positions gathered straight into the warp's shared memory, reduced to the distinct
+// diagonals there and appended to the flat candidate list, in no order: only a candidate that
+// passes the filter needs its place among its read's (3 in 1,000 on the colour workload), and
+// slot_lists_kernel gives it (map_kernels.cu).  Every lane looks up several (seed, position) keys
+// before any result is used, so that a read costs two memory latencies (key table, positions) rather
+// than two per seed.  Reads with more index positions than a warp can hold go to a
+// block-per-read kernel (shared memory up to 4096 positions) and, beyond that, to slices in global
+// memory; these append ascending diagonals.
 #include <type_traits>
 
 #include "gather.cuh"
@@ -50,19 +49,6 @@ __device__ __forceinline__ int seed_npos(const SeedDev& s, int L) {
   return s.n_positions ? s.n_positions : (L - s.span + 1 > 0 ? L - s.span + 1 : 0);
 }
 
-// (index offset, count, read position) of item t of seed si
-__device__ __forceinline__ void seed_item(const SeedSet& gs, const IndexView& ix, int si, int t, const uint8_t* read,
-                                          int L, int& a, int& cnt, int& rp) {
-  const SeedDev& s = gs.s[si];
-  a = 0; cnt = 0; rp = 0;
-  if (t >= seed_npos(s, L)) return;
-  rp = s.n_positions ? s.positions[t] : t;
-  if (rp < 0 || rp >= L) return;
-  const uint32_t key = read_key(s, read, L, rp);
-  a = __ldg(ix.first[si] + key);
-  cnt = __ldg(ix.first[si] + key + 1) - a;
-}
-
 // (index offset, count, read position) of position t of seed s, with that seed's key table;
 // `read` is staged in shared memory (see read_key_window)
 __device__ __forceinline__ void item_lookup(const int32_t* __restrict__ first, const SeedDev& s, int t,
@@ -76,36 +62,21 @@ __device__ __forceinline__ void item_lookup(const int32_t* __restrict__ first, c
   cnt = __ldg(first + key + 1) - a;
 }
 
-__device__ __forceinline__ void warp_bitonic(int32_t* s, int P) {
-  const int lane = threadIdx.x & 31;
-  for (int k = 2; k <= P; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = lane; i < P; i += 32) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const int32_t a = s[i], b = s[ixj];
-          if ((a > b) == ((i & k) == 0)) { s[i] = b; s[ixj] = a; }
-        }
-      }
-      __syncwarp();
-    }
-}
-
-// sorted s[0..H) -> accepted diagonals appended to the flat list (one warp)
-__device__ __forceinline__ void warp_emit(int32_t* s, int H, int I, int r, const GatherOut& go) {
+// Diagonals a[0..U) (distinct, any order; one warp) -> flat list; the smallest, vmin, is dropped when
+// it is not above -I (run.c:617, :648).
+__device__ __forceinline__ void warp_emit(int32_t* a, int U, int32_t vmin, int I, int r, const GatherOut& go) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  int U = 0;
-  for (int t0 = 0; t0 < H; t0 += 32) {
-    const int t = t0 + lane;
-    const int32_t v = t < H ? s[t] : 0;
-    const int32_t prev = t == 0 ? -I : (t < H ? s[t - 1] : 0);
-    const bool keep = t < H && v > prev;
-    const unsigned m = __ballot_sync(0xffffffffu, keep);
-    __syncwarp();
-    if (keep) s[U + __popc(m & lt)] = v;  // compaction in place (writes trail reads)
-    U += __popc(m);
-    __syncwarp();
+  if (U > 0 && vmin <= -I) {
+    int W = 0;
+    for (int k0 = 0; k0 < U; k0 += 32) {
+      const int32_t v = k0 + lane < U ? a[k0 + lane] : vmin;
+      const unsigned m = __ballot_sync(0xffffffffu, v != vmin);
+      if (v != vmin) a[W + __popc(m & lt)] = v;  // writes trail the reads
+      W += __popc(m);
+      __syncwarp();
+    }
+    U = W;
   }
   unsigned long long base = 0;
   if (lane == 0 && U) base = atomicAdd(&go.counters[7], (unsigned long long)U);
@@ -116,102 +87,27 @@ __device__ __forceinline__ void warp_emit(int32_t* s, int H, int I, int r, const
   }
   for (int k = lane; k < U; k += 32) {
     go.fr[base + k] = r;
-    go.fd[base + k] = s[k];
+    go.fd[base + k] = a[k];
   }
-}
-
-// Bitonic sort of 32*E values held E per lane (value k of lane l is element k*32 + l):
-// partners 32 or more apart are in the same lane (register compare-exchange), closer ones are
-// exchanged with __shfl_xor_sync.
-template <int E>
-__device__ __forceinline__ void reg_bitonic(int32_t (&v)[E]) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int kk = 2; kk <= 32 * E; kk <<= 1) {
-#pragma unroll
-    for (int j = kk >> 1; j > 0; j >>= 1) {
-      if (j >= 32) {
-#pragma unroll
-        for (int k = 0; k < E; ++k) {
-          const int k2 = k ^ (j >> 5);
-          if (k2 > k) {
-            const bool up = ((k * 32 + lane) & kk) == 0;
-            const int32_t a = v[k], b = v[k2];
-            const bool sw = (a > b) == up;
-            v[k] = sw ? b : a;
-            v[k2] = sw ? a : b;
-          }
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < E; ++k) {
-          const int32_t o = __shfl_xor_sync(0xffffffffu, v[k], j);
-          const bool up = ((k * 32 + lane) & kk) == 0;
-          const bool lower = (lane & j) == 0;
-          v[k] = (lower == up) ? min(v[k], o) : max(v[k], o);
-        }
-      }
-    }
-  }
-}
-
-// accepted diagonals of the sorted register array (first H valid) -> flat list
-template <int E>
-__device__ __forceinline__ void reg_emit(const int32_t (&v)[E], int H, int I, int r, const GatherOut& go) {
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  unsigned m[E];
-  int U = 0;
-#pragma unroll
-  for (int k = 0; k < E; ++k) {
-    const int32_t up = __shfl_up_sync(0xffffffffu, v[k], 1);
-    const int32_t last = __shfl_sync(0xffffffffu, k ? v[k > 0 ? k - 1 : 0] : 0, 31);
-    const int32_t prev = lane ? up : (k ? last : -I);
-    const bool keep = (k * 32 + lane) < H && v[k] > prev;
-    m[k] = __ballot_sync(0xffffffffu, keep);
-    U += __popc(m[k]);
-  }
-  unsigned long long base = 0;
-  if (lane == 0 && U) base = atomicAdd(&go.counters[7], (unsigned long long)U);
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if ((int64_t)(base + U) > go.cap) {
-    if (lane == 0) atomicExch(&go.counters[8], 1ull);
-    return;
-  }
-  int off = 0;
-#pragma unroll
-  for (int k = 0; k < E; ++k) {
-    if ((m[k] >> lane) & 1u) {
-      const int64_t o = (int64_t)base + off + __popc(m[k] & lt);
-      go.fr[o] = r;
-      go.fd[o] = v[k];
-    }
-    off += __popc(m[k]);
-  }
-}
-
-template <int E>
-__device__ __forceinline__ void sort_emit_regs(const int32_t* s, int H, int I, int r, const GatherOut& go) {
-  const int lane = threadIdx.x & 31;
-  int32_t v[E];
-#pragma unroll
-  for (int k = 0; k < E; ++k) {
-    const int i = k * 32 + lane;
-    v[k] = i < H ? s[i] : 0x7fffffff;
-  }
-  reg_bitonic<E>(v);
-  reg_emit<E>(v, H, I, r, go);
 }
 
 // Drop repeated values from a[0..H) (one warp), keeping one of each, compacted to the front
 // of a (order not kept); tab[0..cap), cap >= H, is the open-addressing set.  The diagonal a read
-// truly maps to comes once per (seed, position) that hits it, so this removes the one large
-// group of equal values before the sort.  Returns the number of distinct values.
+// truly maps to comes once per (seed, position) that hits it.  Returns the number of distinct values.
 constexpr int32_t kEmptySlot = 0x7fffffff;  // no diagonal (position - read position) reaches it
 __device__ __forceinline__ int warp_dedupe(int32_t* a, int H, int32_t* tab, int cap) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  for (int i = lane; i < cap; i += 32) tab[i] = kEmptySlot;
+  if (H <= 32) {
+    const int32_t v = lane < H ? a[lane] : kEmptySlot;
+    const unsigned peers = __match_any_sync(0xffffffffu, v);
+    const unsigned m = __ballot_sync(0xffffffffu, lane < H && (peers & lt) == 0);
+    if ((m >> lane) & 1u) a[__popc(m & lt)] = v;
+    __syncwarp();
+    return __popc(m);
+  }
+  const int size = min(cap, 2 * H);
+  for (int i = lane; i < size; i += 32) tab[i] = kEmptySlot;
   __syncwarp();
   int U = 0;
   for (int i0 = 0; i0 < H; i0 += 32) {
@@ -220,12 +116,12 @@ __device__ __forceinline__ int warp_dedupe(int32_t* a, int H, int32_t* tab, int 
     int32_t v = 0;
     if (i < H) {
       v = a[i];
-      uint32_t h = __umulhi((uint32_t)v * 0x9E3779B1u, (uint32_t)cap);
+      uint32_t h = __umulhi((uint32_t)v * 0x9E3779B1u, (uint32_t)size);
       for (;;) {
         const int32_t old = atomicCAS(&tab[h], kEmptySlot, v);
         if (old == kEmptySlot) { keep = true; break; }
         if (old == v) break;
-        h = h + 1 == (uint32_t)cap ? 0u : h + 1;
+        h = h + 1 == (uint32_t)size ? 0u : h + 1;
       }
     }
     const unsigned m = __ballot_sync(0xffffffffu, keep);
@@ -236,64 +132,32 @@ __device__ __forceinline__ int warp_dedupe(int32_t* a, int H, int32_t* tab, int 
   return U;
 }
 
-// Sort a[0..H) (one warp) into b[0..H) and emit: 32 buckets of equal width over [min, max]
-// (so that bucket order is value order), counted with shared atomics,
-// scattered to b, then every lane insertion-sorts its own bucket.  A bucket holding more than
-// 64 values (clustered diagonals) falls back to the bitonic sort of a, which needs room for
-// the next power of two of H from a on (a and b are adjacent).
-__device__ __forceinline__ void bucket_sort_emit(int32_t* a, int32_t* b, int32_t* hist, int H, int I, int r,
-                                                 const GatherOut& go) {
-  const int lane = threadIdx.x & 31;
-  int32_t vmin = 0x7fffffff, vmax = (int32_t)0x80000000;
-  for (int i = lane; i < H; i += 32) {
-    const int32_t v = a[i];
-    vmin = min(vmin, v);
-    vmax = max(vmax, v);
+// A seed's care positions as runs, for keys from a window of 32 codes whose first code is in the
+// high bits: the key is the OR of (window >> sh) & mask over the runs (4 to 7 of them, where taking
+// the care positions one by one takes 10 to 15 steps).
+struct SeedRuns {
+  int n;
+  uint8_t sh[16];
+  uint32_t mask[16];
+};
+
+__device__ __forceinline__ void make_runs(const SeedDev& s, SeedRuns& o) {
+  int n = 0;
+  for (int c = 0; c < s.n_care;) {
+    int m = 1;
+    while (c + m < s.n_care && s.care[c + m] - s.care[c] == m) ++m;
+    o.sh[n] = (uint8_t)(62 - 2 * (s.care[c] + s.n_care - 1 - c));
+    o.mask[n] = (uint32_t)((1ull << (2 * m)) - 1ull) << (2 * (s.n_care - c - m));
+    ++n;
+    c += m;
   }
-  vmin = __reduce_min_sync(0xffffffffu, vmin);
-  vmax = __reduce_max_sync(0xffffffffu, vmax);
-  // bucket = floor(32 * (v - min) / (range + 1)) as a multiply-high: monotone, all 32 buckets used
-  const uint32_t range = (uint32_t)vmax - (uint32_t)vmin;
-  const uint32_t mul = range < 32u ? 0u : (uint32_t)((32ull << 32) / ((uint64_t)range + 1ull));
-  auto bucket = [&](int32_t v) -> int {
-    const uint32_t x = (uint32_t)v - (uint32_t)vmin;
-    return range < 32u ? (int)x : (int)__umulhi(x, mul);
-  };
-  hist[lane] = 0;
-  __syncwarp();
-  for (int i = lane; i < H; i += 32) atomicAdd(&hist[bucket(a[i])], 1);
-  __syncwarp();
-  const int c = hist[lane];
-  const int incl = warp_incl_scan(c);
-  const int base = incl - c;
-  if (__reduce_max_sync(0xffffffffu, (unsigned)c) > 64u) {
-    int P = 1;
-    while (P < H) P <<= 1;
-    for (int i = H + lane; i < P; i += 32) a[i] = 0x7fffffff;
-    __syncwarp();
-    warp_bitonic(a, P);
-    warp_emit(a, H, I, r, go);
-    return;
-  }
-  __syncwarp();
-  hist[lane] = base;
-  __syncwarp();
-  for (int i = lane; i < H; i += 32) {
-    const int32_t v = a[i];
-    b[atomicAdd(&hist[bucket(v)], 1)] = v;
-  }
-  __syncwarp();
-  for (int x = 1; x < c; ++x) {
-    const int32_t t = b[base + x];
-    int y = x - 1;
-    while (y >= 0 && b[base + y] > t) {
-      b[base + y + 1] = b[base + y];
-      --y;
-    }
-    b[base + y + 1] = t;
-  }
-  __syncwarp();
-  warp_emit(b, H, I, r, go);
+  o.n = n;
+}
+
+// 16 packed codes, first code in the low bits -> first code in the high bits
+__device__ __forceinline__ uint32_t reverse_codes(uint32_t x) {
+  x = __brev(x);
+  return ((x & 0x55555555u) << 1) | ((x >> 1) & 0x55555555u);
 }
 
 constexpr int kGWarps = 4;
@@ -303,28 +167,32 @@ constexpr int kGWarps = 4;
 // read order: a batch whose reads are grouped by length gives a candidate list grouped by
 // length, which the filter needs to keep one read length per SM.
 constexpr int kReadBytes = STORMGPU_MAX_READ_LEN / 4 + 16;
+constexpr int kReadWords = STORMGPU_MAX_READ_LEN / 16 + 3;
 
 constexpr int kItems = 4;  // (seed, position) items per lane and round: 128 key lookups in flight per warp
 
 __global__ void __launch_bounds__(kGWarps * 32, 8) gather_fused_kernel(ReadsDev rd, IndexView ix, int I, GatherOut go,
                                                                    const __grid_constant__ SeedSet gs) {
-  extern __shared__ int32_t sm[];  // per warp 2 * cap: gathered positions, then the set / sorted copy
-  __shared__ int32_t shist[kGWarps][32];
+  extern __shared__ int32_t sm[];  // per warp 2 * cap: gathered positions, then the set
+  __shared__ SeedRuns runs[kMaxSeeds];
+  __shared__ int32_t sspan[kMaxSeeds];
   __shared__ int32_t soff[kGWarps][kMaxSeeds + 1];  // first item of every seed, for the current read
   __shared__ const int32_t* s_first[kMaxSeeds];
   __shared__ const int32_t* s_map[kMaxSeeds];
-  __shared__ __align__(16) uint8_t srd[kGWarps][kReadBytes];
+  __shared__ uint32_t srev[kGWarps][kReadWords];  // the read's codes, first code in the high bits, 0 after its end
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nseeds = gs.n;
   if (threadIdx.x < nseeds) {
     s_first[threadIdx.x] = ix.first[threadIdx.x];
     s_map[threadIdx.x] = ix.map[threadIdx.x];
+    sspan[threadIdx.x] = gs.s[threadIdx.x].span;
+    if (gs.s[threadIdx.x].span <= 32) make_runs(gs.s[threadIdx.x], runs[threadIdx.x]);
   }
   __syncthreads();
   const int cap = go.warp_cap;
   int32_t* s = sm + (size_t)w * 2 * cap;
   int32_t* so = soff[w];
-  uint8_t* rs = srd[w];
+  uint32_t* rv = srev[w];
   unsigned long long lookups = 0, positions = 0;
   for (;;) {
   unsigned long long k0 = 0;
@@ -335,16 +203,23 @@ __global__ void __launch_bounds__(kGWarps * 32, 8) gather_fused_kernel(ReadsDev 
   for (int64_t kr = (int64_t)k0; kr < kend; ++kr) {
     const int64_t r = rd.order ? (int64_t)rd.order[kr] : kr;
     const int L = rd.lengths[r];
+    const uint8_t* src = rd.codes + r * rd.cstride;
     {  // the read's packed codes into shared memory, and the item offsets of the seeds
-      const uint8_t* src = rd.codes + r * rd.cstride;
-      const int nb = (L + 3) >> 2;
-      for (int b = lane; b < nb; b += 32) rs[b] = src[b];
+      const int nb = (L + 3) >> 2, nw = (L + 15) >> 4;
+      for (int k = lane; k < nw + 2; k += 32) {
+        uint32_t x = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          if (4 * k + b < nb) x |= (uint32_t)src[4 * k + b] << (8 * b);
+        const int left = L - 16 * k;  // codes of this word
+        if (left < 16) x &= left > 0 ? (1u << (2 * left)) - 1u : 0u;
+        rv[k] = reverse_codes(x);
+      }
       const int np = lane < nseeds ? seed_npos(gs.s[lane], L) : 0;
       const int incl = warp_incl_scan(np);
       if (lane <= nseeds) so[lane] = incl - np;
       __syncwarp();
     }
-    const uint8_t* read = rs;
     const int T = so[nseeds];
     int H = 0;
     // a read with more positions than the warp holds is only counted from there on and goes to
@@ -356,10 +231,27 @@ __global__ void __launch_bounds__(kGWarps * 32, 8) gather_fused_kernel(ReadsDev 
       for (int m = 0; m < kItems; ++m) {
         const int it = r0 + m * 32 + lane;
         int si = 0;
-        if (it < T)
+        a[m] = 0; cnt[m] = 0; rp[m] = 0;
+        if (it < T) {
           while (it >= so[si + 1]) ++si;
+          rp[m] = it - so[si];
+          if (gs.s[si].n_positions) rp[m] = gs.s[si].positions[rp[m]];
+          if (rp[m] >= 0 && rp[m] < L) {
+            uint32_t key = 0;
+            if (sspan[si] <= 32) {
+              const uint32_t* q = rv + (rp[m] >> 4);
+              const int sh = 2 * (rp[m] & 15);
+              const uint64_t win = (uint64_t)__funnelshift_l(q[1], q[0], sh) << 32 | __funnelshift_l(q[2], q[1], sh);
+              const SeedRuns& R = runs[si];
+              for (int c = 0; c < R.n; ++c) key |= (uint32_t)(win >> R.sh[c]) & R.mask[c];
+            } else {
+              key = read_key(gs.s[si], src, L, rp[m]);
+            }
+            a[m] = __ldg(s_first[si] + key);
+            cnt[m] = __ldg(s_first[si] + key + 1) - a[m];
+          }
+        }
         sid[m] = si;
-        item_lookup(s_first[si], gs.s[si], it < T ? it - so[si] : 0x40000000, read, L, a[m], cnt[m], rp[m]);
       }
       // ... then one scan places all of them, and the position loads go out together
       int tot = 0;
@@ -417,13 +309,10 @@ __global__ void __launch_bounds__(kGWarps * 32, 8) gather_fused_kernel(ReadsDev 
     positions += (unsigned long long)H;
     lookups += (unsigned long long)T;
     __syncwarp();
-    if (H <= 32) {
-      sort_emit_regs<1>(s, H, I, (int)r, go);
-    } else {
-      const int U = warp_dedupe(s, H, s + cap, cap);
-      if (U <= 32) sort_emit_regs<1>(s, U, I, (int)r, go);
-      else bucket_sort_emit(s, s + cap, shist[w], U, I, (int)r, go);
-    }
+    const int U = warp_dedupe(s, H, s + cap, cap);
+    int32_t vmin = 0x7fffffff;
+    for (int k = lane; k < U; k += 32) vmin = min(vmin, s[k]);
+    warp_emit(s, U, __reduce_min_sync(0xffffffffu, vmin), I, (int)r, go);
     __syncwarp();
   }
   }

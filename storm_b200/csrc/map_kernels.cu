@@ -782,18 +782,32 @@ __global__ void slot_starts_kernel(int64_t npass, const int64_t* __restrict__ np
 }
 
 // Per read its number of slots, the list of reads with slots, and with rounds the first round's
-// slots: the first `take` of each read (their bounds exceed -t, the threshold it starts from).
-__global__ void slot_lists_kernel(int64_t npass, const int64_t* __restrict__ npass_dev, PassBuffers pb, int take) {
-  if (npass_dev) npass = *npass_dev;
+// slots: the first `take` of each read (their bounds exceed -t, the threshold it starts from).  A
+// slot's place in its read is the number of smaller diagonals of the read (they are distinct),
+// counted here for reads with few slots; the others go to the long list.
+__global__ void slot_lists_kernel(KeptList kl, int16_t* __restrict__ ub, PassBuffers pb, int take) {
+  const int64_t npass = kl.n_dev ? *kl.n_dev : kl.n;
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < npass; base += stride) {
     const int64_t s = base + lane;
     const bool in = s < npass;
     const int r = in ? pb.p_read[s] : -1;
-    const int rank = in ? (int)(s - pb.pstart[r]) : -1;
+    const int64_t s0 = in ? pb.pstart[r] : 0;
+    const int rank = in ? (int)(s - s0) : -1;
     const bool last = in && (s == npass - 1 || pb.p_read[s + 1] != r);
     if (last) pb.pcount[r] = rank + 1;
+    if (in) {
+      const int32_t d = kl.diag[s];
+      int smaller = 0, k = 0;
+      for (; k <= kShortSlots && s0 + k < npass && pb.p_read[s0 + k] == r; ++k) smaller += kl.diag[s0 + k] < d;
+      if (k <= kShortSlots) {
+        pb.p_diag[s0 + smaller] = d;
+        if (kl.ub) ub[s0 + smaller] = kl.ub[s];
+      } else if (rank == 0) {
+        kl.long_list[atomicAdd(kl.long_count, 1)] = r;
+      }
+    }
     const unsigned mf = __ballot_sync(0xffffffffu, rank == 0);
     if (mf) {
       int b = 0;
@@ -815,11 +829,65 @@ __global__ void slot_lists_kernel(int64_t npass, const int64_t* __restrict__ npa
   }
 }
 
-void launch_slot_lists(int64_t npass, const int64_t* npass_dev, PassBuffers& pb, int take, cudaStream_t st) {
-  if (npass <= 0) return;
-  const int64_t blocks = std::min<int64_t>((npass + 255) / 256, 148 * 32);
-  slot_starts_kernel<<<(unsigned)blocks, 256, 0, st>>>(npass, npass_dev, pb.p_read, pb.pstart);
-  slot_lists_kernel<<<(unsigned)blocks, 256, 0, st>>>(npass, npass_dev, pb, take);
+// The reads of the long list, one warp each: their slots copied when they are ascending already (the
+// block gather's reads), else sorted in shared memory as (diagonal, bound) keys.
+constexpr int kSortWarps = 4;
+__global__ void __launch_bounds__(kSortWarps * 32) slot_sort_kernel(KeptList kl, int16_t* __restrict__ ub, PassBuffers pb,
+                                                                    int cap) {
+  extern __shared__ unsigned long long skeys[];  // cap per warp, a power of two
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned long long* a = skeys + (size_t)w * cap;
+  const int n = *kl.long_count;
+  for (int q = blockIdx.x * kSortWarps + w; q < n; q += gridDim.x * kSortWarps) {
+    const int r = kl.long_list[q];
+    const int P = pb.pcount[r];
+    const int64_t s0 = pb.pstart[r];
+    bool asc = true;
+    for (int k = lane; k < P; k += 32) {
+      const int32_t d = kl.diag[s0 + k];
+      if (k > 0 && kl.diag[s0 + k - 1] > d) asc = false;
+      pb.p_diag[s0 + k] = d;
+      if (kl.ub) ub[s0 + k] = kl.ub[s0 + k];
+    }
+    if (__all_sync(0xffffffffu, asc) || P > cap) continue;  // a read above cap came from the block gather
+    int N = 64;
+    while (N < P) N <<= 1;
+    for (int k = lane; k < N; k += 32)
+      a[k] = k < P ? ((unsigned long long)((uint32_t)kl.diag[s0 + k] ^ 0x80000000u) << 32) |
+                         (kl.ub ? (uint16_t)kl.ub[s0 + k] : 0u)
+                   : ~0ull;
+    __syncwarp();
+    for (int k = 2; k <= N; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int i = lane; i < N; i += 32) {
+          const int x = i ^ j;
+          if (x > i) {
+            const unsigned long long u = a[i], v = a[x];
+            if ((u > v) == ((i & k) == 0)) { a[i] = v; a[x] = u; }
+          }
+        }
+        __syncwarp();
+      }
+    for (int k = lane; k < P; k += 32) {
+      pb.p_diag[s0 + k] = (int32_t)((uint32_t)(a[k] >> 32) ^ 0x80000000u);
+      if (kl.ub) ub[s0 + k] = (int16_t)(uint16_t)a[k];
+    }
+    __syncwarp();
+  }
+}
+
+void launch_slot_lists(const KeptList& kl, int16_t* ub, PassBuffers& pb, int take, cudaStream_t st) {
+  if (kl.n <= 0) return;
+  const int64_t blocks = std::min<int64_t>((kl.n + 255) / 256, 148 * 32);
+  slot_starts_kernel<<<(unsigned)blocks, 256, 0, st>>>(kl.n, kl.n_dev, pb.p_read, pb.pstart);
+  slot_lists_kernel<<<(unsigned)blocks, 256, 0, st>>>(kl, ub, pb, take);
+  int cap = 64;
+  while (cap < kl.sort_cap) cap <<= 1;
+  const size_t smem = (size_t)kSortWarps * cap * sizeof(unsigned long long);
+  set_smem_attribute_once(reinterpret_cast<const void*>(slot_sort_kernel), kSortWarps * 2048 * 8);
+  const int64_t grid = std::min<int64_t>((kl.n / kShortSlots + kSortWarps) / kSortWarps,
+                                         resident_grid(slot_sort_kernel, kSortWarps * 32, smem));
+  slot_sort_kernel<<<(unsigned)grid, kSortWarps * 32, smem, st>>>(kl, ub, pb, cap);
 }
 
 }  // namespace sg

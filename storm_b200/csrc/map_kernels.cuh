@@ -56,8 +56,8 @@ struct PassBuffers {
   int32_t* active;
   int32_t* active_next;
   int32_t* active_count;
-  int32_t* p_read;      // per slot
-  int32_t* p_diag;
+  int32_t* p_read;      // per slot, reads contiguous
+  int32_t* p_diag;      // per slot, ascending within a read
   int64_t p_cap;
   unsigned long long* counters;  // [0] slots used, [1] overflow flag, [2] filter cells, [3] lookups, [4] positions
   // align outputs per slot
@@ -103,10 +103,22 @@ void launch_align(const ReadsDev& r, const ScoreParams& sp, const uint8_t* genom
                   cudaStream_t st);
 // scratch columns of a launch_align with a cursor (the threads of its persistent grid)
 int64_t align_workers(int64_t nslots, const ScoreParams& sp);
-// pstart / pcount and the first active list of the pass's slots (npass of them, or with npass_dev (may
-// be null) an upper bound for the grid and the count is read from there); with rounds the first
-// round's slots, `take` per read.  The counts are zeroed by the caller.
-void launch_slot_lists(int64_t npass, const int64_t* npass_dev, PassBuffers& pb, int take, cudaStream_t st);
+// The candidates of a pass that are aligned, as the filter (and the score bound) left them: reads
+// contiguous, each read's diagonals in any order.
+struct KeptList {
+  int64_t n;                 // or with n_dev (may be null) an upper bound for the grid
+  const int64_t* n_dev;
+  const int32_t* diag;
+  const int16_t* ub;         // may be null
+  int32_t* long_list;        // reads with more than kShortSlots candidates (as many as reads), their number (zeroed)
+  int32_t* long_count;
+  int sort_cap;              // most candidates of a read whose diagonals are not ascending already
+};
+constexpr int kShortSlots = 64;
+// pb.p_diag / pb.ub from the list, ascending within each read; pstart / pcount and the first active
+// list; with rounds the first round's slots, `take` per read.  The counts are zeroed by the caller.
+// pb.p_read is the list's.
+void launch_slot_lists(const KeptList& kl, int16_t* ub, PassBuffers& pb, int take, cudaStream_t st);
 // Replay of the active reads (at most n): the whole read (no rounds), or the ranks selected last and
 // then the selection of up to `take` candidates for the next round.
 void launch_replay(int64_t n, const ScoreParams& sp, int ref_id, int sense, PassBuffers& pb, int take,

@@ -205,7 +205,8 @@ extern "C" void stormgpu_close(stormgpu_ctx* c) {
   c->a_pos.release(); c->a_tb.release(); c->scratch.release(); c->counters.release();
   c->foff.release(); c->fr.release(); c->fd.release(); c->flag.release(); c->flagw.release();
   c->rexp.release();
-  c->q_read.release(); c->q_diag.release(); c->q_ub.release(); c->p_ub.release(); c->bstream.release(); c->wstream.release();
+  c->q_read.release(); c->q_diag.release(); c->q_ub.release(); c->k_ub.release(); c->p_ub.release();
+  c->k_diag.release(); c->long_list.release(); c->bstream.release(); c->wstream.release();
   c->gm_k0.release(); c->gm_v0.release(); c->gm_k1.release(); c->gm_v1.release(); c->gm_tmp.release();
   c->gm_base.release();
   c->ord.release(); c->ord_tmp.release();
@@ -447,7 +448,7 @@ static void launch_bound_pass(stormgpu_ctx* c, const PassSetup& P, const ReadsDe
 
 // Buffers of the replay's lists: two lists of active reads, and with rounds the round's slots.
 static int round_lists_grow(stormgpu_ctx* c, int64_t n, int64_t kept, int rounds) {
-  if (c->active.grow(2 * n) || c->rounds.grow(2 * kRoundCounts)) return STORMGPU_ENOMEM;
+  if (c->active.grow(2 * n) || c->long_list.grow(n) || c->rounds.grow(2 * kRoundCounts + 1)) return STORMGPU_ENOMEM;
   if (rounds > 1 && (c->thr.grow(n) || c->round_cur.grow(2 * n) || c->round_slots.grow(kept))) return STORMGPU_ENOMEM;
   return 0;
 }
@@ -464,7 +465,7 @@ static void round_buffers(stormgpu_ctx* c, int k, PassBuffers& pb) {
 }
 
 static int setup_rounds(stormgpu_ctx* c, int rounds, PassBuffers& pb, cudaStream_t st) {
-  SG_CUDA(cudaMemsetAsync(c->rounds.p, 0, sizeof(unsigned long long) * 2 * kRoundCounts, st));
+  SG_CUDA(cudaMemsetAsync(c->rounds.p, 0, sizeof(unsigned long long) * (2 * kRoundCounts + 1), st));
   round_buffers(c, 0, pb);
   if (rounds > 1) {
     pb.round_slots = c->round_slots.p;
@@ -472,6 +473,18 @@ static int setup_rounds(stormgpu_ctx* c, int rounds, PassBuffers& pb, cudaStream
     pb.thr = c->thr.p;
   }
   return 0;
+}
+
+static KeptList kept_list(stormgpu_ctx* c, const PassSetup& P, int64_t n, const int64_t* n_dev) {
+  KeptList kl;
+  kl.n = n;
+  kl.n_dev = n_dev;
+  kl.diag = c->k_diag.p;
+  kl.ub = P.bound_H ? c->k_ub.p : nullptr;
+  kl.long_list = c->long_list.p;
+  kl.long_count = reinterpret_cast<int32_t*>(c->rounds.p + 2 * kRoundCounts);
+  kl.sort_cap = c->tune.gather_warp_cap;  // more come from the block gather, in order
+  return kl;
 }
 
 // List capacities of a graph call.
@@ -493,9 +506,9 @@ static bool graph_buffers(stormgpu_ctx* c, const PassSetup& P, GraphCaps* caps) 
       c->big_tmp.grow(std::max(grid_b * 2 * (int64_t)kBlockGatherCap, caps->grid_h * 2 * c->huge_cap)))
     return false;
   if (P.bound_H && (c->q_read.grow(want_pass) || c->q_diag.grow(want_pass) || c->q_ub.grow(want_pass) ||
-                    c->p_ub.grow(want_kept)))
+                    c->k_ub.grow(want_kept) || c->p_ub.grow(want_kept)))
     return false;
-  if (c->p_read.grow(want_kept) || c->p_diag.grow(want_kept) || c->a_score.grow(want_kept) ||
+  if (c->p_read.grow(want_kept) || c->p_diag.grow(want_kept) || c->k_diag.grow(want_kept) || c->a_score.grow(want_kept) ||
       c->a_bound.grow(want_kept) || c->a_tblen.grow(want_kept) || c->a_pos.grow(want_kept * 4) ||
       c->a_tb.grow(want_kept * P.tbs))
     return false;
@@ -591,20 +604,20 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const Graph
         exclusive_scan<PassWord, int64_t>(reinterpret_cast<const PassWord*>(c->flagw.p), c->foff.p, nwq,
                                           c->foff.p + nwq, c->scan_tmp64.p, st);
         gate_bound_kernel<<<1, 1, 0, st>>>(c->foff.p + nwq, kept_cap, gs);
-        launch_compact(nwq, c->flagw.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->p_diag.p, kept_cap,
-                       c->q_ub.p, c->p_ub.p, st);
+        launch_compact(nwq, c->flagw.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->k_diag.p, kept_cap,
+                       c->q_ub.p, c->k_ub.p, st);
         pb.ub = c->p_ub.p;
         launches += 6 + scan_launches(nwq);
       } else {
         gate_bound_kernel<<<1, 1, 0, st>>>(c->foff.p + nw, kept_cap, gs);
-        launch_compact(nw, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->p_diag.p, kept_cap, nullptr, nullptr,
+        launch_compact(nw, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->k_diag.p, kept_cap, nullptr, nullptr,
                        st);
         launches += 2;
       }
       const int64_t* np = reinterpret_cast<const int64_t*>(gs + kGsKept);
       setup_rounds(c, rounds, pb, st);
-      launch_slot_lists(kept_cap, np, pb, align_round_take(0, rounds), st);
-      launches += 2;
+      launch_slot_lists(kept_list(c, P, kept_cap, np), c->p_ub.p, pb, align_round_take(0, rounds), st);
+      launches += 3;
       pb.a_score = c->a_score.p; pb.a_bound = c->a_bound.p; pb.a_tblen = c->a_tblen.p;
       pb.a_pos = c->a_pos.p; pb.a_tb = c->a_tb.p; pb.tbs = P.tbs;
       pb.npass_dev = np;
@@ -950,22 +963,22 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
       }
       max_kept = std::max(max_kept, nkept);
       if (nkept > 0) {
-        if (c->p_read.grow(nkept) || c->p_diag.grow(nkept) || c->a_score.grow(nkept) || c->a_bound.grow(nkept) ||
+        if (c->p_read.grow(nkept) || c->p_diag.grow(nkept) || c->k_diag.grow(nkept) || c->a_score.grow(nkept) || c->a_bound.grow(nkept) ||
             c->a_tblen.grow(nkept) || c->a_pos.grow(nkept * 4) || c->a_tb.grow(nkept * tbs) ||
-            (bound_H && c->p_ub.grow(nkept)))
+            (bound_H && (c->k_ub.grow(nkept) || c->p_ub.grow(nkept))))
           return STORMGPU_ENOMEM;
         pb.p_read = c->p_read.p; pb.p_diag = c->p_diag.p; pb.p_cap = c->p_read.cap;
         if (bound_H) {
-          launch_compact((npass + 31) / 32, c->flagw.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->p_diag.p,
-                         c->p_read.cap, c->q_ub.p, c->p_ub.p, st);
+          launch_compact((npass + 31) / 32, c->flagw.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->k_diag.p,
+                         nkept, c->q_ub.p, c->k_ub.p, st);
           pb.ub = c->p_ub.p;
         } else {
-          launch_compact(nwords, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->p_diag.p, c->p_read.cap,
-                         nullptr, nullptr, st);
+          launch_compact(nwords, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->k_diag.p, nkept, nullptr,
+                         nullptr, st);
         }
         if (round_lists_grow(c, n, nkept, rounds) || setup_rounds(c, rounds, pb, st)) return STORMGPU_ENOMEM;
-        launch_slot_lists(nkept, nullptr, pb, align_round_take(0, rounds), st);
-        launches += 3;
+        launch_slot_lists(kept_list(c, P, nkept, nullptr), c->p_ub.p, pb, align_round_take(0, rounds), st);
+        launches += 4;
         pb.a_score = c->a_score.p; pb.a_bound = c->a_bound.p; pb.a_tblen = c->a_tblen.p;
         pb.a_pos = c->a_pos.p; pb.a_tb = c->a_tb.p; pb.tbs = tbs;
         // one persistent launch over all kept candidates; scratch for its threads only

@@ -62,96 +62,86 @@ __device__ __forceinline__ void item_lookup(const int32_t* __restrict__ first, c
   cnt = __ldg(first + key + 1) - a;
 }
 
-// Diagonals a[0..U) (distinct, any order; one warp) -> flat list; the smallest, vmin, is dropped when
-// it is not above -I (run.c:617, :648).
-__device__ __forceinline__ void warp_emit(int32_t* a, int U, int32_t vmin, int I, int r, const GatherOut& go) {
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  if (U > 0 && vmin <= -I) {
-    int W = 0;
-    for (int k0 = 0; k0 < U; k0 += 32) {
-      const int32_t v = k0 + lane < U ? a[k0 + lane] : vmin;
-      const unsigned m = __ballot_sync(0xffffffffu, v != vmin);
-      if (v != vmin) a[W + __popc(m & lt)] = v;  // writes trail the reads
-      W += __popc(m);
-      __syncwarp();
-    }
-    U = W;
-  }
+// Place of U candidates of the warp's read in the flat list (-1: the list is full).
+__device__ __forceinline__ int64_t reserve(const GatherOut& go, int U) {
   unsigned long long base = 0;
-  if (lane == 0 && U) base = atomicAdd(&go.counters[7], (unsigned long long)U);
+  if ((threadIdx.x & 31) == 0 && U) base = atomicAdd(&go.counters[7], (unsigned long long)U);
   base = __shfl_sync(0xffffffffu, base, 0);
   if ((int64_t)(base + U) > go.cap) {
-    if (lane == 0) atomicExch(&go.counters[8], 1ull);
-    return;
+    if ((threadIdx.x & 31) == 0) atomicExch(&go.counters[8], 1ull);
+    return -1;
   }
-  for (int k = lane; k < U; k += 32) {
-    go.fr[base + k] = r;
-    go.fd[base + k] = a[k];
-  }
+  return (int64_t)base;
 }
 
-// Drop repeated values from a[0..H) (one warp), keeping one of each, compacted to the front
-// of a (order not kept); tab[0..cap), cap >= H, is the open-addressing set.  The diagonal a read
-// truly maps to comes once per (seed, position) that hits it.  Returns the number of distinct values.
 constexpr int32_t kEmptySlot = 0x7fffffff;  // no diagonal (position - read position) reaches it
-__device__ __forceinline__ int warp_dedupe(int32_t* a, int H, int32_t* tab, int cap) {
+
+// The distinct values of a[0..H) stay, the repeats become kEmptySlot (one warp).  Rounds of claims
+// without atomics: every undecided entry writes its index to tab[hash], and reads back who wrote
+// last: itself -- it stays; an entry of its own value -- it is a repeat; another value -- it is undecided
+// and goes to the next round, with another hash.  Every slot read was written in the same round, so
+// the table is never cleared; all entries of one value are decided in the same round.  About 85 %
+// are decided in the first.  The diagonal a read truly maps to comes once per (seed, position) that
+// hits it: with an open-addressing set those lanes queue on one shared atomic.  list[0..H): the
+// undecided entries.  Returns the number of distinct values.
+__device__ __forceinline__ int warp_distinct(int32_t* a, int H, uint16_t* tab, int size, uint16_t* list) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  if (H <= 32) {
-    const int32_t v = lane < H ? a[lane] : kEmptySlot;
-    const unsigned peers = __match_any_sync(0xffffffffu, v);
-    const unsigned m = __ballot_sync(0xffffffffu, lane < H && (peers & lt) == 0);
-    if ((m >> lane) & 1u) a[__popc(m & lt)] = v;
-    __syncwarp();
-    return __popc(m);
-  }
-  const int size = min(cap, 2 * H);
-  for (int i = lane; i < size; i += 32) tab[i] = kEmptySlot;
-  __syncwarp();
-  int U = 0;
-  for (int i0 = 0; i0 < H; i0 += 32) {
-    const int i = i0 + lane;
-    bool keep = false;
-    int32_t v = 0;
-    if (i < H) {
-      v = a[i];
-      uint32_t h = __umulhi((uint32_t)v * 0x9E3779B1u, (uint32_t)size);
-      for (;;) {
-        const int32_t old = atomicCAS(&tab[h], kEmptySlot, v);
-        if (old == kEmptySlot) { keep = true; break; }
-        if (old == v) break;
-        h = h + 1 == (uint32_t)size ? 0u : h + 1;
-      }
+  int U = 0, n = H;
+  uint32_t mul = 0x9E3779B1u;
+  for (int round = 0; n > 0; ++round) {
+    for (int k = lane; k < n; k += 32) {
+      const int i = round ? list[k] : k;
+      tab[__umulhi((uint32_t)a[i] * mul, (uint32_t)size)] = (uint16_t)i;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, keep);
-    if (keep) a[U + __popc(m & lt)] = v;  // writes trail the reads of this and later chunks
-    U += __popc(m);
     __syncwarp();
+    int left = 0;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+      const int k = k0 + lane;
+      bool stays = false, undecided = false, repeat = false;
+      int i = 0;
+      if (k < n) {
+        i = round ? list[k] : k;
+        const int32_t v = a[i];
+        const int win = tab[__umulhi((uint32_t)v * mul, (uint32_t)size)];
+        const int32_t wv = a[win];
+        stays = win == i;
+        undecided = wv != v && wv != kEmptySlot;
+        repeat = !stays && !undecided;
+      }
+      // repeats are blanked after the chunk's reads; a blanked winner cannot be: winners stay
+      const unsigned mu = __ballot_sync(0xffffffffu, undecided);
+      U += __popc(__ballot_sync(0xffffffffu, stays));
+      if (repeat) a[i] = kEmptySlot;
+      if (undecided) list[left + __popc(mu & lt)] = (uint16_t)i;  // writes trail the reads
+      left += __popc(mu);
+      __syncwarp();
+    }
+    n = left;
+    mul = mul * 0x85EBCA6Bu + 2u;  // odd
   }
   return U;
 }
 
 // A seed's care positions as runs, for keys from a window of 32 codes whose first code is in the
-// high bits: the key is the OR of (window >> sh) & mask over the runs (4 to 7 of them, where taking
+// high bits: the key is the OR of (window >> shift) & mask over the runs (4 to 7 of them, where taking
 // the care positions one by one takes 10 to 15 steps).
 struct SeedRuns {
-  int n;
-  uint8_t sh[16];
-  uint32_t mask[16];
+  uint2 r[16];  // shift, mask; unused ones have mask 0
 };
 
-__device__ __forceinline__ void make_runs(const SeedDev& s, SeedRuns& o) {
+// returns the number of runs
+__device__ __forceinline__ int make_runs(const SeedDev& s, SeedRuns& o) {
   int n = 0;
+  for (int c = 0; c < 16; ++c) o.r[c] = make_uint2(0, 0);
   for (int c = 0; c < s.n_care;) {
     int m = 1;
     while (c + m < s.n_care && s.care[c + m] - s.care[c] == m) ++m;
-    o.sh[n] = (uint8_t)(62 - 2 * (s.care[c] + s.n_care - 1 - c));
-    o.mask[n] = (uint32_t)((1ull << (2 * m)) - 1ull) << (2 * (s.n_care - c - m));
-    ++n;
+    o.r[n++] = make_uint2((uint32_t)(62 - 2 * (s.care[c] + s.n_care - 1 - c)),
+                          (uint32_t)((1ull << (2 * m)) - 1ull) << (2 * (s.n_care - c - m)));
     c += m;
   }
-  o.n = n;
+  return n;
 }
 
 // 16 packed codes, first code in the low bits -> first code in the high bits
@@ -170,27 +160,48 @@ constexpr int kReadBytes = STORMGPU_MAX_READ_LEN / 4 + 16;
 constexpr int kReadWords = STORMGPU_MAX_READ_LEN / 16 + 3;
 
 constexpr int kItems = 4;  // (seed, position) items per lane and round: 128 key lookups in flight per warp
+constexpr int kChunks = 4; // chunks of 32 index positions loaded before any is used
 
-__global__ void __launch_bounds__(kGWarps * 32, 8) gather_fused_kernel(ReadsDev rd, IndexView ix, int I, GatherOut go,
+// Words of a warp's shared memory for `cap` index positions: the positions; the claims of
+// warp_distinct (16 bits each), whose space holds the item markers before (a byte per position); two
+// words per item of a round, whose space holds the undecided entries (16 bits each) after.
+__host__ __device__ constexpr int gather_half_words(int cap) { return (cap / 2 + 32) & ~31; }
+__host__ __device__ constexpr int gather_item_words(int cap) {
+  return gather_half_words(cap) > 2 * 32 * kItems ? gather_half_words(cap) : 2 * 32 * kItems;
+}
+__host__ __device__ constexpr int gather_warp_words(int cap) {
+  return ((cap + 31) & ~31) + gather_half_words(cap) + gather_item_words(cap);
+}
+
+__global__ void __launch_bounds__(kGWarps * 32, 9) gather_fused_kernel(ReadsDev rd, IndexView ix, int I, GatherOut go,
                                                                    const __grid_constant__ SeedSet gs) {
-  extern __shared__ int32_t sm[];  // per warp 2 * cap: gathered positions, then the set
+  extern __shared__ __align__(16) int32_t sm[];  // gather_warp_words per warp
   __shared__ SeedRuns runs[kMaxSeeds];
   __shared__ int32_t sspan[kMaxSeeds];
+  __shared__ int s_nruns;
   __shared__ int32_t soff[kGWarps][kMaxSeeds + 1];  // first item of every seed, for the current read
   __shared__ const int32_t* s_first[kMaxSeeds];
   __shared__ const int32_t* s_map[kMaxSeeds];
   __shared__ uint32_t srev[kGWarps][kReadWords];  // the read's codes, first code in the high bits, 0 after its end
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
   const int nseeds = gs.n;
+  const int cap = go.warp_cap;
+  int32_t* pos = sm + (size_t)w * gather_warp_words(cap);
+  uint16_t* claims = reinterpret_cast<uint16_t*>(pos + ((cap + 31) & ~31));
+  uint8_t* mark = reinterpret_cast<uint8_t*>(claims);  // item + 1 at the first position of an item, 0 elsewhere
+  int2* item = reinterpret_cast<int2*>(claims + 2 * gather_half_words(cap));  // map offset - slot, read position | seed << 16
+  uint16_t* undecided = reinterpret_cast<uint16_t*>(item);
+  if (threadIdx.x == 0) s_nruns = 0;
+  __syncthreads();
   if (threadIdx.x < nseeds) {
     s_first[threadIdx.x] = ix.first[threadIdx.x];
     s_map[threadIdx.x] = ix.map[threadIdx.x];
     sspan[threadIdx.x] = gs.s[threadIdx.x].span;
-    if (gs.s[threadIdx.x].span <= 32) make_runs(gs.s[threadIdx.x], runs[threadIdx.x]);
+    if (gs.s[threadIdx.x].span <= 32) atomicMax(&s_nruns, make_runs(gs.s[threadIdx.x], runs[threadIdx.x]));
   }
   __syncthreads();
-  const int cap = go.warp_cap;
-  int32_t* s = sm + (size_t)w * 2 * cap;
+  const int nruns = s_nruns;
   int32_t* so = soff[w];
   uint32_t* rv = srev[w];
   unsigned long long lookups = 0, positions = 0;
@@ -222,74 +233,93 @@ __global__ void __launch_bounds__(kGWarps * 32, 8) gather_fused_kernel(ReadsDev 
     }
     const int T = so[nseeds];
     int H = 0;
+    int32_t vmin = kEmptySlot, v1 = kEmptySlot;  // v1: a read of at most 32 positions, one per lane
     // a read with more positions than the warp holds is only counted from there on and goes to
     // the block kernel with its count (its lookups and positions are counted there)
     for (int r0 = 0; r0 < T; r0 += 32 * kItems) {
       // every lane looks up its items (all key-table loads in flight together) ...
-      int a[kItems], cnt[kItems], rp[kItems], sid[kItems];
+      int a[kItems], cnt[kItems], info[kItems];
 #pragma unroll
       for (int m = 0; m < kItems; ++m) {
         const int it = r0 + m * 32 + lane;
-        int si = 0;
-        a[m] = 0; cnt[m] = 0; rp[m] = 0;
+        a[m] = 0; cnt[m] = 0; info[m] = 0;
         if (it < T) {
+          int si = 0;
           while (it >= so[si + 1]) ++si;
-          rp[m] = it - so[si];
-          if (gs.s[si].n_positions) rp[m] = gs.s[si].positions[rp[m]];
-          if (rp[m] >= 0 && rp[m] < L) {
+          int rp = it - so[si];
+          if (gs.s[si].n_positions) rp = gs.s[si].positions[rp];
+          if (rp >= 0 && rp < L) {
             uint32_t key = 0;
             if (sspan[si] <= 32) {
-              const uint32_t* q = rv + (rp[m] >> 4);
-              const int sh = 2 * (rp[m] & 15);
+              const uint32_t* q = rv + (rp >> 4);
+              const int sh = 2 * (rp & 15);
               const uint64_t win = (uint64_t)__funnelshift_l(q[1], q[0], sh) << 32 | __funnelshift_l(q[2], q[1], sh);
-              const SeedRuns& R = runs[si];
-              for (int c = 0; c < R.n; ++c) key |= (uint32_t)(win >> R.sh[c]) & R.mask[c];
+#pragma unroll 4
+              for (int c = 0; c < nruns; ++c) {
+                const uint2 R = runs[si].r[c];
+                key |= (uint32_t)(win >> R.x) & R.y;
+              }
             } else {
-              key = read_key(gs.s[si], src, L, rp[m]);
+              key = read_key(gs.s[si], src, L, rp);
             }
             a[m] = __ldg(s_first[si] + key);
             cnt[m] = __ldg(s_first[si] + key + 1) - a[m];
+            info[m] = rp | si << 16;
           }
         }
-        sid[m] = si;
       }
-      // ... then one scan places all of them, and the position loads go out together
+      // ... then one scan places all of them ...
       int tot = 0;
 #pragma unroll
       for (int m = 0; m < kItems; ++m) tot += cnt[m];
       const int incl = warp_incl_scan(tot);
-      int dst[kItems];
-      dst[0] = H + incl - tot;
-#pragma unroll
-      for (int m = 1; m < kItems; ++m) dst[m] = dst[m - 1] + cnt[m - 1];
-      H += __shfl_sync(0xffffffffu, incl, 31);
+      const int n = __shfl_sync(0xffffffffu, incl, 31);  // positions of this round
+      const int H0 = H;
+      H += n;
       if (H > cap) continue;  // uniform over the warp: counting only
+      if (n == 0) continue;
+      for (int k = lane; 4 * k < n; k += 32) reinterpret_cast<uint32_t*>(mark)[k] = 0;
+      __syncwarp();
+      int dst = incl - tot;
 #pragma unroll
       for (int m = 0; m < kItems; ++m) {
-        if (cnt[m] <= 8) {
-          const int32_t* mp = s_map[sid[m]] + a[m];
-          int32_t tv[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) tv[u] = u < cnt[m] ? __ldg(mp + u) : 0;
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (u < cnt[m] && dst[m] + u < cap) s[dst[m] + u] = tv[u] - rp[m];
+        if (cnt[m] > 0) {
+          mark[dst] = (uint8_t)(lane * kItems + m + 1);
+          item[lane * kItems + m] = make_int2(a[m] - dst, info[m]);
+          dst += cnt[m];
         }
       }
+      __syncwarp();
+      // ... and the positions are spread over the lanes: position s belongs to the last item marked
+      // at or before it
+      int carry = 0;
+      for (int s0 = 0; s0 < n; s0 += 32 * kChunks) {
+        int32_t v[kChunks];
 #pragma unroll
-      for (int m = 0; m < kItems; ++m) {  // long position lists: the whole warp copies each
-        unsigned bm = __ballot_sync(0xffffffffu, cnt[m] > 8);
-        while (bm) {
-          const int j = __ffs(bm) - 1;
-          bm &= bm - 1;
-          const int aj = __shfl_sync(0xffffffffu, a[m], j), cj = __shfl_sync(0xffffffffu, cnt[m], j);
-          const int dj = __shfl_sync(0xffffffffu, dst[m], j), rj = __shfl_sync(0xffffffffu, rp[m], j);
-          const int sj = __shfl_sync(0xffffffffu, sid[m], j);
-          const int32_t* mp = s_map[sj];
-          for (int u = lane; u < cj; u += 32)
-            if (dj + u < cap) s[dj + u] = __ldg(mp + aj + u) - rj;
+        for (int c = 0; c < kChunks; ++c) {
+          const int s = s0 + 32 * c + lane;
+          v[c] = kEmptySlot;
+          if (s0 + 32 * c < n) {  // uniform
+            const int mk = s < n ? mark[s] : 0;
+            const unsigned b = __ballot_sync(0xffffffffu, mk != 0) & (lt | (1u << lane));
+            const int own = __shfl_sync(0xffffffffu, mk, b ? 31 - __clz(b) : lane);
+            const int it = b ? own - 1 : carry;
+            carry = __shfl_sync(0xffffffffu, it, 31);
+            if (s < n) {
+              const int2 e = item[it];
+              v[c] = __ldg(s_map[e.y >> 16] + e.x + s) - (e.y & 0xffff);
+            }
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+          const int s = s0 + 32 * c + lane;
+          vmin = min(vmin, v[c]);
+          if (c == 0 && s0 == 0) v1 = v[0];
+          if (s < n) pos[H0 + s] = v[c];
         }
       }
+      __syncwarp();
     }
     if (H > cap) {
       if (lane == 0) {
@@ -308,11 +338,37 @@ __global__ void __launch_bounds__(kGWarps * 32, 8) gather_fused_kernel(ReadsDev 
     }
     positions += (unsigned long long)H;
     lookups += (unsigned long long)T;
-    __syncwarp();
-    const int U = warp_dedupe(s, H, s + cap, cap);
-    int32_t vmin = 0x7fffffff;
-    for (int k = lane; k < U; k += 32) vmin = min(vmin, s[k]);
-    warp_emit(s, U, __reduce_min_sync(0xffffffffu, vmin), I, (int)r, go);
+    if (H == 0) continue;
+    // the distinct diagonals to the flat list; the smallest is dropped when it is not above -I
+    // (run.c:617, :648)
+    vmin = __reduce_min_sync(0xffffffffu, vmin);
+    const int32_t drop = vmin <= -I ? vmin : kEmptySlot;
+    if (H <= 32) {
+      if (T > 32 * kItems) v1 = lane < H ? pos[lane] : kEmptySlot;  // more than one round
+      const unsigned peers = __match_any_sync(0xffffffffu, v1);
+      const unsigned m = __ballot_sync(0xffffffffu, v1 != kEmptySlot && v1 != drop && (peers & lt) == 0);
+      const int64_t base = reserve(go, __popc(m));
+      if (base >= 0 && ((m >> lane) & 1u)) {
+        const int64_t o = base + __popc(m & lt);
+        go.fr[o] = (int32_t)r;
+        go.fd[o] = v1;
+      }
+    } else {
+      const int U = warp_distinct(pos, H, claims, cap, undecided) - (drop != kEmptySlot ? 1 : 0);
+      int64_t o = reserve(go, U);
+      if (o >= 0) {
+        for (int k0 = 0; k0 < H; k0 += 32) {
+          const int32_t v = k0 + lane < H ? pos[k0 + lane] : kEmptySlot;
+          const bool keep = v != kEmptySlot && v != drop;
+          const unsigned m = __ballot_sync(0xffffffffu, keep);
+          if (keep) {
+            go.fr[o + __popc(m & lt)] = (int32_t)r;
+            go.fd[o + __popc(m & lt)] = v;
+          }
+          o += __popc(m);
+        }
+      }
+    }
     __syncwarp();
   }
   }
@@ -548,8 +604,8 @@ __global__ void __launch_bounds__(kBT) gather_block_kernel(ReadsDev rd, IndexVie
 void launch_gather_fused(const ReadsDev& rd, const IndexView& ix, int I, const GatherOut& go, const SeedSet& seeds,
                          cudaStream_t st) {
   if (rd.n <= 0) return;
-  set_smem_attribute_once(reinterpret_cast<const void*>(gather_fused_kernel), kGWarps * 2 * kMaxWarpCap * 4);
-  const size_t smem = (size_t)kGWarps * 2 * go.warp_cap * sizeof(int32_t);
+  set_smem_attribute_once(reinterpret_cast<const void*>(gather_fused_kernel), kGWarps * gather_warp_words(kMaxWarpCap) * 4);
+  const size_t smem = (size_t)kGWarps * gather_warp_words(go.warp_cap) * sizeof(int32_t);
   const int64_t per_block = (int64_t)kGWarps * go.reads_per_steal;
   const int64_t blocks = std::min<int64_t>((rd.n + per_block - 1) / per_block,
                                           resident_grid(gather_fused_kernel, kGWarps * 32, smem));

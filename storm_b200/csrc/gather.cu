@@ -11,8 +11,7 @@
 // slot_lists_kernel gives it (map_kernels.cu).  Every lane looks up several (seed, position) keys
 // before any result is used, so that a read costs two memory latencies (key table, positions) rather
 // than two per seed.  Reads with more index positions than a warp can hold go to a
-// block-per-read kernel (shared memory up to 4096 positions) and, beyond that, to slices in global
-// memory; these append ascending diagonals.
+// block-per-read kernel (below), which appends ascending diagonals.
 #include <type_traits>
 
 #include "gather.cuh"
@@ -156,7 +155,6 @@ constexpr int kGWarps = 4;
 // reads with many index positions balance out, and warps append their candidates in close to
 // read order: a batch whose reads are grouped by length gives a candidate list grouped by
 // length, which the filter needs to keep one read length per SM.
-constexpr int kReadBytes = STORMGPU_MAX_READ_LEN / 4 + 16;
 constexpr int kReadWords = STORMGPU_MAX_READ_LEN / 16 + 3;
 
 constexpr int kItems = 4;  // (seed, position) items per lane and round: 128 key lookups in flight per warp
@@ -378,229 +376,6 @@ __global__ void __launch_bounds__(kGWarps * 32, 9) gather_fused_kernel(ReadsDev 
   }
 }
 
-// One block per read of the list, for reads with more index positions than a warp holds: the
-// positions go to a block-private slice of a global buffer (scratch: 2 * cap words per block,
-// its working set small enough to stay in L2), then a bucket sort without comparisons across
-// buckets: min / max, buckets of equal power-of-two width over [min, max] (about 8 values each,
-// so that bucket order is value order), counted and scattered with shared atomics, then every
-// thread insertion-sorts its buckets, dropping repeated values on the way.  The surviving
-// diagonals are appended in order; the smallest is dropped when it is not above -I
-// (run.c:617, :648).  Reads with more than `cap` positions are appended to (huge_list,
-// huge_h) for a second launch with a larger cap.  The grid is persistent: blocks take the next
-// read of the list from `cursor` (zeroed), list_count read on the device when given.
-constexpr int kBT = 512;              // threads of a block-gather block
-constexpr int kMaxBuckets = 4096;
-constexpr int kSmallCap = kSmallGatherCap;  // a read with at most this many positions sorts in shared memory
-
-// exclusive scan of a[0..n) in place (n <= kMaxBuckets, every thread of the block); the total
-__device__ __forceinline__ int block_excl_scan(int32_t* a, int n, int* wtot) {
-  constexpr int per = kMaxBuckets / kBT;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int b0 = threadIdx.x * per;
-  int loc = 0;
-#pragma unroll
-  for (int k = 0; k < per; ++k)
-    if (b0 + k < n) loc += a[b0 + k];
-  const int incl = warp_incl_scan(loc);
-  if (lane == 31) wtot[w] = incl;
-  __syncthreads();
-  int before = 0, tot = 0;
-  for (int q = 0; q < kBT / 32; ++q) {
-    if (q < w) before += wtot[q];
-    tot += wtot[q];
-  }
-  int run = before + incl - loc;
-#pragma unroll
-  for (int k = 0; k < per; ++k)
-    if (b0 + k < n) {
-      const int v = a[b0 + k];
-      a[b0 + k] = run;
-      run += v;
-    }
-  __syncthreads();
-  return tot;
-}
-
-// SMEM: the slices in dynamic shared memory (every read of the list has at most kSmallCap
-// positions).  Without it a launch keeps its shared memory small: the L1 cache shares that
-// storage, and the global slices of reads with many positions live off it.
-template <bool SMEM>
-__global__ void __launch_bounds__(kBT) gather_block_kernel(ReadsDev rd, IndexView ix, int I, const int32_t* __restrict__ list,
-                                                           const int32_t* __restrict__ list_h,
-                                                           const int32_t* __restrict__ list_count, int64_t nlist,
-                                                           GatherOut go, int32_t* __restrict__ scratch, int cap,
-                                                           unsigned long long* cursor, int32_t* huge_list, int32_t* huge_h,
-                                                           int32_t* huge_count, const __grid_constant__ SeedSet gs) {
-  __shared__ int32_t cnt[kMaxBuckets];   // per bucket: count, start, then end
-  __shared__ int32_t uoff[kMaxBuckets];  // per bucket: distinct values, then their offset
-  __shared__ int wtot[kBT / 32];
-  __shared__ int s_read, s_H;
-  __shared__ int32_t s_min, s_max;
-  __shared__ unsigned long long s_base;
-  __shared__ __align__(16) uint8_t srd[kReadBytes];
-  extern __shared__ int32_t dsm[];  // 2 * kSmallCap: the slices of a read with few positions
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int32_t* const Ag = scratch + (int64_t)blockIdx.x * 2 * cap;  // the block's slices in global memory
-  int32_t* const Bg = Ag + cap;
-  const int64_t n = list_count ? (int64_t)*list_count : nlist;
-  unsigned long long lookups = 0, positions = 0;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      const unsigned long long k = atomicAdd(cursor, 1ull);
-      s_read = (int64_t)k < n ? list[k] : -1;
-      s_H = (int64_t)k < n ? list_h[k] : 0;
-      s_min = 0x7fffffff;
-      s_max = (int32_t)0x80000000;
-    }
-    __syncthreads();
-    const int r = s_read;
-    if (r < 0) break;
-    const int L = rd.lengths[r];
-    {
-      const uint8_t* src = rd.codes + (int64_t)r * rd.cstride;
-      const int nbytes = (L + 3) >> 2;
-      for (int b = threadIdx.x; b < kReadBytes; b += kBT) srd[b] = b < nbytes ? src[b] : 0;
-    }
-    __syncthreads();
-    // the read's position count came with it (the warp gather counted it), so a read above
-    // `cap` loads none of its positions here
-    int T = 0;
-    for (int si = 0; si < gs.n; ++si) T += seed_npos(gs.s[si], L);
-    const int H = s_H;
-    if (H > cap) {
-      if (threadIdx.x == 0) {
-        const int k = atomicAdd(huge_count, 1);
-        huge_list[k] = r;
-        huge_h[k] = H;
-      }
-      __syncthreads();
-      continue;
-    }
-    lookups += (unsigned long long)T;
-    positions += (unsigned long long)H;
-    if (H == 0) {
-      __syncthreads();
-      continue;
-    }
-    __syncthreads();  // every thread has read s_H
-    if (threadIdx.x == 0) s_H = 0;
-    __syncthreads();
-    // the rest of the read, compiled twice: slices in shared memory (a read with few positions)
-    // or in the block's global slices, each with plain shared or global memory operations
-    auto per_read = [&](auto in_shared) {
-      constexpr bool SMALL = decltype(in_shared)::value;
-      int32_t* const A = SMALL ? dsm : Ag;
-      int32_t* const B = SMALL ? dsm + kSmallCap : Bg;
-      // gather: every (seed, read position) item's CSR range, placed by a block scan; the range
-      // of the values is taken on the way
-      int32_t vmin = 0x7fffffff, vmax = (int32_t)0x80000000;
-      auto put = [&](int k, int32_t v) {
-        vmin = min(vmin, v);
-        vmax = max(vmax, v);
-        A[k] = v;
-      };
-      for (int si = 0; si < gs.n; ++si) {
-        const int np = seed_npos(gs.s[si], L);
-        const int32_t* first = ix.first[si];
-        const int32_t* mp = ix.map[si];
-        for (int t0 = 0; t0 < np; t0 += kBT) {
-          int a, c, rp;
-          item_lookup(first, gs.s[si], t0 + threadIdx.x, srd, L, a, c, rp);
-          const int incl = warp_incl_scan(c);
-          if (lane == 31) wtot[w] = incl;
-          __syncthreads();
-          int before = 0, tot = 0;
-          for (int q = 0; q < kBT / 32; ++q) {
-            if (q < w) before += wtot[q];
-            tot += wtot[q];
-          }
-          const int dst = s_H + before + incl - c;
-          if (c <= 8) {
-            for (int u = 0; u < c; ++u) put(dst + u, __ldg(mp + a + u) - rp);
-          }
-          unsigned bm = __ballot_sync(0xffffffffu, c > 8);  // long lists: the warp copies each
-          while (bm) {
-            const int j = __ffs(bm) - 1;
-            bm &= bm - 1;
-            const int aj = __shfl_sync(0xffffffffu, a, j), cj = __shfl_sync(0xffffffffu, c, j);
-            const int dj = __shfl_sync(0xffffffffu, dst, j), rj = __shfl_sync(0xffffffffu, rp, j);
-            for (int u = lane; u < cj; u += 32) put(dj + u, __ldg(mp + aj + u) - rj);
-          }
-          __syncthreads();
-          if (threadIdx.x == 0) s_H += tot;
-          __syncthreads();
-        }
-      }
-      // range
-      vmin = __reduce_min_sync(0xffffffffu, vmin);
-      vmax = __reduce_max_sync(0xffffffffu, vmax);
-      if (lane == 0) {
-        atomicMin(&s_min, vmin);
-        atomicMax(&s_max, vmax);
-      }
-      __syncthreads();
-      vmin = s_min;
-      const uint32_t range = (uint32_t)s_max - (uint32_t)vmin;
-      int nb = 1;
-      while (nb < kMaxBuckets && nb * 8 < H) nb <<= 1;
-      int shift = 0;
-      while ((range >> shift) >= (uint32_t)nb) ++shift;
-      for (int b = threadIdx.x; b < nb; b += kBT) cnt[b] = 0;
-      __syncthreads();
-      for (int i = threadIdx.x; i < H; i += kBT) atomicAdd(&cnt[((uint32_t)A[i] - (uint32_t)vmin) >> shift], 1);
-      __syncthreads();
-      block_excl_scan(cnt, nb, wtot);
-      for (int i = threadIdx.x; i < H; i += kBT) {
-        const int32_t v = A[i];
-        B[atomicAdd(&cnt[((uint32_t)v - (uint32_t)vmin) >> shift], 1)] = v;
-      }
-      __syncthreads();  // cnt[b] is now the end of bucket b
-      for (int b = threadIdx.x; b < nb; b += kBT) {
-        const int s0 = b ? cnt[b - 1] : 0, e = cnt[b];
-        int u = 0;
-        for (int x = s0; x < e; ++x) {  // insertion into the sorted distinct prefix B[s0, s0 + u)
-          const int32_t t = B[x];
-          int y = u - 1;
-          while (y >= 0 && B[s0 + y] > t) --y;
-          if (y >= 0 && B[s0 + y] == t) continue;
-          for (int z = u - 1; z > y; --z) B[s0 + z + 1] = B[s0 + z];
-          B[s0 + y + 1] = t;
-          ++u;
-        }
-        uoff[b] = u;
-      }
-      __syncthreads();
-      const int U = block_excl_scan(uoff, nb, wtot);
-      for (int b = threadIdx.x; b < nb; b += kBT) {
-        const int s0 = b ? cnt[b - 1] : 0, o = uoff[b];
-        const int u = (b + 1 < nb ? uoff[b + 1] : U) - o;
-        for (int k = 0; k < u; ++k) A[o + k] = B[s0 + k];
-      }
-      __syncthreads();
-      const int drop = A[0] <= -I ? 1 : 0;  // the first diagonal must exceed -I (run.c:617, :648)
-      const int Uo = U - drop;
-      if (threadIdx.x == 0) s_base = Uo ? atomicAdd(&go.counters[7], (unsigned long long)Uo) : 0ull;
-      __syncthreads();
-      const unsigned long long base = s_base;
-      if ((int64_t)(base + Uo) > go.cap) {
-        if (threadIdx.x == 0) atomicExch(&go.counters[8], 1ull);
-      } else {
-        for (int k = threadIdx.x; k < Uo; k += kBT) {
-          go.fr[base + k] = r;
-          go.fd[base + k] = A[k + drop];
-        }
-      }
-    };
-    if constexpr (SMEM) per_read(std::true_type{});
-    else per_read(std::false_type{});
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    atomicAdd(&go.counters[3], lookups);
-    atomicAdd(&go.counters[4], positions);
-  }
-}
-
 void launch_gather_fused(const ReadsDev& rd, const IndexView& ix, int I, const GatherOut& go, const SeedSet& seeds,
                          cudaStream_t st) {
   if (rd.n <= 0) return;
@@ -612,27 +387,353 @@ void launch_gather_fused(const ReadsDev& rd, const IndexView& ix, int I, const G
   gather_fused_kernel<<<(unsigned)blocks, kGWarps * 32, smem, st>>>(rd, ix, I, go, seeds);
 }
 
-constexpr size_t kBlockGatherSmem = 2 * kSmallCap * sizeof(int32_t);
+// ------------------------------------------------------------------ reads with many positions
 
-int64_t gather_block_grid(bool smem) {
-  if (!smem) return resident_grid(gather_block_kernel<false>, kBT, 0);
-  set_smem_attribute_once(reinterpret_cast<const void*>(gather_block_kernel<true>), (int)kBlockGatherSmem);
-  return resident_grid(gather_block_kernel<true>, kBT, kBlockGatherSmem);
+// One block per read of a list, for reads above the warp gather's bucket: a bucket sort without
+// comparisons across buckets.  Buckets of equal power-of-two width (bucket order is value order), about
+// 8 values each, counted and scattered with shared atomics; every thread then sorts its buckets,
+// dropping repeated values, and the surviving diagonals are appended in order; the smallest is dropped
+// when it is not above -I (run.c:617, :648).  The positions are read from the index once to be
+// counted and once to be scattered straight into their buckets, so that one copy of them is held and
+// not two.  The grid is persistent: blocks take the next read of the list from `cursor` (zeroed),
+// list_count read on the device when given.
+//   * kSmall, up to kSmallGatherCap positions: the diagonals in shared memory, buckets over their range,
+//     several blocks per SM.
+//   * kLarge, up to kSortGatherCap positions: buckets over the whole sequence, at most 2^16 codes wide, so
+//     that 16 bits hold a diagonal's place in its bucket and 65,535 of them fit one SM's shared memory
+//     (a 150-bp read meets 50,000 positions in a repeat-rich 100 Mbp genome under three w10 seeds).
+//     Sequences too long for that (2^29 codes) go to (huge_list, huge_h), as do reads with more.
+//   * kHuge, up to `cap` positions: as kSmall with the diagonals in a slice of global memory (scratch: cap
+//     words per block) and more buckets; above cap to (huge_list, huge_h) for a launch with larger slices.
+// What bounds it is the latency of shared memory in the buckets and of the index passes; with two
+// global slices per block (L2-resident), insertion sorts in them and the position lists copied one by
+// one, the same reads took 11.1 ms where this takes 4.3 ms (4,000 mixed reads, both strands).
+
+constexpr int kReadBytes = STORMGPU_MAX_READ_LEN / 4 + 16;
+
+// exclusive scan of a[0..n) in place, n <= NB, by every thread of the block; the total
+template <int THREADS, int NB, class T>
+__device__ __forceinline__ int sort_excl_scan(T* a, int n, int* wtot) {
+  constexpr int per = NB / THREADS;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int b0 = threadIdx.x * per;
+  int loc = 0;
+#pragma unroll
+  for (int k = 0; k < per; ++k)
+    if (b0 + k < n) loc += a[b0 + k];
+  const int incl = warp_incl_scan(loc);
+  if (lane == 31) wtot[w] = incl;
+  __syncthreads();
+  if (w == 0) {
+    const int t = lane < THREADS / 32 ? wtot[lane] : 0;
+    const int i = warp_incl_scan(t);
+    if (lane < THREADS / 32) wtot[lane] = i;
+  }
+  __syncthreads();
+  int run = (w ? wtot[w - 1] : 0) + incl - loc;
+  const int tot = wtot[THREADS / 32 - 1];
+#pragma unroll
+  for (int k = 0; k < per; ++k)
+    if (b0 + k < n) {
+      const int v = a[b0 + k];
+      a[b0 + k] = (T)run;
+      run += v;
+    }
+  __syncthreads();
+  return tot;
 }
 
-void launch_gather_block(const ReadsDev& rd, const IndexView& ix, int I, const int32_t* list, const int32_t* list_h,
-                         int64_t nlist, const int32_t* nlist_dev, const GatherOut& go, int32_t* scratch, int cap,
-                         int64_t grid, unsigned long long* cursor, int32_t* huge_list, int32_t* huge_h,
-                         int32_t* huge_count, bool smem, const SeedSet& seeds, cudaStream_t st) {
-  if (nlist <= 0 || grid <= 0) return;
-  if (smem) {
-    set_smem_attribute_once(reinterpret_cast<const void*>(gather_block_kernel<true>), (int)kBlockGatherSmem);
-    gather_block_kernel<true><<<(unsigned)grid, kBT, kBlockGatherSmem, st>>>(
-        rd, ix, I, list, list_h, nlist_dev, nlist, go, scratch, cap, cursor, huge_list, huge_h, huge_count, seeds);
-  } else {
-    gather_block_kernel<false><<<(unsigned)grid, kBT, 0, st>>>(rd, ix, I, list, list_h, nlist_dev, nlist, go, scratch,
-                                                               cap, cursor, huge_list, huge_h, huge_count, seeds);
+// The items of a read, THREADS at a time, in shared memory, and body(place, diagonal) for every one of
+// its positions, g lanes per item.
+template <int THREADS>
+struct SortItems {
+  int32_t off[THREADS];      // map offset
+  int32_t at[THREADS + 32];  // place of the first position; at[THREADS]: their number
+  int32_t info[THREADS];     // read position | seed << 16
+  int wtot[32];
+};
+
+template <int THREADS, class Body>
+__device__ __forceinline__ void each_position(SortItems<THREADS>& it, const IndexView& ix, const SeedSet& gs,
+                                              const uint8_t* srd, int L, int T, int H, Body body) {
+  // lanes per item: about a third of an item's positions
+  const int g = H >= 64 * T ? 32 : H >= 16 * T ? 8 : 4;
+  const int sub = threadIdx.x & (g - 1), grp = threadIdx.x / g, ngrp = THREADS / g;
+  int H0 = 0;
+  for (int t0 = 0; t0 < T; t0 += THREADS) {
+    int t = t0 + (int)threadIdx.x, si = 0;
+    int a = 0, c = 0, rp = 0;
+    if (t < T) {
+      for (; si < gs.n - 1; ++si) {
+        const int np = seed_npos(gs.s[si], L);
+        if (t < np) break;
+        t -= np;
+      }
+      item_lookup(ix.first[si], gs.s[si], t, srd, L, a, c, rp);
+    }
+    it.off[threadIdx.x] = a;
+    it.info[threadIdx.x] = c > 0 ? rp | si << 16 : 0;
+    it.at[threadIdx.x] = c;
+    __syncthreads();
+    const int tot = sort_excl_scan<THREADS, THREADS>(it.at, THREADS, it.wtot);
+    if (threadIdx.x == 0) it.at[THREADS] = tot;
+    __syncthreads();
+    const int ni = min(THREADS, T - t0);
+    for (int q = grp; q < ni; q += ngrp) {
+      const int o = it.at[q], cq = it.at[q + 1] - o;
+      const int e = it.info[q], rq = e & 0xffff;
+      const int32_t* mp = ix.map[e >> 16] + it.off[q];
+      for (int u = sub; u < cq; u += 4 * g) {
+        int32_t v[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) v[x] = u + x * g < cq ? __ldg(mp + u + x * g) : 0;
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          if (u + x * g < cq) body(H0 + o + u + x * g, v[x] - rq);
+      }
+    }
+    H0 += tot;
+    __syncthreads();
   }
+}
+
+// Batcher's odd-even merge sort of N registers, every index a constant.
+template <int N>
+__device__ __forceinline__ void sort_network(int32_t (&v)[N]) {
+#pragma unroll
+  for (int p = 1; p < N; p <<= 1)
+#pragma unroll
+    for (int k = p; k >= 1; k >>= 1)
+#pragma unroll
+      for (int j = k % p; j + k < N; j += 2 * k)
+#pragma unroll
+        for (int i = 0; i < k; ++i)
+          if (i + j + k < N && (i + j) / (2 * p) == (i + j + k) / (2 * p)) {
+            const int32_t x = v[i + j], y = v[i + j + k];
+            v[i + j] = min(x, y);
+            v[i + j + k] = max(x, y);
+          }
+}
+
+// Sorts and de-duplicates the N - or less - values B[s0, s0 + n) in registers; the number of distinct
+// ones.
+template <int N, class V>
+__device__ __forceinline__ int sort_bucket_regs(V* B, int s0, int n) {
+  int32_t v[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) v[k] = k < n ? (int32_t)B[s0 + k] : kEmptySlot;
+  sort_network<N>(v);
+  int u = 0;
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if (v[k] != kEmptySlot && (k == 0 || v[k] != v[k > 0 ? k - 1 : 0])) B[s0 + u++] = (V)v[k];
+  return u;
+}
+
+// Sorts and de-duplicates B[s0, e) (one thread); the number of distinct values.  Up to 16 values go
+// through a sorting network, the same instructions in every lane (insertion, whose steps differ from
+// lane to lane, ran 13 of 32 lanes: 576 against 441 us for 1,000 mixed reads, one strand).
+template <class V>
+__device__ __forceinline__ int sort_bucket(V* B, int s0, int e) {
+  const int n = e - s0;
+  if (n <= 1) return n;
+  if (n <= 8) return sort_bucket_regs<8>(B, s0, n);
+  if (n <= 16) return sort_bucket_regs<16>(B, s0, n);
+  int u = 0;
+  for (int x = s0; x < e; ++x) {  // insertion into the sorted distinct prefix B[s0, s0 + u)
+    const V t = B[x];
+    int y = u - 1;
+    while (y >= 0 && B[s0 + y] > t) --y;
+    if (y >= 0 && B[s0 + y] == t) continue;
+    for (int z = u - 1; z > y; --z) B[s0 + z + 1] = B[s0 + z];
+    B[s0 + y + 1] = t;
+    ++u;
+  }
+  return u;
+}
+
+enum SortKind { kSmall, kLarge, kHuge };
+
+template <SortKind KIND>
+struct SortConfig {
+  static constexpr int CAP = KIND == kSmall ? kSmallGatherCap : KIND == kLarge ? kSortGatherCap : 0;  // in shared memory
+  static constexpr int THREADS = KIND == kSmall ? 256 : 1024;
+  static constexpr int NB = KIND == kSmall ? 1024 : KIND == kLarge ? 8192 : 16384;
+  using V = typename std::conditional<KIND == kLarge, uint16_t, int32_t>::type;  // a diagonal, or its place in its bucket
+  using U = typename std::conditional<KIND == kHuge, int32_t, uint16_t>::type;   // an offset in the read's list
+  struct Smem {
+    int32_t cnt[NB];  // per bucket: count, start, then end
+    SortItems<THREADS> items;
+    U uoff[NB];  // per bucket: distinct values, then their offset
+    V B[CAP > 0 ? CAP : 1];
+  };
+};
+static_assert(kSortGatherCap < 65536 && sizeof(SortConfig<kLarge>::Smem) <= 226 * 1024 &&
+                  sizeof(SortConfig<kHuge>::Smem) <= 226 * 1024,
+              "16-bit offsets, shared memory of an SM");
+
+template <SortKind KIND>
+__global__ void __launch_bounds__(SortConfig<KIND>::THREADS) gather_sort_kernel(
+    ReadsDev rd, IndexView ix, int I, int64_t n_codes, const int32_t* __restrict__ list, const int32_t* __restrict__ list_h,
+    const int32_t* __restrict__ list_count, int64_t nlist, GatherOut go, int32_t* __restrict__ scratch, int cap,
+    unsigned long long* cursor, int32_t* huge_list, int32_t* huge_h, int32_t* huge_count,
+    const __grid_constant__ SeedSet gs) {
+  using Cf = SortConfig<KIND>;
+  using V = typename Cf::V;
+  constexpr int THREADS = Cf::THREADS, NB = Cf::NB;
+  extern __shared__ __align__(16) uint8_t dsm[];
+  typename Cf::Smem& S = *reinterpret_cast<typename Cf::Smem*>(dsm);
+  V* const B = KIND == kHuge ? reinterpret_cast<V*>(scratch + (int64_t)blockIdx.x * cap) : S.B;
+  __shared__ int s_read, s_H, s_drop;
+  __shared__ int32_t s_min, s_max;
+  __shared__ unsigned long long s_base;
+  __shared__ __align__(16) uint8_t srd[kReadBytes];
+  const int64_t n = list_count ? (int64_t)*list_count : nlist;
+  // the large form's buckets: diagonals from -kMaxReadLen to n_codes
+  int shift_all = 0;
+  while (((n_codes + STORMGPU_MAX_READ_LEN) >> shift_all) >= NB) ++shift_all;
+  unsigned long long lookups = 0, positions = 0;
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const unsigned long long k = atomicAdd(cursor, 1ull);
+      s_read = (int64_t)k < n ? list[k] : -1;
+      s_H = (int64_t)k < n ? list_h[k] : 0;
+      s_min = 0x7fffffff;
+      s_max = (int32_t)0x80000000;
+      s_drop = 0;
+    }
+    __syncthreads();
+    const int r = s_read, H = s_H;
+    if (r < 0) break;
+    if (H > (KIND == kHuge ? cap : Cf::CAP) || (KIND == kLarge && shift_all > 16)) {
+      if (threadIdx.x == 0) {
+        const int k = atomicAdd(huge_count, 1);
+        huge_list[k] = r;
+        huge_h[k] = H;
+      }
+      __syncthreads();
+      continue;
+    }
+    const int L = rd.lengths[r];
+    {
+      const uint8_t* src = rd.codes + (int64_t)r * rd.cstride;
+      const int nbytes = (L + 3) >> 2;
+      for (int b = threadIdx.x; b < kReadBytes; b += THREADS) srd[b] = b < nbytes ? src[b] : 0;
+    }
+    int T = 0;
+    for (int si = 0; si < gs.n; ++si) T += seed_npos(gs.s[si], L);
+    lookups += (unsigned long long)T;
+    positions += (unsigned long long)H;
+    int nb = NB, shift = shift_all;
+    int32_t vmin = -STORMGPU_MAX_READ_LEN;
+    if constexpr (KIND != kLarge) {
+      nb = 1;
+      while (nb < NB && nb * 8 < H) nb <<= 1;
+    }
+    for (int b = threadIdx.x; b < nb; b += THREADS) S.cnt[b] = 0;
+    __syncthreads();
+    if constexpr (KIND != kLarge) {
+      vmin = 0x7fffffff;
+      int32_t vmax = (int32_t)0x80000000;
+      each_position<THREADS>(S.items, ix, gs, srd, L, T, H, [&](int k, int32_t v) {
+        vmin = min(vmin, v);
+        vmax = max(vmax, v);
+        B[k] = v;
+      });
+      vmin = __reduce_min_sync(0xffffffffu, vmin);
+      vmax = __reduce_max_sync(0xffffffffu, vmax);
+      if ((threadIdx.x & 31) == 0) {
+        atomicMin(&s_min, vmin);
+        atomicMax(&s_max, vmax);
+      }
+      __syncthreads();
+      vmin = s_min;
+      const uint32_t range = (uint32_t)s_max - (uint32_t)vmin;
+      shift = 0;
+      while ((range >> shift) >= (uint32_t)nb) ++shift;
+      for (int i = threadIdx.x; i < H; i += THREADS) atomicAdd(&S.cnt[((uint32_t)B[i] - (uint32_t)vmin) >> shift], 1);
+    } else {
+      each_position<THREADS>(S.items, ix, gs, srd, L, T, H,
+                             [&](int, int32_t v) { atomicAdd(&S.cnt[((uint32_t)v - (uint32_t)vmin) >> shift], 1); });
+    }
+    __syncthreads();
+    sort_excl_scan<THREADS, NB>(S.cnt, nb, S.items.wtot);
+    each_position<THREADS>(S.items, ix, gs, srd, L, T, H, [&](int, int32_t v) {
+      const uint32_t x = (uint32_t)v - (uint32_t)vmin;
+      B[atomicAdd(&S.cnt[x >> shift], 1)] = KIND != kLarge ? (V)v : (V)(x & ((1u << shift) - 1u));
+    });
+    // cnt[b] is now the end of bucket b
+    for (int b = threadIdx.x; b < nb; b += THREADS)
+      S.uoff[b] = (typename Cf::U)sort_bucket(B, b ? S.cnt[b - 1] : 0, S.cnt[b]);
+    __syncthreads();
+    const int U = sort_excl_scan<THREADS, NB>(S.uoff, nb, S.items.wtot);
+    // bucket b: its first slot, the offset of its distinct values and their number; the diagonals
+    auto bucket = [&](int b, int& s0, int& o, int& u) {
+      s0 = b ? S.cnt[b - 1] : 0;
+      o = S.uoff[b];
+      u = (b + 1 < nb ? (int)S.uoff[b + 1] : U) - o;
+    };
+    auto value = [&](int b, int at) -> int32_t {
+      return KIND != kLarge ? (int32_t)B[at] : (int32_t)((uint32_t)vmin + ((uint32_t)b << shift) + (uint32_t)B[at]);
+    };
+    for (int b = threadIdx.x; b < nb; b += THREADS) {  // the first diagonal must exceed -I (run.c:617, :648)
+      int s0, o, u;
+      bucket(b, s0, o, u);
+      if (o == 0 && u > 0 && value(b, s0) <= -I) s_drop = 1;
+    }
+    __syncthreads();
+    const int drop = s_drop, Uo = U - drop;
+    if (threadIdx.x == 0) s_base = Uo > 0 ? atomicAdd(&go.counters[7], (unsigned long long)Uo) : 0ull;
+    __syncthreads();
+    const unsigned long long base = s_base;
+    if ((int64_t)(base + Uo) > go.cap) {
+      if (threadIdx.x == 0) atomicExch(&go.counters[8], 1ull);
+    } else {
+      for (int k = threadIdx.x; k < Uo; k += THREADS) go.fr[base + k] = r;
+      for (int b = threadIdx.x; b < nb; b += THREADS) {
+        int s0, o, u;
+        bucket(b, s0, o, u);
+        for (int k = 0; k < u; ++k)
+          if (o + k >= drop) go.fd[base + o + k - drop] = value(b, s0 + k);
+      }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    atomicAdd(&go.counters[3], lookups);
+    atomicAdd(&go.counters[4], positions);
+  }
+}
+
+int64_t gather_huge_grid() {
+  set_smem_attribute_once(reinterpret_cast<const void*>(gather_sort_kernel<kHuge>), (int)sizeof(SortConfig<kHuge>::Smem));
+  return resident_grid(gather_sort_kernel<kHuge>, SortConfig<kHuge>::THREADS, sizeof(SortConfig<kHuge>::Smem));
+}
+
+template <SortKind KIND>
+static void launch_sort(const ReadsDev& rd, const IndexView& ix, int I, int64_t n_codes, const GatherList& l,
+                        const GatherOut& go, int32_t* scratch, int cap, int64_t max_grid, const SeedSet& seeds,
+                        cudaStream_t st) {
+  if (l.n <= 0 || max_grid <= 0) return;
+  constexpr size_t smem = sizeof(typename SortConfig<KIND>::Smem);
+  constexpr int threads = SortConfig<KIND>::THREADS;
+  set_smem_attribute_once(reinterpret_cast<const void*>(gather_sort_kernel<KIND>), (int)smem);
+  const int64_t grid = std::min({l.n, max_grid, resident_grid(gather_sort_kernel<KIND>, threads, smem)});
+  gather_sort_kernel<KIND><<<(unsigned)grid, threads, smem, st>>>(rd, ix, I, n_codes, l.read, l.h, l.n_dev, l.n, go,
+                                                                  scratch, cap, l.cursor, l.above, l.above_h,
+                                                                  l.above_count, seeds);
+}
+
+void launch_gather_sort(const ReadsDev& rd, const IndexView& ix, int I, int64_t n_codes, const GatherList& l, bool small,
+                        const GatherOut& go, const SeedSet& seeds, cudaStream_t st) {
+  if (small) launch_sort<kSmall>(rd, ix, I, n_codes, l, go, nullptr, 0, INT64_MAX, seeds, st);
+  else launch_sort<kLarge>(rd, ix, I, n_codes, l, go, nullptr, 0, INT64_MAX, seeds, st);
+}
+
+void launch_gather_huge(const ReadsDev& rd, const IndexView& ix, int I, int64_t n_codes, const GatherList& l,
+                        int32_t* scratch, int cap, int64_t grid, const GatherOut& go, const SeedSet& seeds,
+                        cudaStream_t st) {
+  launch_sort<kHuge>(rd, ix, I, n_codes, l, go, scratch, cap, grid, seeds, st);
 }
 
 }  // namespace sg

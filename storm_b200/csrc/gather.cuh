@@ -25,23 +25,36 @@ struct GatherOut {
 
 constexpr int kMaxWarpCap = 1536;
 
-constexpr int kBlockGatherCap = 65536;
 
 // The seed family travels with every launch (a kernel parameter), so that mapping calls with
 // different seed families can run concurrently on different streams.
 void launch_gather_fused(const ReadsDev& rd, const IndexView& ix, int I, const GatherOut& go, const SeedSet& seeds,
                          cudaStream_t st);
-// The nlist reads of `list` with their position counts `list_h` (with nlist_dev, which may be
-// null, the count is read from there when the kernel starts and nlist is only nonzero), a
-// persistent grid of `grid` blocks (at most gather_block_grid(smem) useful) taking reads from the
-// zeroed `cursor`; scratch holds 2 * cap words per block.  Reads with more than `cap` positions
-// are appended to (huge_list, huge_h), counted in huge_count.  smem: the slices in shared memory,
-// for lists whose reads have at most kSmallGatherCap positions.
+// Reads the warp gather handed on, with their position counts (with n_dev, which may be null, the
+// number is read from there when the kernel starts and n is only an upper bound), taken from the
+// zeroed `cursor` by a persistent grid; reads with too many positions for the launch are appended to
+// (above, above_h), counted in above_count.
+struct GatherList {
+  const int32_t* read;
+  const int32_t* h;
+  int64_t n;
+  const int32_t* n_dev;
+  unsigned long long* cursor;
+  int32_t* above;
+  int32_t* above_h;
+  int32_t* above_count;
+};
+
+// sorted in shared memory: reads of at most kSmallGatherCap positions (small), else kSortGatherCap
 constexpr int kSmallGatherCap = 4096;
-void launch_gather_block(const ReadsDev& rd, const IndexView& ix, int I, const int32_t* list, const int32_t* list_h,
-                         int64_t nlist, const int32_t* nlist_dev, const GatherOut& go, int32_t* scratch, int cap,
-                         int64_t grid, unsigned long long* cursor, int32_t* huge_list, int32_t* huge_h,
-                         int32_t* huge_count, bool smem, const SeedSet& seeds, cudaStream_t st);
-int64_t gather_block_grid(bool smem);
+constexpr int kSortGatherCap = 65535;
+void launch_gather_sort(const ReadsDev& rd, const IndexView& ix, int I, int64_t n_codes, const GatherList& l, bool small,
+                        const GatherOut& go, const SeedSet& seeds, cudaStream_t st);
+// in global memory: reads of at most `cap` positions, at most `grid` blocks (gather_huge_grid() are
+// useful), scratch of cap words each
+void launch_gather_huge(const ReadsDev& rd, const IndexView& ix, int I, int64_t n_codes, const GatherList& l,
+                        int32_t* scratch, int cap, int64_t grid, const GatherOut& go, const SeedSet& seeds,
+                        cudaStream_t st);
+int64_t gather_huge_grid();
 
 }  // namespace sg

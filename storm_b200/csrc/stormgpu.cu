@@ -487,6 +487,19 @@ static KeptList kept_list(stormgpu_ctx* c, const PassSetup& P, int64_t n, const 
   return kl;
 }
 
+// The lists of reads the warp gather hands on: at most kSmallGatherCap positions, more, and too many for
+// shared memory.  Their cursors are zeroed with the counters of the pass.
+static GatherList small_gather_list(stormgpu_ctx* c, int64_t n, const int32_t* n_dev) {
+  return {c->small_list.p, c->small_h.p, n, n_dev, c->counters.p + 9, c->huge_list.p, c->huge_h.p, c->big_count.p + 1};
+}
+static GatherList large_gather_list(stormgpu_ctx* c, int64_t n, const int32_t* n_dev) {
+  return {c->big_list.p, c->big_h.p, n, n_dev, c->counters.p + 14, c->huge_list.p, c->huge_h.p, c->big_count.p + 1};
+}
+static GatherList huge_gather_list(stormgpu_ctx* c, int64_t reads, int64_t n, const int32_t* n_dev) {
+  return {c->huge_list.p, c->huge_h.p, n, n_dev, c->counters.p + 15, c->huge_list.p + reads, c->huge_h.p + reads,
+          c->big_count.p + 1};
+}
+
 // List capacities of a graph call.
 struct GraphCaps {
   int64_t cand, pass, kept;
@@ -500,10 +513,9 @@ static bool graph_buffers(stormgpu_ctx* c, const PassSetup& P, GraphCaps* caps) 
   const int64_t want_cand = (int64_t)(c->gdens_cand * P.wsum * 1.25) + 61440;  // small calls: one scan block
   const int64_t want_pass = (int64_t)(c->gdens_pass * P.wsum * 1.25) + 4096;
   const int64_t want_kept = P.bound_H ? (int64_t)(c->gdens_kept * P.wsum * 1.25) + 4096 : want_pass;
-  const int64_t grid_b = gather_block_grid(false);
-  caps->grid_h = std::max<int64_t>(1, std::min<int64_t>(grid_b, ((int64_t)1 << 25) / c->huge_cap));
+  caps->grid_h = std::max<int64_t>(1, std::min<int64_t>(gather_huge_grid(), ((int64_t)1 << 25) / c->huge_cap));
   if (c->fr.grow(want_cand) || c->fd.grow(want_cand) || c->big_count.grow(4) || c->gstate.grow(kGsWords) ||
-      c->big_tmp.grow(std::max(grid_b * 2 * (int64_t)kBlockGatherCap, caps->grid_h * 2 * c->huge_cap)))
+      c->big_tmp.grow(caps->grid_h * c->huge_cap))
     return false;
   if (P.bound_H && (c->q_read.grow(want_pass) || c->q_diag.grow(want_pass) || c->q_ub.grow(want_pass) ||
                     c->k_ub.grow(want_kept) || c->p_ub.grow(want_kept)))
@@ -535,7 +547,6 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const Graph
   unsigned long long* gs = c->gstate.p;
   const int64_t nw = (cand_cap + 31) / 32, nwq = (pass_cap + 31) / 32;
   const int rounds = P.rounds;
-  const int64_t grid_s = gather_block_grid(true), grid_b = gather_block_grid(false);
   auto rec = [&](cudaEvent_t e) { return cudaEventRecordWithFlags(e, st, cudaEventRecordExternal); };
   SG_CUDA(cudaMemsetAsync(gs, 0, sizeof(unsigned long long) * kGsWords, st));
   int pi = 0;
@@ -563,15 +574,11 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const Graph
       go.reads_per_steal = c->tune.gather_reads_per_steal;
       go.warp_cap = c->tune.gather_warp_cap;
       launch_gather_fused(rd, ix, sp.I, go, c->seeds, st);
-      launch_gather_block(rd, ix, sp.I, c->small_list.p, c->small_h.p, n, c->big_count.p + 2, go, c->big_tmp.p,
-                          kBlockGatherCap, grid_s, c->counters.p + 9, c->huge_list.p, c->huge_h.p, c->big_count.p + 1,
-                          true, c->seeds, st);
-      launch_gather_block(rd, ix, sp.I, c->big_list.p, c->big_h.p, n, c->big_count.p + 0, go, c->big_tmp.p,
-                          kBlockGatherCap, grid_b, c->counters.p + 14, c->huge_list.p, c->huge_h.p,
-                          c->big_count.p + 1, false, c->seeds, st);
-      launch_gather_block(rd, ix, sp.I, c->huge_list.p, c->huge_h.p, n, c->big_count.p + 1, go, c->big_tmp.p,
-                          (int)c->huge_cap, grid_h, c->counters.p + 15, c->huge_list.p + n, c->huge_h.p + n,
-                          c->big_count.p + 3, false, c->seeds, st);
+      launch_gather_sort(rd, ix, sp.I, R.n, small_gather_list(c, n, c->big_count.p + 2), true, go, c->seeds, st);
+      launch_gather_sort(rd, ix, sp.I, R.n, large_gather_list(c, n, c->big_count.p + 0), false, go, c->seeds, st);
+      GatherList hl = huge_gather_list(c, n, n, c->big_count.p + 1);
+      hl.above_count = c->big_count.p + 3;
+      launch_gather_huge(rd, ix, sp.I, R.n, hl, c->big_tmp.p, (int)c->huge_cap, grid_h, go, c->seeds, st);
       gate_gather_kernel<<<1, 1, 0, st>>>(c->counters.p, c->big_count.p, cand_cap, kMaxCandidatesPerPass, gs);
       launches += 5;
       SG_CUDA(rec(E[1]));
@@ -865,36 +872,28 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
         SG_CUDA(cudaMemcpyAsync(nbig, c->big_count.p, sizeof(nbig), cudaMemcpyDeviceToHost, st));
         SG_CUDA(cudaStreamSynchronize(st));
         if (nbig[2] > 0) {  // reads with few positions: sorted in shared memory
-          const int64_t grid_s = std::min<int64_t>(nbig[2], gather_block_grid(true));
-          launch_gather_block(rd, ix, sp.I, c->small_list.p, c->small_h.p, nbig[2], nullptr, go, c->big_tmp.p, kBlockGatherCap,
-                              grid_s, c->counters.p + 9, c->huge_list.p, c->huge_h.p, c->big_count.p + 1, true,
-                              c->seeds, st);
+          launch_gather_sort(rd, ix, sp.I, R.n, small_gather_list(c, nbig[2], nullptr), true, go, c->seeds, st);
           launches++;
         }
-        if (nbig[0] > 0) {  // reads with many positions: a block each, slices in global memory
-          const int64_t grid = std::min<int64_t>(nbig[0], gather_block_grid(false));
-          if (c->big_tmp.grow(grid * 2 * (int64_t)kBlockGatherCap)) return STORMGPU_ENOMEM;
-          launch_gather_block(rd, ix, sp.I, c->big_list.p, c->big_h.p, nbig[0], nullptr, go, c->big_tmp.p, kBlockGatherCap,
-                              grid, c->counters.p + 14, c->huge_list.p, c->huge_h.p, c->big_count.p + 1, false,
-                              c->seeds, st);
+        if (nbig[0] > 0) {  // reads with many positions: a block with most of an SM's shared memory
+          launch_gather_sort(rd, ix, sp.I, R.n, large_gather_list(c, nbig[0], nullptr), false, go, c->seeds, st);
           launches++;
           SG_CUDA(cudaMemcpyAsync(nbig + 1, c->big_count.p + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
           SG_CUDA(cudaStreamSynchronize(st));
-          if (nbig[1] > 0) {  // beyond kBlockGatherCap: the same with a slice of the largest read's size
+          if (nbig[1] > 0) {  // beyond it: slices of the largest read's size in global memory
             std::vector<int32_t> hh(nbig[1]);
             SG_CUDA(cudaMemcpyAsync(hh.data(), c->huge_h.p, sizeof(int32_t) * nbig[1], cudaMemcpyDeviceToHost, st));
             SG_CUDA(cudaStreamSynchronize(st));
-            int64_t cap2 = kBlockGatherCap;
+            int64_t cap2 = 65536;
             for (int k = 0; k < nbig[1]; ++k) while (cap2 < hh[k]) cap2 <<= 1;
             if (cap2 > (int64_t)1 << 30) { sg_set_error("a read has %lld index positions", (long long)cap2); return STORMGPU_EINVAL; }
             c->huge_cap = std::max<int64_t>(c->huge_cap, cap2);
             // at most 1 GiB of slices
-            const int64_t grid2 = std::max<int64_t>(1, std::min<int64_t>({(int64_t)nbig[1], gather_block_grid(false),
-                                                                           ((int64_t)1 << 27) / cap2}));
-            if (c->big_tmp.grow(grid2 * 2 * cap2)) return STORMGPU_ENOMEM;
-            launch_gather_block(rd, ix, sp.I, c->huge_list.p, c->huge_h.p, nbig[1], nullptr, go, c->big_tmp.p, (int)cap2,
-                                grid2, c->counters.p + 15, c->huge_list.p + n, c->huge_h.p + n, c->big_count.p + 1,
-                                false, c->seeds, st);
+            const int64_t grid2 = std::max<int64_t>(1, std::min<int64_t>({(int64_t)nbig[1], gather_huge_grid(),
+                                                                           ((int64_t)1 << 28) / cap2}));
+            if (c->big_tmp.grow(grid2 * cap2)) return STORMGPU_ENOMEM;
+            launch_gather_huge(rd, ix, sp.I, R.n, huge_gather_list(c, n, nbig[1], nullptr), c->big_tmp.p, (int)cap2, grid2,
+                               go, c->seeds, st);
             launches++;
           }
         }

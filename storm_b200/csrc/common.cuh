@@ -39,6 +39,34 @@ __host__ __device__ __forceinline__ int code_at(const uint8_t* p, int64_t n) {
   return (p[n >> 2] >> ((n & 3) << 1)) & 3;
 }
 
+// A seed's care positions as runs, for keys from a window of 32 codes whose first code is in the
+// high bits: the key is the OR of (window >> shift) & mask over the runs (4 to 7 of them, where taking
+// the care positions one by one takes 10 to 15 steps).  Seeds of span <= 32.
+struct SeedRuns {
+  uint2 r[16];  // shift, mask; unused ones have mask 0
+};
+
+// returns the number of runs
+__host__ __device__ __forceinline__ int make_runs(const SeedDev& s, SeedRuns& o) {
+  int n = 0;
+  for (int c = 0; c < 16; ++c) { o.r[c].x = 0; o.r[c].y = 0; }
+  for (int c = 0; c < s.n_care;) {
+    int m = 1;
+    while (c + m < s.n_care && s.care[c + m] - s.care[c] == m) ++m;
+    o.r[n].x = (uint32_t)(62 - 2 * (s.care[c] + s.n_care - 1 - c));
+    o.r[n].y = (uint32_t)((1ull << (2 * m)) - 1ull) << (2 * (s.n_care - c - m));
+    ++n;
+    c += m;
+  }
+  return n;
+}
+
+// 16 packed codes, first code in the low bits -> first code in the high bits
+__device__ __forceinline__ uint32_t reverse_codes(uint32_t x) {
+  x = __brev(x);
+  return ((x & 0x55555555u) << 1) | ((x >> 1) & 0x55555555u);
+}
+
 __device__ __forceinline__ int warp_incl_scan(int v) {
   const int lane = threadIdx.x & 31;
 #pragma unroll

@@ -122,33 +122,6 @@ __device__ __forceinline__ int warp_distinct(int32_t* a, int H, uint16_t* tab, i
   return U;
 }
 
-// A seed's care positions as runs, for keys from a window of 32 codes whose first code is in the
-// high bits: the key is the OR of (window >> shift) & mask over the runs (4 to 7 of them, where taking
-// the care positions one by one takes 10 to 15 steps).
-struct SeedRuns {
-  uint2 r[16];  // shift, mask; unused ones have mask 0
-};
-
-// returns the number of runs
-__device__ __forceinline__ int make_runs(const SeedDev& s, SeedRuns& o) {
-  int n = 0;
-  for (int c = 0; c < 16; ++c) o.r[c] = make_uint2(0, 0);
-  for (int c = 0; c < s.n_care;) {
-    int m = 1;
-    while (c + m < s.n_care && s.care[c + m] - s.care[c] == m) ++m;
-    o.r[n++] = make_uint2((uint32_t)(62 - 2 * (s.care[c] + s.n_care - 1 - c)),
-                          (uint32_t)((1ull << (2 * m)) - 1ull) << (2 * (s.n_care - c - m)));
-    c += m;
-  }
-  return n;
-}
-
-// 16 packed codes, first code in the low bits -> first code in the high bits
-__device__ __forceinline__ uint32_t reverse_codes(uint32_t x) {
-  x = __brev(x);
-  return ((x & 0x55555555u) << 1) | ((x >> 1) & 0x55555555u);
-}
-
 constexpr int kGWarps = 4;
 // Reads per steal (GatherOut.reads_per_steal, 4 by default): the grid is the resident set, and
 // every warp takes the next reads_per_steal reads (in the order of rd.order, or of the batch) from a work cursor until none is left, so

@@ -4,9 +4,12 @@
 // index.c:212-241).
 //
 // Build = seed keys of every indexed position (kernel) -> stable LSD radix sort of (key, pos)
-// -> per-key runs of the sorted list (start, count) -> repeat filter (exact integer moments;
-// the host turns them into the largest admissible count) -> a scan of the kept counts ->
-// compaction into the CSR.  HBM-streaming work.
+// -> the runs of equal keys in the sorted list: their number and squared lengths (the repeat filter's
+// exact integer moments; the host turns them into the largest admissible count), then the offsets.
+// When the filter erases nothing the sorted positions are the map; else the kept ones are compacted.
+// The key table is written once, from the sorted list (nothing else has its 4^w entries: for a
+// 1 Mbp sequence and w = 12 the passes over them were most of the build).  HBM-streaming work; the
+// seeds of a sequence share one wait for their moments.
 #include <cmath>
 #include <vector>
 
@@ -16,73 +19,165 @@
 namespace sg {
 
 // Indexed positions come as intervals [a, b); t-th indexed position = a_k + (t - before_k).
+// A warp takes consecutive t: the interval of its first is searched, the others walk on from it.
+constexpr int kKeysPerLane = 8;
+struct KeySeed {
+  SeedRuns runs;
+  int nruns;
+  SeedDev seed;  // span above 32: code by code
+};
+
 __global__ void seed_keys_kernel(const uint8_t* __restrict__ codes, const int64_t* __restrict__ ia,
                                  const int64_t* __restrict__ ibefore, int nint, int64_t total,
-                                 SeedDev seed, uint32_t* __restrict__ keys, uint32_t* __restrict__ pos) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= total) return;
+                                 const __grid_constant__ KeySeed ks, uint32_t* __restrict__ keys,
+                                 uint32_t* __restrict__ pos) {
+  const int lane = threadIdx.x & 31;
+  const int64_t tw = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 * kKeysPerLane);
+  if (tw >= total) return;
   int lo = 0, hi = nint - 1;
-  while (lo < hi) {  // last interval with before <= t
-    int mid = (lo + hi + 1) >> 1;
-    if (ibefore[mid] <= t) lo = mid; else hi = mid - 1;
+  while (lo < hi) {  // last interval with before <= the warp's first t
+    const int mid = (lo + hi + 1) >> 1;
+    if (ibefore[mid] <= tw) lo = mid; else hi = mid - 1;
   }
-  int64_t p = ia[lo] + (t - ibefore[lo]);
-  uint32_t key = 0;
-  for (int c = 0; c < seed.n_care; ++c) key = (key << 2) | (uint32_t)code_at(codes, p + seed.care[c]);
-  keys[t] = key;
-  pos[t] = (uint32_t)p;
+#pragma unroll
+  for (int r = 0; r < kKeysPerLane; ++r) {
+    const int64_t t = tw + 32 * r + lane;
+    if (t >= total) return;
+    while (lo + 1 < nint && ibefore[lo + 1] <= t) ++lo;
+    const int64_t p = ia[lo] + (t - ibefore[lo]);
+    uint32_t key = 0;
+    if (ks.seed.span <= 32) {
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(codes) + (p >> 4);
+      const uint32_t w0 = reverse_codes(__ldg(w)), w1 = reverse_codes(__ldg(w + 1)), w2 = reverse_codes(__ldg(w + 2));
+      const int sh = 2 * (int)(p & 15);
+      const uint64_t win = (uint64_t)__funnelshift_l(w1, w0, sh) << 32 | __funnelshift_l(w2, w1, sh);
+      for (int c = 0; c < ks.nruns; ++c) key |= (uint32_t)(win >> ks.runs.r[c].x) & ks.runs.r[c].y;
+    } else {
+      for (int c = 0; c < ks.seed.n_care; ++c) key = (key << 2) | (uint32_t)code_at(codes, p + ks.seed.care[c]);
+    }
+    keys[t] = key;
+    pos[t] = (uint32_t)p;
+  }
 }
 
-// Runs of equal keys in the sorted list: start[k] = first index of key k, end[k] = one past its
-// last (both left at 0 for absent keys), so that count = end - start with no atomics.
-__global__ void key_runs_kernel(const uint32_t* __restrict__ skeys, int64_t n, int32_t* __restrict__ start,
-                                int32_t* __restrict__ end) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const uint32_t k = skeys[t];
-  if (t == 0 || skeys[t - 1] != k) start[k] = (int32_t)t;
-  if (t == n - 1 || skeys[t + 1] != k) end[k] = (int32_t)(t + 1);
+// The key table is written in blocks of kKeyBlock keys; bound[b]: first index of the sorted list whose
+// key is in block b or a later one.
+constexpr int kKeyBlock = 2048;
+
+// length of the run of equal keys that starts at t
+__device__ __forceinline__ int64_t run_length(const uint32_t* __restrict__ skeys, int64_t n, int64_t t, uint32_t k) {
+  int64_t d = 1;
+  while (t + d < n && skeys[t + d] == k) d <<= 1;
+  int64_t lo = d >> 1, hi = min(d, n - t);  // t + lo has the key (or lo = 0), t + hi has not
+  while (hi - lo > 1) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (skeys[t + mid] == k) lo = mid; else hi = mid;
+  }
+  return hi;
 }
 
-__global__ void run_counts_kernel(const int32_t* __restrict__ start, int64_t nkeys, int32_t* __restrict__ counts) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < nkeys) counts[k] -= start[k];
-}
-
-__global__ void moments_kernel(const int32_t* __restrict__ counts, int64_t nkeys,
-                               unsigned long long* __restrict__ out) {
-  unsigned long long s2 = 0, nocc = 0;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nkeys; k += (int64_t)gridDim.x * blockDim.x) {
-    long long c = counts[k];
-    if (c > 0) { s2 += (unsigned long long)(c * c); nocc++; }
+// out[0] += squared run lengths, out[1] += runs, out[2] = longest run; the blocks' bounds.
+__global__ void run_stats_kernel(const uint32_t* __restrict__ skeys, int64_t n, int64_t nblocks,
+                                 unsigned long long* __restrict__ out, int32_t* __restrict__ bound) {
+  unsigned long long s2 = 0, runs = 0, longest = 0;
+  const int lane = threadIdx.x & 31;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
+    const int64_t t = base + lane;
+    const uint32_t k = t < n ? skeys[t] : 0u;
+    uint32_t prev = __shfl_up_sync(0xffffffffu, k, 1);
+    if (lane == 0 && t) prev = skeys[t - 1];
+    const bool head = t < n && (t == 0 || prev != k);
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    if (!head) continue;
+    // up to the next head of the warp, else on from the warp's end
+    const unsigned later = lane < 31 ? heads >> (lane + 1) : 0u;
+    unsigned long long c;
+    if (later) c = (unsigned long long)__ffs(later);
+    else if (base + 32 >= n) c = (unsigned long long)(n - t);
+    else c = skeys[base + 32] == k ? (unsigned long long)(32 - lane) + (unsigned long long)run_length(skeys, n, base + 32, k)
+                                   : (unsigned long long)(32 - lane);
+    s2 += c * c;
+    runs++;
+    longest = max(longest, c);
+    for (int64_t b = t ? (int64_t)(prev / kKeyBlock) + 1 : 0; b <= (int64_t)(k / kKeyBlock); ++b) bound[b] = (int32_t)t;
+    if (t + (int64_t)c == n)
+      for (int64_t b = (int64_t)(k / kKeyBlock) + 1; b <= nblocks; ++b) bound[b] = (int32_t)n;
   }
   for (int o = 16; o > 0; o >>= 1) {
     s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-    nocc += __shfl_xor_sync(0xffffffffu, nocc, o);
+    runs += __shfl_xor_sync(0xffffffffu, runs, o);
+    longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
   }
-  if ((threadIdx.x & 31) == 0) {
+  if ((threadIdx.x & 31) == 0 && runs) {
     atomicAdd(&out[0], s2);
-    atomicAdd(&out[1], nocc);
+    atomicAdd(&out[1], runs);
+    atomicMax(&out[2], longest);
   }
 }
 
-__global__ void kept_kernel(const int32_t* __restrict__ counts, int64_t nkeys, int32_t cmax,
-                            int32_t* __restrict__ kept) {
-  int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < nkeys) {
-    int32_t c = counts[k];
-    kept[k] = c <= cmax ? c : 0;
+// keep[t] = 0 for the positions of keys with more than cmax (all 1 before)
+__global__ void erase_runs_kernel(const uint32_t* __restrict__ skeys, int64_t n, int32_t cmax, uint8_t* __restrict__ keep) {
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t k = skeys[t];
+    if (t && skeys[t - 1] == k) continue;
+    const int64_t c = run_length(skeys, n, t, k);
+    if (c > cmax)
+      for (int64_t u = t; u < t + c; ++u) keep[u] = 0;
   }
 }
 
-__global__ void csr_fill_kernel(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ spos,
-                                int64_t n, const int32_t* __restrict__ counts,
-                                const int32_t* __restrict__ allstart, const int32_t* __restrict__ first,
-                                int32_t cmax, int32_t* __restrict__ map) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  uint32_t k = skeys[t];
-  if (counts[k] <= cmax) map[first[k] + (t - allstart[k])] = (int32_t)spos[t];
+__global__ void kept_positions_kernel(const uint8_t* __restrict__ keep, const int32_t* __restrict__ off,
+                                      const uint32_t* __restrict__ spos, int64_t n, int32_t* __restrict__ map) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n && keep[t]) map[off[t]] = (int32_t)spos[t];
+}
+
+// first[k] of a block of keys: the offset (off[t], or t without off) of the first position t whose key is
+// k or a later one: the first positions of the keys present go to shared memory, and a suffix
+// minimum gives the others theirs.  total: the offset after the last position.
+__global__ void __launch_bounds__(256) key_table_kernel(const uint32_t* __restrict__ skeys, int64_t n, int64_t nkeys,
+                                                        const int32_t* __restrict__ bound,
+                                                        const int32_t* __restrict__ off, const int32_t* __restrict__ total,
+                                                        int32_t* __restrict__ first) {
+  constexpr int PER = kKeyBlock / 256;
+  __shared__ int32_t at[kKeyBlock];
+  __shared__ int32_t wmin[8];
+  const int64_t k0 = (int64_t)blockIdx.x * kKeyBlock;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t lo = bound[blockIdx.x], hi = bound[blockIdx.x + 1];
+  for (int k = threadIdx.x; k < kKeyBlock; k += 256) at[k] = 0x7fffffff;
+  __syncthreads();
+  for (int64_t t = lo + threadIdx.x; t < hi; t += 256) {
+    const uint32_t k = skeys[t];
+    if (t == 0 || skeys[t - 1] != k) at[k - (uint32_t)k0] = (int32_t)t;
+  }
+  __syncthreads();
+  int32_t v[PER], m = 0x7fffffff;
+#pragma unroll
+  for (int i = PER - 1; i >= 0; --i) {  // thread-local suffix minima
+    m = min(m, at[threadIdx.x * PER + i]);
+    v[i] = m;
+  }
+  int32_t x = m;  // of the lanes from this one on
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t y = __shfl_down_sync(0xffffffffu, x, o);
+    if (lane + o < 32) x = min(x, y);
+  }
+  if (lane == 0) wmin[w] = x;
+  int32_t after = __shfl_down_sync(0xffffffffu, x, 1);
+  if (lane == 31) after = 0x7fffffff;
+  __syncthreads();
+  for (int q = w + 1; q < 8; ++q) after = min(after, wmin[q]);
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int64_t t = min((int64_t)min(v[i], after), hi);
+    at[threadIdx.x * PER + i] = !off ? (int32_t)t : t < n ? off[t] : *total;
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < kKeyBlock; k += 256)
+    if (k0 + k <= nkeys) first[k0 + k] = at[k];
 }
 
 // Host simulation of the position loop of index.c:65-96 at interval granularity: windows are
@@ -131,79 +226,136 @@ int32_t repeat_cutoff(int stdev_distance, int64_t N, unsigned long long s2, unsi
   return (int32_t)c;
 }
 
-int build_one_index(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, const int32_t* re,
-                    int nreg, const SeedDev& seed, int stdev_distance, DevIndex* out,
-                    cudaStream_t st, int64_t* launches) {
+namespace {
+
+// one seed's build between its sort and its fill
+struct Sorted {
+  uint32_t *keys = nullptr, *pos = nullptr;
+  int32_t* bound = nullptr;
+  int64_t total = 0, nblocks = 0;
+};
+
+unsigned blocks_of(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
+
+int sort_seed(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, const int32_t* re, int nreg,
+              const SeedDev& seed, DevIndex* out, Sorted* so, unsigned long long* mom, uint32_t* scratch, cudaStream_t st,
+              int64_t& L) {
   std::vector<int64_t> a, b;
   indexed_intervals(n_codes, seed.span, rs, re, nreg, a, b);
   const int64_t nkeys = (int64_t)1 << (2 * seed.weight);
   out->weight = seed.weight;
   out->nkeys = nkeys;
-  std::vector<int64_t> before(a.size());
-  int64_t total = 0;
-  for (size_t k = 0; k < a.size(); ++k) { before[k] = total; total += b[k] - a[k]; }
-  SG_CUDA(cudaMallocAsync(&out->first, sizeof(int32_t) * (nkeys + 1), st));
-  SG_CUDA(cudaMemsetAsync(out->first, 0, sizeof(int32_t) * (nkeys + 1), st));
   out->map = nullptr;
   out->n = 0;
-  if (total == 0) return 0;
+  std::vector<int64_t> iv(a);  // starts, then positions before each interval
+  int64_t total = 0;
+  for (size_t k = 0; k < a.size(); ++k) { iv.push_back(total); total += b[k] - a[k]; }
   if (total > INT32_MAX) { sg_set_error("sequence too long for 32-bit positions"); return STORMGPU_EINVAL; }
+  SG_CUDA(cudaMallocAsync(&out->first, sizeof(int32_t) * (nkeys + 1), st));
+  if (total == 0) {
+    SG_CUDA(cudaMemsetAsync(out->first, 0, sizeof(int32_t) * (nkeys + 1), st));
+    return 0;
+  }
+  so->total = total;
+  so->nblocks = nkeys / kKeyBlock + 1;  // the last one: the table's closing entry
+  // The sorted list ends in its own arrays, whichever way the passes go; the other side of the sort is
+  // scratch that every seed of the sequence uses.
   int64_t* d_iv;
-  uint32_t *k0, *v0, *k1, *v1;
-  int32_t *counts, *kept, *allstart;
-  unsigned long long* mom;
-  void* tmp;
-  const int64_t tmpb = std::max<int64_t>(radix_tmp_bytes(total), (scan_tmp_elems(nkeys + 1) + 8) * 4);
-  SG_CUDA(cudaMallocAsync(&d_iv, sizeof(int64_t) * 2 * a.size(), st));
-  SG_CUDA(cudaMallocAsync(&k0, sizeof(uint32_t) * total, st));
-  SG_CUDA(cudaMallocAsync(&v0, sizeof(uint32_t) * total, st));
-  SG_CUDA(cudaMallocAsync(&k1, sizeof(uint32_t) * total, st));
-  SG_CUDA(cudaMallocAsync(&v1, sizeof(uint32_t) * total, st));
-  SG_CUDA(cudaMallocAsync(&counts, sizeof(int32_t) * nkeys, st));
-  SG_CUDA(cudaMallocAsync(&kept, sizeof(int32_t) * (nkeys + 1), st));
-  SG_CUDA(cudaMallocAsync(&allstart, sizeof(int32_t) * (nkeys + 1), st));
-  SG_CUDA(cudaMallocAsync(&mom, sizeof(unsigned long long) * 2, st));
-  SG_CUDA(cudaMallocAsync(&tmp, tmpb, st));
-  SG_CUDA(cudaMemcpyAsync(d_iv, a.data(), sizeof(int64_t) * a.size(), cudaMemcpyHostToDevice, st));
-  SG_CUDA(cudaMemcpyAsync(d_iv + a.size(), before.data(), sizeof(int64_t) * a.size(), cudaMemcpyHostToDevice, st));
-  int64_t L = 0;
+  SG_CUDA(cudaMallocAsync(&so->keys, sizeof(uint32_t) * total, st));
+  SG_CUDA(cudaMallocAsync(&so->pos, sizeof(uint32_t) * total, st));
+  SG_CUDA(cudaMallocAsync(&so->bound, sizeof(int32_t) * (so->nblocks + 1), st));
+  SG_CUDA(cudaMallocAsync(&d_iv, sizeof(int64_t) * iv.size(), st));
+  const int passes = (2 * seed.weight + kRadixBits - 1) / kRadixBits;
+  uint32_t* const sk = scratch;
+  uint32_t* const sv = sk + n_codes;
+  void* const tmp = sv + n_codes;
+  uint32_t *k0 = passes & 1 ? sk : so->keys, *v0 = passes & 1 ? sv : so->pos;
+  uint32_t *k1 = passes & 1 ? so->keys : sk, *v1 = passes & 1 ? so->pos : sv;
+  SG_CUDA(cudaMemcpyAsync(d_iv, iv.data(), sizeof(int64_t) * iv.size(), cudaMemcpyHostToDevice, st));
+  KeySeed ks;
+  ks.seed = seed;
+  ks.nruns = seed.span <= 32 ? make_runs(seed, ks.runs) : 0;
   const int TB = 256;
-  seed_keys_kernel<<<(unsigned)((total + TB - 1) / TB), TB, 0, st>>>(d_codes, d_iv, d_iv + a.size(),
-                                                                       (int)a.size(), total, seed, k0, v0);
-  L++;
-  int which = radix_sort_pairs(k0, v0, k1, v1, total, 2 * seed.weight, tmp, st);
-  L += 3 * ((2 * seed.weight + kRadixBits - 1) / kRadixBits);
-  uint32_t* sk = which ? k1 : k0;
-  uint32_t* sv = which ? v1 : v0;
-  SG_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * nkeys, st));
-  SG_CUDA(cudaMemsetAsync(allstart, 0, sizeof(int32_t) * nkeys, st));
-  key_runs_kernel<<<(unsigned)((total + TB - 1) / TB), TB, 0, st>>>(sk, total, allstart, counts);
-  run_counts_kernel<<<(unsigned)((nkeys + TB - 1) / TB), TB, 0, st>>>(allstart, nkeys, counts);
-  SG_CUDA(cudaMemsetAsync(mom, 0, sizeof(unsigned long long) * 2, st));
-  moments_kernel<<<592, TB, 0, st>>>(counts, nkeys, mom);
-  L += 3;
-  unsigned long long hm[2];
-  SG_CUDA(cudaMemcpyAsync(hm, mom, sizeof(hm), cudaMemcpyDeviceToHost, st));
-  SG_CUDA(cudaStreamSynchronize(st));
-  int32_t cmax = repeat_cutoff(stdev_distance, total, hm[0], hm[1]);
-  kept_kernel<<<(unsigned)((nkeys + TB - 1) / TB), TB, 0, st>>>(counts, nkeys, cmax, kept);
-  exclusive_scan<int32_t, int32_t>(kept, out->first, nkeys, out->first + nkeys, (int32_t*)tmp, st);
-  L += 1 + 3;
-  int32_t nmap = 0;
-  SG_CUDA(cudaMemcpyAsync(&nmap, out->first + nkeys, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  SG_CUDA(cudaStreamSynchronize(st));
-  out->n = nmap;
-  SG_CUDA(cudaMallocAsync(&out->map, sizeof(int32_t) * std::max<int64_t>(nmap, 1), st));
-  csr_fill_kernel<<<(unsigned)((total + TB - 1) / TB), TB, 0, st>>>(sk, sv, total, counts, allstart,
-                                                                      out->first, cmax, out->map);
-  L++;
+  seed_keys_kernel<<<blocks_of(total, TB * kKeysPerLane), TB, 0, st>>>(d_codes, d_iv, d_iv + a.size(), (int)a.size(), total, ks, k0, v0);
+  radix_sort_pairs(k0, v0, k1, v1, total, 2 * seed.weight, tmp, st);
+  cudaFreeAsync(d_iv, st);
+  run_stats_kernel<<<(unsigned)std::min<int64_t>(blocks_of(total, TB), 148 * 16), TB, 0, st>>>(so->keys, total,
+                                                                                           so->nblocks, mom, so->bound);
+  L += 2 + 3 * passes;
   SG_CUDA(cudaGetLastError());
-  cudaFreeAsync(d_iv, st); cudaFreeAsync(k0, st); cudaFreeAsync(v0, st); cudaFreeAsync(k1, st);
-  cudaFreeAsync(v1, st); cudaFreeAsync(counts, st); cudaFreeAsync(kept, st);
-  cudaFreeAsync(allstart, st); cudaFreeAsync(mom, st); cudaFreeAsync(tmp, st);
+  return 0;
+}
+
+int fill_seed(DevIndex* out, const Sorted& so, int32_t cmax, int64_t longest, cudaStream_t st, int64_t& L) {
+  const int TB = 256;
+  int32_t *off = nullptr, *total = nullptr;
+  if (longest <= cmax) {  // nothing erased: the sorted positions are the map
+    out->map = reinterpret_cast<int32_t*>(so.pos);
+    out->n = so.total;
+  } else {
+    uint8_t* keep;
+    int32_t* tmp;  // scan
+    SG_CUDA(cudaMallocAsync(&keep, so.total, st));
+    SG_CUDA(cudaMallocAsync(&off, sizeof(int32_t) * (so.total + 1), st));
+    SG_CUDA(cudaMallocAsync(&tmp, sizeof(int32_t) * (scan_tmp_elems(so.total) + 8), st));
+    SG_CUDA(cudaMallocAsync(&out->map, sizeof(int32_t) * so.total, st));
+    total = off + so.total;
+    SG_CUDA(cudaMemsetAsync(keep, 1, so.total, st));
+    erase_runs_kernel<<<(unsigned)std::min<int64_t>(blocks_of(so.total, TB), 148 * 16), TB, 0, st>>>(so.keys, so.total, cmax,
+                                                                                                  keep);
+    exclusive_scan<uint8_t, int32_t>(keep, off, so.total, total, tmp, st);
+    kept_positions_kernel<<<blocks_of(so.total, TB), TB, 0, st>>>(keep, off, so.pos, so.total, out->map);
+    L += 2 + scan_launches(so.total);
+    int32_t n = 0;
+    SG_CUDA(cudaMemcpyAsync(&n, total, sizeof(n), cudaMemcpyDeviceToHost, st));
+    SG_CUDA(cudaStreamSynchronize(st));
+    out->n = n;
+    cudaFreeAsync(keep, st);
+    cudaFreeAsync(tmp, st);
+    cudaFreeAsync(so.pos, st);
+  }
+  key_table_kernel<<<(unsigned)so.nblocks, 256, 0, st>>>(so.keys, so.total, out->nkeys, so.bound, off, total, out->first);
+  L++;
+  if (off) cudaFreeAsync(off, st);
+  cudaFreeAsync(so.keys, st);
+  cudaFreeAsync(so.bound, st);
+  SG_CUDA(cudaGetLastError());
+  return 0;
+}
+
+}  // namespace
+
+int build_indexes(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, const int32_t* re, int nreg,
+                  const SeedDev* seeds, int nseeds, int stdev_distance, DevIndex* out, cudaStream_t st,
+                  int64_t* launches) {
+  constexpr int kGroup = 4;  // seeds whose sorted lists are held at once (8 bytes per position each)
+  unsigned long long* mom;
+  uint32_t* scratch;
+  const int64_t room = std::max<int64_t>(n_codes, 1);  // indexed positions of a seed
+  SG_CUDA(cudaMallocAsync(&scratch, sizeof(uint32_t) * 2 * room + radix_tmp_bytes(room), st));
+  SG_CUDA(cudaMallocAsync(&mom, sizeof(unsigned long long) * 3 * kGroup, st));
+  int64_t L = 0;
+  for (int s0 = 0; s0 < nseeds; s0 += kGroup) {
+    const int ng = std::min(kGroup, nseeds - s0);
+    Sorted so[kGroup];
+    SG_CUDA(cudaMemsetAsync(mom, 0, sizeof(unsigned long long) * 3 * kGroup, st));
+    for (int q = 0; q < ng; ++q)
+      if (const int rc = sort_seed(d_codes, n_codes, rs, re, nreg, seeds[s0 + q], &out[s0 + q], &so[q], mom + 3 * q, scratch, st, L))
+        return rc;
+    unsigned long long hm[3 * kGroup];
+    SG_CUDA(cudaMemcpyAsync(hm, mom, sizeof(hm), cudaMemcpyDeviceToHost, st));
+    SG_CUDA(cudaStreamSynchronize(st));
+    for (int q = 0; q < ng; ++q) {
+      if (so[q].total == 0) continue;
+      DevIndex* o = &out[s0 + q];
+      o->positions_indexed = so[q].total;
+      o->cmax = repeat_cutoff(stdev_distance, so[q].total, hm[3 * q], hm[3 * q + 1]);
+      if (const int rc = fill_seed(o, so[q], o->cmax, (int64_t)hm[3 * q + 2], st, L)) return rc;
+    }
+  }
+  cudaFreeAsync(mom, st);
+  cudaFreeAsync(scratch, st);
   if (launches) *launches += L;
-  out->positions_indexed = total;
-  out->cmax = cmax;
   return 0;
 }
 

@@ -258,13 +258,14 @@ extern "C" int stormgpu_build_index(stormgpu_ctx* c) {
   SG_CUDA(cudaEventRecord(c->ev[0], c->st));
   int64_t launches = 0;
   for (auto& r : c->refs) {
-    for (auto& ix : r.idx) { cudaFree(ix.first); cudaFree(ix.map); }
-    r.idx.assign(c->seeds.n, DevIndex());
-    for (int si = 0; si < c->seeds.n; ++si) {
-      int rc = build_one_index(r.d_codes, r.n, r.rs.data(), r.re.data(), (int)r.rs.size(), c->seeds.s[si],
-                               c->p.stdev_distance, &r.idx[si], c->st, &launches);
-      if (rc) return rc;
+    for (auto& ix : r.idx) {  // of the last build, from the stream-ordered pool
+      if (ix.first) cudaFreeAsync(ix.first, c->st);
+      if (ix.map) cudaFreeAsync(ix.map, c->st);
     }
+    r.idx.assign(c->seeds.n, DevIndex());
+    const int rc = build_indexes(r.d_codes, r.n, r.rs.data(), r.re.data(), (int)r.rs.size(), c->seeds.s, c->seeds.n,
+                                 c->p.stdev_distance, r.idx.data(), c->st, &launches);
+    if (rc) return rc;
   }
   SG_CUDA(cudaEventRecord(c->ev[1], c->st));
   SG_CUDA(cudaStreamSynchronize(c->st));
@@ -1389,7 +1390,7 @@ extern "C" int stormgpu_index_one(const char* seed, int32_t stdev_distance, cons
   uint8_t *ga, *gb;
   if (upload_padded(codes, n_codes, pad, 0, &ga, &gb)) return STORMGPU_ECUDA;
   DevIndex ix;
-  int rc = build_one_index(gb, n_codes, rs, re, n_regions, ss.s[0], stdev_distance, &ix, 0, nullptr);
+  int rc = build_indexes(gb, n_codes, rs, re, n_regions, ss.s, 1, stdev_distance, &ix, 0, nullptr);
   if (rc) { cudaFree(ga); return rc; }
   SG_CUDA(cudaDeviceSynchronize());
   SG_CUDA(cudaMemcpy(first, ix.first, sizeof(int32_t) * (ix.nkeys + 1), cudaMemcpyDeviceToHost));

@@ -81,6 +81,32 @@ __device__ __forceinline__ int st_make(int from, int ind, int chk, int ac, int f
 
 constexpr int kMaxBand = 2 * STORMGPU_MAX_INDELS + 1;
 
+// The colour state of a corner step (alignment.c:535-603, and the condition of the SNP adjustment
+// :465-468) as a table: index = state of the corner cell (checksum | auto-correct << 2 | freshness << 4)
+// | checksum of the cell's own colours << 7 | quality level << 9; entry = the new state, bit 7 the
+// condition.  The branches of the state machine, taken differently in every lane, were most of the
+// colour alignment's time (one round of 300 reads of 49 colours, both strands: 0.58 -> 0.31 ms).
+constexpr int kColourTable = 2048;
+__device__ __forceinline__ uint8_t colour_step(int idx) {
+  const int cchk = idx & 3, cac = (idx >> 2) & 3, cfr = (idx >> 4) & 7, chk0 = (idx >> 7) & 3, q = (idx >> 9) & 3;
+  int chk = chk0 ^ cchk, ac = chk0, fr = chk0 ? q : 0;
+  if (cchk != chk) {
+    if (cchk == 0) { ac = chk; fr = q; }
+    else if (chk == cac) { ac = 0; chk = 0; fr = 0; }
+    else if (chk == 0) { if (cfr - 1 > 0) { ac = cac; fr = cfr - 1; } else { ac = 0; fr = 0; } }
+    else { if (cfr - 1 > 0) { ac = cac; fr = cfr - 1; } else { ac = chk; fr = q; } }
+  } else {
+    if (cac != 0) {
+      if (cfr - 1 > 0) {
+        if (chk == 0) { ac = 0; fr = 0; } else { ac = cac; fr = cfr - 1; }
+      }
+    } else { chk = 0; ac = 0; fr = 0; }
+  }
+  const int cmp = cchk ^ chk0;
+  const bool adjust = cchk && (cmp == 0 || cmp == cac);
+  return (uint8_t)(chk | (ac << 2) | (fr << 4) | (adjust ? 0x80 : 0));
+}
+
 // alignment.c:326-360 (init), :488-632 (rows 1..L-1, corner > top > left on ties, gaps only
 // while indels < I, affine through the predecessor's direction, colour checksum state
 // machine :535-603 with the SNP adjustment :465-468), best cell on the last row (:621-630),
@@ -121,8 +147,42 @@ struct BandWindow {
   __device__ __forceinline__ int mcode(int c) const { return (int)((m[c >> 5] >> (2 * (c & 31))) & 3u); }
 };
 
+// Traceback over the direction words of the rows from i (cell c) up: emit(i, c, words of the row,
+// direction) for every cell of the path.  A path leaves a row once (every step but LEFT goes up), so the
+// rows' words are loaded four rows ahead whatever the path does; walked one cell at a time, each
+// step waited for its own word.
+template <int WPR, int WDIR, int LEFT, int TOP, class Emit>
+__device__ __forceinline__ void trace_rows(const uint32_t* scr, int64_t ns, int64_t sl, int i, int c, int BW, Emit emit) {
+  constexpr int PF = 4;
+  uint32_t w[PF][WPR];
+  auto load = [&](int q, int row) {
+#pragma unroll
+    for (int k = 0; k < WPR; ++k) w[q][k] = row >= 0 ? scr[((int64_t)row * WPR + k) * ns + sl] : 0u;
+  };
+#pragma unroll
+  for (int q = 0; q < PF; ++q) load(q, i - q);
+  for (;;) {
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      int from;
+      for (;;) {
+        uint32_t x = w[q][0];
+        if (WDIR > 1 && c >= 16) x = w[q][WDIR > 1 ? 1 : 0];
+        if (WDIR > 2 && c >= 32) x = w[q][WDIR > 2 ? 2 : 0];
+        from = (x >> ((2 * c) & 31)) & 3;
+        emit(i, c, w[q], from);
+        if (from != LEFT) break;
+        if (--c < 0) return;
+      }
+      if (from == TOP) ++c;
+      if (--i < 0 || c >= BW) return;
+      load(q, i - (PF - 1));
+    }
+  }
+}
+
 // BWT > 0: the band width 2I + 1 as a constant, so that the row arrays live in registers;
-// BWT = 0: any width up to kMaxBand (arrays in local memory).  CM: 0 nucleotide, 1 colour
+// BWT = 0: any width up to kMaxBand (arrays in local memory).  ctab: the table of colour_step.  CM: 0 nucleotide, 1 colour
 // space (the colour state machine compiled in), -1 either (sp.colour); the kernel's CM = 2 runs
 // the packed nucleotide form below (align_one_nuc).
 // A candidate whose running abort bound falls below the replay's threshold stops at that row:
@@ -133,7 +193,7 @@ struct BandWindow {
 template <int BWT, int CM>
 __device__ __forceinline__ int align_one(const ReadsDev& rd, const ScoreParams& sp, const uint8_t* __restrict__ genome,
                                          const uint8_t* __restrict__ mask, int64_t slot, int64_t sl, int64_t ns,
-                                         const PassBuffers& pb) {
+                                         const PassBuffers& pb, const uint8_t* ctab) {
   constexpr int NB = BWT > 0 ? BWT : kMaxBand;
   const int r = pb.p_read[slot];
   // the first round, and a launch without rounds, stop at -t only: pb.thr holds the read's
@@ -193,49 +253,27 @@ __device__ __forceinline__ int align_one(const ReadsDev& rd, const ScoreParams& 
       const int csc = sc[c], cst = stt[c];
       const int tsc = c + 1 < BW ? sc[c + 1] : kMinScore;
       const int tst = c + 1 < BW ? stt[c + 1] : st_make(3, I, 0, 0, 0);
-      int ms = s0;
+      int ms = s0, step = 0;
       if (colour) {
-        const int prev = st_chk(cst), cmp = prev ^ chk0;
-        if (prev && (cmp == 0 || cmp == st_ac(cst)) && s0 != kMinScore && s0 < 0) ms = -2 * s0;
+        step = ctab[(cst >> 9) | (chk0 << 7) | (q << 9)];
+        if ((step & 0x80) && s0 != kMinScore && s0 < 0) ms = -2 * s0;
       }
       int score = csc + ms, it = 0, tmp;
       if (st_ind(tst) < I && (tmp = tsc + ((st_from(tst) ^ 2) ? sp.gap_open : sp.gap_ext)) > score) { it = 1; score = tmp; }
       if (st_ind(lst) < I && (tmp = lsc + ((st_from(lst) ^ 1) ? sp.gap_open : sp.gap_ext)) > score) { it = 2; score = tmp; }
-      int from = 3, ind, chk = chk0, ac = ac0, fr = fr0;
-      if (it == 0) {
-        ind = st_ind(cst);
-        if (colour) {
-          const int cchk = st_chk(cst), cac = st_ac(cst), cfr = st_fr(cst);
-          chk = chk0 ^ cchk;
-          if (cchk != chk) {
-            if (cchk == 0) { ac = chk; fr = q; }
-            else if (chk == cac) { ac = 0; chk = 0; fr = 0; }
-            else if (chk == 0) { if (cfr - 1 > 0) { ac = cac; fr = cfr - 1; } else { ac = 0; fr = 0; } }
-            else { if (cfr - 1 > 0) { ac = cac; fr = cfr - 1; } else { ac = chk; fr = q; } }
-          } else {
-            if (cac != 0) {
-              if (cfr - 1 > 0) {
-                if (chk == 0) { ac = 0; fr = 0; } else { ac = cac; fr = cfr - 1; }
-              }
-            } else { chk = 0; ac = 0; fr = 0; }
-          }
-        }
-      } else if (it == 1) {
-        from = 2;
-        ind = st_ind(tst) + 1;
-        if (colour) {
-          chk = st_chk(tst) ^ rc;
-          if (st_fr(tst) - 1 > 0) { fr = st_fr(tst) - 1; ac = st_ac(cst); }
-        }
+      // the state after a corner, or after a gap: one more indel, the gap's own checksum, and the
+      // source's freshness less one while it lasts
+      const int gst = it == 1 ? tst : lst;
+      int nst;
+      if (colour) {
+        const bool fresh = st_fr(gst) > 1;
+        const int gap = st_make(it == 1 ? 2 : 1, st_ind(gst) + 1, st_chk(gst) ^ (it == 1 ? rc : f),
+                                fresh ? st_ac(cst) : ac0, fresh ? st_fr(gst) - 1 : fr0);
+        nst = it == 0 ? (3 | (cst & 0x1FC) | ((step & 0x7F) << 9)) : gap;
       } else {
-        from = 1;
-        ind = st_ind(lst) + 1;
-        if (colour) {
-          chk = st_chk(lst) ^ f;
-          if (st_fr(lst) - 1 > 0) { fr = st_fr(lst) - 1; ac = st_ac(cst); }
-        }
+        nst = it == 0 ? (3 | (cst & 0x1FC)) : (3 - it) | ((st_ind(gst) + 1) << 2);
       }
-      const int nst = st_make(from, ind, chk, ac, fr);
+      const int from = nst & 3;
       sc[c] = score;
       stt[c] = nst;
       lsc = score;
@@ -264,39 +302,45 @@ __device__ __forceinline__ int align_one(const ReadsDev& rd, const ScoreParams& 
   int i0 = bi, j0 = bj, tl = 0;
   uint8_t* tb = pb.a_tb + slot * pb.tbs;
   if (bi >= 0 && bnd >= thr && best > thr) {
-    int i = bi, c = bj - bi, colr = 0;
+    int colr = 0;
     uint8_t cur = 0;
-    while (i >= 0 && i < L && c >= 0 && c < BW) {
-      const int j = i + c;
-      i0 = i;
-      j0 = j;
-      const uint32_t wdir = scr[((int64_t)i * wpr + ((2 * c) >> 5)) * ns + sl];
-      const int from = (wdir >> ((2 * c) & 31)) & 3;
-      const int rc = code_at(rdc, i);
-      int op;
-      if (from == 2) op = 0xC | rc;
-      else if (from == 1) op = 0x1;
-      else {
-        const int f = code_at(genome, (int64_t)win + j);
-        if (rc != f) {
-          if (!colour) op = 0x4 | rc;
-          else {
-            bool adj = false;
-            if (i != 0 && j != 0) {
-              const uint32_t wcol = scr[((int64_t)i * wpr + wpr_dir + (c >> 5)) * ns + sl];
-              adj = (wcol >> (c & 31)) & 1u;
-            }
-            if (colr || adj) { op = 0x8 | rc; colr ^= rc ^ f; }
-            else op = 0x4 | rc;
-          }
-        } else op = 0x3;
-      }
+    auto put = [&](int op) {
       if (tl & 1) { cur |= (uint8_t)op; tb[tl >> 1] = cur; }
       else { cur = (uint8_t)(op << 4); tb[tl >> 1] = cur; }
       tl++;
-      if (from == 2) { i--; c++; }
-      else if (from == 1) { c--; }
-      else { i--; }
+    };
+    // one cell: its operation; adj: its pair score was made positive by the SNP adjustment
+    auto cell = [&](int i, int c, int from, bool adj) {
+      const int j = i + c;
+      i0 = i;
+      j0 = j;
+      const int rc = code_at(rdc, i);
+      if (from == 2) { put(0xC | rc); return; }
+      if (from == 1) { put(0x1); return; }
+      const int f = code_at(genome, (int64_t)win + j);
+      if (rc == f) put(0x3);
+      else if (!colour || !(colr || (adj && i != 0 && j != 0))) put(0x4 | rc);
+      else { put(0x8 | rc); colr ^= rc ^ f; }
+    };
+    if constexpr (BWT > 0) {
+      constexpr int WD = (2 * BWT + 31) / 32, WC = CM == 0 ? 0 : (BWT + 31) / 32;
+      trace_rows<WD + WC, WD, 1, 2>(scr, ns, sl, bi, bj - bi, BW, [&](int i, int c, const uint32_t* w, int from) {
+        uint32_t x = 0;
+        if (WC > 0) x = w[WC > 0 ? WD : 0];
+        if (WC > 1 && c >= 32) x = w[WC > 1 ? WD + 1 : 0];
+        cell(i, c, from, WC > 0 && ((x >> (c & 31)) & 1u));
+      });
+    } else {
+      int i = bi, c = bj - bi;
+      while (i >= 0 && i < L && c >= 0 && c < BW) {
+        const uint32_t wdir = scr[((int64_t)i * wpr + ((2 * c) >> 5)) * ns + sl];
+        const int from = (wdir >> ((2 * c) & 31)) & 3;
+        const bool adj = colour && ((scr[((int64_t)i * wpr + wpr_dir + (c >> 5)) * ns + sl] >> (c & 31)) & 1u);
+        cell(i, c, from, adj);
+        if (from == 2) { i--; c++; }
+        else if (from == 1) { c--; }
+        else { i--; }
+      }
     }
   }
   pb.a_tblen[slot] = tl;
@@ -469,14 +513,12 @@ __device__ __forceinline__ int align_one_nuc(const ReadsDev& rd, const ScorePara
   int i0 = bi, j0 = bj, tl = 0;
   uint8_t* tb = pb.a_tb + slot * pb.tbs;
   if (bi >= 0 && bnd >= thr && best > thr) {  // alignment.c:642-734
-    int i = bi, c = bj - bi;
     uint8_t cur = 0;
-    while (i >= 0 && i < L && c >= 0 && c < BW) {
+    // directions: 2 corner, 1 top, 0 left
+    trace_rows<wpr, wpr, 0, 1>(scr, ns, sl, bi, bj - bi, BW, [&](int i, int c, const uint32_t*, int from) {
       const int j = i + c;
       i0 = i;
       j0 = j;
-      const uint32_t wdir = scr[((int64_t)i * wpr + ((2 * c) >> 5)) * ns + sl];
-      const int from = (wdir >> ((2 * c) & 31)) & 3;  // 2 corner, 1 top, 0 left
       const int rc = code_at(rdc, i);
       int op;
       if (from == 1) op = 0xC | rc;
@@ -485,10 +527,7 @@ __device__ __forceinline__ int align_one_nuc(const ReadsDev& rd, const ScorePara
       if (tl & 1) { cur |= (uint8_t)op; tb[tl >> 1] = cur; }
       else { cur = (uint8_t)(op << 4); tb[tl >> 1] = cur; }
       tl++;
-      if (from == 1) { i--; c++; }
-      else if (from == 0) { c--; }
-      else { i--; }
-    }
+    });
   }
   pb.a_tblen[slot] = tl;
   pb.a_pos[slot * 4 + 0] = (int16_t)bi;
@@ -502,10 +541,22 @@ __device__ __forceinline__ int align_one_nuc(const ReadsDev& rd, const ScorePara
 // pb.cursor a persistent grid whose warps take the next 32 slots from the cursor (the slot
 // count read from pb.npass_dev when it is given; scratch column = the thread's index in the
 // grid, so the scratch holds align_workers() columns).
+// whether any code of [a, b) is masked
+__device__ __forceinline__ bool window_masked(const uint8_t* __restrict__ mask, int64_t a, int64_t b) {
+  unsigned any = 0;
+  for (int64_t k = a >> 2; k <= (b - 1) >> 2; ++k) {
+    unsigned x = mask[k];
+    if (k == a >> 2) x &= 0xFFu << (2 * (a & 3));
+    if (k == (b - 1) >> 2) x &= 0xFFu >> (6 - 2 * ((b - 1) & 3));
+    any |= x;
+  }
+  return any != 0;
+}
+
 // Resident blocks of 128 threads per SM the registers are bounded for: the packed form holds about
 // BWT registers of cells, the general one (scores and states apart) twice that.
 constexpr int align_blocks(int bw, int cm) {
-  return bw <= 0 ? 1 : cm == 2 ? (bw <= 15 ? 7 : bw <= 23 ? 6 : bw <= 31 ? 5 : 4) : (bw <= 15 ? 5 : bw <= 31 ? 4 : 3);
+  return bw <= 0 ? 1 : cm == 3 ? 2 : cm == 2 ? (bw <= 15 ? 7 : bw <= 23 ? 6 : bw <= 31 ? 5 : 4) : (bw <= 15 ? 5 : bw <= 31 ? 4 : 3);
 }
 
 template <int BWT, int CM>
@@ -513,6 +564,11 @@ __global__ void __launch_bounds__(128, align_blocks(BWT, CM)) align_kernel(Reads
                                                     const uint8_t* __restrict__ genome,
                                                     const uint8_t* __restrict__ mask, int64_t slot0, int64_t nslots,
                                                     PassBuffers pb) {
+  __shared__ uint8_t ctab[CM == 1 || CM == -1 ? kColourTable : 1];
+  if (CM == 1 || CM == -1) {
+    for (int k = threadIdx.x; k < kColourTable; k += blockDim.x) ctab[k] = colour_step(k);
+    __syncthreads();
+  }
   // one call site of align_one (its band code is large and fully unrolled)
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool steal = pb.cursor != nullptr;
@@ -534,10 +590,19 @@ __global__ void __launch_bounds__(128, align_blocks(BWT, CM)) align_kernel(Reads
     }
     if (s < n) {
       const int64_t slot = pb.round_slots ? (int64_t)pb.round_slots[s] : slot0 + s;
-      if constexpr (CM == 2)
+      if constexpr (CM == 2) {
         rows += (unsigned long long)align_one_nuc<BWT>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb);
-      else
-        rows += (unsigned long long)align_one<BWT, CM>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb);
+      } else if constexpr (CM == 3) {
+        // every cell exact: without masked codes no cell comes near the packed form's floor
+        const int r = pb.p_read[slot];
+        const int64_t win = max(pb.p_diag[slot] - sp.I, -sp.Is);
+        if (window_masked(mask, win, win + rd.lengths[r] + 2 * sp.I))
+          rows += (unsigned long long)align_one<BWT, 0>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb, ctab);
+        else
+          rows += (unsigned long long)align_one_nuc<BWT>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb);
+      } else {
+        rows += (unsigned long long)align_one<BWT, CM>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb, ctab);
+      }
     }
     if (!steal) break;
     s += 32;
@@ -552,7 +617,11 @@ __global__ void __launch_bounds__(128, align_blocks(BWT, CM)) align_kernel(Reads
 // memory ran -i 5 at 50 GCUPS, a twentieth of the packed form's rate); the others the widths of the
 // filter's own limits and of -i 20.
 static const void* align_kernel_of(const ScoreParams& sp) {
-  if (sp.packed) {
+  if (sp.packed == 2) {
+#define SG_ALIGN(BW) case BW: return (const void*)align_kernel<BW, 3>;
+    switch (2 * sp.I + 1) { SG_ALIGN(7) SG_ALIGN(11) SG_ALIGN(15) SG_ALIGN(21) SG_ALIGN(31) SG_ALIGN(41) }
+#undef SG_ALIGN
+  } else if (sp.packed) {
 #define SG_ALIGN(BW) case BW: return (const void*)align_kernel<BW, 2>;
     switch (2 * sp.I + 1) {
       SG_ALIGN(3) SG_ALIGN(5) SG_ALIGN(7) SG_ALIGN(9) SG_ALIGN(11) SG_ALIGN(13) SG_ALIGN(15) SG_ALIGN(17)
@@ -565,6 +634,7 @@ static const void* align_kernel_of(const ScoreParams& sp) {
   case BW: return sp.colour ? (const void*)align_kernel<BW, 1> : (const void*)align_kernel<BW, 0>;
   switch (2 * sp.I + 1) {
     SG_ALIGN(7)
+    SG_ALIGN(11)
     SG_ALIGN(15)
     SG_ALIGN(31)
     SG_ALIGN(41)
@@ -583,9 +653,11 @@ void launch_align(const ReadsDev& r, const ScoreParams& sp, const uint8_t* genom
                   cudaStream_t st) {
   if (nslots <= 0) return;
   const void* k = align_kernel_of(sp);
-  const unsigned blocks = (unsigned)(pb.cursor ? align_workers(nslots, sp) / 128 : (nslots + 127) / 128);
+  // one slot per thread: few slots as warps on as many SMs as there are
+  const int threads = !pb.cursor && nslots <= 148 * 64 ? 32 : 128;
+  const unsigned blocks = (unsigned)(pb.cursor ? align_workers(nslots, sp) / 128 : (nslots + threads - 1) / threads);
   void* args[] = {(void*)&r, (void*)&sp, (void*)&genome, (void*)&mask, (void*)&slot0, (void*)&nslots, (void*)&pb};
-  cudaLaunchKernel(k, dim3(blocks), dim3(128), args, 0, st);  // errors surface at the caller's next check
+  cudaLaunchKernel(k, dim3(blocks), dim3(threads), args, 0, st);  // errors surface at the caller's next check
 }
 
 // ------------------------------------------------------------------------------ replay

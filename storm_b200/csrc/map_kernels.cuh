@@ -18,7 +18,9 @@ struct ScoreParams {
   int min_score;      // -t
   // the packed nucleotide alignment (align_one_nuc): used when `packed`; its constants come
   // through the kernel parameters so that the multiply-adds stay multiply-adds
-  int packed;
+  // (1: in every window; 2, the unit entry points: in windows without masked codes; small: its scores
+  // allow it)
+  int packed, small;
   uint32_t one;       // 1
   uint32_t open1;     // (gap_open << 13) + 1
   uint32_t open1_tc;  // open1 + (1 << 11) - (1 << 12): a corner-labelled cell as a top gap source

@@ -574,6 +574,7 @@ __global__ void __launch_bounds__(128, align_blocks(BWT, CM)) align_kernel(Reads
   const bool steal = pb.cursor != nullptr;
   int64_t n = steal && pb.npass_dev ? *pb.npass_dev : nslots;
   if (pb.round_slots) n = (int64_t)*pb.round_count;  // with rounds: round_slots[0 .. n)
+  if (n <= pb.wave) return;                          // align_wave_kernel's
   const int64_t ns = steal ? (int64_t)gridDim.x * blockDim.x : nslots;
   const int lane = threadIdx.x & 31;
   const int take = pb.steal >= 32 ? pb.steal & ~31 : 32;
@@ -646,6 +647,188 @@ static const void* align_kernel_of(const ScoreParams& sp) {
 int64_t align_workers(int64_t nslots, const ScoreParams& sp) {
   const int64_t g = resident_grid_of(align_kernel_of(sp), 128, 0) * 128;
   return std::min<int64_t>(g, (nslots + 127) / 128 * 128);
+}
+
+// ------------------------------------------------------------------------------ align, few slots
+
+// The alignment of align_one by a warp per slot, for calls with so few slots that a thread each leaves
+// the GPU idle while every thread walks its rows cell by cell: lane c holds cell c of the band and
+// is at row i at time 2i + c, when the cell to its left (lane c - 1, same row) and the one above
+// (lane c + 1, the row before) are one time step old.  The row maximum travels along with the row.
+// Directions stay in shared memory (a byte per cell: direction, bit 2 the SNP adjustment), where lane
+// 0 walks them back.  Every lane runs the same instructions in every step (those whose turn it is not
+// discard the result).  2L + 2I + 1 steps of about 60 instructions, against L (2I + 1) cells of 25 to 40:
+// 800 windows of 101 codes take 75 us at -i 15 where a thread each takes 148, 88 us in colours at -i 7
+// against 260 (the whole call).  The chain of a step (shuffle, sums, state, next row's codes) is what
+// bounds it: 31 % of the issue slots are taken with 5 warps an SM.
+template <bool COLOUR>
+__global__ void __launch_bounds__(32) align_wave_kernel(ReadsDev rd, ScoreParams sp, const uint8_t* __restrict__ genome,
+                                                        const uint8_t* __restrict__ mask, int64_t slot0, int64_t nslots,
+                                                        PassBuffers pb, int maxL) {
+  extern __shared__ __align__(16) uint8_t wsm[];
+  __shared__ uint8_t ctab[COLOUR ? kColourTable : 1];
+  const int lane = threadIdx.x;
+  const int64_t n = pb.npass_dev ? *pb.npass_dev : nslots;
+  if (n > wave_slots(sp) || (int64_t)blockIdx.x >= n) return;
+  const int I = sp.I, BW = 2 * I + 1;
+  constexpr bool colour = COLOUR;
+  int2* const pair_s = reinterpret_cast<int2*>(wsm);       // per read position: match and mismatch score
+  uint8_t* const dir = wsm + sizeof(int2) * maxL;          // 32 per row
+  uint8_t* const rc_s = dir + 32 * maxL;                   // per read position: code | level << 2
+  uint8_t* const gc_s = rc_s + maxL;                       // per window position: code | masked << 2
+  if (colour) {
+    for (int k = lane; k < kColourTable; k += 32) ctab[k] = colour_step(k);
+    __syncwarp();
+  }
+  const int mbest = sp.pair[0][3];
+  unsigned long long rows = 0;
+  for (int64_t s = blockIdx.x; s < n; s += gridDim.x) {
+    const int64_t slot = slot0 + s;
+    const int r = pb.p_read[slot];
+    const int L = rd.lengths[r];
+    const int64_t win = max(pb.p_diag[slot] - I, -sp.Is);  // run.c:667
+    const uint8_t* rdc = rd.codes + (int64_t)r * rd.cstride;
+    const uint8_t* rdq = rd.levels ? rd.levels + (int64_t)r * rd.lstride : nullptr;
+    __syncwarp();
+    for (int i = lane; i < L; i += 32) {
+      const int q = rdq ? code_at(rdq, i) : 3;
+      rc_s[i] = (uint8_t)(code_at(rdc, i) | q << 2);
+      pair_s[i] = make_int2(sp.pair[0][q], sp.pair[1][q]);
+    }
+    for (int i = lane; i < L + 2 * I; i += 32)
+      gc_s[i] = (uint8_t)(code_at(genome, win + i) | (code_at(mask, win + i) ? 4 : 0));
+    __syncwarp();
+    // row 0
+    int sc = kMinScore, st = st_make(3, 0, 0, 0, 0);
+    if (lane < BW) {
+      const int x = rc_s[0], rc = x & 3, q = x >> 2, g = gc_s[lane], f = g & 3;
+      int chk = 0;
+      if (!(g & 4)) {
+        chk = colour ? (rc ^ f) : 0;
+        sc = sp.pair[colour ? (chk ? 1 : 0) : (rc != f)][q];
+      }
+      st = st_make(3, 0, chk, chk, (colour && chk) ? q : 0);
+      dir[lane] = 3;
+    }
+    long long bound = 0x7fffffffLL;
+    int best_possible = (colour ? (L - 2) : L) * mbest;
+    int mol = kMinScore;  // of the row this lane was last at, its cells up to this lane's
+    const int last_t = 2 * (L - 1) + BW - 1;
+    const int border = st_make(3, I, 0, 0, 0);
+    const bool first = lane == 0, last = lane == BW - 1, inband = lane < BW;
+    int i = 1;  // the row this lane is at next, at time 2i + lane; its read and window codes
+    int x = rc_s[min(1, L - 1)], g = gc_s[min(1 + lane, L + 2 * I - 1)];
+    int2 pr = pair_s[min(1, L - 1)];
+    for (int t = 2; t <= last_t; ++t) {
+      int lsc = __shfl_up_sync(0xffffffffu, sc, 1), lst = __shfl_up_sync(0xffffffffu, st, 1);
+      int tsc = __shfl_down_sync(0xffffffffu, sc, 1), tst = __shfl_down_sync(0xffffffffu, st, 1);
+      int lmol = __shfl_up_sync(0xffffffffu, mol, 1);
+      if (first) { lsc = kMinScore; lst = border; lmol = kMinScore; }
+      if (last) { tsc = kMinScore; tst = border; }
+      const bool now = inband && t == 2 * i + lane && i < L;
+      const int rc = x & 3, q = x >> 2, f = g & 3;
+      const bool masked = (g & 4) != 0;
+      const int chk0 = colour && !masked ? rc ^ f : 0;
+      const int s0 = masked ? kMinScore : rc != f ? pr.y : pr.x;
+      int ms = s0, step = 0;
+      if (colour) {
+        step = ctab[(st >> 9) | (chk0 << 7) | (q << 9)];
+        ms = (step & 0x80) && !masked && s0 < 0 ? -2 * s0 : s0;
+      }
+      const int cs = sc + ms;
+      const int ts = tsc + (st_from(tst) == 2 ? sp.gap_ext : sp.gap_open);
+      const int ls = lsc + (st_from(lst) == 1 ? sp.gap_ext : sp.gap_open);
+      const bool top = st_ind(tst) < I && ts > cs;
+      const int m1 = top ? ts : cs;
+      const bool left = st_ind(lst) < I && ls > m1;
+      const int score = left ? ls : m1;
+      const int gst = left ? lst : tst;
+      int gap = (left ? 1 : 2) | ((st_ind(gst) + 1) << 2);
+      int cor = 3 | (st & 0x1FC);
+      if (colour) {
+        const bool fresh = st_fr(gst) > 1;
+        const int ac = fresh ? st_ac(st) : chk0, fr = fresh ? st_fr(gst) - 1 : chk0 ? q : 0;
+        gap |= ((st_chk(gst) ^ (left ? f : rc)) << 9) | (ac << 11) | (fr << 13);
+        cor |= (step & 0x7F) << 9;
+      }
+      const bool corner = !top && !left;
+      const int nst = corner ? cor : gap;
+      if (now) {
+        st = nst;
+        sc = score;
+        dir[32 * i + lane] = (uint8_t)((nst & 3) | (colour && corner && ms > 0 ? 4 : 0));
+        mol = max(lmol, score);
+        if (last) {  // the row is complete
+          bound = min(bound, (long long)mol + best_possible);
+          best_possible -= mbest;
+        }
+        ++i;
+        const int in = min(i, L - 1);
+        x = rc_s[in];
+        pr = pair_s[in];
+        g = gc_s[in + lane];
+      }
+    }
+    __syncwarp();
+    // the first of the largest cells of the last row
+    const int top = __reduce_max_sync(0xffffffffu, lane < BW ? sc : kMinScore);
+    const unsigned at = __ballot_sync(0xffffffffu, lane < BW && sc == top);
+    const int bi = top > kMinScore ? L - 1 : -1, bc = top > kMinScore ? __ffs(at) - 1 : 0;
+    const int32_t bnd = (int32_t)__shfl_sync(0xffffffffu, (int)bound, BW - 1);
+    if (lane == 0) {
+      const int bj = bi < 0 ? -1 : L - 1 + bc;
+      int i0 = bi, j0 = bj, tl = 0;
+      if (bi >= 0 && bnd >= sp.min_score && top > sp.min_score) {
+        uint8_t* tb = pb.a_tb + slot * pb.tbs;
+        uint8_t cur = 0;
+        int c = bc, colr = 0;
+        i = bi;
+        while (i >= 0 && c >= 0 && c < BW) {
+          const int d = dir[32 * i + c], from = d & 3, rc = rc_s[i] & 3, f = gc_s[i + c] & 3;
+          i0 = i;
+          j0 = i + c;
+          int op;
+          if (from == 2) op = 0xC | rc;
+          else if (from == 1) op = 0x1;
+          else if (rc == f) op = 0x3;
+          else if (!colour || !(colr || ((d & 4) && i != 0 && i + c != 0))) op = 0x4 | rc;
+          else { op = 0x8 | rc; colr ^= rc ^ f; }
+          if (tl & 1) { cur |= (uint8_t)op; tb[tl >> 1] = cur; }
+          else { cur = (uint8_t)(op << 4); tb[tl >> 1] = cur; }
+          tl++;
+          if (from == 2) { i--; c++; }
+          else if (from == 1) { c--; }
+          else { i--; }
+        }
+      }
+      pb.a_score[slot] = top;
+      pb.a_bound[slot] = bnd;
+      pb.a_tblen[slot] = tl;
+      pb.a_pos[slot * 4 + 0] = (int16_t)bi;
+      pb.a_pos[slot * 4 + 1] = (int16_t)bj;
+      pb.a_pos[slot * 4 + 2] = (int16_t)i0;
+      pb.a_pos[slot * 4 + 3] = (int16_t)j0;
+    }
+    rows += (unsigned long long)L;
+  }
+  if (pb.cells && lane == 0 && rows) atomicAdd(pb.cells, rows * (unsigned long long)BW);
+}
+
+void launch_align_wave(const ReadsDev& r, const ScoreParams& sp, const uint8_t* genome, const uint8_t* mask,
+                       int64_t slot0, int64_t nslots, PassBuffers& pb, int maxL, cudaStream_t st) {
+  if (nslots <= 0) return;
+  const size_t smem = (size_t)maxL * (33 + sizeof(int2)) + maxL + 2 * sp.I + 32;
+  const int most = STORMGPU_MAX_READ_LEN * (34 + (int)sizeof(int2)) + 64;
+  // a graph launches it for a whole list capacity
+  const unsigned grid = (unsigned)std::min<int64_t>(nslots, wave_slots(sp));
+  if (!grid) return;
+  if (sp.colour) {
+    set_smem_attribute_once(reinterpret_cast<const void*>(align_wave_kernel<true>), most);
+    align_wave_kernel<true><<<grid, 32, smem, st>>>(r, sp, genome, mask, slot0, nslots, pb, maxL);
+  } else {
+    set_smem_attribute_once(reinterpret_cast<const void*>(align_wave_kernel<false>), most);
+    align_wave_kernel<false><<<grid, 32, smem, st>>>(r, sp, genome, mask, slot0, nslots, pb, maxL);
+  }
 }
 
 void launch_align(const ReadsDev& r, const ScoreParams& sp, const uint8_t* genome,

@@ -75,6 +75,7 @@ struct PassBuffers {
   // align_workers() threads (scratch columns) taking slots from it
   unsigned long long* cursor;
   const int64_t* npass_dev;  // may be null; else the slot count is read from here
+  int wave;                  // with a cursor: up to so many slots are left to align_wave_kernel
   int steal;                 // with a cursor: slots a warp takes at a time, a multiple of 32 (0 = 32)
   // Rounds (all null for one round over every slot).  The candidates of a read are aligned in rounds:
   // each takes its next candidates that may still exceed the read's running threshold (see
@@ -103,6 +104,18 @@ void launch_init_results(int64_t n, stormgpu_hit* hits, uint8_t* mapped, uint8_t
 void launch_align(const ReadsDev& r, const ScoreParams& sp, const uint8_t* genome,
                   const uint8_t* mask, int64_t slot0, int64_t nslots, PassBuffers& pb,
                   cudaStream_t st);
+// The same by a warp per slot (no scratch, no rounds), for bands of at most 32 cells: every slot when
+// there are at most wave_slots() of them (read from pb.npass_dev when given), else none.  maxL: longest
+// read.  Up to so many slots the warp form is the faster one: it takes 75 to 100 us for up to 1,000
+// windows of 101 codes whatever the band (all at once) and about 35 us more per further 1,000, a thread
+// per slot the same time from 64 to 8,000 windows: 88 us and 111 us in nucleotides at -i 3 and 7 (crossing
+// near 1,300 and 2,200), 149 us at -i 15 (near 3,700), 190 us at -i 1; 223, 260, 432 and 735 us in colours.
+constexpr int wave_slots(const ScoreParams& sp) {
+  const int bw = 2 * sp.I + 1;
+  return bw > 32 ? 0 : !sp.colour && bw >= 7 && bw <= 15 ? 148 * 8 : 4096;
+}
+void launch_align_wave(const ReadsDev& r, const ScoreParams& sp, const uint8_t* genome, const uint8_t* mask,
+                       int64_t slot0, int64_t nslots, PassBuffers& pb, int maxL, cudaStream_t st);
 // scratch columns of a launch_align with a cursor (the threads of its persistent grid)
 int64_t align_workers(int64_t nslots, const ScoreParams& sp);
 // The candidates of a pass that are aligned, as the filter (and the score bound) left them: reads

@@ -633,8 +633,10 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const Graph
       pb.a_scratch = c->scratch.p;
       pb.cells = c->counters.p + 13;
       if (rounds == 1) {
+        pb.wave = wave_slots(sp);
+        if (pb.wave) launch_align_wave(rd, sp, R.d_codes, R.d_mask, 0, kept_cap, pb, P.maxL, st);
         launch_align(rd, sp, R.d_codes, R.d_mask, 0, kept_cap, pb, st);
-        launches++;
+        launches += pb.wave ? 2 : 1;
         SG_CUDA(rec(E[3]));
         launch_replay(n, sp, (int)ref_id, strand ? -1 : 1, pb, 0, P.out->hits, P.out->tb, P.out->tb_stride,
                       P.out->mapped, st);
@@ -988,7 +990,8 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
         pb.a_scratch = c->scratch.p;
         pb.cells = c->counters.p + 13;
         if (rounds == 1) {
-          launch_align(rd, sp, R.d_codes, R.d_mask, 0, nkept, pb, st);
+          if (nkept <= wave_slots(sp)) launch_align_wave(rd, sp, R.d_codes, R.d_mask, 0, nkept, pb, maxL, st);
+          else launch_align(rd, sp, R.d_codes, R.d_mask, 0, nkept, pb, st);
           launches++;
         } else {
           // rounds, each of the candidates the replay of the round before selected
@@ -1361,7 +1364,8 @@ extern "C" int stormgpu_align(const stormgpu_params* params, const uint8_t* read
   pb.tbs = tbs;
   SG_CUDA(cudaMemcpy(pb.p_read, zeros.data(), sizeof(int32_t) * nn, cudaMemcpyHostToDevice));
   SG_CUDA(cudaMemcpy(pb.p_diag, diag.data(), sizeof(int32_t) * nn, cudaMemcpyHostToDevice));
-  launch_align(rd, sp, gb, mb, 0, n, pb, 0);
+  if (n <= wave_slots(sp)) launch_align_wave(rd, sp, gb, mb, 0, n, pb, read_len, 0);
+  else launch_align(rd, sp, gb, mb, 0, n, pb, 0);
   SG_CUDA(cudaGetLastError());
   SG_CUDA(cudaDeviceSynchronize());
   if (n) {

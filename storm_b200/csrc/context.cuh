@@ -86,12 +86,11 @@ struct stormgpu_ctx {
   sg::DevBuf<stormgpu_hit> hits;
   sg::DevBuf<uint8_t> tb, mapped;
   // pass buffers
-  sg::DevBuf<int32_t> pstart, pcount, p_read, p_diag, big_list, big_h, small_list, small_h, big_count, huge_list,
+  sg::DevBuf<int32_t> pstart, pcount, p_read, p_diag, big_list, big_h, small_list, small_h, huge_list,
       huge_h;
-  sg::DevBuf<int64_t> scan_tmp64, foff;
+  sg::DevBuf<int64_t> foff;       // places of the selections' tiles
   sg::DevBuf<int32_t> fr, fd;
   sg::DevBuf<uint8_t> flag;       // pass byte per candidate
-  sg::DevBuf<uint32_t> flagw;     // pass bits, one word per 32 candidates
   sg::DevBuf<uint8_t> rexp;
   // score bound: passing candidates before it (p_read / p_diag hold those it keeps); read streams of
   // the banded core, its constants for the filter and the bound (band_set: computed for this
@@ -108,9 +107,8 @@ struct stormgpu_ctx {
   sg::DevBuf<uint8_t> a_tb;
   sg::DevBuf<uint32_t> scratch;
   // replay: two lists of reads with candidates left; alignment rounds: per-read threshold and range of
-  // the last selection, the round's slots; per round the counts of both lists
+  // the last selection, the round's slots
   sg::DevBuf<int32_t> active, thr, round_cur, round_slots;
-  sg::DevBuf<unsigned long long> rounds;
   sg::DevBuf<unsigned long long> counters;
   sg::DevBuf<uint32_t> ord, ord_tmp;  // length order of a mixed-length batch: sort keys and values, sort scratch
   cudaEvent_t ev[8];
@@ -122,20 +120,15 @@ struct stormgpu_ctx {
   // call: a batch that would exceed a pass's bounds at that density is cut up front instead of
   // after its gather
   double dens_cand = 0, dens_pass = 0;
-  // the same densities, and that of the aligned candidates, for the list sizes of a graph call: the
+  // the same densities, and that of the aligned candidates, for the list sizes of passes enqueued ahead: the
   // larger of the last call's and 0.9 x the value before it, so that calls of different densities
   // in turn (one read length after another) do not outgrow their lists each time
   double gdens_cand = 0, gdens_pass = 0, gdens_kept = 0;
-  // CUDA graph of the strand passes: on unless turned off (stormgpu_set_graphs, STORMGPU_GRAPHS=0)
-  // or broken (a capture or instantiation that failed turns it off for the context); the
-  // executable graph of the last call, updated in place by the next call of the same shape; its
-  // stage events; its device state (list sizes, status, sums of the counters)
+  // strand passes enqueued ahead, without a host wait between them: on unless turned off
+  // (stormgpu_set_graphs, STORMGPU_GRAPHS=0); their stage events
   bool graphs = true;
-  bool graph_broken = false;
-  cudaGraphExec_t gexec = nullptr;
   std::vector<cudaEvent_t> gev;
-  sg::DevBuf<unsigned long long> gstate;
-  // slice size (index positions) of the graph's launch for reads with the most positions: the
+  // slice size (index positions) of their launch for reads with the most positions: the
   // largest the host-synced passes needed so far
   int64_t huge_cap = 1 << 17;
   // genome_map placement
@@ -145,6 +138,7 @@ struct stormgpu_ctx {
 namespace sg {
 
 // One batch on c's stream (every pointer in reads / out on the device); synchronous.
-int map_device_impl(stormgpu_ctx* c, const stormgpu_reads* reads, stormgpu_results* out);
+// reads and results in device memory; lengths: the reads' lengths on the host, or null (then copied here)
+int map_device_impl(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, stormgpu_results* out);
 
 }  // namespace sg

@@ -25,6 +25,18 @@ namespace {
 
 using namespace sg;
 
+// A word of bits, counted as its number of set bits when scanned.
+struct BitWord {
+  uint32_t bits;
+  __host__ __device__ explicit operator int64_t() const {
+#if defined(__CUDA_ARCH__)
+    return __popc(bits);
+#else
+    return __builtin_popcount(bits);
+#endif
+  }
+};
+
 constexpr uint32_t kNoRank = 0xffffffffu;
 constexpr int32_t kPending = (int32_t)0xfefefefe;  // a rank not placed yet (a byte fill)
 constexpr int kCodes = 4;        // BASE_CODE_COUNT / COLOR_CODE_COUNT (codes.h:25-29)
@@ -496,7 +508,7 @@ extern "C" int stormgpu_genome_map_contextual(stormgpu_ctx* c, int32_t uniquenes
   if (!bits || !woff || !wtmp) return nomem();
   SG_CUDA(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * nwords, st));
   ctx_mark_kernel<<<grid_for(nm * 32, 256), 256, 0, st>>>(nm, M, bits);
-  exclusive_scan<PassWord, int64_t>(reinterpret_cast<const PassWord*>(bits), woff, nwords, woff + nwords, wtmp, st);
+  exclusive_scan<BitWord, int64_t>(reinterpret_cast<const BitWord*>(bits), woff, nwords, woff + nwords, wtmp, st);
   int64_t cov = 0;
   SG_CUDA(cudaMemcpyAsync(&cov, woff + nwords, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   SG_CUDA(cudaStreamSynchronize(st));

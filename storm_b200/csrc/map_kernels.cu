@@ -819,7 +819,7 @@ void launch_align_wave(const ReadsDev& r, const ScoreParams& sp, const uint8_t* 
   if (nslots <= 0) return;
   const size_t smem = (size_t)maxL * (33 + sizeof(int2)) + maxL + 2 * sp.I + 32;
   const int most = STORMGPU_MAX_READ_LEN * (34 + (int)sizeof(int2)) + 64;
-  // a graph launches it for a whole list capacity
+  // passes enqueued ahead launch it for a whole list capacity
   const unsigned grid = (unsigned)std::min<int64_t>(nslots, wave_slots(sp));
   if (!grid) return;
   if (sp.colour) {

@@ -92,7 +92,7 @@ struct Request {
 struct Slot {
   stormgpu_ctx* ws = nullptr;
   // candidates, passing and aligned candidates per unit of work weight of the densest pass of the last
-  // batch, per chain step (each step's seeds have their own): the sizes of a step's graph
+  // batch, per chain step (each step's seeds have their own): the list sizes of a step's passes
   double dens[16][5] = {};
   uint8_t* staging = nullptr;  // pinned host memory
   int64_t staging_cap = 0;
@@ -275,7 +275,7 @@ int run_chain(stormgpu_server* s, Slot* sl, Request* q, std::string& err) {
     const int ks = std::min(k, 15);
     double* dk = sl->dens[ks];
     ws->dens_cand = dk[0]; ws->dens_pass = dk[1]; ws->gdens_cand = dk[2]; ws->gdens_pass = dk[3]; ws->gdens_kept = dk[4];
-    if (const int rc = map_device_impl(ws, &r, &o)) return fail(rc);
+    if (const int rc = map_device_impl(ws, &r, k == 0 ? R.lengths : nullptr, &o)) return fail(rc);
     dk[0] = ws->dens_cand; dk[1] = ws->dens_pass; dk[2] = ws->gdens_cand; dk[3] = ws->gdens_pass; dk[4] = ws->gdens_kept;
     chain_scatter_kernel<<<grid_for(m), 256, 0, st>>>(m, cv.ids[cur], cv.hits, cv.tb, cv.mapped, tbs, k,
                                                       cv.hits_all, cv.tb_all, cv.mapped_all,

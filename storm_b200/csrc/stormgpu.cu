@@ -197,20 +197,18 @@ extern "C" void stormgpu_close(stormgpu_ctx* c) {
   c->mapped.release();
   c->pstart.release(); c->pcount.release(); c->p_read.release(); c->p_diag.release();
   c->big_list.release(); c->big_h.release(); c->small_list.release(); c->small_h.release();
-  c->big_count.release(); c->huge_list.release(); c->huge_h.release(); c->gstate.release();
-  if (c->gexec) cudaGraphExecDestroy(c->gexec);
+  c->huge_list.release(); c->huge_h.release(); 
   for (auto& e : c->gev) cudaEventDestroy(e);
-  c->scan_tmp64.release();
   c->a_score.release(); c->a_bound.release(); c->a_tblen.release(); c->big_tmp.release();
   c->a_pos.release(); c->a_tb.release(); c->scratch.release(); c->counters.release();
-  c->foff.release(); c->fr.release(); c->fd.release(); c->flag.release(); c->flagw.release();
+  c->foff.release(); c->fr.release(); c->fd.release(); c->flag.release();
   c->rexp.release();
   c->q_read.release(); c->q_diag.release(); c->q_ub.release(); c->k_ub.release(); c->p_ub.release();
   c->k_diag.release(); c->long_list.release(); c->bstream.release(); c->wstream.release();
   c->gm_k0.release(); c->gm_v0.release(); c->gm_k1.release(); c->gm_v1.release(); c->gm_tmp.release();
   c->gm_base.release();
   c->ord.release(); c->ord_tmp.release();
-  c->thr.release(); c->active.release(); c->round_cur.release(); c->round_slots.release(); c->rounds.release();
+  c->thr.release(); c->active.release(); c->round_cur.release(); c->round_slots.release();
   for (auto& e : c->ev) cudaEventDestroy(e);
   for (auto& e : c->rev) cudaEventDestroy(e);
   cudaStreamDestroy(c->st);
@@ -304,40 +302,47 @@ static __global__ void length_keys_kernel(const int16_t* __restrict__ lengths, i
 // Work weight of a read: its seed positions, about L - 15 (candidates grow with them).
 static inline double read_weight(int L) { return L > 16 ? (double)(L - 15) : 1.0; }
 
-// ------------------------------------------------------------------------------ graph passes
+// ------------------------------------------------------------------------------ passes ahead
 //
-// Every strand pass of a call as one CUDA graph: the lists are sized up front (from the densest
-// pass of the last call, +25 %), every launch takes its list size from device memory, and a
-// one-thread gate after the gather and after the filter writes the size the next stages take,
-// or 0 with a status when a list would not fit (or the batch must be cut): the passes from there
-// on then do nothing, and the host, reading the status once after the graph, maps the call
-// again with the host-synced passes.
+// Every strand pass of a call enqueued without waiting for the device: the lists are sized up front
+// (from the densest pass of the last calls, +25 %), every launch takes its list size from device
+// memory, and a gate after the gather, the filter and the score bound writes the size the next stages
+// take, or 0 with a status when a list would not fit (or the batch must be cut): the passes from there
+// on then do nothing, and the host, reading the status once at the end, maps the call again with the
+// host-synced passes.
+//
+// Plain launches, not a graph: a graph has to be captured again for every batch (its sizes and pointers
+// are the batch's), which takes the host as long as launching, and the device waits for it; a batch of
+// another size often has another number of scan launches and a new executable graph (a chain served in
+// batches of 100 to 4,000 reads: 21 ms with graphs, 15 with plain launches; 400,000 reads: the same).
 
-constexpr int kGraphRetry = 2;
+constexpr int kHostSynced = 2;
 
-// words of the graph's device state (c->gstate)
+// Words of c->counters.  The stage counters, which passes enqueued ahead add up; what a pass starts
+// with zeroed; and their state.
 enum : int {
-  kGsCand = 0,    // candidates the filter of the current pass takes (0: skipped)
-  kGsPass,        // passing candidates the score bound of the current pass takes (0: skipped)
-  kGsStatus,      // 1: a list outgrew its capacity, 2: the batch must be cut, 4: too many passing
-  kGsLookups,     // sums over the passes of the stage counters
-  kGsPositions,
-  kGsCandidates,
-  kGsCells,
-  kGsBand,
-  kGsAlignCells,
-  kGsPassed,
-  kGsMaxCand,     // densest pass
+  kCntAlign = 1,   // band cells of the alignments ([2] to [6]: filter cells, index lookups, index positions,
+                   // candidates, band cells of the filter)
+  kCntSums = 7,
+  kCntPass = 7,    // [7] candidates listed, [8] list overflow, [9..15] work cursors, [16..] those of the rounds
+  kCntSelect = 24, // tickets of the two selections
+  kCntBig = 26,    // int32: reads on the gather's large, huge and small lists, and above the huge slices
+  kCntRounds = 28, // round_count, then int32 active_count, then the long list's count
+  kGsCand = 44,    // candidates the filter of the current pass takes (0: skipped)
+  kGsPass,         // passing candidates the score bound of the current pass takes (0: skipped)
+  kGsKept,         // candidates the alignment of the current pass takes (0: skipped)
+  kGsStatus,       // 1: a list outgrew its capacity, 2: the batch must be cut, 4: too many passing
+  kGsPassed,       // sums over the passes
+  kGsAligned,
+  kGsMaxCand,      // densest pass
   kGsMaxPass,
-  kGsKept,        // candidates the alignment of the current pass takes (0: skipped)
-  kGsAligned,     // their sum over the passes
   kGsMaxKept,
-  kGsWords = 16
+  kCounters = 56
 };
 
-static __global__ void gate_gather_kernel(const unsigned long long* __restrict__ counters,
-                                          const int32_t* __restrict__ big_count, int64_t cand_cap, int64_t cand_max,
-                                          unsigned long long* __restrict__ gs) {
+static __global__ void gate_gather_kernel(const unsigned long long* __restrict__ counters, int64_t cand_cap,
+                                          int64_t cand_max, unsigned long long* __restrict__ gs) {
+  const int32_t* big_count = reinterpret_cast<const int32_t*>(counters + kCntBig);
   const unsigned long long u = counters[7];
   unsigned long long s = gs[kGsStatus];
   // candidate list overflow, a read above the slices of the last gather launch, or a full list
@@ -345,41 +350,7 @@ static __global__ void gate_gather_kernel(const unsigned long long* __restrict__
   if (u > (unsigned long long)cand_max) s |= 2;
   gs[kGsStatus] = s;
   gs[kGsCand] = s ? 0 : u;
-  gs[kGsLookups] += counters[3];
-  gs[kGsPositions] += counters[4];
   if (u > gs[kGsMaxCand]) gs[kGsMaxCand] = u;
-}
-
-static __global__ void gate_filter_kernel(const int64_t* __restrict__ total, int64_t pass_cap, int64_t pass_max,
-                                          int64_t nreads, unsigned long long* __restrict__ gs) {
-  const int64_t p = *total;
-  unsigned long long s = gs[kGsStatus];
-  if (p > pass_cap) s |= 4;
-  if (p > pass_max && nreads > 1) s |= 2;
-  gs[kGsStatus] = s;
-  gs[kGsPass] = s ? 0 : (unsigned long long)p;
-  if (!s) gs[kGsPassed] += (unsigned long long)p;
-  if ((unsigned long long)p > gs[kGsMaxPass]) gs[kGsMaxPass] = (unsigned long long)p;
-}
-
-// total: candidates the score bound kept
-static __global__ void gate_bound_kernel(const int64_t* __restrict__ total, int64_t kept_cap,
-                                         unsigned long long* __restrict__ gs) {
-  const int64_t p = *total;
-  unsigned long long s = gs[kGsStatus];
-  if (p > kept_cap) s |= 4;
-  gs[kGsStatus] = s;
-  gs[kGsKept] = s ? 0 : (unsigned long long)p;
-  if (!s) gs[kGsAligned] += (unsigned long long)p;
-  if ((unsigned long long)p > gs[kGsMaxKept]) gs[kGsMaxKept] = (unsigned long long)p;
-}
-
-static __global__ void pass_sums_kernel(const unsigned long long* __restrict__ counters,
-                                        unsigned long long* __restrict__ gs) {
-  gs[kGsCandidates] += counters[5];
-  gs[kGsCells] += counters[2];
-  gs[kGsBand] += counters[6];
-  gs[kGsAlignCells] += counters[13];
 }
 
 static void set_densities(stormgpu_ctx* c, double cand, double pass, double kept) {
@@ -449,7 +420,7 @@ static void launch_bound_pass(stormgpu_ctx* c, const PassSetup& P, const ReadsDe
 
 // Buffers of the replay's lists: two lists of active reads, and with rounds the round's slots.
 static int round_lists_grow(stormgpu_ctx* c, int64_t n, int64_t kept, int rounds) {
-  if (c->active.grow(2 * n) || c->long_list.grow(n) || c->rounds.grow(2 * kRoundCounts + 1)) return STORMGPU_ENOMEM;
+  if (c->active.grow(2 * n) || c->long_list.grow(n)) return STORMGPU_ENOMEM;
   if (rounds > 1 && (c->thr.grow(n) || c->round_cur.grow(2 * n) || c->round_slots.grow(kept))) return STORMGPU_ENOMEM;
   return 0;
 }
@@ -458,22 +429,20 @@ static int round_lists_grow(stormgpu_ctx* c, int64_t n, int64_t kept, int rounds
 static void round_buffers(stormgpu_ctx* c, int k, PassBuffers& pb) {
   const int64_t half = c->active.cap / 2;
   pb.round = k;
-  pb.round_count = c->rounds.p + k;
+  pb.round_count = c->counters.p + kCntRounds + k;  // zeroed with the counters of the pass
   pb.active = c->active.p + (k & 1 ? half : 0);
   pb.active_next = c->active.p + (k & 1 ? 0 : half);
-  pb.active_count = reinterpret_cast<int32_t*>(c->rounds.p + kRoundCounts) + k;
-  pb.cursor = c->counters.p + 16 + k;  // zeroed with the counters of the pass
+  pb.active_count = reinterpret_cast<int32_t*>(c->counters.p + kCntRounds + kRoundCounts) + k;
+  pb.cursor = c->counters.p + 16 + k;
 }
 
-static int setup_rounds(stormgpu_ctx* c, int rounds, PassBuffers& pb, cudaStream_t st) {
-  SG_CUDA(cudaMemsetAsync(c->rounds.p, 0, sizeof(unsigned long long) * (2 * kRoundCounts + 1), st));
+static void setup_rounds(stormgpu_ctx* c, int rounds, PassBuffers& pb) {
   round_buffers(c, 0, pb);
   if (rounds > 1) {
     pb.round_slots = c->round_slots.p;
     pb.round_cur = c->round_cur.p;
     pb.thr = c->thr.p;
   }
-  return 0;
 }
 
 static KeptList kept_list(stormgpu_ctx* c, const PassSetup& P, int64_t n, const int64_t* n_dev) {
@@ -483,39 +452,41 @@ static KeptList kept_list(stormgpu_ctx* c, const PassSetup& P, int64_t n, const 
   kl.diag = c->k_diag.p;
   kl.ub = P.bound_H ? c->k_ub.p : nullptr;
   kl.long_list = c->long_list.p;
-  kl.long_count = reinterpret_cast<int32_t*>(c->rounds.p + 2 * kRoundCounts);
+  kl.long_count = reinterpret_cast<int32_t*>(c->counters.p + kCntRounds + 2 * kRoundCounts);
   kl.sort_cap = c->tune.gather_warp_cap;  // more come from the block gather, in order
   return kl;
 }
 
+static int32_t* big_count(stormgpu_ctx* c) { return reinterpret_cast<int32_t*>(c->counters.p + kCntBig); }
+
 // The lists of reads the warp gather hands on: at most kSmallGatherCap positions, more, and too many for
 // shared memory.  Their cursors are zeroed with the counters of the pass.
 static GatherList small_gather_list(stormgpu_ctx* c, int64_t n, const int32_t* n_dev) {
-  return {c->small_list.p, c->small_h.p, n, n_dev, c->counters.p + 9, c->huge_list.p, c->huge_h.p, c->big_count.p + 1};
+  return {c->small_list.p, c->small_h.p, n, n_dev, c->counters.p + 9, c->huge_list.p, c->huge_h.p, big_count(c) + 1};
 }
 static GatherList large_gather_list(stormgpu_ctx* c, int64_t n, const int32_t* n_dev) {
-  return {c->big_list.p, c->big_h.p, n, n_dev, c->counters.p + 14, c->huge_list.p, c->huge_h.p, c->big_count.p + 1};
+  return {c->big_list.p, c->big_h.p, n, n_dev, c->counters.p + 14, c->huge_list.p, c->huge_h.p, big_count(c) + 1};
 }
 static GatherList huge_gather_list(stormgpu_ctx* c, int64_t reads, int64_t n, const int32_t* n_dev) {
   return {c->huge_list.p, c->huge_h.p, n, n_dev, c->counters.p + 15, c->huge_list.p + reads, c->huge_h.p + reads,
-          c->big_count.p + 1};
+          big_count(c) + 1};
 }
 
-// List capacities of a graph call.
-struct GraphCaps {
+// List capacities of a call whose passes are enqueued ahead.
+struct AheadCaps {
   int64_t cand, pass, kept;
   int64_t grid_h;  // blocks of the gather for the reads with the most positions
 };
 
-// The lists a graph call needs (false: they could not be allocated, and the call runs without a
-// graph).
-static bool graph_buffers(stormgpu_ctx* c, const PassSetup& P, GraphCaps* caps) {
+// The lists such a call needs (false: they could not be allocated, and the call runs host-synced).
+static bool ahead_buffers(stormgpu_ctx* c, const PassSetup& P, AheadCaps* caps) {
   const int64_t n = P.n;
   const int64_t want_cand = (int64_t)(c->gdens_cand * P.wsum * 1.25) + 61440;  // small calls: one scan block
-  const int64_t want_pass = (int64_t)(c->gdens_pass * P.wsum * 1.25) + 4096;
-  const int64_t want_kept = P.bound_H ? (int64_t)(c->gdens_kept * P.wsum * 1.25) + 4096 : want_pass;
+  const int64_t spare = std::min<int64_t>(4096, 64 * n);  // few reads: few enough for the wave alignment alone
+  const int64_t want_pass = (int64_t)(c->gdens_pass * P.wsum * 1.25) + spare;
+  const int64_t want_kept = P.bound_H ? (int64_t)(c->gdens_kept * P.wsum * 1.25) + spare : want_pass;
   caps->grid_h = std::max<int64_t>(1, std::min<int64_t>(gather_huge_grid(), ((int64_t)1 << 25) / c->huge_cap));
-  if (c->fr.grow(want_cand) || c->fd.grow(want_cand) || c->big_count.grow(4) || c->gstate.grow(kGsWords) ||
+  if (c->fr.grow(want_cand) || c->fd.grow(want_cand) ||
       c->big_tmp.grow(caps->grid_h * c->huge_cap))
     return false;
   if (P.bound_H && (c->q_read.grow(want_pass) || c->q_diag.grow(want_pass) || c->q_ub.grow(want_pass) ||
@@ -529,27 +500,25 @@ static bool graph_buffers(stormgpu_ctx* c, const PassSetup& P, GraphCaps* caps) 
   caps->cand = want_cand;
   caps->kept = want_kept;
   caps->pass = P.bound_H ? want_pass : caps->kept;
-  const int64_t nw = (std::max(caps->cand, caps->pass) + 31) / 32;
-  if (c->flag.grow(nw * 32) || c->flagw.grow(nw) || c->foff.grow(nw + 1) ||
-      c->scan_tmp64.grow(scan_tmp_elems(std::max<int64_t>(nw, n)) + 8) ||
+  const int64_t longest = std::max(caps->cand, caps->pass);
+  if (c->flag.grow(longest) || c->foff.grow(select_tiles(longest) + 1) ||
       c->scratch.grow(align_workers(caps->kept, P.sp) * (int64_t)P.maxL * P.wpr))
     return false;
   return round_lists_grow(c, n, caps->kept, P.rounds) == 0;
 }
 
-// The launches of every pass on c's stream, each list size read from the device (captured into
-// the graph; nothing here waits for the device).  E: the stage events, per_pass per pass.
-static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const GraphCaps& caps, int per_pass,
+// The launches of every pass on c's stream, each list size read from the device; nothing here waits for
+// the device.  E: the stage events, per_pass per pass.
+static int enqueue_passes(stormgpu_ctx* c, const PassSetup& P, const AheadCaps& caps, int per_pass,
                                 int64_t& launches) {
   cudaStream_t st = c->st;
   const int64_t cand_cap = caps.cand, pass_cap = caps.pass, kept_cap = caps.kept, grid_h = caps.grid_h;
   const ScoreParams& sp = P.sp;
   const int64_t n = P.n;
-  unsigned long long* gs = c->gstate.p;
-  const int64_t nw = (cand_cap + 31) / 32, nwq = (pass_cap + 31) / 32;
+  unsigned long long* gs = c->counters.p;
   const int rounds = P.rounds;
-  auto rec = [&](cudaEvent_t e) { return cudaEventRecordWithFlags(e, st, cudaEventRecordExternal); };
-  SG_CUDA(cudaMemsetAsync(gs, 0, sizeof(unsigned long long) * kGsWords, st));
+  auto rec = [&](cudaEvent_t e) { return cudaEventRecord(e, st); };
+  SG_CUDA(cudaMemsetAsync(gs, 0, sizeof(unsigned long long) * kCounters, st));
   int pi = 0;
   for (size_t ref_id = 0; ref_id < c->refs.size(); ++ref_id) {
     RefSeq& R = c->refs[ref_id];
@@ -563,24 +532,24 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const Graph
       ++pi;
       SG_CUDA(rec(E[0]));
       // hit gather: the warp kernel, then the block kernels over the lists it filled, then the
-      // reads above the block kernel's slices (reads above this launch's slices end the graph
+      // reads above the block kernel's slices (reads above this launch's slices end the
       // call: the host-synced passes size their slices to fit)
-      SG_CUDA(cudaMemsetAsync(c->counters.p, 0, sizeof(unsigned long long) * 32, st));
-      SG_CUDA(cudaMemsetAsync(c->big_count.p, 0, sizeof(int32_t) * 4, st));
+      if (pi > 1)
+        SG_CUDA(cudaMemsetAsync(c->counters.p + kCntPass, 0, sizeof(unsigned long long) * (kGsCand - kCntPass), st));
       GatherOut go;
       go.fr = c->fr.p; go.fd = c->fd.p; go.cap = cand_cap; go.counters = c->counters.p;
       go.big_list = c->big_list.p; go.big_h = c->big_h.p; go.small_list = c->small_list.p;
-      go.small_h = c->small_h.p; go.big_count = c->big_count.p;
+      go.small_h = c->small_h.p; go.big_count = big_count(c);
       go.cursor = c->counters.p + 12;
       go.reads_per_steal = c->tune.gather_reads_per_steal;
       go.warp_cap = c->tune.gather_warp_cap;
       launch_gather_fused(rd, ix, sp.I, go, c->seeds, st);
-      launch_gather_sort(rd, ix, sp.I, R.n, small_gather_list(c, n, c->big_count.p + 2), true, go, c->seeds, st);
-      launch_gather_sort(rd, ix, sp.I, R.n, large_gather_list(c, n, c->big_count.p + 0), false, go, c->seeds, st);
-      GatherList hl = huge_gather_list(c, n, n, c->big_count.p + 1);
-      hl.above_count = c->big_count.p + 3;
+      launch_gather_sort(rd, ix, sp.I, R.n, small_gather_list(c, n, big_count(c) + 2), true, go, c->seeds, st);
+      launch_gather_sort(rd, ix, sp.I, R.n, large_gather_list(c, n, big_count(c) + 0), false, go, c->seeds, st);
+      GatherList hl = huge_gather_list(c, n, n, big_count(c) + 1);
+      hl.above_count = big_count(c) + 3;
       launch_gather_huge(rd, ix, sp.I, R.n, hl, c->big_tmp.p, (int)c->huge_cap, grid_h, go, c->seeds, st);
-      gate_gather_kernel<<<1, 1, 0, st>>>(c->counters.p, c->big_count.p, cand_cap, kMaxCandidatesPerPass, gs);
+      gate_gather_kernel<<<1, 1, 0, st>>>(c->counters.p, cand_cap, kMaxCandidatesPerPass, gs);
       launches += 5;
       SG_CUDA(rec(E[1]));
       // filter over the gate's candidate count
@@ -593,12 +562,13 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const Graph
       launch_filter_flat_job(job, sp, filter_dpx_ok(sp, P.maxL), st);
       launches += 2;
       SG_CUDA(rec(E[2]));
-      // passing candidates, in order, over the whole capacity (the words past the count are zero)
-      launch_pack_flags(cand_cap, gs + kGsCand, c->flag.p, c->flagw.p, st);
-      exclusive_scan<PassWord, int64_t>(reinterpret_cast<const PassWord*>(c->flagw.p), c->foff.p, nw, c->foff.p + nw,
-                                        c->scan_tmp64.p, st);
-      gate_filter_kernel<<<1, 1, 0, st>>>(c->foff.p + nw, pass_cap, kMaxPassingPerPass, n, gs);
-      launches += 2 + scan_launches(nw);
+      // the passing candidates, in order
+      const SelectGate passing{gs + kGsStatus, gs + kGsPass, gs + kGsPassed, gs + kGsMaxPass, pass_cap,
+                               n > 1 ? kMaxPassingPerPass : INT64_MAX};
+      const SelectGate kept{gs + kGsStatus, gs + kGsKept, gs + kGsAligned, gs + kGsMaxKept, kept_cap, INT64_MAX};
+      launch_select_count(cand_cap, gs + kGsCand, c->flag.p, c->foff.p, gs + kCntSelect, passing,
+                          P.bound_H ? SelectGate{} : kept, st);
+      launches++;
       PassBuffers pb;
       memset(&pb, 0, sizeof(pb));
       pb.pstart = c->pstart.p; pb.pcount = c->pcount.p;
@@ -606,24 +576,21 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const Graph
       pb.p_read = c->p_read.p; pb.p_diag = c->p_diag.p; pb.p_cap = kept_cap;
       if (P.bound_H) {
         // the candidates whose score can exceed -t, in order
-        launch_compact(nw, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->q_read.p, c->q_diag.p, pass_cap, nullptr, nullptr, st);
+        launch_select_write(cand_cap, gs + kGsCand, c->flag.p, c->foff.p, c->fr.p, c->fd.p, c->q_read.p, c->q_diag.p,
+                            pass_cap, nullptr, nullptr, st);
         launch_bound_pass(c, P, rd, R, pass_cap, reinterpret_cast<const int64_t*>(gs + kGsPass), st);
-        launch_pack_flags(pass_cap, gs + kGsPass, c->flag.p, c->flagw.p, st);
-        exclusive_scan<PassWord, int64_t>(reinterpret_cast<const PassWord*>(c->flagw.p), c->foff.p, nwq,
-                                          c->foff.p + nwq, c->scan_tmp64.p, st);
-        gate_bound_kernel<<<1, 1, 0, st>>>(c->foff.p + nwq, kept_cap, gs);
-        launch_compact(nwq, c->flagw.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->k_diag.p, kept_cap,
-                       c->q_ub.p, c->k_ub.p, st);
+        launch_select_count(pass_cap, gs + kGsPass, c->flag.p, c->foff.p, gs + kCntSelect + 1, kept, SelectGate{}, st);
+        launch_select_write(pass_cap, gs + kGsPass, c->flag.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->k_diag.p,
+                            kept_cap, c->q_ub.p, c->k_ub.p, st);
         pb.ub = c->p_ub.p;
-        launches += 6 + scan_launches(nwq);
+        launches += 4;
       } else {
-        gate_bound_kernel<<<1, 1, 0, st>>>(c->foff.p + nw, kept_cap, gs);
-        launch_compact(nw, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->k_diag.p, kept_cap, nullptr, nullptr,
-                       st);
-        launches += 2;
+        launch_select_write(cand_cap, gs + kGsCand, c->flag.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->k_diag.p,
+                            kept_cap, nullptr, nullptr, st);
+        launches++;
       }
       const int64_t* np = reinterpret_cast<const int64_t*>(gs + kGsKept);
-      setup_rounds(c, rounds, pb, st);
+      setup_rounds(c, rounds, pb);
       launch_slot_lists(kept_list(c, P, kept_cap, np), c->p_ub.p, pb, align_round_take(0, rounds), st);
       launches += 3;
       pb.a_score = c->a_score.p; pb.a_bound = c->a_bound.p; pb.a_tblen = c->a_tblen.p;
@@ -631,12 +598,12 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const Graph
       pb.npass_dev = np;
       pb.steal = c->tune.align_steal;
       pb.a_scratch = c->scratch.p;
-      pb.cells = c->counters.p + 13;
+      pb.cells = c->counters.p + kCntAlign;
       if (rounds == 1) {
         pb.wave = wave_slots(sp);
         if (pb.wave) launch_align_wave(rd, sp, R.d_codes, R.d_mask, 0, kept_cap, pb, P.maxL, st);
-        launch_align(rd, sp, R.d_codes, R.d_mask, 0, kept_cap, pb, st);
-        launches += pb.wave ? 2 : 1;
+        if (kept_cap > pb.wave) launch_align(rd, sp, R.d_codes, R.d_mask, 0, kept_cap, pb, st);
+        launches += (pb.wave > 0) + (kept_cap > pb.wave);
         SG_CUDA(rec(E[3]));
         launch_replay(n, sp, (int)ref_id, strand ? -1 : 1, pb, 0, P.out->hits, P.out->tb, P.out->tb_stride,
                       P.out->mapped, st);
@@ -654,24 +621,22 @@ static int enqueue_graph_passes(stormgpu_ctx* c, const PassSetup& P, const Graph
         }
         SG_CUDA(rec(E[3]));
       }
-      pass_sums_kernel<<<1, 1, 0, st>>>(c->counters.p, gs);
-      launches++;
       SG_CUDA(rec(E[4]));
     }
   }
   return 0;
 }
 
-// Every pass of the call as one graph.  0: done (results in P.out, stats in c->stats);
-// kGraphRetry: the results are not usable (a list did not fit, or graphs do not work here) and
-// the call must run the host-synced passes; else an error code.
-static int map_passes_graph(stormgpu_ctx* c, const PassSetup& P, int64_t launches) {
+// Every pass of the call enqueued ahead.  0: done (results in P.out, stats in c->stats); kHostSynced: the
+// results are not usable (a list did not fit) and the call must run the host-synced passes; else an
+// error code.
+static int map_passes_ahead(stormgpu_ctx* c, const PassSetup& P, int64_t launches) {
   cudaStream_t st = c->st;
-  GraphCaps caps;
-  if (!graph_buffers(c, P, &caps)) {
+  AheadCaps caps;
+  if (!ahead_buffers(c, P, &caps)) {
     cudaGetLastError();
     c->work.over = false;  // the host-synced passes allocate what they need, no more
-    return kGraphRetry;
+    return kHostSynced;
   }
   const int rounds = P.rounds;
   const int per_pass = 5 + (rounds > 1 ? 1 + 2 * rounds : 0);
@@ -683,55 +648,26 @@ static int map_passes_graph(stormgpu_ctx* c, const PassSetup& P, int64_t launche
     SG_CUDA(cudaEventCreate(&e));
     c->gev.push_back(e);
   }
-  // capture (nothing runs), then update the last call's executable graph in place when the
-  // shape is the same, else instantiate anew
-  cudaGraph_t g = nullptr;
-  auto broken = [&]() {
-    cudaGetLastError();
-    if (g) cudaGraphDestroy(g);
-    c->graph_broken = true;
-    return kGraphRetry;
-  };
-  if (cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed) != cudaSuccess) return broken();
-  const int erc = enqueue_graph_passes(c, P, caps, per_pass, launches);
-  const cudaError_t ece = cudaStreamEndCapture(st, &g);
-  if (erc || ece != cudaSuccess || !g) return broken();
-  bool ready = false;
-  if (c->gexec) {
-    cudaGraphExecUpdateResultInfo info;
-    ready = cudaGraphExecUpdate(c->gexec, g, &info) == cudaSuccess;
-    if (!ready) {
-      cudaGetLastError();
-      cudaGraphExecDestroy(c->gexec);
-      c->gexec = nullptr;
-    }
-  }
-  if (!ready && cudaGraphInstantiate(&c->gexec, g, 0) != cudaSuccess) {
-    c->gexec = nullptr;
-    return broken();
-  }
-  cudaGraphDestroy(g);
-  g = nullptr;
-  unsigned long long h[kGsWords];
+  unsigned long long h[kCounters];
   SG_CUDA(cudaEventRecord(c->ev[6], st));
-  SG_CUDA(cudaGraphLaunch(c->gexec, st));
+  if (const int e = enqueue_passes(c, P, caps, per_pass, launches)) return e;
   SG_CUDA(cudaEventRecord(c->ev[7], st));
-  SG_CUDA(cudaMemcpyAsync(h, c->gstate.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+  SG_CUDA(cudaMemcpyAsync(h, c->counters.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   SG_CUDA(cudaStreamSynchronize(st));
   SG_CUDA(cudaGetLastError());
-  if (h[kGsStatus]) return kGraphRetry;
+  if (h[kGsStatus]) return kHostSynced;
   stormgpu_stats& S = c->stats;
-  S.candidates = (int64_t)h[kGsCandidates];
-  S.filter_cells = (int64_t)h[kGsCells];
-  S.filter_band_cells = (int64_t)h[kGsBand];
-  S.seed_lookups = (int64_t)h[kGsLookups];
-  S.hit_positions = (int64_t)h[kGsPositions];
+  S.candidates = (int64_t)h[5];
+  S.filter_cells = (int64_t)h[2];
+  S.filter_band_cells = (int64_t)h[6];
+  S.seed_lookups = (int64_t)h[3];
+  S.hit_positions = (int64_t)h[4];
   S.filter_passed = (int64_t)h[kGsPassed];
   S.aligned = (int64_t)h[kGsAligned];
-  S.align_cells = (int64_t)h[kGsAlignCells];
+  S.align_cells = (int64_t)h[kCntAlign];
   S.passes = npasses;
   S.graph_passes = npasses;
-  // stage times from the graph's events (as the host-synced passes split them)
+  // stage times (as the host-synced passes split them)
   float tg = 0, tf = 0, ta = 0, tr = 0, tt = 0;
   for (int pi = 0; pi < npasses; ++pi) {
     const cudaEvent_t* E = c->gev.data() + (size_t)pi * per_pass;
@@ -756,7 +692,7 @@ static int map_passes_graph(stormgpu_ctx* c, const PassSetup& P, int64_t launche
   return 0;
 }
 
-static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgpu_results* out) {
+static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, stormgpu_results* out) {
   if (!c->indexed) { sg_set_error("stormgpu_build_index must be called before mapping"); return STORMGPU_ESTATE; }
   cudaStream_t st = c->st;
   const int64_t n = reads->n;
@@ -768,17 +704,12 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
   int64_t launches = 0;
   int maxL = 0, minL = STORMGPU_MAX_READ_LEN;
   double wsum = 0;  // the batch's work weight (read_weight)
-  {
-    std::vector<int16_t> hl(n > 0 ? n : 1);
-    if (n > 0) SG_CUDA(cudaMemcpyAsync(hl.data(), reads->lengths, sizeof(int16_t) * n, cudaMemcpyDeviceToHost, st));
-    SG_CUDA(cudaStreamSynchronize(st));
-    for (int64_t r = 0; r < n; ++r) {
-      maxL = std::max<int>(maxL, hl[r]);
-      minL = std::min<int>(minL, hl[r]);
-      wsum += read_weight(hl[r]);
-    }
-    if (maxL > STORMGPU_MAX_READ_LEN) { sg_set_error("read longer than %d", STORMGPU_MAX_READ_LEN); return STORMGPU_EINVAL; }
+  for (int64_t r = 0; r < n; ++r) {
+    maxL = std::max<int>(maxL, lengths[r]);
+    minL = std::min<int>(minL, lengths[r]);
+    wsum += read_weight(lengths[r]);
   }
+  if (maxL > STORMGPU_MAX_READ_LEN) { sg_set_error("read longer than %d", STORMGPU_MAX_READ_LEN); return STORMGPU_EINVAL; }
   if (out->tb_stride < (maxL + c->p.allowed_indels + 1) / 2) { sg_set_error("tb_stride too small"); return STORMGPU_EINVAL; }
   launch_init_results(n, out->hits, out->mapped, out->tb, out->tb_stride, st);
   launches++;
@@ -806,10 +737,10 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
     rev.codes = c->rcodes.p;
     rev.levels = reads->levels ? c->rlevels.p : nullptr;
   }
-  if (c->pstart.grow(n) || c->pcount.grow(n) || c->scan_tmp64.grow(scan_tmp_elems(n) + 8) ||
+  if (c->pstart.grow(n) || c->pcount.grow(n) ||
       c->big_list.grow(n) || c->big_h.grow(n) || c->small_list.grow(n) || c->small_h.grow(n) ||
-      c->huge_list.grow(2 * n) || c->huge_h.grow(2 * n) || c->big_count.grow(3) ||
-      c->counters.grow(32) || c->fr.grow(std::max<int64_t>(n * 64, 1 << 20)) ||
+      c->huge_list.grow(2 * n) || c->huge_h.grow(2 * n) || c->counters.grow(kCounters) ||
+      c->fr.grow(std::max<int64_t>(n * 64, 1 << 20)) ||
       c->fd.grow(std::max<int64_t>(n * 64, 1 << 20)))
     return STORMGPU_ENOMEM;
   const int BW = 2 * sp.I + 1;
@@ -836,11 +767,11 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
   // an alignment's latency each (300 colour reads: alignment and replay 0.70 -> 0.60 ms), as they do in a call of a few reads.
   const int rounds = !bound_H || n <= 256 ? 1 : std::max(1, std::min<int>(c->tune.align_rounds, kMaxAlignRounds));
   const PassSetup P{sp, fwd, rev, n, maxL, minL, wsum, wpr, tbs, rounds, filter_H, bound_H, out};
-  if (c->graphs && !c->graph_broken && c->gdens_cand > 0 && c->huge_cap <= ((int64_t)1 << 22)) {
-    const int g = map_passes_graph(c, P, launches);
-    if (g != kGraphRetry) return g;
-    // a list outgrew its capacity: the passes again, each sized by the host (the graph's
-    // replays may have updated the results of its first passes)
+  if (c->graphs && c->gdens_cand > 0 && c->huge_cap <= ((int64_t)1 << 22)) {
+    const int g = map_passes_ahead(c, P, launches);
+    if (g != kHostSynced) return g;
+    // a list outgrew its capacity: the passes again, each sized by the host (the replays of the
+    // first passes may have updated the results)
     launch_init_results(n, out->hits, out->mapped, out->tb, out->tb_stride, st);
     launches++;
   }
@@ -860,19 +791,18 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
       for (int attempt = 0;; ++attempt) {
         // fused hit gather: sorted, de-duplicated diagonals of every read, appended to the flat
         // candidate list (fr, fd); reads with many index positions go to the block kernel
-        SG_CUDA(cudaMemsetAsync(c->counters.p, 0, sizeof(unsigned long long) * 32, st));
-        SG_CUDA(cudaMemsetAsync(c->big_count.p, 0, sizeof(int32_t) * 3, st));
+        SG_CUDA(cudaMemsetAsync(c->counters.p, 0, sizeof(unsigned long long) * kCounters, st));
         GatherOut go;
         go.fr = c->fr.p; go.fd = c->fd.p; go.cap = c->fr.cap; go.counters = c->counters.p;
         go.big_list = c->big_list.p; go.big_h = c->big_h.p; go.small_list = c->small_list.p;
-        go.small_h = c->small_h.p; go.big_count = c->big_count.p;
+        go.small_h = c->small_h.p; go.big_count = big_count(c);
         go.cursor = c->counters.p + 12;  // zeroed just above
         go.reads_per_steal = c->tune.gather_reads_per_steal;
         go.warp_cap = c->tune.gather_warp_cap;
         launch_gather_fused(rd, ix, sp.I, go, c->seeds, st);
         launches++;
         int32_t nbig[3] = {0, 0, 0};  // handed to the block gather with many positions, above its slice, with few
-        SG_CUDA(cudaMemcpyAsync(nbig, c->big_count.p, sizeof(nbig), cudaMemcpyDeviceToHost, st));
+        SG_CUDA(cudaMemcpyAsync(nbig, big_count(c), sizeof(nbig), cudaMemcpyDeviceToHost, st));
         SG_CUDA(cudaStreamSynchronize(st));
         if (nbig[2] > 0) {  // reads with few positions: sorted in shared memory
           launch_gather_sort(rd, ix, sp.I, R.n, small_gather_list(c, nbig[2], nullptr), true, go, c->seeds, st);
@@ -881,7 +811,7 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
         if (nbig[0] > 0) {  // reads with many positions: a block with most of an SM's shared memory
           launch_gather_sort(rd, ix, sp.I, R.n, large_gather_list(c, nbig[0], nullptr), false, go, c->seeds, st);
           launches++;
-          SG_CUDA(cudaMemcpyAsync(nbig + 1, c->big_count.p + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+          SG_CUDA(cudaMemcpyAsync(nbig + 1, big_count(c) + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
           SG_CUDA(cudaStreamSynchronize(st));
           if (nbig[1] > 0) {  // beyond it: slices of the largest read's size in global memory
             std::vector<int32_t> hh(nbig[1]);
@@ -910,11 +840,8 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
         if (attempt > 2) { sg_set_error("internal: candidate list overflow"); return STORMGPU_EINVAL; }
         if (c->fr.grow(utot + utot / 4 + 1024) || c->fd.grow(utot + utot / 4 + 1024)) return STORMGPU_ENOMEM;
       }
-      const int64_t nwords = (utot + 31) / 32;
-      if (c->flag.grow(std::max<int64_t>(nwords * 32, 1)) || c->flagw.grow(std::max<int64_t>(nwords, 1)) ||
-          c->foff.grow(nwords + 1) ||
-          c->scan_tmp64.grow(scan_tmp_elems(std::max<int64_t>(nwords, n)) + 8))
-        return STORMGPU_ENOMEM;
+      const int64_t tiles = select_tiles(utot);
+      if (c->flag.grow(std::max<int64_t>(utot, 1)) || c->foff.grow(tiles + 1)) return STORMGPU_ENOMEM;
       SG_CUDA(cudaEventRecord(c->ev[1], st));
       FilterJob job;
       memset(&job, 0, sizeof(job));
@@ -926,16 +853,13 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
       launches += 2;
       S.passes++;
       SG_CUDA(cudaEventRecord(c->ev[2], st));
-      launch_pack_flags(utot, nullptr, c->flag.p, c->flagw.p, st);
-      launches += (utot > 0 ? 1 : 0) + scan_launches(nwords);
-      exclusive_scan<PassWord, int64_t>(reinterpret_cast<const PassWord*>(c->flagw.p), c->foff.p, nwords,
-                                        c->foff.p + nwords, c->scan_tmp64.p, st);
+      launch_select_count(utot, nullptr, c->flag.p, c->foff.p, c->counters.p + kCntSelect, {}, {}, st);
+      launches++;
       unsigned long long cnt[8];
       int64_t npass = 0;
-      SG_CUDA(cudaMemcpyAsync(&npass, c->foff.p + nwords, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+      SG_CUDA(cudaMemcpyAsync(&npass, c->foff.p + tiles, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
       SG_CUDA(cudaMemcpyAsync(cnt, c->counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, st));
       SG_CUDA(cudaStreamSynchronize(st));
-      if (utot == 0) npass = 0;
       S.candidates += (int64_t)cnt[5];
       S.filter_cells += (int64_t)cnt[2];
       S.filter_band_cells += (int64_t)cnt[6];
@@ -951,16 +875,13 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
       int64_t nkept = npass;  // candidates that are aligned
       if (npass > 0 && bound_H) {
         // those whose score can exceed -t, in order
-        const int64_t nwq = (npass + 31) / 32;
         if (c->q_read.grow(npass) || c->q_diag.grow(npass) || c->q_ub.grow(npass)) return STORMGPU_ENOMEM;
-        launch_compact(nwords, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->q_read.p, c->q_diag.p, c->q_read.cap,
-                       nullptr, nullptr, st);
+        launch_select_write(utot, nullptr, c->flag.p, c->foff.p, c->fr.p, c->fd.p, c->q_read.p, c->q_diag.p,
+                            c->q_read.cap, nullptr, nullptr, st);
         launch_bound_pass(c, P, rd, R, npass, nullptr, st);
-        launch_pack_flags(npass, nullptr, c->flag.p, c->flagw.p, st);
-        exclusive_scan<PassWord, int64_t>(reinterpret_cast<const PassWord*>(c->flagw.p), c->foff.p, nwq,
-                                          c->foff.p + nwq, c->scan_tmp64.p, st);
-        launches += 4 + scan_launches(nwq);
-        SG_CUDA(cudaMemcpyAsync(&nkept, c->foff.p + nwq, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        launch_select_count(npass, nullptr, c->flag.p, c->foff.p, c->counters.p + kCntSelect + 1, {}, {}, st);
+        launches += 4;
+        SG_CUDA(cudaMemcpyAsync(&nkept, c->foff.p + select_tiles(npass), sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         SG_CUDA(cudaStreamSynchronize(st));
       }
       max_kept = std::max(max_kept, nkept);
@@ -971,14 +892,15 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
           return STORMGPU_ENOMEM;
         pb.p_read = c->p_read.p; pb.p_diag = c->p_diag.p; pb.p_cap = c->p_read.cap;
         if (bound_H) {
-          launch_compact((npass + 31) / 32, c->flagw.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->k_diag.p,
-                         nkept, c->q_ub.p, c->k_ub.p, st);
+          launch_select_write(npass, nullptr, c->flag.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->k_diag.p,
+                              nkept, c->q_ub.p, c->k_ub.p, st);
           pb.ub = c->p_ub.p;
         } else {
-          launch_compact(nwords, c->flagw.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->k_diag.p, nkept, nullptr,
-                         nullptr, st);
+          launch_select_write(utot, nullptr, c->flag.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->k_diag.p, nkept,
+                              nullptr, nullptr, st);
         }
-        if (round_lists_grow(c, n, nkept, rounds) || setup_rounds(c, rounds, pb, st)) return STORMGPU_ENOMEM;
+        if (round_lists_grow(c, n, nkept, rounds)) return STORMGPU_ENOMEM;
+        setup_rounds(c, rounds, pb);
         launch_slot_lists(kept_list(c, P, nkept, nullptr), c->p_ub.p, pb, align_round_take(0, rounds), st);
         launches += 4;
         pb.a_score = c->a_score.p; pb.a_bound = c->a_bound.p; pb.a_tblen = c->a_tblen.p;
@@ -988,7 +910,7 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
         const int64_t per_slot = (int64_t)maxL * wpr;
         if (c->scratch.grow(align_workers(nkept, sp) * per_slot)) return STORMGPU_ENOMEM;
         pb.a_scratch = c->scratch.p;
-        pb.cells = c->counters.p + 13;
+        pb.cells = c->counters.p + kCntAlign;
         if (rounds == 1) {
           if (nkept <= wave_slots(sp)) launch_align_wave(rd, sp, R.d_codes, R.d_mask, 0, nkept, pb, maxL, st);
           else launch_align(rd, sp, R.d_codes, R.d_mask, 0, nkept, pb, st);
@@ -1031,7 +953,7 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
       tg += a; tf += b; ta += d; tr += e;
       if (nkept > 0) {
         unsigned long long cells = 0;
-        SG_CUDA(cudaMemcpyAsync(&cells, c->counters.p + 13, sizeof(cells), cudaMemcpyDeviceToHost, st));
+        SG_CUDA(cudaMemcpyAsync(&cells, c->counters.p + kCntAlign, sizeof(cells), cudaMemcpyDeviceToHost, st));
         SG_CUDA(cudaStreamSynchronize(st));
         S.align_cells += (int64_t)cells;
       }
@@ -1049,7 +971,8 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, stormgp
 }
 
 // Maps reads[lo, hi) into the matching part of out.
-static int map_range(stormgpu_ctx* c, const stormgpu_reads* reads, stormgpu_results* out, int64_t lo, int64_t hi) {
+static int map_range(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, stormgpu_results* out,
+                     int64_t lo, int64_t hi) {
   stormgpu_reads r = *reads;
   stormgpu_results o = *out;
   r.n = hi - lo;
@@ -1060,17 +983,17 @@ static int map_range(stormgpu_ctx* c, const stormgpu_reads* reads, stormgpu_resu
   o.hits += 4 * lo;
   o.tb += 4 * lo * out->tb_stride;
   o.mapped += lo;
-  return sg::map_device_impl(c, &r, &o);
+  return sg::map_device_impl(c, &r, lengths + lo, &o);
 }
 
 // Maps the batch as consecutive pieces [cuts[q], cuts[q + 1]), the stats summed.
-static int map_cuts(stormgpu_ctx* c, const stormgpu_reads* reads, stormgpu_results* out,
+static int map_cuts(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, stormgpu_results* out,
                     const std::vector<int64_t>& cuts) {
   stormgpu_stats acc;
   memset(&acc, 0, sizeof(acc));
   for (size_t q = 0; q + 1 < cuts.size(); ++q) {
     if (cuts[q + 1] <= cuts[q]) continue;
-    if (const int e = map_range(c, reads, out, cuts[q], cuts[q + 1])) return e;
+    if (const int e = map_range(c, reads, lengths, out, cuts[q], cuts[q + 1])) return e;
     add_stats(acc, c->stats);
   }
   acc.ms_index = c->stats.ms_index;
@@ -1079,28 +1002,36 @@ static int map_cuts(stormgpu_ctx* c, const stormgpu_reads* reads, stormgpu_resul
 }
 
 // k consecutive pieces of (nearly) equal size
-static int map_pieces(stormgpu_ctx* c, const stormgpu_reads* reads, stormgpu_results* out, int64_t k) {
+static int map_pieces(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, stormgpu_results* out,
+                      int64_t k) {
   std::vector<int64_t> cuts;
   for (int64_t q = 0; q <= k; ++q) cuts.push_back(reads->n * q / k);
-  return map_cuts(c, reads, out, cuts);
+  return map_cuts(c, reads, lengths, out, cuts);
 }
 
-int sg::map_device_impl(stormgpu_ctx* c, const stormgpu_reads* reads, stormgpu_results* out) {
+int sg::map_device_impl(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, stormgpu_results* out) {
+  std::vector<int16_t> hl;
+  if (!lengths) {
+    hl.resize(std::max<int64_t>(reads->n, 1));
+    if (reads->n > 0) {
+      SG_CUDA(cudaMemcpyAsync(hl.data(), reads->lengths, sizeof(int16_t) * reads->n, cudaMemcpyDeviceToHost, c->st));
+      SG_CUDA(cudaStreamSynchronize(c->st));
+    }
+    lengths = hl.data();
+  }
   if (reads->n > 1 && (c->dens_cand > 0 || c->dens_pass > 0)) {
     // at the last call's density per unit of work weight the batch would be cut after its
     // gather: cut it now, into pieces of equal weight (a batch's reads need not be mixed: a file
     // of several lengths often lists them one length after the other).  0.8: the pieces still
     // differ in repeat content; one that overflows is cut after its gather.
     const int64_t n = reads->n;
-    std::vector<int16_t> hl(n);
-    SG_CUDA(cudaMemcpyAsync(hl.data(), reads->lengths, sizeof(int16_t) * n, cudaMemcpyDeviceToHost, c->st));
-    SG_CUDA(cudaStreamSynchronize(c->st));
-    std::vector<double> cum(n + 1, 0.0);
-    for (int64_t r = 0; r < n; ++r) cum[r + 1] = cum[r] + read_weight(hl[r]);
-    const double W = cum[n];
+    double W = 0.0;
+    for (int64_t r = 0; r < n; ++r) W += read_weight(lengths[r]);
     const double need = std::max(c->dens_cand * W / (0.8 * (double)kMaxCandidatesPerPass),
                                  c->dens_pass * W / (0.8 * (double)kMaxPassingPerPass));
     if (need > 1.0) {
+      std::vector<double> cum(n + 1, 0.0);
+      for (int64_t r = 0; r < n; ++r) cum[r + 1] = cum[r] + read_weight(lengths[r]);
       const int64_t k = std::min<int64_t>(n, (int64_t)std::ceil(need));
       std::vector<int64_t> cuts(1, 0);
       for (int64_t q = 1; q < k; ++q) {  // strictly increasing, every piece smaller than the batch
@@ -1109,13 +1040,13 @@ int sg::map_device_impl(stormgpu_ctx* c, const stormgpu_reads* reads, stormgpu_r
         cuts.push_back(cut);
       }
       cuts.push_back(n);
-      return map_cuts(c, reads, out, cuts);
+      return map_cuts(c, reads, lengths, out, cuts);
     }
   }
   WorkBudget* saved = g_work_budget;
   g_work_budget = &c->work;
   c->work.over = false;
-  int rc = map_device_once(c, reads, out);
+  int rc = map_device_once(c, reads, lengths, out);
   g_work_budget = saved;
   const int64_t n = reads->n;
   if (rc == STORMGPU_ENOMEM && c->work.over) {
@@ -1130,7 +1061,7 @@ int sg::map_device_impl(stormgpu_ctx* c, const stormgpu_reads* reads, stormgpu_r
     sg_set_error("one read has more than %lld candidate diagonals", (long long)kMaxCandidatesPerPass);
     return STORMGPU_ENOMEM;
   }
-  return map_pieces(c, reads, out, 2);
+  return map_pieces(c, reads, lengths, out, 2);
 }
 
 extern "C" int stormgpu_map_device(stormgpu_ctx* c, const stormgpu_reads* reads, stormgpu_results* out,
@@ -1145,7 +1076,7 @@ extern "C" int stormgpu_map_device(stormgpu_ctx* c, const stormgpu_reads* reads,
     SG_CUDA(cudaStreamWaitEvent(c->st, e, 0));
     cudaEventDestroy(e);
   }
-  int rc = map_device_impl(c, reads, out);
+  int rc = map_device_impl(c, reads, nullptr, out);
   if (rc == 0 && user) {
     cudaEvent_t e;
     SG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1189,7 +1120,7 @@ extern "C" int stormgpu_map(stormgpu_ctx* c, const stormgpu_reads* reads, stormg
   dres.tb = c->tb.p;
   dres.tb_stride = out->tb_stride;
   dres.mapped = c->mapped.p;
-  int rc = map_device_impl(c, &dr, &dres);
+  int rc = map_device_impl(c, &dr, reads->lengths, &dres);
   if (rc) return rc;
   c->last_n = n;
   c->last_tbs = out->tb_stride;

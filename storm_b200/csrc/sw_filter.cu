@@ -19,6 +19,8 @@
 // hit passes in both; cells are masked before they propagate, so an unmasked run and a
 // saturating one agree on pass/fail.  Values stay below 2^15 when L * match < 32000 (checked
 // by the host, which otherwise uses the plain 32-bit kernel).
+#include <algorithm>
+
 #include "map_kernels.cuh"
 #include "sw_filter.cuh"
 #include "filter_ref.cuh"
@@ -265,69 +267,143 @@ void launch_filter_flat_job(const FilterJob& job, const ScoreParams& sp, bool dp
 
 // ------------------------------------------------------------------ compaction of passing candidates
 
-// pass bytes -> pass bits, one word per 32 candidates (the scan then runs over words); the
-// words of [n_dev, ncap) (all of them from n_dev on, when it is given) are zero
-__global__ void pack_flags_kernel(int64_t ncap, const unsigned long long* __restrict__ n_dev,
-                                  const uint8_t* __restrict__ flag, uint32_t* __restrict__ words) {
-  const int64_t nw = (ncap + 31) / 32;
+// ------------------------------------------------------------------------------ selection
+//
+// The flagged candidates in order: a count per tile of 4,096 flag bytes, whose last block to finish scans
+// the counts (it waits for nothing, the others are done) and applies the gates, then the writes.  The
+// bytes are read twice where pass words, their scan (one to three launches), a gate and the writes took
+// four to six launches: 10 us for 16 reads (269 candidates) against 14, 50 us for 12 million.  Launches
+// count where a call is small: one of 16 reads went from 432 to 379 us with half of them gone.
+
+constexpr int kSelectThreads = 256;
+static_assert(kSelectTile == kSelectThreads * 16, "a thread takes 16 flag bytes");
+
+// flags [t0, t0 + 16) of n as bits
+__device__ __forceinline__ uint32_t flags16(const uint8_t* __restrict__ flag, int64_t t0, int64_t n) {
+  uint32_t bits = 0;
+  if (t0 + 16 <= n) {
+    const uint4 q = *reinterpret_cast<const uint4*>(flag + t0);
+    const uint32_t v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) bits |= ((v[k] >> (8 * b)) & 1u) << (4 * k + b);
+  } else {
+    for (int64_t t = t0; t < n; ++t) bits |= (uint32_t)(flag[t] & 1) << (t - t0);
+  }
+  return bits;
+}
+
+// exclusive scan over the block; *total the sum
+template <class T>
+__device__ __forceinline__ T select_scan(T v, T* wsum, T* total) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  T incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const T x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
+  }
+  __syncthreads();  // wsum is free again
+  if (lane == 31) wsum[w] = incl;
+  __syncthreads();
+  T before = 0, all = 0;
+#pragma unroll
+  for (int k = 0; k < kSelectThreads / 32; ++k) {
+    if (k < w) before += wsum[k];
+    all += wsum[k];
+  }
+  *total = all;
+  return before + incl - v;
+}
+
+__device__ __forceinline__ void apply_gate(const SelectGate& g, int64_t total) {
+  if (!g.status) return;
+  unsigned long long s = *g.status;
+  if (total > g.cap) s |= 4;
+  if (total > g.limit) s |= 2;
+  *g.status = s;
+  *g.take = s ? 0 : (unsigned long long)total;
+  if (!s) *g.sum += (unsigned long long)total;
+  if ((unsigned long long)total > *g.most) *g.most = (unsigned long long)total;
+}
+
+__global__ void __launch_bounds__(kSelectThreads) select_count_kernel(int64_t ncap, const unsigned long long* __restrict__ n_dev,
+                                                                      const uint8_t* __restrict__ flag, int64_t* tile,
+                                                                      unsigned long long* ticket, SelectGate g0, SelectGate g1) {
+  __shared__ int64_t wsum[kSelectThreads / 32];
+  __shared__ bool last;
   const int64_t n = n_dev ? min(ncap, (int64_t)*n_dev) : ncap;
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t bits = 0;
-    const int64_t t0 = w * 32;
-    if (t0 >= n) {
-      words[w] = 0;
-      continue;
-    }
-    if (t0 + 32 <= n) {
-      const uint4* p = reinterpret_cast<const uint4*>(flag + t0);  // flag is 16-byte aligned, t0 a multiple of 32
-      const uint4 q0 = p[0], q1 = p[1];
-      const uint32_t v[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) bits |= ((v[k] >> (8 * b)) & 1u) << (4 * k + b);
-    } else {
-      for (int64_t t = t0; t < n; ++t) bits |= (uint32_t)(flag[t] & 1) << (t - t0);
-    }
-    words[w] = bits;
+  const int64_t nt = (n + kSelectTile - 1) / kSelectTile;
+  for (int64_t t = blockIdx.x; t < nt; t += gridDim.x) {
+    const int64_t mine = __popc(flags16(flag, t * kSelectTile + threadIdx.x * 16, n));
+    int64_t all;
+    select_scan<int64_t>(mine, wsum, &all);
+    if (threadIdx.x == 0) tile[t] = all;
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1ull) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int64_t per = (nt + kSelectThreads - 1) / kSelectThreads;
+  const int64_t a = min(nt, threadIdx.x * per), b = min(nt, a + per);
+  int64_t sum = 0;
+  for (int64_t t = a; t < b; ++t) sum += __ldcg(reinterpret_cast<const long long*>(tile + t));
+  int64_t total;
+  int64_t off = select_scan<int64_t>(sum, wsum, &total);
+  for (int64_t t = a; t < b; ++t) {
+    const int64_t c = __ldcg(reinterpret_cast<const long long*>(tile + t));
+    tile[t] = off;
+    off += c;
+  }
+  if (threadIdx.x == 0) {
+    tile[(ncap + kSelectTile - 1) / kSelectTile] = total;
+    apply_gate(g0, total);
+    apply_gate(g1, total);
   }
 }
 
-void launch_pack_flags(int64_t ncap, const unsigned long long* n_dev, const uint8_t* flag, uint32_t* words,
-                       cudaStream_t st) {
-  if (ncap <= 0) return;
-  int64_t blocks = ((ncap + 31) / 32 + 255) / 256;
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  pack_flags_kernel<<<(unsigned)blocks, 256, 0, st>>>(ncap, n_dev, flag, words);
-}
-
-// passing candidates, in order, into (p_read, p_diag): one thread per word of pass bits
-// (slots from pcap on are not written)
-__global__ void compact_kernel(int64_t nwords, const uint32_t* __restrict__ flag, const int64_t* __restrict__ woff,
-                               const int32_t* __restrict__ fr, const int32_t* __restrict__ fd,
-                               int32_t* __restrict__ p_read, int32_t* __restrict__ p_diag, int64_t pcap,
-                               const int16_t* __restrict__ ub, int16_t* __restrict__ p_ub) {
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t m = flag[w];
-    if (!m) continue;
-    int64_t o = woff[w];
+__global__ void __launch_bounds__(kSelectThreads) select_write_kernel(
+    int64_t ncap, const unsigned long long* __restrict__ n_dev, const uint8_t* __restrict__ flag,
+    const int64_t* __restrict__ tile, const int32_t* __restrict__ fr, const int32_t* __restrict__ fd,
+    int32_t* __restrict__ p_read, int32_t* __restrict__ p_diag, int64_t pcap, const int16_t* __restrict__ ub,
+    int16_t* __restrict__ p_ub) {
+  __shared__ int wsum[kSelectThreads / 32];
+  const int64_t n = n_dev ? min(ncap, (int64_t)*n_dev) : ncap;
+  const int64_t nt = (n + kSelectTile - 1) / kSelectTile, end = (ncap + kSelectTile - 1) / kSelectTile;
+  for (int64_t t = blockIdx.x; t < nt; t += gridDim.x) {
+    const int64_t base = tile[t], next = tile[t + 1 < nt ? t + 1 : end];
+    if (next == base) continue;  // uniform over the block
+    const int64_t t0 = t * kSelectTile + threadIdx.x * 16;
+    uint32_t m = flags16(flag, t0, n);
+    int all;
+    int64_t o = base + select_scan<int>(__popc(m), wsum, &all);
     while (m && o < pcap) {
-      const int64_t t = w * 32 + (__ffs(m) - 1);
-      p_read[o] = fr[t];
-      p_diag[o] = fd[t];
-      if (p_ub) p_ub[o] = ub[t];
+      const int64_t c = t0 + (__ffs(m) - 1);
+      p_read[o] = fr[c];
+      p_diag[o] = fd[c];
+      if (p_ub) p_ub[o] = ub[c];
       ++o;
       m &= m - 1;
     }
   }
 }
 
-void launch_compact(int64_t nwords, const uint32_t* flag, const int64_t* woff, const int32_t* fr, const int32_t* fd,
-                    int32_t* p_read, int32_t* p_diag, int64_t pcap, const int16_t* ub, int16_t* p_ub, cudaStream_t st) {
-  if (nwords <= 0) return;
-  int64_t blocks = (nwords + 255) / 256;
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  compact_kernel<<<(unsigned)blocks, 256, 0, st>>>(nwords, flag, woff, fr, fd, p_read, p_diag, pcap, ub, p_ub);
+static unsigned select_grid(int64_t ncap) { return (unsigned)std::clamp<int64_t>(select_tiles(ncap), 1, 148 * 8); }
+
+void launch_select_count(int64_t ncap, const unsigned long long* n_dev, const uint8_t* flag, int64_t* tile,
+                         unsigned long long* ticket, const SelectGate& g0, const SelectGate& g1, cudaStream_t st) {
+  select_count_kernel<<<select_grid(ncap), kSelectThreads, 0, st>>>(ncap, n_dev, flag, tile, ticket, g0, g1);
+}
+
+void launch_select_write(int64_t ncap, const unsigned long long* n_dev, const uint8_t* flag, const int64_t* tile,
+                         const int32_t* fr, const int32_t* fd, int32_t* p_read, int32_t* p_diag, int64_t pcap,
+                         const int16_t* ub, int16_t* p_ub, cudaStream_t st) {
+  select_write_kernel<<<select_grid(ncap), kSelectThreads, 0, st>>>(ncap, n_dev, flag, tile, fr, fd, p_read, p_diag, pcap, ub,
+                                                                    p_ub);
 }
 
 }  // namespace sg

@@ -48,23 +48,21 @@ void launch_expand_reads(const ReadsDev& rd, uint8_t* rexp, int64_t rstride, cud
 
 bool filter_dpx_ok(const ScoreParams& sp, int max_len);
 void launch_filter_flat_job(const FilterJob& job, const ScoreParams& sp, bool dpx, cudaStream_t st);
-// pass bytes of the ncap candidates -> words of 32 pass bits (bit t & 31 of word t >> 5); with
-// n_dev (may be null) only the first *n_dev candidates count, the words after them are zero
-void launch_pack_flags(int64_t ncap, const unsigned long long* n_dev, const uint8_t* flag, uint32_t* words,
-                       cudaStream_t st);
-// A word of pass bits, counted as its number of passing candidates when scanned.
-struct PassWord {
-  uint32_t bits;
-  __host__ __device__ explicit operator int64_t() const {
-#if defined(__CUDA_ARCH__)
-    return __popc(bits);
-#else
-    return __builtin_popcount(bits);
-#endif
-  }
+// What a selection does with its total on the device (all null: nothing): above cap (the lists' size)
+// *status gets bit 2, above limit bit 1; *take becomes the total, or 0 with a status; without one *sum grows
+// by it; *most keeps the largest.
+struct SelectGate {
+  unsigned long long *status, *take, *sum, *most;
+  int64_t cap, limit;
 };
-// passing candidates, in order: word w's set bits go to woff[w], woff[w] + 1, ... (those below
-// pcap: the capacity of p_read / p_diag); with p_ub (may be null) their score bounds too
-void launch_compact(int64_t nwords, const uint32_t* flag, const int64_t* woff, const int32_t* fr, const int32_t* fd,
-                    int32_t* p_read, int32_t* p_diag, int64_t pcap, const int16_t* ub, int16_t* p_ub, cudaStream_t st);
+constexpr int kSelectTile = 4096;  // flag bytes per tile
+inline int64_t select_tiles(int64_t ncap) { return (ncap + kSelectTile - 1) / kSelectTile; }
+// The flagged of the first n_dev (null: all ncap) candidates, in order, in two launches.  tile: select_tiles(ncap)
+// + 1 words, the last of which gets their number; ticket: a zeroed word; flag 16-byte aligned.  The
+// second writes those below pcap (the lists' capacity), with p_ub (may be null) their score bounds too.
+void launch_select_count(int64_t ncap, const unsigned long long* n_dev, const uint8_t* flag, int64_t* tile,
+                         unsigned long long* ticket, const SelectGate& g0, const SelectGate& g1, cudaStream_t st);
+void launch_select_write(int64_t ncap, const unsigned long long* n_dev, const uint8_t* flag, const int64_t* tile,
+                         const int32_t* fr, const int32_t* fd, int32_t* p_read, int32_t* p_diag, int64_t pcap,
+                         const int16_t* ub, int16_t* p_ub, cudaStream_t st);
 }  // namespace sg

@@ -692,6 +692,14 @@ static int map_passes_ahead(stormgpu_ctx* c, const PassSetup& P, int64_t launche
   return 0;
 }
 
+// Alignment rounds of a pass that aligns about `kept` candidates of n reads, at most `most`.  Rounds pay
+// where reads have so many candidates that each round lets the bound drop most of what is left: mixed
+// reads of a repeat-rich genome at -i 15, 360 per read and strand, alignment 17.1 -> 13.1 ms with 4 rounds
+// (23 % of the cells).  With few per read all the rounds do is to align them a part at a time, each
+// taking as long as its longest read: 14 per read 4.8 -> 9.6 ms (ragged reads at -i 5), 1.6 per read
+// 0.61 -> 0.86 ms (48 Mbp), as in a call of a few reads.
+static int align_rounds(int most, int64_t n, double kept) { return n <= 256 || kept < 32.0 * (double)n ? 1 : most; }
+
 static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, stormgpu_results* out) {
   if (!c->indexed) { sg_set_error("stormgpu_build_index must be called before mapping"); return STORMGPU_ESTATE; }
   cudaStream_t st = c->st;
@@ -762,11 +770,9 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const i
         (!filter_H && c->rexp.grow(n * rexp_stride(maxL))))
       return STORMGPU_ENOMEM;
   }
-  // Rounds pay where the bound lets each round drop most of what is left (mixed reads at -i 15: 45 % of
-  // the cells of one round); without it they only shorten alignments that stop early (3 %) and cost
-  // an alignment's latency each (300 colour reads: alignment and replay 0.70 -> 0.60 ms), as they do in a call of a few reads.
-  const int rounds = !bound_H || n <= 256 ? 1 : std::max(1, std::min<int>(c->tune.align_rounds, kMaxAlignRounds));
-  const PassSetup P{sp, fwd, rev, n, maxL, minL, wsum, wpr, tbs, rounds, filter_H, bound_H, out};
+  const int most_rounds = !bound_H ? 1 : std::max(1, std::min<int>(c->tune.align_rounds, kMaxAlignRounds));
+  const int rounds_ahead = align_rounds(most_rounds, n, c->gdens_kept * wsum);
+  const PassSetup P{sp, fwd, rev, n, maxL, minL, wsum, wpr, tbs, rounds_ahead, filter_H, bound_H, out};
   if (c->graphs && c->gdens_cand > 0 && c->huge_cap <= ((int64_t)1 << 22)) {
     const int g = map_passes_ahead(c, P, launches);
     if (g != kHostSynced) return g;
@@ -885,6 +891,7 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const i
         SG_CUDA(cudaStreamSynchronize(st));
       }
       max_kept = std::max(max_kept, nkept);
+      const int rounds = align_rounds(most_rounds, n, (double)nkept);
       if (nkept > 0) {
         if (c->p_read.grow(nkept) || c->p_diag.grow(nkept) || c->k_diag.grow(nkept) || c->a_score.grow(nkept) || c->a_bound.grow(nkept) ||
             c->a_tblen.grow(nkept) || c->a_pos.grow(nkept * 4) || c->a_tb.grow(nkept * tbs) ||

@@ -137,8 +137,8 @@ struct stormgpu_ctx {
 
 namespace sg {
 
-// One batch on c's stream (every pointer in reads / out on the device); synchronous.
-// reads and results in device memory; lengths: the reads' lengths on the host, or null (then copied here)
+// One batch on c's stream (every pointer in reads / out on the device); synchronous.  lengths: the
+// reads' lengths on the host, or null (then measured on the device).
 int map_device_impl(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, stormgpu_results* out);
 
 }  // namespace sg

@@ -300,7 +300,32 @@ static __global__ void length_keys_kernel(const int16_t* __restrict__ lengths, i
 }
 
 // Work weight of a read: its seed positions, about L - 15 (candidates grow with them).
-static inline double read_weight(int L) { return L > 16 ? (double)(L - 15) : 1.0; }
+__host__ __device__ static inline int read_weight(int L) { return L > 16 ? L - 15 : 1; }
+
+// What a call needs of its reads' lengths: the longest, 1024 less the shortest (both from 0 up, so that
+// one maximum gives them), and the batch's weight.
+struct LengthStats {
+  unsigned long long longest, shortest_c, weight;
+};
+
+__global__ void __launch_bounds__(256) length_stats_kernel(const int16_t* __restrict__ lengths, int64_t n, LengthStats* out) {
+  int hi = 0, lo_c = 0;
+  unsigned long long w = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int L = lengths[i];
+    hi = max(hi, L);
+    lo_c = max(lo_c, STORMGPU_MAX_READ_LEN - L);
+    w += (unsigned long long)read_weight(L);
+  }
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  lo_c = __reduce_max_sync(0xffffffffu, lo_c);
+  for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&out->longest, (unsigned long long)hi);
+    atomicMax(&out->shortest_c, (unsigned long long)lo_c);
+    atomicAdd(&out->weight, w);
+  }
+}
 
 // ------------------------------------------------------------------------------ passes ahead
 //
@@ -700,7 +725,34 @@ static int map_passes_ahead(stormgpu_ctx* c, const PassSetup& P, int64_t launche
 // 0.61 -> 0.86 ms (48 Mbp), as in a call of a few reads.
 static int align_rounds(int most, int64_t n, double kept) { return n <= 256 || kept < 32.0 * (double)n ? 1 : most; }
 
-static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, stormgpu_results* out) {
+// The lengths' measures: from the host's copy when there is one, else by a kernel (400,000 lengths copied
+// and walked by the host took 1 ms of a 31 ms call).
+static int length_stats(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, LengthStats* out) {
+  memset(out, 0, sizeof(*out));
+  const int64_t n = reads->n;
+  if (n <= 0) return 0;
+  if (lengths) {
+    int hi = 0, lo_c = 0;
+    int64_t w = 0;
+    for (int64_t r = 0; r < n; ++r) {
+      const int L = lengths[r];
+      hi = std::max(hi, L);
+      lo_c = std::max(lo_c, STORMGPU_MAX_READ_LEN - L);
+      w += read_weight(L);
+    }
+    *out = {(unsigned long long)hi, (unsigned long long)lo_c, (unsigned long long)w};
+    return 0;
+  }
+  if (c->counters.grow(kCounters)) return STORMGPU_ENOMEM;
+  LengthStats* d = reinterpret_cast<LengthStats*>(c->counters.p);
+  SG_CUDA(cudaMemsetAsync(d, 0, sizeof(*d), c->st));
+  length_stats_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 148 * 4), 256, 0, c->st>>>(reads->lengths, n, d);
+  SG_CUDA(cudaMemcpyAsync(out, d, sizeof(*d), cudaMemcpyDeviceToHost, c->st));
+  SG_CUDA(cudaStreamSynchronize(c->st));
+  return 0;
+}
+
+static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const LengthStats& ls, stormgpu_results* out) {
   if (!c->indexed) { sg_set_error("stormgpu_build_index must be called before mapping"); return STORMGPU_ESTATE; }
   cudaStream_t st = c->st;
   const int64_t n = reads->n;
@@ -710,13 +762,8 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const i
   memset(&S, 0, sizeof(S));
   S.ms_index = ms_index;
   int64_t launches = 0;
-  int maxL = 0, minL = STORMGPU_MAX_READ_LEN;
-  double wsum = 0;  // the batch's work weight (read_weight)
-  for (int64_t r = 0; r < n; ++r) {
-    maxL = std::max<int>(maxL, lengths[r]);
-    minL = std::min<int>(minL, lengths[r]);
-    wsum += read_weight(lengths[r]);
-  }
+  const int maxL = (int)ls.longest, minL = STORMGPU_MAX_READ_LEN - (int)ls.shortest_c;
+  const double wsum = (double)ls.weight;  // the batch's work weight (read_weight)
   if (maxL > STORMGPU_MAX_READ_LEN) { sg_set_error("read longer than %d", STORMGPU_MAX_READ_LEN); return STORMGPU_EINVAL; }
   if (out->tb_stride < (maxL + c->p.allowed_indels + 1) / 2) { sg_set_error("tb_stride too small"); return STORMGPU_EINVAL; }
   launch_init_results(n, out->hits, out->mapped, out->tb, out->tb_stride, st);
@@ -990,7 +1037,7 @@ static int map_range(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t
   o.hits += 4 * lo;
   o.tb += 4 * lo * out->tb_stride;
   o.mapped += lo;
-  return sg::map_device_impl(c, &r, lengths + lo, &o);
+  return sg::map_device_impl(c, &r, lengths ? lengths + lo : nullptr, &o);
 }
 
 // Maps the batch as consecutive pieces [cuts[q], cuts[q + 1]), the stats summed.
@@ -1017,26 +1064,25 @@ static int map_pieces(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_
 }
 
 int sg::map_device_impl(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, stormgpu_results* out) {
-  std::vector<int16_t> hl;
-  if (!lengths) {
-    hl.resize(std::max<int64_t>(reads->n, 1));
-    if (reads->n > 0) {
-      SG_CUDA(cudaMemcpyAsync(hl.data(), reads->lengths, sizeof(int16_t) * reads->n, cudaMemcpyDeviceToHost, c->st));
-      SG_CUDA(cudaStreamSynchronize(c->st));
-    }
-    lengths = hl.data();
-  }
+  LengthStats ls;
+  if (const int e = length_stats(c, reads, lengths, &ls)) return e;
   if (reads->n > 1 && (c->dens_cand > 0 || c->dens_pass > 0)) {
     // at the last call's density per unit of work weight the batch would be cut after its
     // gather: cut it now, into pieces of equal weight (a batch's reads need not be mixed: a file
     // of several lengths often lists them one length after the other).  0.8: the pieces still
     // differ in repeat content; one that overflows is cut after its gather.
     const int64_t n = reads->n;
-    double W = 0.0;
-    for (int64_t r = 0; r < n; ++r) W += read_weight(lengths[r]);
+    const double W = (double)ls.weight;
     const double need = std::max(c->dens_cand * W / (0.8 * (double)kMaxCandidatesPerPass),
                                  c->dens_pass * W / (0.8 * (double)kMaxPassingPerPass));
     if (need > 1.0) {
+      std::vector<int16_t> hl;
+      if (!lengths) {
+        hl.resize(n);
+        SG_CUDA(cudaMemcpyAsync(hl.data(), reads->lengths, sizeof(int16_t) * n, cudaMemcpyDeviceToHost, c->st));
+        SG_CUDA(cudaStreamSynchronize(c->st));
+        lengths = hl.data();
+      }
       std::vector<double> cum(n + 1, 0.0);
       for (int64_t r = 0; r < n; ++r) cum[r + 1] = cum[r] + read_weight(lengths[r]);
       const int64_t k = std::min<int64_t>(n, (int64_t)std::ceil(need));
@@ -1053,7 +1099,7 @@ int sg::map_device_impl(stormgpu_ctx* c, const stormgpu_reads* reads, const int1
   WorkBudget* saved = g_work_budget;
   g_work_budget = &c->work;
   c->work.over = false;
-  int rc = map_device_once(c, reads, lengths, out);
+  int rc = map_device_once(c, reads, ls, out);
   g_work_budget = saved;
   const int64_t n = reads->n;
   if (rc == STORMGPU_ENOMEM && c->work.over) {

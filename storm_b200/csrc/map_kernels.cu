@@ -1027,9 +1027,7 @@ void launch_replay(int64_t n, const ScoreParams& sp, int ref_id, int sense, Pass
 
 // ------------------------------------------------------------------------------ slots of a read
 
-__global__ void slot_starts_kernel(int64_t npass, const int64_t* __restrict__ npass_dev,
-                                   const int32_t* __restrict__ p_read, int32_t* __restrict__ pstart) {
-  if (npass_dev) npass = *npass_dev;
+__device__ __forceinline__ void slot_starts(int64_t npass, const int32_t* p_read, int32_t* pstart) {
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < npass; s += (int64_t)gridDim.x * blockDim.x) {
     const int r = p_read[s];
     if (s == 0 || p_read[s - 1] != r) pstart[r] = (int32_t)s;
@@ -1040,8 +1038,7 @@ __global__ void slot_starts_kernel(int64_t npass, const int64_t* __restrict__ np
 // slots: the first `take` of each read (their bounds exceed -t, the threshold it starts from).  A
 // slot's place in its read is the number of smaller diagonals of the read (they are distinct),
 // counted here for reads with few slots; the others go to the long list.
-__global__ void slot_lists_kernel(KeptList kl, int16_t* __restrict__ ub, PassBuffers pb, int take) {
-  const int64_t npass = kl.n_dev ? *kl.n_dev : kl.n;
+__device__ __forceinline__ void slot_lists(int64_t npass, const KeptList& kl, int16_t* ub, const PassBuffers& pb, int take) {
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < npass; base += stride) {
@@ -1087,9 +1084,8 @@ __global__ void slot_lists_kernel(KeptList kl, int16_t* __restrict__ ub, PassBuf
 // The reads of the long list, one warp each: their slots copied when they are ascending already (the
 // block gather's reads), else sorted in shared memory as (diagonal, bound) keys.
 constexpr int kSortWarps = 4;
-__global__ void __launch_bounds__(kSortWarps * 32) slot_sort_kernel(KeptList kl, int16_t* __restrict__ ub, PassBuffers pb,
-                                                                    int cap) {
-  extern __shared__ unsigned long long skeys[];  // cap per warp, a power of two
+__device__ __forceinline__ void slot_sort(const KeptList& kl, int16_t* ub, const PassBuffers& pb, int cap,
+                                          unsigned long long* skeys) {  // cap per warp, a power of two
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   unsigned long long* a = skeys + (size_t)w * cap;
   const int n = *kl.long_count;
@@ -1131,14 +1127,45 @@ __global__ void __launch_bounds__(kSortWarps * 32) slot_sort_kernel(KeptList kl,
   }
 }
 
+__global__ void slot_starts_kernel(KeptList kl, PassBuffers pb) {
+  slot_starts(kl.n_dev ? *kl.n_dev : kl.n, pb.p_read, pb.pstart);
+}
+
+__global__ void slot_lists_kernel(KeptList kl, int16_t* __restrict__ ub, PassBuffers pb, int take) {
+  slot_lists(kl.n_dev ? *kl.n_dev : kl.n, kl, ub, pb, take);
+}
+
+__global__ void __launch_bounds__(kSortWarps * 32) slot_sort_kernel(KeptList kl, int16_t* __restrict__ ub, PassBuffers pb,
+                                                                    int cap) {
+  extern __shared__ unsigned long long skeys[];
+  slot_sort(kl, ub, pb, cap, skeys);
+}
+
+// The three by one block, for a call of few reads (three launches of 2.5 to 5 us each).
+__global__ void __launch_bounds__(kSortWarps * 32) slots_small_kernel(KeptList kl, int16_t* ub, PassBuffers pb, int take,
+                                                                      int cap) {
+  extern __shared__ unsigned long long skeys[];
+  const int64_t n = kl.n_dev ? *kl.n_dev : kl.n;
+  slot_starts(n, pb.p_read, pb.pstart);
+  __syncthreads();
+  slot_lists(n, kl, ub, pb, take);
+  __syncthreads();
+  slot_sort(kl, ub, pb, cap, skeys);
+}
+
 void launch_slot_lists(const KeptList& kl, int16_t* ub, PassBuffers& pb, int take, cudaStream_t st) {
   if (kl.n <= 0) return;
-  const int64_t blocks = std::min<int64_t>((kl.n + 255) / 256, 148 * 32);
-  slot_starts_kernel<<<(unsigned)blocks, 256, 0, st>>>(kl.n, kl.n_dev, pb.p_read, pb.pstart);
-  slot_lists_kernel<<<(unsigned)blocks, 256, 0, st>>>(kl, ub, pb, take);
   int cap = 64;
   while (cap < kl.sort_cap) cap <<= 1;
   const size_t smem = (size_t)kSortWarps * cap * sizeof(unsigned long long);
+  if (kl.n <= kSlotsSmall) {
+    set_smem_attribute_once(reinterpret_cast<const void*>(slots_small_kernel), kSortWarps * 2048 * 8);
+    slots_small_kernel<<<1, kSortWarps * 32, smem, st>>>(kl, ub, pb, take, cap);
+    return;
+  }
+  const int64_t blocks = std::min<int64_t>((kl.n + 255) / 256, 148 * 32);
+  slot_starts_kernel<<<(unsigned)blocks, 256, 0, st>>>(kl, pb);
+  slot_lists_kernel<<<(unsigned)blocks, 256, 0, st>>>(kl, ub, pb, take);
   set_smem_attribute_once(reinterpret_cast<const void*>(slot_sort_kernel), kSortWarps * 2048 * 8);
   const int64_t grid = std::min<int64_t>((kl.n / kShortSlots + kSortWarps) / kSortWarps,
                                          resident_grid(slot_sort_kernel, kSortWarps * 32, smem));

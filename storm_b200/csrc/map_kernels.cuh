@@ -133,6 +133,7 @@ constexpr int kShortSlots = 64;
 // pb.p_diag / pb.ub from the list, ascending within each read; pstart / pcount and the first active
 // list; with rounds the first round's slots, `take` per read.  The counts are zeroed by the caller.
 // pb.p_read is the list's.
+constexpr int64_t kSlotsSmall = 2048;  // up to so many by one launch of one block, else by three
 void launch_slot_lists(const KeptList& kl, int16_t* ub, PassBuffers& pb, int take, cudaStream_t st);
 // Replay of the active reads (at most n): the whole read (no rounds), or the ranks selected last and
 // then the selection of up to `take` candidates for the next round.

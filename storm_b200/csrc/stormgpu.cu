@@ -591,9 +591,17 @@ static int enqueue_passes(stormgpu_ctx* c, const PassSetup& P, const AheadCaps& 
       const SelectGate passing{gs + kGsStatus, gs + kGsPass, gs + kGsPassed, gs + kGsMaxPass, pass_cap,
                                n > 1 ? kMaxPassingPerPass : INT64_MAX};
       const SelectGate kept{gs + kGsStatus, gs + kGsKept, gs + kGsAligned, gs + kGsMaxKept, kept_cap, INT64_MAX};
-      launch_select_count(cand_cap, gs + kGsCand, c->flag.p, c->foff.p, gs + kCntSelect, passing,
-                          P.bound_H ? SelectGate{} : kept, st);
-      launches++;
+      auto select = [&](int64_t cap, int take, int which, const SelectGate& g0, const SelectGate& g1, const int32_t* fr,
+                        const int32_t* fd, int32_t* o_read, int32_t* o_diag, int64_t ocap, const int16_t* ub, int16_t* o_ub) {
+        if (cand_cap <= kSelectSmall) {
+          launch_select_small(cap, gs + take, c->flag.p, g0, g1, fr, fd, o_read, o_diag, ocap, ub, o_ub, st);
+          launches++;
+          return;
+        }
+        launch_select_count(cap, gs + take, c->flag.p, c->foff.p, gs + kCntSelect + which, g0, g1, st);
+        launch_select_write(cap, gs + take, c->flag.p, c->foff.p, fr, fd, o_read, o_diag, ocap, ub, o_ub, st);
+        launches += 2;
+      };
       PassBuffers pb;
       memset(&pb, 0, sizeof(pb));
       pb.pstart = c->pstart.p; pb.pcount = c->pcount.p;
@@ -601,23 +609,19 @@ static int enqueue_passes(stormgpu_ctx* c, const PassSetup& P, const AheadCaps& 
       pb.p_read = c->p_read.p; pb.p_diag = c->p_diag.p; pb.p_cap = kept_cap;
       if (P.bound_H) {
         // the candidates whose score can exceed -t, in order
-        launch_select_write(cand_cap, gs + kGsCand, c->flag.p, c->foff.p, c->fr.p, c->fd.p, c->q_read.p, c->q_diag.p,
-                            pass_cap, nullptr, nullptr, st);
+        select(cand_cap, kGsCand, 0, passing, {}, c->fr.p, c->fd.p, c->q_read.p, c->q_diag.p, pass_cap, nullptr, nullptr);
         launch_bound_pass(c, P, rd, R, pass_cap, reinterpret_cast<const int64_t*>(gs + kGsPass), st);
-        launch_select_count(pass_cap, gs + kGsPass, c->flag.p, c->foff.p, gs + kCntSelect + 1, kept, SelectGate{}, st);
-        launch_select_write(pass_cap, gs + kGsPass, c->flag.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->k_diag.p,
-                            kept_cap, c->q_ub.p, c->k_ub.p, st);
+        select(pass_cap, kGsPass, 1, kept, {}, c->q_read.p, c->q_diag.p, c->p_read.p, c->k_diag.p, kept_cap, c->q_ub.p,
+               c->k_ub.p);
         pb.ub = c->p_ub.p;
-        launches += 4;
-      } else {
-        launch_select_write(cand_cap, gs + kGsCand, c->flag.p, c->foff.p, c->fr.p, c->fd.p, c->p_read.p, c->k_diag.p,
-                            kept_cap, nullptr, nullptr, st);
         launches++;
+      } else {
+        select(cand_cap, kGsCand, 0, passing, kept, c->fr.p, c->fd.p, c->p_read.p, c->k_diag.p, kept_cap, nullptr, nullptr);
       }
       const int64_t* np = reinterpret_cast<const int64_t*>(gs + kGsKept);
       setup_rounds(c, rounds, pb);
       launch_slot_lists(kept_list(c, P, kept_cap, np), c->p_ub.p, pb, align_round_take(0, rounds), st);
-      launches += 3;
+      launches += kept_cap <= kSlotsSmall ? 1 : 3;
       pb.a_score = c->a_score.p; pb.a_bound = c->a_bound.p; pb.a_tblen = c->a_tblen.p;
       pb.a_pos = c->a_pos.p; pb.a_tb = c->a_tb.p; pb.tbs = P.tbs;
       pb.npass_dev = np;
@@ -720,7 +724,7 @@ static int map_passes_ahead(stormgpu_ctx* c, const PassSetup& P, int64_t launche
 // Alignment rounds of a pass that aligns about `kept` candidates of n reads, at most `most`.  Rounds pay
 // where reads have so many candidates that each round lets the bound drop most of what is left: mixed
 // reads of a repeat-rich genome at -i 15, 360 per read and strand, alignment 17.1 -> 13.1 ms with 4 rounds
-// (23 % of the cells).  With few per read all the rounds do is to align them a part at a time, each
+// (43 % of the cells).  With few per read all the rounds do is to align them a part at a time, each
 // taking as long as its longest read: 14 per read 4.8 -> 9.6 ms (ragged reads at -i 5), 1.6 per read
 // 0.61 -> 0.86 ms (48 Mbp), as in a call of a few reads.
 static int align_rounds(int most, int64_t n, double kept) { return n <= 256 || kept < 32.0 * (double)n ? 1 : most; }
@@ -956,7 +960,7 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const L
         if (round_lists_grow(c, n, nkept, rounds)) return STORMGPU_ENOMEM;
         setup_rounds(c, rounds, pb);
         launch_slot_lists(kept_list(c, P, nkept, nullptr), c->p_ub.p, pb, align_round_take(0, rounds), st);
-        launches += 4;
+        launches += nkept <= kSlotsSmall ? 2 : 4;
         pb.a_score = c->a_score.p; pb.a_bound = c->a_bound.p; pb.a_tblen = c->a_tblen.p;
         pb.a_pos = c->a_pos.p; pb.a_tb = c->a_tb.p; pb.tbs = tbs;
         // one persistent launch over all kept candidates; scratch for its threads only

@@ -392,6 +392,42 @@ __global__ void __launch_bounds__(kSelectThreads) select_write_kernel(
   }
 }
 
+// The same by one block in one launch, tile after tile, for the lists of a call of few reads.
+__global__ void __launch_bounds__(kSelectThreads) select_small_kernel(
+    int64_t ncap, const unsigned long long* __restrict__ n_dev, const uint8_t* __restrict__ flag, SelectGate g0, SelectGate g1,
+    const int32_t* __restrict__ fr, const int32_t* __restrict__ fd, int32_t* __restrict__ p_read,
+    int32_t* __restrict__ p_diag, int64_t pcap, const int16_t* __restrict__ ub, int16_t* __restrict__ p_ub) {
+  __shared__ int wsum[kSelectThreads / 32];
+  const int64_t n = min(ncap, (int64_t)*n_dev);
+  int64_t total = 0;
+  for (int64_t base = 0; base < n; base += kSelectTile) {
+    const int64_t t0 = base + threadIdx.x * 16;
+    uint32_t m = flags16(flag, t0, n);
+    int all;
+    int64_t o = total + select_scan<int>(__popc(m), wsum, &all);
+    total += all;
+    while (m && o < pcap) {
+      const int64_t c = t0 + (__ffs(m) - 1);
+      p_read[o] = fr[c];
+      p_diag[o] = fd[c];
+      if (p_ub) p_ub[o] = ub[c];
+      ++o;
+      m &= m - 1;
+    }
+  }
+  __syncthreads();  // every thread has its n
+  if (threadIdx.x == 0) {
+    apply_gate(g0, total);
+    apply_gate(g1, total);
+  }
+}
+
+void launch_select_small(int64_t ncap, const unsigned long long* n_dev, const uint8_t* flag, const SelectGate& g0,
+                         const SelectGate& g1, const int32_t* fr, const int32_t* fd, int32_t* p_read, int32_t* p_diag,
+                         int64_t pcap, const int16_t* ub, int16_t* p_ub, cudaStream_t st) {
+  select_small_kernel<<<1, kSelectThreads, 0, st>>>(ncap, n_dev, flag, g0, g1, fr, fd, p_read, p_diag, pcap, ub, p_ub);
+}
+
 static unsigned select_grid(int64_t ncap) { return (unsigned)std::clamp<int64_t>(select_tiles(ncap), 1, 148 * 8); }
 
 void launch_select_count(int64_t ncap, const unsigned long long* n_dev, const uint8_t* flag, int64_t* tile,

@@ -65,4 +65,11 @@ void launch_select_count(int64_t ncap, const unsigned long long* n_dev, const ui
 void launch_select_write(int64_t ncap, const unsigned long long* n_dev, const uint8_t* flag, const int64_t* tile,
                          const int32_t* fr, const int32_t* fd, int32_t* p_read, int32_t* p_diag, int64_t pcap,
                          const int16_t* ub, int16_t* p_ub, cudaStream_t st);
+// Both in one launch of one block, for candidate lists of a capacity up to kSelectSmall (a call of few
+// reads: the spare 61,440 places and at most 3,300 expected candidates, so one tile of about 5 us where
+// the two launches take 10; a full list would take 30).
+constexpr int64_t kSelectSmall = 1 << 16;
+void launch_select_small(int64_t ncap, const unsigned long long* n_dev, const uint8_t* flag, const SelectGate& g0,
+                         const SelectGate& g1, const int32_t* fr, const int32_t* fd, int32_t* p_read, int32_t* p_diag,
+                         int64_t pcap, const int16_t* ub, int16_t* p_ub, cudaStream_t st);
 }  // namespace sg

@@ -208,21 +208,22 @@ int stormgpu_genome_map_contextual(stormgpu_ctx *ctx, int32_t uniqueness, int32_
 typedef struct stormgpu_stats {
   int64_t candidates;        /* diagonals produced by the hit gather */
   int64_t filter_passed;     /* diagonals passing the banded SW filter */
-  int64_t aligned;           /* full alignments computed */
+  int64_t aligned;           /* candidates the full alignment is for: those that pass the filter
+                                and, in nucleotide space, whose score bound exceeds -t */
   int64_t seed_lookups;      /* (seed, read position) key lookups */
   int64_t hit_positions;     /* index positions read by the hit gather */
   int64_t filter_cells;      /* filter cell updates: W * 2 * (L + W - 1) per candidate, W = 2..16 */
   int64_t align_cells;       /* band cells the full alignment computed: 2*i+1 per row, L rows for
                                 a candidate that runs to its last row, fewer for one that stops
-                                once it can no longer be accepted */
+                                once it can no longer be accepted, none for one that a round
+                                leaves out */
   int64_t kernels;           /* kernel launches */
   int64_t filter_band_cells; /* band cells of the filtered diagonals: L * (2*min(i,15)+1) each */
   double  ms_index, ms_gather, ms_filter, ms_align, ms_replay, ms_total;
   int64_t passes;            /* strand passes run (one filter launch each; a batch cut into pieces
                                 runs one per piece, sequence and strand) */
-  int64_t graph_passes;      /* of them, passes that ran inside a CUDA graph (every pass of a call
-                                captured as one graph and launched once, no host read between
-                                its launches) */
+  int64_t graph_passes;      /* of them, passes enqueued ahead: no host read between the launches
+                                of a call, list sizes read on the device */
   int64_t placement_waves;   /* waves of the last stormgpu_genome_map_contextual call on the
                                 context (reads placed together in one wave share no position) */
 } stormgpu_stats;
@@ -241,17 +242,20 @@ typedef struct stormgpu_tuning {
                                      a multiple of 32 */
   int32_t filter_cursor;          /* 1: the filter runs as a persistent grid whose blocks take tiles
                                      from a work cursor; 0: one block per tile */
-  int32_t align_rounds;           /* 1..6: a read's passing candidates are aligned in this many
-                                     rounds of increasing rank (the first 8, then up to 32, 128,
-                                     512, 2048, then the rest), each followed by the replay of its
-                                     ranks; a later round's alignment stops as soon as it cannot
-                                     reach the read's running threshold.  1: one round */
+  int32_t align_rounds;           /* 1..6: a read's candidates are aligned in at most this many
+                                     rounds (its next 8, 16, 32, 64, 128 candidates whose score
+                                     bound exceeds the read's running threshold, then the rest of
+                                     them), each followed by the replay of its candidates.  One
+                                     round without a bound (colour space, bands above 47 cells),
+                                     for at most 256 reads, and where a pass has fewer than 32
+                                     candidates per read */
 } stormgpu_tuning;
-/* CUDA graphs (default on, unless the environment sets STORMGPU_GRAPHS=0 when the context
- * opens): from the second mapping call of a context on, all strand passes of a call are
- * captured as one graph, with every list sized from the densest pass seen so far (+25 %), and
- * launched once; a call whose lists outgrow those sizes is run again as separate launches with
- * the host reading each list size (the results are the same either way).  0 turns them off. */
+/* Passes enqueued ahead (default on, unless the environment sets STORMGPU_GRAPHS=0 when the
+ * context opens; earlier versions captured them as a CUDA graph, hence the names): from the
+ * second mapping call of a context on, all strand passes of a call are launched without a host
+ * wait between them, with every list sized from the densest pass seen so far (+25 %); a call
+ * whose lists outgrow those sizes is run again with the host reading each list size (the
+ * results are the same either way).  0 turns this off. */
 int stormgpu_set_graphs(stormgpu_ctx *ctx, int enable);
 /* The context's parameters (defaults 768, 4, 8, 32, 0, 4). */
 int stormgpu_get_tuning(stormgpu_ctx *ctx, stormgpu_tuning *out);

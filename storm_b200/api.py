@@ -245,7 +245,7 @@ class Mapper:
         return read[:npl.value], rank[:npl.value]
 
     def set_graphs(self, enable: bool):
-        """CUDA graphs for the strand passes (on by default; the results are the same)."""
+        """Strand passes enqueued ahead, without host waits (on by default; the results are the same)."""
         _check(lib().stormgpu_set_graphs(self._ctx, 1 if enable else 0))
 
     def autotune(self, batch: ReadBatch, sample: int = 200000) -> dict:

@@ -84,10 +84,13 @@ __device__ __forceinline__ void add_filter_counters(unsigned long long* counters
 }
 
 // Calls body(t) for the block's candidates t < n: with a cursor (CURSOR) tiles of `rows` rows
-// taken from it one after the other, else the one tile blockIdx.x of kFilterTile rows.  One
+// taken from it one after the other, else the one tile blockIdx.x of kFilterTile rows, or, where the
+// list does not fill the GPU with such tiles, of as few rows as spread it over the grid (a thread takes
+// its rows one after the other: 117,000 candidates of 300 colour reads 116 us with 8 rows, 34 with
+// 2; beyond that size fewer rows than 8 ran the colour workload's filter 1 % slower).  One
 // call site of body per instantiation (it is the long unrolled band code).  The one-tile form
-// has no barrier and a constant row count, which keeps the W = 8 kernel within 64 registers
-// without spilling; run through the cursor loop it measured 3 % slower.
+// has no barrier; run through the cursor loop it measured 3 % slower.
+constexpr int64_t kFilterShort = 148 * 3 * 256 * 8;
 template <bool CURSOR, class Body>
 __device__ __forceinline__ void for_filter_tiles(const FilterJob& job, int64_t n, int rows, Body body) {
   if constexpr (CURSOR) {
@@ -99,9 +102,11 @@ __device__ __forceinline__ void for_filter_tiles(const FilterJob& job, int64_t n
         body(t);
       }
   } else {
-    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x * kFilterTile + threadIdx.x;
-    for (int i = 0; i < kFilterTile; ++i) {
-      const int64_t t = t0 + (int64_t)i * blockDim.x;
+    const int64_t row = 256 * (int64_t)gridDim.x;  // candidates of one row of the grid
+    const int mine = n > kFilterShort ? kFilterTile : (int)min((int64_t)kFilterTile, (n + row - 1) / row);
+    const int64_t t0 = (int64_t)blockIdx.x * 256 * mine + threadIdx.x;
+    for (int i = 0; i < mine; ++i) {
+      const int64_t t = t0 + (int64_t)i * 256;
       if (t >= n) break;
       body(t);
     }
@@ -227,7 +232,9 @@ bool filter_dpx_ok(const ScoreParams& sp, int max_len) {
 void launch_filter_flat_job(const FilterJob& job, const ScoreParams& sp, bool dpx, cudaStream_t st) {
   if (job.n <= 0) return;
   const int64_t tile = 256 * (int64_t)(job.cursor && job.rows > 0 ? job.rows : kFilterTile);
-  const int64_t blocks = (job.n + tile - 1) / tile;
+  int64_t blocks = (job.n + tile - 1) / tile;
+  // a short list over every SM, down to one row per block
+  if (!job.cursor) blocks = std::max(blocks, std::min<int64_t>((job.n + 255) / 256, kFilterShort / (256 * kFilterTile)));
   auto grid = [&](const void* k) {
     return (unsigned)(job.cursor ? std::min<int64_t>(blocks, resident_grid_of(k, 256, 0)) : blocks);
   };

@@ -238,10 +238,11 @@ int32_t repeat_cutoff(int stdev_distance, int64_t N, unsigned long long s2, unsi
 
 namespace {
 
-// one seed's build between its sort and its fill
+// one seed's build between its sort and its fill; keys, bound and iv are in the build's one scratch block
 struct Sorted {
   uint32_t *keys = nullptr, *pos = nullptr;
   int32_t* bound = nullptr;
+  int64_t* iv = nullptr;
   int64_t total = 0, nblocks = 0;
 };
 
@@ -270,17 +271,15 @@ int sort_seed(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, const 
   so->nblocks = nkeys / kKeyBlock + 1;  // the last one: the table's closing entry
   // The sorted list ends in its own arrays, whichever way the passes go; the other side of the sort is
   // scratch that every seed of the sequence uses.
-  int64_t* d_iv;
-  SG_CUDA(cudaMallocAsync(&so->keys, sizeof(uint32_t) * total, st));
+  int64_t* const d_iv = so->iv;
   SG_CUDA(cudaMallocAsync(&so->pos, sizeof(uint32_t) * total, st));
-  SG_CUDA(cudaMallocAsync(&so->bound, sizeof(int32_t) * (so->nblocks + 1), st));
-  SG_CUDA(cudaMallocAsync(&d_iv, sizeof(int64_t) * iv.size(), st));
   const int passes = (2 * seed.weight + kRadixBits - 1) / kRadixBits;
   uint32_t* const sk = scratch;
   uint32_t* const sv = sk + n_codes;
   void* const tmp = sv + n_codes;
   uint32_t *k0 = passes & 1 ? sk : so->keys, *v0 = passes & 1 ? sv : so->pos;
   uint32_t *k1 = passes & 1 ? so->keys : sk, *v1 = passes & 1 ? so->pos : sv;
+  if ((int64_t)iv.size() > 4 * ((int64_t)nreg + 2)) { sg_set_error("internal: %zu index intervals", iv.size() / 2); return STORMGPU_EINVAL; }
   SG_CUDA(cudaMemcpyAsync(d_iv, iv.data(), sizeof(int64_t) * iv.size(), cudaMemcpyHostToDevice, st));
   KeySeed ks;
   ks.seed = seed;
@@ -288,7 +287,6 @@ int sort_seed(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, const 
   const int TB = 256;
   seed_keys_kernel<<<blocks_of(total, TB * kKeysPerLane), TB, 0, st>>>(d_codes, d_iv, d_iv + a.size(), (int)a.size(), total, ks, k0, v0);
   radix_sort_pairs(k0, v0, k1, v1, total, 2 * seed.weight, tmp, st);
-  cudaFreeAsync(d_iv, st);
   run_stats_kernel<<<(unsigned)std::min<int64_t>(blocks_of(total, kStatsThreads), 148 * 16), kStatsThreads, 0, st>>>(so->keys, total,
                                                                                            so->nblocks, mom, so->bound);
   L += 2 + 3 * passes;
@@ -327,8 +325,6 @@ int fill_seed(DevIndex* out, const Sorted& so, int32_t cmax, int64_t longest, cu
   key_table_kernel<<<(unsigned)so.nblocks, 256, 0, st>>>(so.keys, so.total, out->nkeys, so.bound, off, total, out->first);
   L++;
   if (off) cudaFreeAsync(off, st);
-  cudaFreeAsync(so.keys, st);
-  cudaFreeAsync(so.bound, st);
   SG_CUDA(cudaGetLastError());
   return 0;
 }
@@ -339,19 +335,39 @@ int build_indexes(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, co
                   const SeedDev* seeds, int nseeds, int stdev_distance, DevIndex* out, cudaStream_t st,
                   int64_t* launches) {
   constexpr int kGroup = 4;  // seeds whose sorted lists are held at once (8 bytes per position each)
-  unsigned long long* mom;
-  uint32_t* scratch;
   const int64_t room = std::max<int64_t>(n_codes, 1);  // indexed positions of a seed
-  SG_CUDA(cudaMallocAsync(&scratch, sizeof(uint32_t) * 2 * room + radix_tmp_bytes(room), st));
-  SG_CUDA(cudaMallocAsync(&mom, sizeof(unsigned long long) * 3 * kGroup, st));
+  // One block for everything a build needs only while it runs: with a block for each, the pool had to map
+  // new memory in one build of thirty (10 to 50 ms against 6; none in 300 builds of 48 Mbp since).
+  const int held = std::min(kGroup, nseeds);
+  int64_t most_keys = 0;
+  for (int q = 0; q < nseeds; ++q) most_keys = std::max(most_keys, (int64_t)1 << (2 * seeds[q].weight));
+  int64_t size = 0;
+  auto take = [&](int64_t bytes) { const int64_t at = size; size += (bytes + 255) & ~255LL; return at; };
+  const int64_t at_scratch = take(sizeof(uint32_t) * 2 * room + radix_tmp_bytes(room));
+  const int64_t at_mom = take(sizeof(unsigned long long) * 3 * kGroup);
+  const int64_t at_keys = take(0), key_bytes = ((int64_t)sizeof(uint32_t) * room + 255) & ~255LL;
+  take(key_bytes * held);
+  const int64_t at_bound = take(0), bound_bytes = ((int64_t)sizeof(int32_t) * (most_keys / kKeyBlock + 2) + 255) & ~255LL;
+  take(bound_bytes * held);
+  const int64_t at_iv = take(0), iv_bytes = ((int64_t)sizeof(int64_t) * 4 * (nreg + 2) + 255) & ~255LL;
+  // (at most two intervals per masked region and one after them, two words each)
+  take(iv_bytes * held);
+  uint8_t* block;
+  SG_CUDA(cudaMallocAsync(&block, size, st));
+  uint32_t* const scratch = reinterpret_cast<uint32_t*>(block + at_scratch);
+  unsigned long long* const mom = reinterpret_cast<unsigned long long*>(block + at_mom);
   int64_t L = 0;
   for (int s0 = 0; s0 < nseeds; s0 += kGroup) {
     const int ng = std::min(kGroup, nseeds - s0);
     Sorted so[kGroup];
     SG_CUDA(cudaMemsetAsync(mom, 0, sizeof(unsigned long long) * 3 * kGroup, st));
-    for (int q = 0; q < ng; ++q)
+    for (int q = 0; q < ng; ++q) {
+      so[q].keys = reinterpret_cast<uint32_t*>(block + at_keys + q * key_bytes);
+      so[q].bound = reinterpret_cast<int32_t*>(block + at_bound + q * bound_bytes);
+      so[q].iv = reinterpret_cast<int64_t*>(block + at_iv + q * iv_bytes);
       if (const int rc = sort_seed(d_codes, n_codes, rs, re, nreg, seeds[s0 + q], &out[s0 + q], &so[q], mom + 3 * q, scratch, st, L))
         return rc;
+    }
     unsigned long long hm[3 * kGroup];
     SG_CUDA(cudaMemcpyAsync(hm, mom, sizeof(hm), cudaMemcpyDeviceToHost, st));
     SG_CUDA(cudaStreamSynchronize(st));
@@ -363,8 +379,7 @@ int build_indexes(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, co
       if (const int rc = fill_seed(o, so[q], o->cmax, (int64_t)hm[3 * q + 2], st, L)) return rc;
     }
   }
-  cudaFreeAsync(mom, st);
-  cudaFreeAsync(scratch, st);
+  cudaFreeAsync(block, st);
   if (launches) *launches += L;
   return 0;
 }

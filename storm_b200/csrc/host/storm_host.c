@@ -1379,18 +1379,21 @@ int sh_write_sam(FILE *f, const sh_sam_opts *o, const sh_refs *refs, const sh_re
   int64_t CH = count / (8 * (int64_t)nthreads);
   CH = CH < 256 ? 256 : CH > 4096 ? 4096 : CH;
   const int64_t nchunks = (count + CH - 1) / CH;
-  int nomem = colour && !chk;
-  if (!nomem) {
-#pragma omp parallel reduction(|| : nomem) if (nchunks > 1)
+  int rc = colour && !chk ? STORMGPU_ENOMEM : 0;  /* once set, nothing more is written (read and set in chunk order) */
+  if (!rc) {
+#pragma omp parallel if (nchunks > 1)
     {
       growbuf g = {0};
 #pragma omp for schedule(dynamic, 1) ordered
       for (int64_t c = 0; c < nchunks; ++c) {
         const int64_t a = first + c * CH, e = a + CH < first + count ? a + CH : first + count;
         g.n = 0;
-        if (write_sam_records(&g, o, refs, reads, res, a, e - a, chk, &qt)) nomem = 1;
+        const int formatted = write_sam_records(&g, o, refs, reads, res, a, e - a, chk, &qt);
 #pragma omp ordered
-        if (g.n) fwrite(g.p, 1, g.n, f);
+        if (!rc) {
+          if (formatted) rc = formatted;
+          else if (g.n && fwrite(g.p, 1, g.n, f) != g.n) rc = STORMGPU_EINVAL;
+        }
       }
       free(g.p);
     }
@@ -1399,7 +1402,10 @@ int sh_write_sam(FILE *f, const sh_sam_opts *o, const sh_refs *refs, const sh_re
     for (int s = 0; s < refs->n; ++s) free(chk[s]);
     free(chk);
   }
-  if (nomem) return fail(STORMGPU_ENOMEM, "Out of memory while writing the SAM output.");
+  if (rc == STORMGPU_ENOMEM) return fail(STORMGPU_ENOMEM, "Out of memory while writing the SAM output.");
+  /* a chunk goes past stdio's buffer: a write that failed leaves nothing there for the caller's fclose to
+   * fail on */
+  if (rc || fflush(f) != 0 || ferror(f)) return fail(STORMGPU_EINVAL, "Cannot write the SAM output.");
   return 0;
 }
 

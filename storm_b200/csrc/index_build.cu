@@ -248,20 +248,22 @@ struct Sorted {
 
 unsigned blocks_of(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
 
-int sort_seed(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, const int32_t* re, int nreg,
-              const SeedDev& seed, DevIndex* out, Sorted* so, unsigned long long* mom, uint32_t* scratch, cudaStream_t st,
-              int64_t& L) {
-  std::vector<int64_t> a, b;
-  indexed_intervals(n_codes, seed.span, rs, re, nreg, a, b);
-  const int64_t nkeys = (int64_t)1 << (2 * seed.weight);
+// A seed's indexed positions: the intervals' starts, then the positions before each; their number.  With
+// masked regions in ascending order it is at most the sequence's length; with regions out of order the
+// walk jumps back and indexes positions again.
+struct Positions {
+  std::vector<int64_t> iv;
+  int nint = 0;
+  int64_t total = 0;
+};
+
+int sort_seed(const uint8_t* d_codes, const Positions& at, const SeedDev& seed, DevIndex* out, Sorted* so,
+              unsigned long long* mom, uint32_t* scratch, int64_t room, cudaStream_t st, int64_t& L) {
+  const int64_t nkeys = (int64_t)1 << (2 * seed.weight), total = at.total;
   out->weight = seed.weight;
   out->nkeys = nkeys;
   out->map = nullptr;
   out->n = 0;
-  std::vector<int64_t> iv(a);  // starts, then positions before each interval
-  int64_t total = 0;
-  for (size_t k = 0; k < a.size(); ++k) { iv.push_back(total); total += b[k] - a[k]; }
-  if (total > INT32_MAX) { sg_set_error("sequence too long for 32-bit positions"); return STORMGPU_EINVAL; }
   SG_CUDA(cudaMallocAsync(&out->first, sizeof(int32_t) * (nkeys + 1), st));
   if (total == 0) {
     SG_CUDA(cudaMemsetAsync(out->first, 0, sizeof(int32_t) * (nkeys + 1), st));
@@ -275,17 +277,16 @@ int sort_seed(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, const 
   SG_CUDA(cudaMallocAsync(&so->pos, sizeof(uint32_t) * total, st));
   const int passes = (2 * seed.weight + kRadixBits - 1) / kRadixBits;
   uint32_t* const sk = scratch;
-  uint32_t* const sv = sk + n_codes;
-  void* const tmp = sv + n_codes;
+  uint32_t* const sv = sk + room;
+  void* const tmp = sv + room;
   uint32_t *k0 = passes & 1 ? sk : so->keys, *v0 = passes & 1 ? sv : so->pos;
   uint32_t *k1 = passes & 1 ? so->keys : sk, *v1 = passes & 1 ? so->pos : sv;
-  if ((int64_t)iv.size() > 4 * ((int64_t)nreg + 2)) { sg_set_error("internal: %zu index intervals", iv.size() / 2); return STORMGPU_EINVAL; }
-  SG_CUDA(cudaMemcpyAsync(d_iv, iv.data(), sizeof(int64_t) * iv.size(), cudaMemcpyHostToDevice, st));
+  SG_CUDA(cudaMemcpyAsync(d_iv, at.iv.data(), sizeof(int64_t) * at.iv.size(), cudaMemcpyHostToDevice, st));
   KeySeed ks;
   ks.seed = seed;
   ks.nruns = seed.span <= 32 ? make_runs(seed, ks.runs) : 0;
   const int TB = 256;
-  seed_keys_kernel<<<blocks_of(total, TB * kKeysPerLane), TB, 0, st>>>(d_codes, d_iv, d_iv + a.size(), (int)a.size(), total, ks, k0, v0);
+  seed_keys_kernel<<<blocks_of(total, TB * kKeysPerLane), TB, 0, st>>>(d_codes, d_iv, d_iv + at.nint, at.nint, total, ks, k0, v0);
   radix_sort_pairs(k0, v0, k1, v1, total, 2 * seed.weight, tmp, st);
   run_stats_kernel<<<(unsigned)std::min<int64_t>(blocks_of(total, kStatsThreads), 148 * 16), kStatsThreads, 0, st>>>(so->keys, total,
                                                                                            so->nblocks, mom, so->bound);
@@ -335,7 +336,19 @@ int build_indexes(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, co
                   const SeedDev* seeds, int nseeds, int stdev_distance, DevIndex* out, cudaStream_t st,
                   int64_t* launches) {
   constexpr int kGroup = 4;  // seeds whose sorted lists are held at once (8 bytes per position each)
-  const int64_t room = std::max<int64_t>(n_codes, 1);  // indexed positions of a seed
+  std::vector<Positions> at(nseeds);
+  int64_t room = 1, iv_words = 0;  // most indexed positions, interval words of a seed
+  for (int q = 0; q < nseeds; ++q) {
+    std::vector<int64_t> a, b;
+    indexed_intervals(n_codes, seeds[q].span, rs, re, nreg, a, b);
+    Positions& x = at[q];
+    x.nint = (int)a.size();
+    x.iv = a;
+    for (size_t k = 0; k < a.size(); ++k) { x.iv.push_back(x.total); x.total += b[k] - a[k]; }
+    if (x.total > INT32_MAX) { sg_set_error("sequence too long for 32-bit positions"); return STORMGPU_EINVAL; }
+    room = std::max(room, x.total);
+    iv_words = std::max(iv_words, (int64_t)x.iv.size());
+  }
   // One block for everything a build needs only while it runs: with a block for each, the pool had to map
   // new memory in one build of thirty (10 to 50 ms against 6; none in 300 builds of 48 Mbp since).
   const int held = std::min(kGroup, nseeds);
@@ -349,8 +362,7 @@ int build_indexes(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, co
   take(key_bytes * held);
   const int64_t at_bound = take(0), bound_bytes = ((int64_t)sizeof(int32_t) * (most_keys / kKeyBlock + 2) + 255) & ~255LL;
   take(bound_bytes * held);
-  const int64_t at_iv = take(0), iv_bytes = ((int64_t)sizeof(int64_t) * 4 * (nreg + 2) + 255) & ~255LL;
-  // (at most two intervals per masked region and one after them, two words each)
+  const int64_t at_iv = take(0), iv_bytes = ((int64_t)sizeof(int64_t) * iv_words + 255) & ~255LL;
   take(iv_bytes * held);
   uint8_t* block;
   SG_CUDA(cudaMallocAsync(&block, size, st));
@@ -365,7 +377,7 @@ int build_indexes(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, co
       so[q].keys = reinterpret_cast<uint32_t*>(block + at_keys + q * key_bytes);
       so[q].bound = reinterpret_cast<int32_t*>(block + at_bound + q * bound_bytes);
       so[q].iv = reinterpret_cast<int64_t*>(block + at_iv + q * iv_bytes);
-      if (const int rc = sort_seed(d_codes, n_codes, rs, re, nreg, seeds[s0 + q], &out[s0 + q], &so[q], mom + 3 * q, scratch, st, L))
+      if (const int rc = sort_seed(d_codes, at[s0 + q], seeds[s0 + q], &out[s0 + q], &so[q], mom + 3 * q, scratch, room, st, L))
         return rc;
     }
     unsigned long long hm[3 * kGroup];

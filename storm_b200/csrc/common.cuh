@@ -7,6 +7,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <vector>
 #include <cuda_runtime.h>
 
 #include "../../include/stormgpu.h"
@@ -121,12 +122,48 @@ inline int64_t resident_grid(K* k, int threads, size_t smem = 0) {
   return resident_grid_of(reinterpret_cast<const void*>(k), threads, smem);
 }
 
+// Allocations from the stream-ordered pool, given back where the scope ends, whichever way.
+struct StreamScratch {
+  cudaStream_t st;
+  std::vector<void*> ptrs;
+  explicit StreamScratch(cudaStream_t s) : st(s) {}
+  StreamScratch(const StreamScratch&) = delete;
+  StreamScratch& operator=(const StreamScratch&) = delete;
+  template <typename T>
+  cudaError_t alloc(T** p, int64_t n) {
+    void* q = nullptr;
+    const cudaError_t e = cudaMallocAsync(&q, sizeof(T) * (size_t)std::max<int64_t>(n, 1), st);
+    *p = static_cast<T*>(q);
+    if (e == cudaSuccess) ptrs.push_back(q);
+    return e;
+  }
+  // null when there is no room for it
+  template <typename T>
+  T* get(int64_t n) {
+    T* p;
+    if (alloc(&p, n) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+  }
+  // p has another owner from here on
+  void keep(void* p) { ptrs.erase(std::remove(ptrs.begin(), ptrs.end(), p), ptrs.end()); }
+  void give_back(void* p) {
+    keep(p);
+    cudaFreeAsync(p, st);
+  }
+  ~StreamScratch() {
+    for (void* p : ptrs) cudaFreeAsync(p, st);
+  }
+};
+
 }  // namespace sg
 
+// The error is cleared where it is reported: a call that follows must not find it as its own.
 #define SG_CUDA(call)                                                                      \
   do {                                                                                     \
     cudaError_t e_ = (call);                                                               \
     if (e_ != cudaSuccess) {                                                               \
+      cudaGetLastError();                                                                  \
       sg_set_error("%s:%d: %s: %s", __FILE__, __LINE__, #call, cudaGetErrorString(e_));    \
       return STORMGPU_ECUDA;                                                               \
     }                                                                                      \

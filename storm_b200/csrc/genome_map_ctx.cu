@@ -414,30 +414,6 @@ unsigned grid_for(int64_t items, int per_block) {
 
 }  // namespace
 
-namespace {
-
-// device allocations of one call, from the stream-ordered pool, given back when it ends
-struct Scratch {
-  cudaStream_t st;
-  std::vector<void*> ptrs;
-  explicit Scratch(cudaStream_t s) : st(s) {}
-  template <typename T>
-  T* get(int64_t n) {
-    void* p = nullptr;
-    if (cudaMallocAsync(&p, sizeof(T) * (size_t)std::max<int64_t>(n, 1), st) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    ptrs.push_back(p);
-    return static_cast<T*>(p);
-  }
-  ~Scratch() {
-    for (void* p : ptrs) cudaFreeAsync(p, st);
-  }
-};
-
-}  // namespace
-
 extern "C" int stormgpu_genome_map_contextual(stormgpu_ctx* c, int32_t uniqueness, int32_t uniqueness_threshold,
                                               int32_t* read, int32_t* rank, int64_t* n_placed) {
   if (!c || !read || !rank || !n_placed) {
@@ -467,7 +443,7 @@ extern "C" int stormgpu_genome_map_contextual(stormgpu_ctx* c, int32_t uniquenes
     return STORMGPU_EINVAL;
   }
   cudaStream_t st = c->st;
-  Scratch S(st);
+  StreamScratch S(st);
   auto nomem = [&]() {
     sg_set_error("stormgpu_genome_map_contextual: device allocation failed");
     return STORMGPU_ENOMEM;

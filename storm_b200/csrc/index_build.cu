@@ -258,7 +258,8 @@ struct Positions {
 };
 
 int sort_seed(const uint8_t* d_codes, const Positions& at, const SeedDev& seed, DevIndex* out, Sorted* so,
-              unsigned long long* mom, uint32_t* scratch, int64_t room, cudaStream_t st, int64_t& L) {
+              unsigned long long* mom, uint32_t* scratch, int64_t room, StreamScratch& S, int64_t& L) {
+  cudaStream_t st = S.st;
   const int64_t nkeys = (int64_t)1 << (2 * seed.weight), total = at.total;
   out->weight = seed.weight;
   out->nkeys = nkeys;
@@ -274,7 +275,7 @@ int sort_seed(const uint8_t* d_codes, const Positions& at, const SeedDev& seed, 
   // The sorted list ends in its own arrays, whichever way the passes go; the other side of the sort is
   // scratch that every seed of the sequence uses.
   int64_t* const d_iv = so->iv;
-  SG_CUDA(cudaMallocAsync(&so->pos, sizeof(uint32_t) * total, st));
+  SG_CUDA(S.alloc(&so->pos, total));
   const int passes = (2 * seed.weight + kRadixBits - 1) / kRadixBits;
   uint32_t* const sk = scratch;
   uint32_t* const sv = sk + room;
@@ -295,18 +296,21 @@ int sort_seed(const uint8_t* d_codes, const Positions& at, const SeedDev& seed, 
   return 0;
 }
 
-int fill_seed(DevIndex* out, const Sorted& so, int32_t cmax, int64_t longest, cudaStream_t st, int64_t& L) {
+int fill_seed(DevIndex* out, const Sorted& so, int32_t cmax, int64_t longest, StreamScratch& S, int64_t& L) {
+  cudaStream_t st = S.st;
+  StreamScratch own(st);
   const int TB = 256;
   int32_t *off = nullptr, *total = nullptr;
   if (longest <= cmax) {  // nothing erased: the sorted positions are the map
+    S.keep(so.pos);
     out->map = reinterpret_cast<int32_t*>(so.pos);
     out->n = so.total;
   } else {
     uint8_t* keep;
     int32_t* tmp;  // scan
-    SG_CUDA(cudaMallocAsync(&keep, so.total, st));
-    SG_CUDA(cudaMallocAsync(&off, sizeof(int32_t) * (so.total + 1), st));
-    SG_CUDA(cudaMallocAsync(&tmp, sizeof(int32_t) * (scan_tmp_elems(so.total) + 8), st));
+    SG_CUDA(own.alloc(&keep, so.total));
+    SG_CUDA(own.alloc(&off, so.total + 1));
+    SG_CUDA(own.alloc(&tmp, scan_tmp_elems(so.total) + 8));
     SG_CUDA(cudaMallocAsync(&out->map, sizeof(int32_t) * so.total, st));
     total = off + so.total;
     SG_CUDA(cudaMemsetAsync(keep, 1, so.total, st));
@@ -319,13 +323,10 @@ int fill_seed(DevIndex* out, const Sorted& so, int32_t cmax, int64_t longest, cu
     SG_CUDA(cudaMemcpyAsync(&n, total, sizeof(n), cudaMemcpyDeviceToHost, st));
     SG_CUDA(cudaStreamSynchronize(st));
     out->n = n;
-    cudaFreeAsync(keep, st);
-    cudaFreeAsync(tmp, st);
-    cudaFreeAsync(so.pos, st);
+    S.give_back(so.pos);
   }
   key_table_kernel<<<(unsigned)so.nblocks, 256, 0, st>>>(so.keys, so.total, out->nkeys, so.bound, off, total, out->first);
   L++;
-  if (off) cudaFreeAsync(off, st);
   SG_CUDA(cudaGetLastError());
   return 0;
 }
@@ -364,8 +365,9 @@ int build_indexes(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, co
   take(bound_bytes * held);
   const int64_t at_iv = take(0), iv_bytes = ((int64_t)sizeof(int64_t) * iv_words + 255) & ~255LL;
   take(iv_bytes * held);
+  StreamScratch S(st);
   uint8_t* block;
-  SG_CUDA(cudaMallocAsync(&block, size, st));
+  SG_CUDA(S.alloc(&block, size));
   uint32_t* const scratch = reinterpret_cast<uint32_t*>(block + at_scratch);
   unsigned long long* const mom = reinterpret_cast<unsigned long long*>(block + at_mom);
   int64_t L = 0;
@@ -377,7 +379,7 @@ int build_indexes(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, co
       so[q].keys = reinterpret_cast<uint32_t*>(block + at_keys + q * key_bytes);
       so[q].bound = reinterpret_cast<int32_t*>(block + at_bound + q * bound_bytes);
       so[q].iv = reinterpret_cast<int64_t*>(block + at_iv + q * iv_bytes);
-      if (const int rc = sort_seed(d_codes, at[s0 + q], seeds[s0 + q], &out[s0 + q], &so[q], mom + 3 * q, scratch, room, st, L))
+      if (const int rc = sort_seed(d_codes, at[s0 + q], seeds[s0 + q], &out[s0 + q], &so[q], mom + 3 * q, scratch, room, S, L))
         return rc;
     }
     unsigned long long hm[3 * kGroup];
@@ -388,10 +390,9 @@ int build_indexes(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, co
       DevIndex* o = &out[s0 + q];
       o->positions_indexed = so[q].total;
       o->cmax = repeat_cutoff(stdev_distance, so[q].total, hm[3 * q], hm[3 * q + 1]);
-      if (const int rc = fill_seed(o, so[q], o->cmax, (int64_t)hm[3 * q + 2], st, L)) return rc;
+      if (const int rc = fill_seed(o, so[q], o->cmax, (int64_t)hm[3 * q + 2], S, L)) return rc;
     }
   }
-  cudaFreeAsync(block, st);
   if (launches) *launches += L;
   return 0;
 }

@@ -255,6 +255,7 @@ extern "C" int stormgpu_build_index(stormgpu_ctx* c) {
   SG_CUDA(cudaSetDevice(c->p.device));
   SG_CUDA(cudaEventRecord(c->ev[0], c->st));
   int64_t launches = 0;
+  c->indexed = false;  // until every table is there again
   for (auto& r : c->refs) {
     for (auto& ix : r.idx) {  // of the last build, from the stream-ordered pool
       if (ix.first) cudaFreeAsync(ix.first, c->st);

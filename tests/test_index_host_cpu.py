@@ -71,3 +71,49 @@ def test_arrays_of_the_index_build(fake, n_codes, regions):
     total = _build(fake, n_codes, regs)
     # regions out of order send the walk back: more positions than the sequence has
     assert total > n_codes if regions in ("descending", "repeated") else 0 < total <= n_codes
+
+
+@pytest.mark.parametrize("erase", [False, True])
+@pytest.mark.parametrize("rebuild", [False, True])
+def test_a_build_that_runs_out_of_memory(fake, rebuild, erase):
+    """Every allocation of a build refused in turn: nothing is left over, mapping is refused until a build
+    goes through, and the next build does.  erase: the moments read back have a key above the repeat
+    filter's cutoff, so that the maps are compacted."""
+    def moments(name, args):
+        if erase and "run_stats_kernel" in name:
+            ctypes.cast(fakert.arg(args, 3, ctypes.c_void_p), ctypes.POINTER(ctypes.c_uint64))[2] = 5
+
+    with fake.hook(moments):
+        _refuse_each_allocation(fake, rebuild)
+
+
+def _refuse_each_allocation(fake, rebuild):
+    n = 5000
+    packed = np.zeros((n + 3) // 4, np.uint8)
+    reads = api.ReadBatch(np.zeros((2, 16), np.uint8), np.array([40, 50], np.int16))
+    before = fake.live()
+    refused = 0
+    for k in range(100):
+        m = api.Mapper(api.params(stdev=100), SEEDS + ";#######;########")  # five seeds: two groups
+        m.add_reference(packed, packed, n, [])
+        if rebuild:
+            m.build_index()
+        fake.fail_in(k)
+        try:
+            m.build_index()
+            done = True
+        except api.StormError:
+            done = False
+        failed = fake.fail_left() < 0
+        fake.fail_in(-1)
+        assert done != failed
+        if failed:
+            refused += 1
+            with pytest.raises(api.StormError, match="build_index"):
+                m.map(reads)
+            m.build_index()
+        m.close()
+        assert fake.live() == before, k
+        if done:
+            break
+    assert refused > 10 and done

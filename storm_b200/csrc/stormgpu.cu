@@ -851,7 +851,8 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const L
         // candidate list (fr, fd); reads with many index positions go to the block kernel
         SG_CUDA(cudaMemsetAsync(c->counters.p, 0, sizeof(unsigned long long) * kCounters, st));
         GatherOut go;
-        go.fr = c->fr.p; go.fd = c->fd.p; go.cap = c->fr.cap; go.counters = c->counters.p;
+        // (a call that ran out of memory between the two leaves them of different lengths)
+        go.fr = c->fr.p; go.fd = c->fd.p; go.cap = std::min(c->fr.cap, c->fd.cap); go.counters = c->counters.p;
         go.big_list = c->big_list.p; go.big_h = c->big_h.p; go.small_list = c->small_list.p;
         go.small_h = c->small_h.p; go.big_count = big_count(c);
         go.cursor = c->counters.p + 12;  // zeroed just above

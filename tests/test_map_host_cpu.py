@@ -1,0 +1,68 @@
+"""The mapping call's host code on the stand-in runtime: the lists its kernels are given are as long as
+they are told, also after a call that ran out of memory half-way through growing them."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import fakert
+from storm_b200 import api
+
+pytestmark = pytest.mark.skipif(not fakert.have_compiler(), reason="no CUDA headers or compiler")
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    with fakert.loaded(fakert.make(tmp_path_factory.mktemp("fake"))) as f:
+        yield f
+
+
+class GatherOut(ctypes.Structure):  # the head of gather.cuh's
+    _fields_ = [("fr", ctypes.c_void_p), ("fd", ctypes.c_void_p), ("cap", ctypes.c_int64),
+                ("counters", ctypes.POINTER(ctypes.c_uint64))]
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_candidate_lists_after_a_call_that_ran_out_of_memory(fake, graphs):
+    found = 3_000_000  # candidates of a pass: more than the lists start with
+    n = 5000
+    packed = np.zeros((n + 3) // 4, np.uint8)
+    reads = api.ReadBatch(np.zeros((2, 16), np.uint8), np.array([40, 50], np.int16))
+    passes = [0]
+
+    def gather(name, args):
+        if "gather_fused_kernel" not in name:
+            return
+        go = fakert.arg(args, 3, GatherOut)
+        passes[0] += 1
+        assert fake.room(go.fr)[0] >= 4 * go.cap and fake.room(go.fd)[0] >= 4 * go.cap
+        go.counters[7] = found
+        go.counters[8] = 1 if found > go.cap else 0
+
+    refused = 0
+    before = fake.live()
+    for k in range(200):
+        m = api.Mapper(api.params(), "######")
+        m.set_graphs(graphs)
+        m.add_reference(packed, packed, n, [])
+        m.build_index()
+        with fake.hook(gather):
+            fake.fail_in(k)
+            try:
+                m.map(reads)
+                done = True
+            except api.StormError:
+                done = False
+            failed = fake.fail_left() < 0
+            fake.fail_in(-1)
+            assert done != failed
+            passes[0] = 0
+            m.map(reads)
+            m.map(reads)
+            assert passes[0] >= 4  # two calls, two strands
+        m.close()
+        assert fake.live() == before
+        if done:
+            break
+        refused += 1
+    assert refused > 20 and done

@@ -1157,6 +1157,7 @@ extern "C" int stormgpu_map(stormgpu_ctx* c, const stormgpu_reads* reads, stormg
   SG_CUDA(cudaSetDevice(c->p.device));
   const int64_t n = reads->n;
   cudaStream_t st = c->st;
+  c->last_n = -1;  // the last call's results may go with their buffers: none until this call has its own
   if (c->fcodes.grow(std::max<int64_t>(n * reads->code_stride, 1)) || c->lengths.grow(std::max<int64_t>(n, 1)) ||
       c->hits.grow(std::max<int64_t>(n * 4, 1)) || c->tb.grow(std::max<int64_t>(n * 4 * out->tb_stride, 1)) ||
       c->mapped.grow(std::max<int64_t>(n, 1)))

@@ -66,3 +66,39 @@ def test_candidate_lists_after_a_call_that_ran_out_of_memory(fake, graphs):
             break
         refused += 1
     assert refused > 20 and done
+
+
+def test_placement_after_a_call_whose_results_had_no_room(fake):
+    """The results of the last call are gone when a later call freed them to grow and could not: the
+    placement refuses, and does not read them."""
+    n = 5000
+    packed = np.zeros((n + 3) // 4, np.uint8)
+
+    def reads(k):
+        return api.ReadBatch(np.zeros((k, 16), np.uint8), np.full(k, 50, np.int16))
+
+    gone = 0
+    for k in range(12):
+        m = api.Mapper(api.params(), "######")
+        m.add_reference(packed, packed, n, [])
+        m.build_index()
+        m.map(reads(4))
+        fake.fail_in(k)
+        try:
+            m.map(reads(400))
+        except api.StormError:
+            pass
+        fake.fail_in(-1)
+
+        def look(name, args):
+            if "mapped_flags_kernel" in name:
+                assert fake.room(fakert.arg(args, 1, ctypes.c_void_p))[0] >= fakert.arg(args, 0)
+
+        with fake.hook(look):
+            try:
+                m.genome_map(400)
+            except api.StormError as e:
+                assert "no stormgpu_map call" in str(e)
+                gone += 1
+        m.close()
+    assert gone > 0

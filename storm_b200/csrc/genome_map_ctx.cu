@@ -414,6 +414,36 @@ unsigned grid_for(int64_t items, int per_block) {
 
 }  // namespace
 
+namespace {
+
+// The device's pool keeps what is given back to it (for the index builds, whose blocks it then has at
+// hand).  A placement that made it grow by up to kKeepBytes (sequences to about 700 Mbp) leaves it so for the
+// next call; the scratch of a longer one goes back to the device.
+constexpr uint64_t kKeepBytes = (uint64_t)256 << 20;
+struct PoolTrim {
+  cudaStream_t st;
+  cudaMemPool_t pool = nullptr;
+  uint64_t before = 0;
+  PoolTrim(int device, cudaStream_t s) : st(s) {
+    if (cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess) pool = nullptr;
+    before = reserved();
+  }
+  uint64_t reserved() {
+    uint64_t v = 0;
+    if (pool) cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &v);
+    return v;
+  }
+  ~PoolTrim() {
+    if (reserved() > before + kKeepBytes) {
+      cudaStreamSynchronize(st);  // the frees are done
+      cudaMemPoolTrimTo(pool, before);
+    }
+    cudaGetLastError();
+  }
+};
+
+}  // namespace
+
 extern "C" int stormgpu_genome_map_contextual(stormgpu_ctx* c, int32_t uniqueness, int32_t uniqueness_threshold,
                                               int32_t* read, int32_t* rank, int64_t* n_placed) {
   if (!c || !read || !rank || !n_placed) {
@@ -443,6 +473,7 @@ extern "C" int stormgpu_genome_map_contextual(stormgpu_ctx* c, int32_t uniquenes
     return STORMGPU_EINVAL;
   }
   cudaStream_t st = c->st;
+  PoolTrim trim(c->p.device, st);  // after S has given its allocations back
   StreamScratch S(st);
   auto nomem = [&]() {
     sg_set_error("stormgpu_genome_map_contextual: device allocation failed");

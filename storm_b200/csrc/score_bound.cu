@@ -18,7 +18,7 @@
 //
 // Bound by the integer ALU pipe as the filter is, with the filter's recurrence: 3.5 ALU
 // instructions per two cells where the full alignment needs about 28 and writes direction bits.
-#include "score_bound.cuh"
+#include "bound_kernel.cuh"
 
 namespace sg {
 
@@ -48,49 +48,12 @@ void launch_band_streams(const ReadsDev& rd, int H, int64_t words, uint32_t* rs,
   band_streams_kernel<<<(unsigned)blocks, 256, 0, st>>>(rd, H, words, rs, ws, c);
 }
 
-// One candidate per thread, blocks in list order (neighbouring candidates are of one read, or of
-// reads of one length).
-// C: the constants, BandBoundDefault for the default scores.
-template <int H, bool WTD, class C>
-__global__ void __launch_bounds__(128, H <= 4 ? 8 : H <= 8 ? 4 : 3)
-    score_bound_kernel(BoundJob job, const __grid_constant__ BandConst bc) {
-  const C c(bc);
-  const int64_t n = job.n_dev ? *job.n_dev : job.n;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int r = job.read[t];
-  const int L = job.lengths[r];
-  int ub = 32767;
-  const int lim = band_bound_limit(job.match, job.mismatch, L);
-  if (lim > kBoundFloor - kBoundZero) {
-    const int64_t win = max(job.diag[t] - job.I, -job.Is);  // run.c:667
-    const int v = band_last_row<H, WTD>(job.gexp, win, job.rs + (int64_t)r * job.words,
-                                        WTD ? job.ws + (int64_t)r * job.words : nullptr, L, c);
-    if (v - kBoundZero < lim) ub = v - kBoundZero;
-  }
-  job.flag[t] = ub > job.min_score ? 1 : 0;
-  job.ub[t] = (int16_t)ub;
-}
-
 void launch_score_bound(const BoundJob& job, const BandConst& c, cudaStream_t st) {
   if (job.n <= 0) return;
-  const unsigned blocks = (unsigned)((job.n + 127) / 128);
-#define SG_BOUND(H, C)                                                                  \
-  case H:                                                                               \
-    if (job.ws) score_bound_kernel<H, true, C><<<blocks, 128, 0, st>>>(job, c);         \
-    else score_bound_kernel<H, false, C><<<blocks, 128, 0, st>>>(job, c);               \
-    break;
-#define SG_BOUNDS(C) \
-  switch (job.H) {   \
-    SG_BOUND(2, C)   \
-    SG_BOUND(4, C)   \
-    SG_BOUND(8, C)   \
-    SG_BOUND(12, C)  \
-  default: break;    \
-  }
-  if (band_is_default_bound(c)) { SG_BOUNDS(BandBoundDefault) } else { SG_BOUNDS(BandConst) }
-#undef SG_BOUNDS
-#undef SG_BOUND
+  const void* k = band_is_default_bound(c) ? bound_kernel_of<BandBoundDefault>(job) : bound_form(job);
+  if (!k) return;
+  void* args[] = {(void*)&job, (void*)&c};
+  cudaLaunchKernel(k, dim3((unsigned)((job.n + 127) / 128)), dim3(128), args, 0, st);  // errors surface at the caller's next check
 }
 
 }  // namespace sg

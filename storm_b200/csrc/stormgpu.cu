@@ -527,7 +527,8 @@ static bool ahead_buffers(stormgpu_ctx* c, const PassSetup& P, AheadCaps* caps) 
   caps->kept = want_kept;
   caps->pass = P.bound_H ? want_pass : caps->kept;
   const int64_t longest = std::max(caps->cand, caps->pass);
-  if (c->flag.grow(longest) || c->foff.grow(select_tiles(longest) + 1) ||
+  if (c->flag.grow(longest) || c->foff.grow(select_tiles(longest) + 1)) return false;
+  if ((P.rounds > 1 || caps->kept > wave_slots(P.sp)) &&
       c->scratch.grow(align_workers(caps->kept, P.sp) * (int64_t)P.maxL * P.wpr))
     return false;
   return round_lists_grow(c, n, caps->kept, P.rounds) == 0;
@@ -967,12 +968,12 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const L
         pb.a_pos = c->a_pos.p; pb.a_tb = c->a_tb.p; pb.tbs = tbs;
         // one persistent launch over all kept candidates; scratch for its threads only
         pb.steal = c->tune.align_steal;
-        const int64_t per_slot = (int64_t)maxL * wpr;
-        if (c->scratch.grow(align_workers(nkept, sp) * per_slot)) return STORMGPU_ENOMEM;
+        const bool wave = rounds == 1 && nkept <= wave_slots(sp);
+        if (!wave && c->scratch.grow(align_workers(nkept, sp) * (int64_t)maxL * wpr)) return STORMGPU_ENOMEM;
         pb.a_scratch = c->scratch.p;
         pb.cells = c->counters.p + kCntAlign;
         if (rounds == 1) {
-          if (nkept <= wave_slots(sp)) launch_align_wave(rd, sp, R.d_codes, R.d_mask, 0, nkept, pb, maxL, st);
+          if (wave) launch_align_wave(rd, sp, R.d_codes, R.d_mask, 0, nkept, pb, maxL, st);
           else launch_align(rd, sp, R.d_codes, R.d_mask, 0, nkept, pb, st);
           launches++;
         } else {

@@ -13,7 +13,11 @@
 namespace {
 std::recursive_mutex mu;
 std::map<char*, size_t> live;                // device allocations
-std::map<const void*, std::string> kernels;  // by their host stub
+struct Kernel { std::string name; int module; };
+std::map<const void*, Kernel> kernels;  // by their host stub
+int modules = 0;                        // in the order their objects are linked
+void* handles[256];
+bool used[256];                         // modules whose kernels were launched or asked about
 long long fail_in = -1;                      // allocations until one fails (-1: none does)
 long long bytes = 0;
 cudaError_t last = cudaSuccess;
@@ -63,13 +67,15 @@ long long fake_room(void* p, void** base) {
   return c <= it->first + it->second ? (long long)(it->first + it->second - c) : -1;
 }
 
+int fake_module_used(int k) { return k < modules ? used[k] : -1; }
+
 // ---- what nvcc's stubs call
-void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
+void** __cudaRegisterFatBinary(void*) { return &handles[modules++]; }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
-void __cudaRegisterFunction(void**, const char* stub, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) {
-  kernels[stub] = name;
+void __cudaRegisterFunction(void** h, const char* stub, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) {
+  kernels[stub] = {name, (int)(h - handles)};
 }
 unsigned __cudaPushCallConfiguration(dim3 grid, dim3 block, size_t smem, struct CUstream_st* st) {
   config = {grid, block, smem, st};
@@ -84,7 +90,8 @@ cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* smem, vo
 }
 cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cudaStream_t) {
   std::lock_guard<std::recursive_mutex> l(mu);
-  if (hook) hook(kernels[f].c_str(), args);
+  used[kernels[f].module] = true;
+  if (hook) hook(kernels[f].name.c_str(), args);
   return cudaSuccess;
 }
 
@@ -120,8 +127,12 @@ cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 0; return cudaSuccess; }
-cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
+cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute, int) { used[kernels[f].module] = true; return cudaSuccess; }
 cudaError_t cudaGetSymbolAddress(void** p, const void*) { *p = nullptr; return set(cudaErrorInvalidSymbol); }
-cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t) { *n = 2; return cudaSuccess; }
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void* f, int, size_t) {
+  used[kernels[f].module] = true;
+  *n = 2;
+  return cudaSuccess;
+}
 
 }  // extern "C"

@@ -1,12 +1,15 @@
 """The mapping call's host code on the stand-in runtime: the lists its kernels are given are as long as
 they are told, also after a call that ran out of memory half-way through growing them."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
 
 import fakert
-from storm_b200 import api
+from storm_b200 import api, build
 
 pytestmark = pytest.mark.skipif(not fakert.have_compiler(), reason="no CUDA headers or compiler")
 
@@ -102,3 +105,46 @@ def test_placement_after_a_call_whose_results_had_no_room(fake):
                 gone += 1
         m.close()
     assert gone > 0
+
+
+LOADS = r"""
+import ctypes, sys
+import numpy as np
+import fakert
+from storm_b200 import api, build
+from test_map_host_cpu import GatherOut
+so, colour, indels, found, kept = sys.argv[1], *map(int, sys.argv[2:])
+with fakert.loaded(so) as fake:
+    def lists(name, args):  # what the kernels would leave: `found` candidates, `kept` of them pass
+        if "gather_fused_kernel" in name:
+            fakert.arg(args, 3, GatherOut).counters[7] = found
+        if "select_count_kernel" in name:
+            tiles = ctypes.cast(fakert.arg(args, 3, ctypes.c_void_p), ctypes.POINTER(ctypes.c_int64))
+            n = fakert.arg(args, 0)
+            tiles[(n + 4095) // 4096] = min(n, kept)
+    m = api.Mapper(api.params(colour=colour, indels=indels), "####--#-#--##--####")
+    packed = np.zeros(1250, np.uint8)
+    m.add_reference(packed, packed, 5000, [])
+    m.build_index()
+    reads = api.ReadBatch(np.zeros((16, 16), np.uint8), np.full(16, 50, np.int16), np.zeros((16, 16), np.uint8))
+    with fake.hook(lists):
+        for _ in range(3):
+            m.map(reads)
+    m.close()
+    print(*[s for k, s in enumerate(build.CU_SOURCES) if fake.L.fake_module_used(k)])
+"""
+
+
+@pytest.mark.parametrize("colour,indels,found,kept,most", [(0, 3, 260, 20, 6), (1, 7, 300, 20, 6), (0, 15, 9000, 8000, 10)])
+def test_modules_that_a_call_loads(tmp_path_factory, colour, indels, found, kept, most):
+    """A process loads a module's code with the first use of a kernel of it, about 0.35 ms per MB: the
+    objects that a call's kernels are in, in MB.  (All of them are 17.)"""
+    so = fakert.make(tmp_path_factory.mktemp("loads"))
+    here = os.path.dirname(os.path.abspath(__file__))
+    p = subprocess.run([sys.executable, "-c", LOADS, so, str(colour), str(indels), str(found), str(kept)], capture_output=True,
+                       text=True, timeout=300, env=dict(os.environ, PYTHONPATH=here + os.pathsep + os.path.dirname(here)))
+    assert p.returncode == 0, p.stderr
+    files = p.stdout.split()
+    assert "gather.cu" in files and "map_kernels.cu" in files
+    size = sum(os.path.getsize(os.path.join(build.PKG, "_build", f.replace(".cu", ".o"))) for f in files)
+    assert size < most * 1e6, (size, files)

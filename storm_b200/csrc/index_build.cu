@@ -61,8 +61,10 @@ __global__ void seed_keys_kernel(const uint8_t* __restrict__ codes, const int64_
 }
 
 // The key table is written in blocks of kKeyBlock keys; bound[b]: first index of the sorted list whose
-// key is in block b or a later one.
+// key is in block b or a later one.  A block with up to kKeyScan positions goes over them, 256 at a time;
+// with more (a key of a long repeat: 4 million positions took 7 ms) it searches for each of its keys.
 constexpr int kKeyBlock = 2048;
+constexpr int64_t kKeyScan = 1 << 15;
 
 // length of the run of equal keys that starts at t
 __device__ __forceinline__ int64_t run_length(const uint32_t* __restrict__ skeys, int64_t n, int64_t t, uint32_t k) {
@@ -126,14 +128,27 @@ __global__ void run_stats_kernel(const uint32_t* __restrict__ skeys, int64_t n, 
   }
 }
 
-// keep[t] = 0 for the positions of keys with more than cmax (all 1 before)
-__global__ void erase_runs_kernel(const uint32_t* __restrict__ skeys, int64_t n, int32_t cmax, uint8_t* __restrict__ keep) {
+// keys equal to k at t and before it
+__device__ __forceinline__ int64_t run_length_back(const uint32_t* __restrict__ skeys, int64_t t, uint32_t k) {
+  int64_t d = 1;
+  while (t - d >= 0 && skeys[t - d] == k) d <<= 1;
+  int64_t lo = d >> 1, hi = min(d, t + 1);  // t - lo has the key, t - hi has not
+  while (hi - lo > 1) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (skeys[t - mid] == k) lo = mid; else hi = mid;
+  }
+  return hi;
+}
+
+// keep[t]: whether the key at t has at most cmax positions.  Every position looks for its run's ends by
+// itself, unless the key cmax places on or back settles it: erased run by run, by the thread at its head, a
+// key with 8 of 16 million positions took 120 ms.
+__global__ void keep_runs_kernel(const uint32_t* __restrict__ skeys, int64_t n, int32_t cmax, uint8_t* __restrict__ keep) {
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t k = skeys[t];
-    if (t && skeys[t - 1] == k) continue;
-    const int64_t c = run_length(skeys, n, t, k);
-    if (c > cmax)
-      for (int64_t u = t; u < t + c; ++u) keep[u] = 0;
+    const bool more = (t + cmax < n && skeys[t + cmax] == k) || (t - cmax >= 0 && skeys[t - cmax] == k) ||
+                      run_length(skeys, n, t, k) + run_length_back(skeys, t, k) - 1 > cmax;
+    keep[t] = more ? 0 : 1;
   }
 }
 
@@ -156,11 +171,23 @@ __global__ void __launch_bounds__(256) key_table_kernel(const uint32_t* __restri
   const int64_t k0 = (int64_t)blockIdx.x * kKeyBlock;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t lo = bound[blockIdx.x], hi = bound[blockIdx.x + 1];
-  for (int k = threadIdx.x; k < kKeyBlock; k += 256) at[k] = 0x7fffffff;
-  __syncthreads();
-  for (int64_t t = lo + threadIdx.x; t < hi; t += 256) {
-    const uint32_t k = skeys[t];
-    if (t == 0 || skeys[t - 1] != k) at[k - (uint32_t)k0] = (int32_t)t;
+  if (hi - lo <= kKeyScan) {
+    for (int k = threadIdx.x; k < kKeyBlock; k += 256) at[k] = 0x7fffffff;
+    __syncthreads();
+    for (int64_t t = lo + threadIdx.x; t < hi; t += 256) {
+      const uint32_t k = skeys[t];
+      if (t == 0 || skeys[t - 1] != k) at[k - (uint32_t)k0] = (int32_t)t;
+    }
+  } else {
+    for (int k = threadIdx.x; k < kKeyBlock; k += 256) {
+      const uint32_t key = (uint32_t)(k0 + k);
+      int64_t a = lo, b = hi;  // the first position in [lo, hi] whose key is `key` or a later one
+      while (a < b) {
+        const int64_t mid = (a + b) >> 1;
+        if (skeys[mid] < key) a = mid + 1; else b = mid;
+      }
+      at[k] = (int32_t)a;
+    }
   }
   __syncthreads();
   int32_t v[PER], m = 0x7fffffff;
@@ -313,9 +340,8 @@ int fill_seed(DevIndex* out, const Sorted& so, int32_t cmax, int64_t longest, St
     SG_CUDA(own.alloc(&tmp, scan_tmp_elems(so.total) + 8));
     SG_CUDA(cudaMallocAsync(&out->map, sizeof(int32_t) * so.total, st));
     total = off + so.total;
-    SG_CUDA(cudaMemsetAsync(keep, 1, so.total, st));
-    erase_runs_kernel<<<(unsigned)std::min<int64_t>(blocks_of(so.total, TB), 148 * 16), TB, 0, st>>>(so.keys, so.total, cmax,
-                                                                                                  keep);
+    keep_runs_kernel<<<(unsigned)std::min<int64_t>(blocks_of(so.total, TB), 148 * 16), TB, 0, st>>>(so.keys, so.total, cmax,
+                                                                                                 keep);
     exclusive_scan<uint8_t, int32_t>(keep, off, so.total, total, tmp, st);
     kept_positions_kernel<<<blocks_of(so.total, TB), TB, 0, st>>>(keep, off, so.pos, so.total, out->map);
     L += 2 + scan_launches(so.total);

@@ -246,9 +246,9 @@ typedef struct stormgpu_tuning {
                                      rounds (its next 8, 16, 32, 64, 128 candidates whose score
                                      bound exceeds the read's running threshold, then the rest of
                                      them), each followed by the replay of its candidates.  One
-                                     round without a bound (colour space, bands above 47 cells),
-                                     for at most 256 reads, and where a pass has fewer than 32
-                                     candidates per read */
+                                     round without a bound (colour space, bands above 47 cells,
+                                     reads too long for one above -t), for at most 256 reads, and
+                                     where a pass has fewer than 32 candidates per read */
 } stormgpu_tuning;
 /* Passes enqueued ahead (default on, unless the environment sets STORMGPU_GRAPHS=0 when the
  * context opens; earlier versions captured them as a CUDA graph, hence the names): from the

@@ -148,3 +148,31 @@ def test_modules_that_a_call_loads(tmp_path_factory, colour, indels, found, kept
     assert "gather.cu" in files and "map_kernels.cu" in files
     size = sum(os.path.getsize(os.path.join(build.PKG, "_build", f.replace(".cu", ".o"))) for f in files)
     assert size < most * 1e6, (size, files)
+
+
+@pytest.mark.parametrize("length,rounds", [(50, 4), (150, 4), (250, 4), (300, 1), (400, 1), (1000, 1)])
+def test_rounds_only_for_reads_that_have_a_score_bound(fake, length, rounds):
+    """Reads too long for a score bound above -t (from 287 codes on with the default scores and -t 100): a
+    round drops nothing, and the candidates go through one."""
+    n, found = 300, 300 * 100
+    replays = [0]
+
+    def lists(name, args):
+        if "gather_fused_kernel" in name:
+            fakert.arg(args, 3, GatherOut).counters[7] = found
+        if "select_count_kernel" in name:  # every candidate passes
+            tiles = ctypes.cast(fakert.arg(args, 3, ctypes.c_void_p), ctypes.POINTER(ctypes.c_int64))
+            m = fakert.arg(args, 0)
+            tiles[(m + 4095) // 4096] = min(m, found)
+        replays[0] += "replay_kernel" in name
+
+    m = api.Mapper(api.params(indels=15, min_score=100), "######")
+    m.set_graphs(False)
+    packed = np.zeros(1250, np.uint8)
+    m.add_reference(packed, packed, 5000, [])
+    m.build_index()
+    reads = api.ReadBatch(np.zeros((n, 256), np.uint8), np.full(n, length, np.int16))
+    with fake.hook(lists):
+        m.map(reads)
+    m.close()
+    assert replays[0] == 2 * rounds

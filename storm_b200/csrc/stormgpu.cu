@@ -280,6 +280,9 @@ extern "C" int stormgpu_build_index(stormgpu_ctx* c) {
 // halves (reads are independent, so the results are the same).
 constexpr int64_t kMaxCandidatesPerPass = 1000000000;
 constexpr int64_t kMaxPassingPerPass = 100000000;  // their tracebacks are kept until the replay
+// Read streams of the banded core held at once: 1.3 KB a read of 150 codes with qualities, which a batch of
+// a hundred million reads has no room for.  A larger batch is cut up front, into pieces of 3 million reads.
+constexpr int64_t kMaxStreamBytes = (int64_t)4 << 30;
 constexpr int kSplitBatch = 1;
 
 // S += s (everything but the index build time)
@@ -758,6 +761,27 @@ static int length_stats(stormgpu_ctx* c, const stormgpu_reads* reads, const int1
   return 0;
 }
 
+// Band registers of the banded core for the filter and for the score bound (nucleotide space, a band it is
+// instantiated for), 0 where it is not used.
+struct BandWidths {
+  int filter, bound;
+  // bytes of the read streams of n reads, the longest of max_len
+  int64_t stream_bytes(int64_t n, int max_len, bool levels) const {
+    const int64_t words = std::max(filter ? band_stream_words(max_len, filter) : 0, bound ? band_stream_words(max_len, bound) : 0);
+    return n * words * (int64_t)sizeof(uint32_t) * (bound && levels ? 2 : 1);
+  }
+};
+
+static BandWidths band_widths(stormgpu_ctx* c, const ScoreParams& sp) {
+  if (!c->band_set) {
+    c->filter_c = band_filter_consts(sp.fm, sp.fx, sp.fo, sp.fe, sp.fthr);
+    memset(&c->bound_c, 0, sizeof(c->bound_c));
+    if (!sp.colour && sp.I <= kMaxBoundIndels) c->bound_c = band_bound_consts(sp.pair, sp.gap_open, sp.gap_ext);
+    c->band_set = true;
+  }
+  return {filter_band_registers(sp.W, c->filter_c), c->bound_c.ok ? bound_registers(sp.I) : 0};
+}
+
 static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const LengthStats& ls, stormgpu_results* out) {
   if (!c->indexed) { sg_set_error("stormgpu_build_index must be called before mapping"); return STORMGPU_ESTATE; }
   cudaStream_t st = c->st;
@@ -807,15 +831,8 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const L
   const int BW = 2 * sp.I + 1;
   const int wpr = (2 * BW + 31) / 32 + (sp.colour ? (BW + 31) / 32 : 0);
   const int64_t tbs = ((maxL + sp.I + 1) / 2 + 7) & ~7LL;
-  // the banded core's constants; score bound: nucleotide space, a band it is instantiated for
-  if (!c->band_set) {
-    c->filter_c = band_filter_consts(sp.fm, sp.fx, sp.fo, sp.fe, sp.fthr);
-    memset(&c->bound_c, 0, sizeof(c->bound_c));
-    if (!sp.colour && sp.I <= kMaxBoundIndels) c->bound_c = band_bound_consts(sp.pair, sp.gap_open, sp.gap_ext);
-    c->band_set = true;
-  }
-  const int filter_H = filter_band_registers(sp.W, c->filter_c);
-  const int bound_H = c->bound_c.ok ? bound_registers(sp.I) : 0;
+  const BandWidths bw = band_widths(c, sp);
+  const int filter_H = bw.filter, bound_H = bw.bound;
   {
     const int64_t words = n * std::max(filter_H ? band_stream_words(maxL, filter_H) : 0,
                                        bound_H ? band_stream_words(maxL, bound_H) : 0);
@@ -1078,15 +1095,17 @@ static int map_pieces(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_
 int sg::map_device_impl(stormgpu_ctx* c, const stormgpu_reads* reads, const int16_t* lengths, stormgpu_results* out) {
   LengthStats ls;
   if (const int e = length_stats(c, reads, lengths, &ls)) return e;
-  if (reads->n > 1 && (c->dens_cand > 0 || c->dens_pass > 0)) {
+  if (reads->n > 1 && ls.longest <= STORMGPU_MAX_READ_LEN) {
     // at the last call's density per unit of work weight the batch would be cut after its
     // gather: cut it now, into pieces of equal weight (a batch's reads need not be mixed: a file
     // of several lengths often lists them one length after the other).  0.8: the pieces still
     // differ in repeat content; one that overflows is cut after its gather.
     const int64_t n = reads->n;
     const double W = (double)ls.weight;
-    const double need = std::max(c->dens_cand * W / (0.8 * (double)kMaxCandidatesPerPass),
-                                 c->dens_pass * W / (0.8 * (double)kMaxPassingPerPass));
+    const int64_t streams = band_widths(c, make_score_params(c->p)).stream_bytes(n, (int)ls.longest, reads->levels != nullptr);
+    const double need = std::max({c->dens_cand * W / (0.8 * (double)kMaxCandidatesPerPass),
+                                  c->dens_pass * W / (0.8 * (double)kMaxPassingPerPass),
+                                  (double)streams / (double)kMaxStreamBytes});
     if (need > 1.0) {
       std::vector<int16_t> hl;
       if (!lengths) {

@@ -176,3 +176,40 @@ def test_rounds_only_for_reads_that_have_a_score_bound(fake, length, rounds):
         m.map(reads)
     m.close()
     assert replays[0] == 2 * rounds
+
+
+class ReadsDev(ctypes.Structure):  # the head of map_kernels.cuh's
+    _fields_ = [("n", ctypes.c_int64), ("codes", ctypes.c_void_p)]
+
+
+@pytest.mark.parametrize("n,pieces", [(1_000_000, 1), (1_200_000, 2), (2_400_000, 3)])
+def test_read_streams_of_a_large_batch(fake, n, pieces):
+    """The read streams held at once are at most 4 GB (a read of 1,000 codes has 4 KB): a larger batch is
+    mapped in pieces, which together are the batch."""
+    stride, tbs = 250, 512
+    codes, lengths = np.zeros((n, stride), np.uint8), np.full(n, 1000, np.int16)
+    hits, tb, mapped = np.empty(n * 4 * 28, np.uint8), np.empty(n * 4 * tbs, np.uint8), np.empty(n, np.uint8)
+    parts = []
+
+    def streams(name, args):
+        if "length_stats_kernel" in name:  # longest, 1024 less the shortest, weight
+            out = ctypes.cast(fakert.arg(args, 2, ctypes.c_void_p), ctypes.POINTER(ctypes.c_uint64))
+            out[0], out[1], out[2] = 1000, 24, 985 * fakert.arg(args, 1)
+        if "band_streams_kernel" in name:
+            rd, words, rs = fakert.arg(args, 0, ReadsDev), fakert.arg(args, 2), fakert.arg(args, 3, ctypes.c_void_p)
+            assert rd.n * words * 4 <= 4 << 30
+            assert fake.room(rs)[0] >= rd.n * words * 4
+            if codes.ctypes.data <= rd.codes < codes.ctypes.data + codes.nbytes:  # the forward strand
+                parts.append(((rd.codes - codes.ctypes.data) // stride, rd.n))
+
+    m = api.Mapper(api.params(indels=15), "######")
+    m.add_reference(np.zeros(1250, np.uint8), np.zeros(1250, np.uint8), 5000, [])
+    m.build_index()
+    reads = api.Reads(n, codes.ctypes.data, stride, None, 0, lengths.ctypes.data, None)
+    results = api.Results(hits.ctypes.data, tb.ctypes.data, tbs, mapped.ctypes.data)
+    with fake.hook(streams):
+        m.map_device(reads, results)
+    m.close()
+    assert len(parts) == pieces
+    assert [a for a, _ in parts] == [sum(k for _, k in parts[:q]) for q in range(pieces)]
+    assert sum(k for _, k in parts) == n

@@ -12,7 +12,7 @@ namespace sg {
 // The instantiated kernels by band width (null: none for it).
 const void* align_packed_kernel(int bw);              // CM 2: nucleotides, every odd width from 3 to 41
 const void* align_unit_kernel(int bw);                // CM 3: the unit entry points
-const void* align_general_kernel(int bw, int colour); // CM 0, 1; -1 for widths that have none of their own
+const void* align_general_kernel(int bw, int colour); // CM 0, 1; any width
 
 // Cell state packed in 16 bits: from (2) | indels (7) | colour checksum (2) | auto-correct (2)
 // | freshness (3).  "from": 3 corner, 2 top, 1 left (alignment.c:13-19).
@@ -93,44 +93,11 @@ struct BandWindow {
   __device__ __forceinline__ int mcode(int c) const { return (int)((m[c >> 5] >> (2 * (c & 31))) & 3u); }
 };
 
-// Traceback over the direction words of the rows from i (cell c) up: emit(i, c, words of the row,
-// direction) for every cell of the path.  A path leaves a row once (every step but LEFT goes up), so the
-// rows' words are loaded four rows ahead whatever the path does; walked one cell at a time, each
-// step waited for its own word.
-template <int WPR, int WDIR, int LEFT, int TOP, class Emit>
-__device__ __forceinline__ void trace_rows(const uint32_t* scr, int64_t ns, int64_t sl, int i, int c, int BW, Emit emit) {
-  constexpr int PF = 4;
-  uint32_t w[PF][WPR];
-  auto load = [&](int q, int row) {
-#pragma unroll
-    for (int k = 0; k < WPR; ++k) w[q][k] = row >= 0 ? scr[((int64_t)row * WPR + k) * ns + sl] : 0u;
-  };
-#pragma unroll
-  for (int q = 0; q < PF; ++q) load(q, i - q);
-  for (;;) {
-#pragma unroll
-    for (int q = 0; q < PF; ++q) {
-      int from;
-      for (;;) {
-        uint32_t x = w[q][0];
-        if (WDIR > 1 && c >= 16) x = w[q][WDIR > 1 ? 1 : 0];
-        if (WDIR > 2 && c >= 32) x = w[q][WDIR > 2 ? 2 : 0];
-        from = (x >> ((2 * c) & 31)) & 3;
-        emit(i, c, w[q], from);
-        if (from != LEFT) break;
-        if (--c < 0) return;
-      }
-      if (from == TOP) ++c;
-      if (--i < 0 || c >= BW) return;
-      load(q, i - (PF - 1));
-    }
-  }
-}
-
 // BWT > 0: the band width 2I + 1 as a constant, so that the row arrays live in registers;
-// BWT = 0: any width up to kMaxBand (arrays in local memory).  ctab: the table of colour_step.  CM: 0 nucleotide, 1 colour
-// space (the colour state machine compiled in), -1 either (sp.colour); the kernel's CM = 2 runs
-// the packed nucleotide form below (align_one_nuc).
+// BWT = 0: any width up to kMaxBand (arrays in local memory).  CM: 0 nucleotide, 1 colour space (the
+// colour state machine compiled in; ctab: the table of colour_step); the kernel's CM = 2 and 3 run the
+// packed nucleotide form below (align_one_nuc).  (With the space a run-time value the widths without a
+// constant ran at less than half the rate in nucleotides: one window at -i 16 1.05 ms, now 0.43.)
 // A candidate whose running abort bound falls below the replay's threshold stops at that row:
 // -t, or with rounds the running threshold its read had after the rounds before (the replay's
 // threshold only rises, so the candidate is aborted whatever comes before it), and neither its
@@ -146,7 +113,7 @@ __device__ __forceinline__ int align_one(const ReadsDev& rd, const ScoreParams& 
   // threshold after the rounds before this one (in the first round, a previous pass's value)
   const int thr = (pb.thr && pb.round > 0) ? max(sp.min_score, pb.thr[r]) : sp.min_score;
   const int d = pb.p_diag[slot];
-  const int I = sp.I, BW = BWT > 0 ? BWT : 2 * I + 1, colour = CM >= 0 ? CM : sp.colour;
+  const int I = sp.I, BW = BWT > 0 ? BWT : 2 * I + 1, colour = CM;
   const int L = rd.lengths[r];
   const uint8_t* rdc = rd.codes + (int64_t)r * rd.cstride;
   const uint8_t* rdq = rd.levels ? rd.levels + (int64_t)r * rd.lstride : nullptr;
@@ -268,25 +235,16 @@ __device__ __forceinline__ int align_one(const ReadsDev& rd, const ScoreParams& 
       else if (!colour || !(colr || (adj && i != 0 && j != 0))) put(0x4 | rc);
       else { put(0x8 | rc); colr ^= rc ^ f; }
     };
-    if constexpr (BWT > 0) {
-      constexpr int WD = (2 * BWT + 31) / 32, WC = CM == 0 ? 0 : (BWT + 31) / 32;
-      trace_rows<WD + WC, WD, 1, 2>(scr, ns, sl, bi, bj - bi, BW, [&](int i, int c, const uint32_t* w, int from) {
-        uint32_t x = 0;
-        if (WC > 0) x = w[WC > 0 ? WD : 0];
-        if (WC > 1 && c >= 32) x = w[WC > 1 ? WD + 1 : 0];
-        cell(i, c, from, WC > 0 && ((x >> (c & 31)) & 1u));
-      });
-    } else {
-      int i = bi, c = bj - bi;
-      while (i >= 0 && i < L && c >= 0 && c < BW) {
-        const uint32_t wdir = scr[((int64_t)i * wpr + ((2 * c) >> 5)) * ns + sl];
-        const int from = (wdir >> ((2 * c) & 31)) & 3;
-        const bool adj = colour && ((scr[((int64_t)i * wpr + wpr_dir + (c >> 5)) * ns + sl] >> (c & 31)) & 1u);
-        cell(i, c, from, adj);
-        if (from == 2) { i--; c++; }
-        else if (from == 1) { c--; }
-        else { i--; }
-      }
+    // (the direction words loaded rows ahead, whatever the path does, were slower at every width)
+    int i = bi, c = bj - bi;
+    while (i >= 0 && i < L && c >= 0 && c < BW) {
+      const uint32_t wdir = scr[((int64_t)i * wpr + ((2 * c) >> 5)) * ns + sl];
+      const int from = (wdir >> ((2 * c) & 31)) & 3;
+      const bool adj = colour && ((scr[((int64_t)i * wpr + wpr_dir + (c >> 5)) * ns + sl] >> (c & 31)) & 1u);
+      cell(i, c, from, adj);
+      if (from == 2) { i--; c++; }
+      else if (from == 1) { c--; }
+      else { i--; }
     }
   }
   pb.a_tblen[slot] = tl;
@@ -460,8 +418,10 @@ __device__ __forceinline__ int align_one_nuc(const ReadsDev& rd, const ScorePara
   uint8_t* tb = pb.a_tb + slot * pb.tbs;
   if (bi >= 0 && bnd >= thr && best > thr) {  // alignment.c:642-734
     uint8_t cur = 0;
-    // directions: 2 corner, 1 top, 0 left
-    trace_rows<wpr, wpr, 0, 1>(scr, ns, sl, bi, bj - bi, BW, [&](int i, int c, const uint32_t*, int from) {
+    int i = bi, c = bj - bi;
+    while (i >= 0 && i < L && c >= 0 && c < BW) {
+      const uint32_t wdir = scr[((int64_t)i * wpr + ((2 * c) >> 5)) * ns + sl];
+      const int from = (wdir >> ((2 * c) & 31)) & 3;  // 2 corner, 1 top, 0 left
       const int j = i + c;
       i0 = i;
       j0 = j;
@@ -473,7 +433,10 @@ __device__ __forceinline__ int align_one_nuc(const ReadsDev& rd, const ScorePara
       if (tl & 1) { cur |= (uint8_t)op; tb[tl >> 1] = cur; }
       else { cur = (uint8_t)(op << 4); tb[tl >> 1] = cur; }
       tl++;
-    });
+      if (from == 1) { i--; c++; }
+      else if (from == 0) { c--; }
+      else { i--; }
+    }
   }
   pb.a_tblen[slot] = tl;
   pb.a_pos[slot * 4 + 0] = (int16_t)bi;
@@ -510,8 +473,8 @@ __global__ void __launch_bounds__(128, align_blocks(BWT, CM)) align_kernel(Reads
                                                     const uint8_t* __restrict__ genome,
                                                     const uint8_t* __restrict__ mask, int64_t slot0, int64_t nslots,
                                                     PassBuffers pb) {
-  __shared__ uint8_t ctab[CM == 1 || CM == -1 ? kColourTable : 1];
-  if (CM == 1 || CM == -1) {
+  __shared__ uint8_t ctab[CM == 1 ? kColourTable : 1];
+  if (CM == 1) {
     for (int k = threadIdx.x; k < kColourTable; k += blockDim.x) ctab[k] = colour_step(k);
     __syncthreads();
   }
@@ -535,15 +498,25 @@ __global__ void __launch_bounds__(128, align_blocks(BWT, CM)) align_kernel(Reads
       end = s + take;
       s += lane;
     }
+    bool masked = false;
+    if constexpr (CM == 3) {
+      // every cell exact: without masked codes no cell comes near the packed form's floor.  A warp with one
+      // masked window runs the general form for all of its windows, not both forms one after the other
+      // (3,000 windows of 101 codes, 2 % of the codes masked, -i 3: 198 us, now 109)
+      if (s < n) {
+        const int64_t slot = slot0 + s;
+        const int r = pb.p_read[slot];
+        const int64_t win = max(pb.p_diag[slot] - sp.I, -sp.Is);
+        masked = window_masked(mask, win, win + rd.lengths[r] + 2 * sp.I);
+      }
+      masked = __any_sync(0xffffffffu, masked);
+    }
     if (s < n) {
       const int64_t slot = pb.round_slots ? (int64_t)pb.round_slots[s] : slot0 + s;
       if constexpr (CM == 2) {
         rows += (unsigned long long)align_one_nuc<BWT>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb);
       } else if constexpr (CM == 3) {
-        // every cell exact: without masked codes no cell comes near the packed form's floor
-        const int r = pb.p_read[slot];
-        const int64_t win = max(pb.p_diag[slot] - sp.I, -sp.Is);
-        if (window_masked(mask, win, win + rd.lengths[r] + 2 * sp.I))
+        if (masked)
           rows += (unsigned long long)align_one<BWT, 0>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb, ctab);
         else
           rows += (unsigned long long)align_one_nuc<BWT>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb);

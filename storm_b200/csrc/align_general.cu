@@ -12,7 +12,7 @@ const void* align_general_kernel(int bw, int colour) {
     SG_ALIGN(15)
     SG_ALIGN(31)
     SG_ALIGN(41)
-  default: return (const void*)align_kernel<0, -1>;
+  default: return colour ? (const void*)align_kernel<0, 1> : (const void*)align_kernel<0, 0>;
   }
 #undef SG_ALIGN
 }

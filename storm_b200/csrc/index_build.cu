@@ -179,15 +179,21 @@ __global__ void __launch_bounds__(256) key_table_kernel(const uint32_t* __restri
       if (t == 0 || skeys[t - 1] != k) at[k - (uint32_t)k0] = (int32_t)t;
     }
   } else {
-    for (int k = threadIdx.x; k < kKeyBlock; k += 256) {
-      const uint32_t key = (uint32_t)(k0 + k);
-      int64_t a = lo, b = hi;  // the first position in [lo, hi] whose key is `key` or a later one
-      while (a < b) {
-        const int64_t mid = (a + b) >> 1;
-        if (skeys[mid] < key) a = mid + 1; else b = mid;
+    // the first position in [lo, hi] whose key is this one or a later one, the thread's searches side by side
+    int32_t a[PER], b[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) { a[i] = (int32_t)lo; b[i] = (int32_t)hi; }
+    for (int64_t left = hi - lo; left > 0; left >>= 1) {
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int32_t mid = (int32_t)(((int64_t)a[i] + b[i]) >> 1);
+        const bool before = a[i] < b[i] && skeys[mid] < (uint32_t)(k0 + threadIdx.x + 256 * i);
+        if (before) a[i] = mid + 1;
+        else b[i] = min(b[i], mid);
       }
-      at[k] = (int32_t)a;
     }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) at[threadIdx.x + 256 * i] = a[i];
   }
   __syncthreads();
   int32_t v[PER], m = 0x7fffffff;
@@ -284,25 +290,14 @@ struct Positions {
   int64_t total = 0;
 };
 
-int sort_seed(const uint8_t* d_codes, const Positions& at, const SeedDev& seed, DevIndex* out, Sorted* so,
-              unsigned long long* mom, uint32_t* scratch, int64_t room, StreamScratch& S, int64_t& L) {
-  cudaStream_t st = S.st;
-  const int64_t nkeys = (int64_t)1 << (2 * seed.weight), total = at.total;
-  out->weight = seed.weight;
-  out->nkeys = nkeys;
-  out->map = nullptr;
-  out->n = 0;
-  SG_CUDA(cudaMallocAsync(&out->first, sizeof(int32_t) * (nkeys + 1), st));
-  if (total == 0) {
-    SG_CUDA(cudaMemsetAsync(out->first, 0, sizeof(int32_t) * (nkeys + 1), st));
-    return 0;
-  }
+int sort_seed(const uint8_t* d_codes, const Positions& at, const SeedDev& seed, Sorted* so, unsigned long long* mom,
+              uint32_t* scratch, int64_t room, cudaStream_t st, int64_t& L) {
+  const int64_t total = at.total;
   so->total = total;
-  so->nblocks = nkeys / kKeyBlock + 1;  // the last one: the table's closing entry
+  so->nblocks = ((int64_t)1 << (2 * seed.weight)) / kKeyBlock + 1;  // the last one: the table's closing entry
   // The sorted list ends in its own arrays, whichever way the passes go; the other side of the sort is
   // scratch that every seed of the sequence uses.
   int64_t* const d_iv = so->iv;
-  SG_CUDA(S.alloc(&so->pos, total));
   const int passes = (2 * seed.weight + kRadixBits - 1) / kRadixBits;
   uint32_t* const sk = scratch;
   uint32_t* const sv = sk + room;
@@ -323,32 +318,27 @@ int sort_seed(const uint8_t* d_codes, const Positions& at, const SeedDev& seed, 
   return 0;
 }
 
-int fill_seed(DevIndex* out, const Sorted& so, int32_t cmax, int64_t longest, StreamScratch& S, int64_t& L) {
+// The map and the key table; where the repeat filter erases, `total` (on the device) gets the map's length.
+// scratch, room: of the sorts, which are done.
+int fill_seed(DevIndex* out, const Sorted& so, int32_t cmax, int64_t longest, int32_t* total, uint32_t* scratch, int64_t room,
+              StreamScratch& S, int64_t& L) {
   cudaStream_t st = S.st;
-  StreamScratch own(st);
   const int TB = 256;
-  int32_t *off = nullptr, *total = nullptr;
+  int32_t* off = nullptr;
   if (longest <= cmax) {  // nothing erased: the sorted positions are the map
     S.keep(so.pos);
     out->map = reinterpret_cast<int32_t*>(so.pos);
     out->n = so.total;
   } else {
-    uint8_t* keep;
-    int32_t* tmp;  // scan
-    SG_CUDA(own.alloc(&keep, so.total));
-    SG_CUDA(own.alloc(&off, so.total + 1));
-    SG_CUDA(own.alloc(&tmp, scan_tmp_elems(so.total) + 8));
+    off = reinterpret_cast<int32_t*>(scratch);
+    uint8_t* const keep = reinterpret_cast<uint8_t*>(scratch + room);
+    int32_t* const tmp = reinterpret_cast<int32_t*>(scratch + 2 * room);  // the scan's: fewer words than the sort's
     SG_CUDA(cudaMallocAsync(&out->map, sizeof(int32_t) * so.total, st));
-    total = off + so.total;
     keep_runs_kernel<<<(unsigned)std::min<int64_t>(blocks_of(so.total, TB), 148 * 16), TB, 0, st>>>(so.keys, so.total, cmax,
                                                                                                  keep);
     exclusive_scan<uint8_t, int32_t>(keep, off, so.total, total, tmp, st);
     kept_positions_kernel<<<blocks_of(so.total, TB), TB, 0, st>>>(keep, off, so.pos, so.total, out->map);
     L += 2 + scan_launches(so.total);
-    int32_t n = 0;
-    SG_CUDA(cudaMemcpyAsync(&n, total, sizeof(n), cudaMemcpyDeviceToHost, st));
-    SG_CUDA(cudaStreamSynchronize(st));
-    out->n = n;
     S.give_back(so.pos);
   }
   key_table_kernel<<<(unsigned)so.nblocks, 256, 0, st>>>(so.keys, so.total, out->nkeys, so.bound, off, total, out->first);
@@ -376,26 +366,39 @@ int build_indexes(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, co
     room = std::max(room, x.total);
     iv_words = std::max(iv_words, (int64_t)x.iv.size());
   }
-  // One block for everything a build needs only while it runs: with a block for each, the pool had to map
-  // new memory in one build of thirty (10 to 50 ms against 6; none in 300 builds of 48 Mbp since).
+  // The tables and the lists that become maps come first, in one order, then one block for everything that a
+  // build needs only while it runs: a rebuild then finds in the pool what the build before gave back.  With the
+  // block first it was cut from the place of a table, and with a block for each the pool's order changed from
+  // build to build; new memory was mapped (10 to 120 ms) now and then, or with tables of 1 GB and more each time.
+  StreamScratch S(st);
+  for (int q = 0; q < nseeds; ++q) {
+    out[q].weight = seeds[q].weight;
+    out[q].nkeys = (int64_t)1 << (2 * seeds[q].weight);
+    SG_CUDA(cudaMallocAsync(&out[q].first, sizeof(int32_t) * (out[q].nkeys + 1), st));
+  }
+  std::vector<uint32_t*> pos(nseeds, nullptr);
+  for (int q = 0; q < nseeds; ++q) {
+    if (at[q].total > 0) SG_CUDA(S.alloc(&pos[q], at[q].total));
+    else SG_CUDA(cudaMemsetAsync(out[q].first, 0, sizeof(int32_t) * (out[q].nkeys + 1), st));
+  }
   const int held = std::min(kGroup, nseeds);
   int64_t most_keys = 0;
   for (int q = 0; q < nseeds; ++q) most_keys = std::max(most_keys, (int64_t)1 << (2 * seeds[q].weight));
   int64_t size = 0;
   auto take = [&](int64_t bytes) { const int64_t at = size; size += (bytes + 255) & ~255LL; return at; };
   const int64_t at_scratch = take(sizeof(uint32_t) * 2 * room + radix_tmp_bytes(room));
-  const int64_t at_mom = take(sizeof(unsigned long long) * 3 * kGroup);
+  const int64_t at_mom = take((sizeof(unsigned long long) * 3 + sizeof(int32_t)) * kGroup);
   const int64_t at_keys = take(0), key_bytes = ((int64_t)sizeof(uint32_t) * room + 255) & ~255LL;
   take(key_bytes * held);
   const int64_t at_bound = take(0), bound_bytes = ((int64_t)sizeof(int32_t) * (most_keys / kKeyBlock + 2) + 255) & ~255LL;
   take(bound_bytes * held);
   const int64_t at_iv = take(0), iv_bytes = ((int64_t)sizeof(int64_t) * iv_words + 255) & ~255LL;
   take(iv_bytes * held);
-  StreamScratch S(st);
   uint8_t* block;
   SG_CUDA(S.alloc(&block, size));
   uint32_t* const scratch = reinterpret_cast<uint32_t*>(block + at_scratch);
   unsigned long long* const mom = reinterpret_cast<unsigned long long*>(block + at_mom);
+  int32_t* const lengths = reinterpret_cast<int32_t*>(mom + 3 * kGroup);  // of the maps with erased keys
   int64_t L = 0;
   for (int s0 = 0; s0 < nseeds; s0 += kGroup) {
     const int ng = std::min(kGroup, nseeds - s0);
@@ -405,19 +408,28 @@ int build_indexes(const uint8_t* d_codes, int64_t n_codes, const int32_t* rs, co
       so[q].keys = reinterpret_cast<uint32_t*>(block + at_keys + q * key_bytes);
       so[q].bound = reinterpret_cast<int32_t*>(block + at_bound + q * bound_bytes);
       so[q].iv = reinterpret_cast<int64_t*>(block + at_iv + q * iv_bytes);
-      if (const int rc = sort_seed(d_codes, at[s0 + q], seeds[s0 + q], &out[s0 + q], &so[q], mom + 3 * q, scratch, room, S, L))
-        return rc;
+      so[q].pos = pos[s0 + q];
+      if (at[s0 + q].total == 0) continue;
+      if (const int rc = sort_seed(d_codes, at[s0 + q], seeds[s0 + q], &so[q], mom + 3 * q, scratch, room, st, L)) return rc;
     }
     unsigned long long hm[3 * kGroup];
     SG_CUDA(cudaMemcpyAsync(hm, mom, sizeof(hm), cudaMemcpyDeviceToHost, st));
     SG_CUDA(cudaStreamSynchronize(st));
+    bool erased = false;
     for (int q = 0; q < ng; ++q) {
       if (so[q].total == 0) continue;
       DevIndex* o = &out[s0 + q];
       o->positions_indexed = so[q].total;
       o->cmax = repeat_cutoff(stdev_distance, so[q].total, hm[3 * q], hm[3 * q + 1]);
-      if (const int rc = fill_seed(o, so[q], o->cmax, (int64_t)hm[3 * q + 2], S, L)) return rc;
+      if (const int rc = fill_seed(o, so[q], o->cmax, (int64_t)hm[3 * q + 2], lengths + q, scratch, room, S, L)) return rc;
+      erased |= (int64_t)hm[3 * q + 2] > o->cmax;
     }
+    if (!erased) continue;
+    int32_t hl[kGroup];
+    SG_CUDA(cudaMemcpyAsync(hl, lengths, sizeof(hl), cudaMemcpyDeviceToHost, st));
+    SG_CUDA(cudaStreamSynchronize(st));
+    for (int q = 0; q < ng; ++q)
+      if (so[q].total > 0 && (int64_t)hm[3 * q + 2] > out[s0 + q].cmax) out[s0 + q].n = hl[q];
   }
   if (launches) *launches += L;
   return 0;

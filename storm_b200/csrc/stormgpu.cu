@@ -181,6 +181,23 @@ extern "C" int stormgpu_set_graphs(stormgpu_ctx* c, int enable) {
   return 0;
 }
 
+// Every buffer that a mapping call grows for itself (what its working memory limit counts).
+static void release_work(stormgpu_ctx* c) {
+  c->rcodes.release(); c->rlevels.release();
+  c->pstart.release(); c->pcount.release(); c->p_read.release(); c->p_diag.release();
+  c->big_list.release(); c->big_h.release(); c->small_list.release(); c->small_h.release();
+  c->huge_list.release(); c->huge_h.release();
+  c->a_score.release(); c->a_bound.release(); c->a_tblen.release(); c->big_tmp.release();
+  c->a_pos.release(); c->a_tb.release(); c->scratch.release(); c->counters.release();
+  c->foff.release(); c->fr.release(); c->fd.release(); c->flag.release();
+  c->rexp.release();
+  c->q_read.release(); c->q_diag.release(); c->q_ub.release(); c->k_ub.release(); c->p_ub.release();
+  c->k_diag.release(); c->long_list.release(); c->bstream.release(); c->wstream.release();
+  c->ord.release(); c->ord_tmp.release();
+  c->thr.release(); c->active.release(); c->round_cur.release(); c->round_slots.release();
+  c->work.used = 0;
+}
+
 extern "C" void stormgpu_close(stormgpu_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->p.device);
@@ -192,23 +209,12 @@ extern "C" void stormgpu_close(stormgpu_ctx* c) {
       cudaFree(r.d_gexp_alloc);
       for (auto& ix : r.idx) { cudaFree(ix.first); cudaFree(ix.map); }
     }
-  c->rcodes.release(); c->rlevels.release(); c->fcodes.release(); c->flevels.release();
-  c->first_levels.release(); c->lengths.release(); c->hits.release(); c->tb.release();
-  c->mapped.release();
-  c->pstart.release(); c->pcount.release(); c->p_read.release(); c->p_diag.release();
-  c->big_list.release(); c->big_h.release(); c->small_list.release(); c->small_h.release();
-  c->huge_list.release(); c->huge_h.release(); 
-  for (auto& e : c->gev) cudaEventDestroy(e);
-  c->a_score.release(); c->a_bound.release(); c->a_tblen.release(); c->big_tmp.release();
-  c->a_pos.release(); c->a_tb.release(); c->scratch.release(); c->counters.release();
-  c->foff.release(); c->fr.release(); c->fd.release(); c->flag.release();
-  c->rexp.release();
-  c->q_read.release(); c->q_diag.release(); c->q_ub.release(); c->k_ub.release(); c->p_ub.release();
-  c->k_diag.release(); c->long_list.release(); c->bstream.release(); c->wstream.release();
+  release_work(c);
+  c->fcodes.release(); c->flevels.release(); c->first_levels.release(); c->lengths.release();
+  c->hits.release(); c->tb.release(); c->mapped.release();
   c->gm_k0.release(); c->gm_v0.release(); c->gm_k1.release(); c->gm_v1.release(); c->gm_tmp.release();
   c->gm_base.release();
-  c->ord.release(); c->ord_tmp.release();
-  c->thr.release(); c->active.release(); c->round_cur.release(); c->round_slots.release();
+  for (auto& e : c->gev) cudaEventDestroy(e);
   for (auto& e : c->ev) cudaEventDestroy(e);
   for (auto& e : c->rev) cudaEventDestroy(e);
   cudaStreamDestroy(c->st);
@@ -1127,18 +1133,28 @@ int sg::map_device_impl(stormgpu_ctx* c, const stormgpu_reads* reads, const int1
       return map_cuts(c, reads, lengths, out, cuts);
     }
   }
-  WorkBudget* saved = g_work_budget;
-  g_work_budget = &c->work;
-  c->work.over = false;
-  int rc = map_device_once(c, reads, ls, out);
-  g_work_budget = saved;
+  int rc;
   const int64_t n = reads->n;
-  if (rc == STORMGPU_ENOMEM && c->work.over) {
-    if (n <= 1) {
+  for (;;) {
+    const bool fresh = c->work.used == 0;
+    WorkBudget* saved = g_work_budget;
+    g_work_budget = &c->work;
+    c->work.over = false;
+    rc = map_device_once(c, reads, ls, out);
+    g_work_budget = saved;
+    if (rc != STORMGPU_ENOMEM || !c->work.over) break;
+    if (n > 1) {
+      rc = kSplitBatch;
+      break;
+    }
+    // A single read with no room beside the buffers that larger batches, given up or of another shape, have
+    // left (reads whose streams fill most of the limit): once more without them.
+    if (fresh) {
       sg_set_error("one read needs more than the working memory limit of %lld bytes", (long long)c->work.limit);
       return STORMGPU_ENOMEM;
     }
-    rc = kSplitBatch;
+    SG_CUDA(cudaStreamSynchronize(c->st));
+    release_work(c);
   }
   if (rc != kSplitBatch) return rc;
   if (n <= 1) {

@@ -213,3 +213,38 @@ def test_read_streams_of_a_large_batch(fake, n, pieces):
     assert len(parts) == pieces
     assert [a for a, _ in parts] == [sum(k for _, k in parts[:q]) for q in range(pieces)]
     assert sum(k for _, k in parts) == n
+
+
+@pytest.mark.parametrize("n", [1, 300, 4000])
+@pytest.mark.parametrize("budget", [20, 24, 32, 48, 64])
+def test_batches_of_a_server_within_its_budget(fake, n, budget):
+    """A batch that needs more working memory than its slot has is mapped in halves, and those in halves
+    again: the buffers of an attempt that was given up don't take the room of its halves, so that the budget
+    which one read fits takes every batch."""
+    packed = np.zeros(1250, np.uint8)
+    mapped = [0]
+
+    def lists(name, args):  # 200 candidates a read (a single read: 8,000), a fifth of them pass
+        if "gather_fused_kernel" in name:
+            rd = fakert.arg(args, 0, ReadsDev)
+            rd.n = rd.n if rd.n > 1 else 40
+            go = fakert.arg(args, 3, GatherOut)
+            assert fake.room(go.fr)[0] >= 4 * go.cap and fake.room(go.fd)[0] >= 4 * go.cap
+            go.counters[7] = 200 * rd.n
+            go.counters[8] = 1 if 200 * rd.n > go.cap else 0
+            mapped[0] = rd.n
+        if "select_count_kernel" in name:
+            tiles = ctypes.cast(fakert.arg(args, 3, ctypes.c_void_p), ctypes.POINTER(ctypes.c_int64))
+            m = fakert.arg(args, 0)
+            tiles[(m + 4095) // 4096] = min(m, 40 * mapped[0])
+
+    s = api.Server(api.params(indels=15), ["######"], slots=1, budget_bytes=budget << 20)
+    s.add_reference(packed, packed, 5000, [])
+    s.build()
+    stride = 40
+    reads = api.ReadBatch(np.zeros((n, stride), np.uint8), np.full(n, 150, np.int16), np.zeros((n, stride), np.uint8))
+    one = api.ReadBatch(reads.codes[:1], reads.lengths[:1], reads.levels[:1])
+    with fake.hook(lists):
+        for batch in (reads, one, reads, reads, one):
+            s.poll(s.submit(batch))
+    s.close()

@@ -1,4 +1,6 @@
 // align_general.cu -- the general form of the alignment: colour space, and scores the packed form has no room for.
+// Widths of -i 3, 5, 7, 15 and 20 with their cells in registers; the others have them in local memory: 3,000
+// windows of 101 colours 674 us at -i 10, 535 at -i 15, 292 at -i 7.
 #include "align_core.cuh"
 
 namespace sg {

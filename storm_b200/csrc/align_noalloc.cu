@@ -141,7 +141,6 @@ extern "C" int stormgpu_align_noalloc(const stormgpu_params* params, const uint8
   pb.a_tb = tb;
   pb.tbs = tb_stride;
   pb.a_scratch = reinterpret_cast<uint32_t*>(scr + off_dir);
-  pb.scratch_words = (int64_t)read_len * wpr * n;
   if (n <= wave_slots(sp)) launch_align_wave(rd, sp, genome, mask, 0, n, pb, read_len, st);
   else launch_align(rd, sp, genome, mask, 0, n, pb, st);
   SG_CUDA(cudaGetLastError());

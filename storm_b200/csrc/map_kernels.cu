@@ -1,7 +1,8 @@
 // map_kernels.cu -- the kernels of one mapping pass (one reference sequence x one strand).
 //
-//  (hit gather: gather.cu; banded filter: sw_filter.cu)
-//  align                                            banded DP + traceback (alignment.c:488-734)
+//  (hit gather: gather.cu; banded filter: sw_filter.cu; score bound: score_bound.cu)
+//  align                                            banded DP + traceback (alignment.c:488-734): a thread per
+//                                                   candidate in align_core.cuh, a warp here
 //  replay                                           per-read top-4 update (run.c:664-691,
 //                                                   hit_map.c:50-144)
 #include "map_kernels.cuh"
@@ -70,7 +71,7 @@ void launch_init_results(int64_t n, stormgpu_hit* hits, uint8_t* mapped, uint8_t
 // ------------------------------------------------------------------------------ align
 
 // The packed nucleotide form has every band width up to 41 as a constant (the general form in local
-// memory ran -i 5 at 50 GCUPS, a twentieth of the packed form's rate); the others those listed with them.
+// memory ran -i 5 at 50 GCUPS, a twentieth of the packed form's rate); the others the widths listed with them.
 static const void* align_kernel_of(const ScoreParams& sp) {
   const int bw = 2 * sp.I + 1;
   const void* k = sp.packed == 2 ? align_unit_kernel(bw) : sp.packed ? align_packed_kernel(bw) : nullptr;
@@ -91,8 +92,8 @@ int64_t align_workers(int64_t nslots, const ScoreParams& sp) {
 // Directions stay in shared memory (a byte per cell: direction, bit 2 the SNP adjustment), where lane
 // 0 walks them back.  Every lane runs the same instructions in every step (those whose turn it is not
 // discard the result).  2L + 2I + 1 steps of about 60 instructions, against L (2I + 1) cells of 25 to 40:
-// 800 windows of 101 codes take 75 us at -i 15 where a thread each takes 148, 88 us in colours at -i 7
-// against 260 (the whole call).  The chain of a step (shuffle, sums, state, next row's codes) is what
+// 800 windows of 101 codes take 85 us at -i 15 where a thread each takes 127, 95 us in colours at -i 7
+// against 290 (the whole call).  The chain of a step (shuffle, sums, state, next row's codes) is what
 // bounds it: 31 % of the issue slots are taken with 5 warps an SM.
 template <bool COLOUR>
 __global__ void __launch_bounds__(32) align_wave_kernel(ReadsDev rd, ScoreParams sp, const uint8_t* __restrict__ genome,

@@ -60,8 +60,6 @@ struct PassBuffers {
   int32_t* active_count;
   int32_t* p_read;      // per slot, reads contiguous
   int32_t* p_diag;      // per slot, ascending within a read
-  int64_t p_cap;
-  unsigned long long* counters;  // [0] slots used, [1] overflow flag, [2] filter cells, [3] lookups, [4] positions
   // align outputs per slot
   int32_t* a_score;
   int32_t* a_bound;
@@ -70,7 +68,6 @@ struct PassBuffers {
   uint8_t* a_tb;        // tbs bytes per slot (end-to-start order)
   int64_t tbs;
   uint32_t* a_scratch;  // direction bits, see align kernel
-  int64_t scratch_words;
   // may be null; else a zeroed work cursor, and the align launch is a persistent grid of
   // align_workers() threads (scratch columns) taking slots from it
   unsigned long long* cursor;
@@ -106,10 +103,12 @@ void launch_align(const ReadsDev& r, const ScoreParams& sp, const uint8_t* genom
                   cudaStream_t st);
 // The same by a warp per slot (no scratch, no rounds), for bands of at most 32 cells: every slot when
 // there are at most wave_slots() of them (read from pb.npass_dev when given), else none.  maxL: longest
-// read.  Up to so many slots the warp form is the faster one: it takes 75 to 100 us for up to 1,000
-// windows of 101 codes whatever the band (all at once) and about 35 us more per further 1,000, a thread
-// per slot the same time from 64 to 8,000 windows: 88 us and 111 us in nucleotides at -i 3 and 7 (crossing
-// near 1,300 and 2,200), 149 us at -i 15 (near 3,700), 190 us at -i 1; 223, 260, 432 and 735 us in colours.
+// read.  The warp form takes 80 us for up to 1,000 windows of 101 codes whatever the band (all at once), 105
+// for 2,000, 140 for 3,000 and 153 for 4,000 (colours 95, 140, 178, 202); a thread per slot the same time from 64
+// to 8,000 windows: in nucleotides 80 us at -i 3, 93 at 7, 127 at 15, 115 at 1 (crossing near 700, 1,300, 2,600
+// and 2,500 windows), in colours 165, 292, 525 and 190 (near 2,700, 5,500, above, and 3,500).  The lines were
+// laid where these crossed when the thread form's traceback took longer (88, 111, 149, 190; 223, 260, 432, 735
+// us); between the crossing and the line the warp form takes up to 1.3 times as long.
 constexpr int wave_slots(const ScoreParams& sp) {
   const int bw = 2 * sp.I + 1;
   return bw > 32 ? 0 : !sp.colour && bw >= 7 && bw <= 15 ? 148 * 8 : 4096;

@@ -2,7 +2,7 @@
 //
 // Per pass: (1) per-tile digit histograms, stored digit-major so that (2) one exclusive scan
 // gives every (digit, tile) its output offset, then (3) each tile re-reads its items and
-// scatters them, ranking equal digits in input order with __match_any_sync inside a warp and
+// scatters them, ranking equal digits in input order with a ballot per digit bit inside a warp and
 // per-(warp, digit) offsets across the warps of the tile, through shared memory so that the
 // writes of one digit are contiguous.  Stability is what the
 // seed index needs: positions are generated in increasing order and must stay so per key.

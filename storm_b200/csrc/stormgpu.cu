@@ -616,8 +616,7 @@ static int enqueue_passes(stormgpu_ctx* c, const PassSetup& P, const AheadCaps& 
       PassBuffers pb;
       memset(&pb, 0, sizeof(pb));
       pb.pstart = c->pstart.p; pb.pcount = c->pcount.p;
-      pb.counters = c->counters.p;
-      pb.p_read = c->p_read.p; pb.p_diag = c->p_diag.p; pb.p_cap = kept_cap;
+      pb.p_read = c->p_read.p; pb.p_diag = c->p_diag.p;
       if (P.bound_H) {
         // the candidates whose score can exceed -t, in order
         select(cand_cap, kGsCand, 0, passing, {}, c->fr.p, c->fd.p, c->q_read.p, c->q_diag.p, pass_cap, nullptr, nullptr);
@@ -959,7 +958,6 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const L
       PassBuffers pb;
       memset(&pb, 0, sizeof(pb));
       pb.pstart = c->pstart.p; pb.pcount = c->pcount.p;
-      pb.counters = c->counters.p;
       int64_t nkept = npass;  // candidates that are aligned
       if (npass > 0 && bound_H) {
         // those whose score can exceed -t, in order
@@ -979,7 +977,7 @@ static int map_device_once(stormgpu_ctx* c, const stormgpu_reads* reads, const L
             c->a_tblen.grow(nkept) || c->a_pos.grow(nkept * 4) || c->a_tb.grow(nkept * tbs) ||
             (bound_H && (c->k_ub.grow(nkept) || c->p_ub.grow(nkept))))
           return STORMGPU_ENOMEM;
-        pb.p_read = c->p_read.p; pb.p_diag = c->p_diag.p; pb.p_cap = c->p_read.cap;
+        pb.p_read = c->p_read.p; pb.p_diag = c->p_diag.p;
         if (bound_H) {
           launch_select_write(npass, nullptr, c->flag.p, c->foff.p, c->q_read.p, c->q_diag.p, c->p_read.p, c->k_diag.p,
                               nkept, c->q_ub.p, c->k_ub.p, st);

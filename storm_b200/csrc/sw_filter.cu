@@ -3,8 +3,10 @@
 // candidates that pass.
 //
 // Semantics: those of alignment_avx2__align_{hexa,octa,quad,pair} (alignment_simd.c:2613-3404)
-// for one hit of W cells, as restated in filter_ref.cuh (sw_filter_one).  Here the W cells of
-// one anti-diagonal step live in W/2 registers, two signed 16-bit cells each (filter_core.cuh):
+// for one hit of W cells, as restated in filter_ref.cuh (sw_filter_one).  Bands of 4 cells and more with
+// scores that have score bytes run on band_core.cuh, whose head describes its cells.  W = 2 and other scores
+// run on filter_core.cuh, where the W cells of one anti-diagonal step live in W/2 registers, two signed
+// 16-bit cells each:
 //   * the per-cell score is one prmt whose selector is the difference of a read byte and a
 //     genome byte (no compare, no branch);
 //   * I = max(P, P of the neighbour cell, 0) with P = max(I[l-1] - ext, M[l-1] - open), and

@@ -38,7 +38,7 @@ struct FilterJob {
   BandConst band;
   const uint32_t* bs;
   int64_t bwords;  // of a row of bs
-  int rows;  // with a cursor: rows of 256 candidates in a block's tile (0 = 8); without: 8
+  int rows;  // with a cursor: rows of 256 candidates in a block's tile (0 = 8); without: 8, fewer for short lists
 };
 
 constexpr int64_t kGexpPad = 4096;   // bytes of padding around a byte-expanded sequence

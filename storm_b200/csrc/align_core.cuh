@@ -93,6 +93,42 @@ struct BandWindow {
   __device__ __forceinline__ int mcode(int c) const { return (int)((m[c >> 5] >> (2 * (c & 31))) & 3u); }
 };
 
+// Traceback over the direction words of the rows from i (cell c) up: emit(i, c, direction) for every cell of
+// the path.  A path leaves a row once (every step but LEFT goes up), so the rows' words are loaded four rows
+// ahead whatever the path does; walked one cell at a time, each step waits for its own word.  For the
+// candidates that a mapping aligns, whose paths are long and have few gaps: 9,001 reads of up to 251 codes at
+// -i 5, alignments 4.95 ms, 5.18 without (12,000 of 100 codes at -i 20: 17.3 and 16.8).  In windows whose paths wander, as the unit entry points get them, the
+// lanes of a warp part in it, and every form is faster without (see align_one).
+template <int WPR, int LEFT, int TOP, class Emit>
+__device__ __forceinline__ void trace_rows(const uint32_t* scr, int64_t ns, int64_t sl, int i, int c, int BW, Emit emit) {
+  constexpr int PF = 4;
+  uint32_t w[PF][WPR];
+  auto load = [&](int q, int row) {
+#pragma unroll
+    for (int k = 0; k < WPR; ++k) w[q][k] = row >= 0 ? scr[((int64_t)row * WPR + k) * ns + sl] : 0u;
+  };
+#pragma unroll
+  for (int q = 0; q < PF; ++q) load(q, i - q);
+  for (;;) {
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      int from;
+      for (;;) {
+        uint32_t x = w[q][0];
+        if (WPR > 1 && c >= 16) x = w[q][WPR > 1 ? 1 : 0];
+        if (WPR > 2 && c >= 32) x = w[q][WPR > 2 ? 2 : 0];
+        from = (x >> ((2 * c) & 31)) & 3;
+        emit(i, c, from);
+        if (from != LEFT) break;
+        if (--c < 0) return;
+      }
+      if (from == TOP) ++c;
+      if (--i < 0 || c >= BW) return;
+      load(q, i - (PF - 1));
+    }
+  }
+}
+
 // BWT > 0: the band width 2I + 1 as a constant, so that the row arrays live in registers;
 // BWT = 0: any width up to kMaxBand (arrays in local memory).  CM: 0 nucleotide, 1 colour space (the
 // colour state machine compiled in; ctab: the table of colour_step); the kernel's CM = 2 and 3 run the
@@ -235,7 +271,8 @@ __device__ __forceinline__ int align_one(const ReadsDev& rd, const ScoreParams& 
       else if (!colour || !(colr || (adj && i != 0 && j != 0))) put(0x4 | rc);
       else { put(0x8 | rc); colr ^= rc ^ f; }
     };
-    // (the direction words loaded rows ahead, whatever the path does, were slower at every width)
+    // (with the direction words loaded rows ahead as in trace_rows: 10,000 windows at -i 15 464 us, without 231;
+    // 5,000 of 101 colours at -i 7 445 and 300)
     int i = bi, c = bj - bi;
     while (i >= 0 && i < L && c >= 0 && c < BW) {
       const uint32_t wdir = scr[((int64_t)i * wpr + ((2 * c) >> 5)) * ns + sl];
@@ -333,7 +370,7 @@ __device__ __forceinline__ int packed_row(int (&v)[BW], uint32_t (&wd)[(2 * BW +
   return mol;
 }
 
-template <int BW>
+template <int BW, bool AHEAD>
 __device__ __forceinline__ int align_one_nuc(const ReadsDev& rd, const ScoreParams& sp,
                                              const uint8_t* __restrict__ genome, const uint8_t* __restrict__ mask,
                                              int64_t slot, int64_t sl, int64_t ns, const PassBuffers& pb) {
@@ -418,10 +455,8 @@ __device__ __forceinline__ int align_one_nuc(const ReadsDev& rd, const ScorePara
   uint8_t* tb = pb.a_tb + slot * pb.tbs;
   if (bi >= 0 && bnd >= thr && best > thr) {  // alignment.c:642-734
     uint8_t cur = 0;
-    int i = bi, c = bj - bi;
-    while (i >= 0 && i < L && c >= 0 && c < BW) {
-      const uint32_t wdir = scr[((int64_t)i * wpr + ((2 * c) >> 5)) * ns + sl];
-      const int from = (wdir >> ((2 * c) & 31)) & 3;  // 2 corner, 1 top, 0 left
+    // directions: 2 corner, 1 top, 0 left
+    auto cell = [&](int i, int c, int from) {
       const int j = i + c;
       i0 = i;
       j0 = j;
@@ -433,9 +468,19 @@ __device__ __forceinline__ int align_one_nuc(const ReadsDev& rd, const ScorePara
       if (tl & 1) { cur |= (uint8_t)op; tb[tl >> 1] = cur; }
       else { cur = (uint8_t)(op << 4); tb[tl >> 1] = cur; }
       tl++;
-      if (from == 1) { i--; c++; }
-      else if (from == 0) { c--; }
-      else { i--; }
+    };
+    if (AHEAD) {
+      trace_rows<wpr, 0, 1>(scr, ns, sl, bi, bj - bi, BW, cell);
+    } else {
+      int i = bi, c = bj - bi;
+      while (i >= 0 && i < L && c >= 0 && c < BW) {
+        const uint32_t wdir = scr[((int64_t)i * wpr + ((2 * c) >> 5)) * ns + sl];
+        const int from = (wdir >> ((2 * c) & 31)) & 3;
+        cell(i, c, from);
+        if (from == 1) { i--; c++; }
+        else if (from == 0) { c--; }
+        else { i--; }
+      }
     }
   }
   pb.a_tblen[slot] = tl;
@@ -514,12 +559,12 @@ __global__ void __launch_bounds__(128, align_blocks(BWT, CM)) align_kernel(Reads
     if (s < n) {
       const int64_t slot = pb.round_slots ? (int64_t)pb.round_slots[s] : slot0 + s;
       if constexpr (CM == 2) {
-        rows += (unsigned long long)align_one_nuc<BWT>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb);
+        rows += (unsigned long long)align_one_nuc<BWT, CM == 2>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb);
       } else if constexpr (CM == 3) {
         if (masked)
           rows += (unsigned long long)align_one<BWT, 0>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb, ctab);
         else
-          rows += (unsigned long long)align_one_nuc<BWT>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb);
+          rows += (unsigned long long)align_one_nuc<BWT, CM == 2>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb);
       } else {
         rows += (unsigned long long)align_one<BWT, CM>(rd, sp, genome, mask, slot, steal ? tid : s, ns, pb, ctab);
       }

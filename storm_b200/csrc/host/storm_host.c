@@ -1352,6 +1352,10 @@ static int write_sam_records(growbuf *g, const sh_sam_opts *o, const sh_refs *re
   return 0;
 }
 
+/* Whether everything written to f has gone out: a chunk goes past stdio's buffer, and a write of it that
+ * failed leaves nothing there for the caller's fclose to fail on. */
+static int gone_out(FILE *f) { return fflush(f) == 0 && !ferror(f); }
+
 int sh_write_sam(FILE *f, const sh_sam_opts *o, const sh_refs *refs, const sh_reads *reads,
                  const stormgpu_results *res, int64_t first, int64_t count, int header) {
   const int colour = o->colour;
@@ -1403,9 +1407,7 @@ int sh_write_sam(FILE *f, const sh_sam_opts *o, const sh_refs *refs, const sh_re
     free(chk);
   }
   if (rc == STORMGPU_ENOMEM) return fail(STORMGPU_ENOMEM, "Out of memory while writing the SAM output.");
-  /* a chunk goes past stdio's buffer: a write that failed leaves nothing there for the caller's fclose to
-   * fail on */
-  if (rc || fflush(f) != 0 || ferror(f)) return fail(STORMGPU_EINVAL, "Cannot write the SAM output.");
+  if (rc || !gone_out(f)) return fail(STORMGPU_EINVAL, "Cannot write the SAM output.");
   return 0;
 }
 
@@ -1731,6 +1733,7 @@ int sh_write_genome_map_sam(FILE *f, const sh_sam_opts *o, const sh_refs *refs, 
     free(chk);
   }
   if (nomem) return fail(STORMGPU_ENOMEM, "Out of memory while writing the SAM output.");
+  if (!gone_out(f)) return fail(STORMGPU_EINVAL, "Cannot write the SAM output.");
   return 0;
 }
 
@@ -1817,6 +1820,7 @@ int sh_write_unmapped_fastq(FILE *f, const sh_sam_opts *o, const sh_reads *reads
   free(bufs);
   free(lens);
   if (nomem) return fail(STORMGPU_ENOMEM, "Out of memory while writing the unmapped reads.");
+  if (!gone_out(f)) return fail(STORMGPU_EINVAL, "Cannot write the unmapped reads.");
   return 0;
 }
 

@@ -1,4 +1,4 @@
-"""A SAM file that cannot be written whole is an error: the writer under a limit on the file's size
+"""A SAM or FASTQ file that cannot be written whole is an error: the writers under a limit on the file's size
 (SIGXFSZ ignored, so that a write past it fails as on a full disk), with outputs of several chunks cut
 inside the first chunk, between chunks and inside the last one."""
 import subprocess
@@ -26,7 +26,10 @@ tb, mapped = np.zeros((n * 4, stride), np.uint8), np.zeros(n, np.uint8)
 res = api.MapResults(n, stride, (hits, tb, mapped)).cstruct()
 o = pipeline.ShSamOpts(0, 1, 1, 0, 0, 100, 9, 33, 1, (C.c_char_p * 1)(b"x"))  # -A: every read a record
 L = pipeline._bind()
-rc = L.sh_write_sam_path(b"o.sam", C.byref(o), C.byref(ref._s), C.byref(reads._s), C.byref(res))
+if sys.argv[2] == "sam":
+    rc = L.sh_write_sam_path(b"o.sam", C.byref(o), C.byref(ref._s), C.byref(reads._s), C.byref(res))
+else:  # the unmapped reads as FASTQ
+    rc = L.sh_write_unmapped_fastq_path(b"o.sam", C.byref(o), C.byref(reads._s), C.byref(res))
 print(rc, L.sh_last_error().decode() if rc else "")
 """
 
@@ -41,8 +44,8 @@ def inputs(tmp_path_factory):
     return d
 
 
-def _write(d, limit):
-    p = subprocess.run([sys.executable, "-c", CHILD, str(limit)], cwd=d, env={"PYTHONPATH": ROOT, "OMP_NUM_THREADS": "4"},
+def _write(d, limit, what="sam"):
+    p = subprocess.run([sys.executable, "-c", CHILD, str(limit), what], cwd=d, env={"PYTHONPATH": ROOT, "OMP_NUM_THREADS": "4"},
                        capture_output=True, text=True, timeout=300)
     assert p.returncode == 0, p.stderr
     rc, _, msg = p.stdout.strip().partition(" ")
@@ -56,5 +59,14 @@ def test_a_sam_file_cut_short_is_an_error(inputs):
     # within the header's chunk, at multiples of a page (nothing is left in stdio's buffer), within the last one
     for limit in (50, 4096, 65536, 1_000_000, 2_000_896, size - 4097, size - 1):
         rc, msg, got = _write(inputs, limit)
+        assert got <= limit < size
+        assert rc != 0 and msg, limit
+
+
+def test_an_unmapped_read_file_cut_short_is_an_error(inputs):
+    rc, _, size = _write(inputs, 0, "fastq")
+    assert rc == 0 and size > 3_000_000
+    for limit in (4096, 1_000_000, size - 4097, size - 1):
+        rc, msg, got = _write(inputs, limit, "fastq")
         assert got <= limit < size
         assert rc != 0 and msg, limit

@@ -129,7 +129,8 @@ int stormgpu_add_reference(stormgpu_ctx *ctx, const uint8_t *codes, const uint8_
 
 /* Build the device-resident spaced-seed index of every reference sequence for every seed.
  * Replaces: index__build_reference (index.c:19-195), called per sequence per seed
- * (run.c:876-884). */
+ * (run.c:876-884).  After a build that failed mapping is refused (STORMGPU_ESTATE) until one goes
+ * through. */
 int stormgpu_build_index(stormgpu_ctx *ctx);
 
 /* Map a batch: every read against every sequence, forward then reverse, the top-4 table
@@ -185,7 +186,8 @@ void stormgpu_server_close(stormgpu_server *s);
  * genome_map.c:551-796): the reads whose rank-0 alignment exists -- and, when
  * uniqueness_threshold > 0 (-u), whose rank-0 score leads the rank-1 score by at least that --
  * in (sequence, rank-0 start) order, reads of one position in read order.  Works on the results
- * of the last stormgpu_map call on ctx, which stay on the device; order (host) holds n int32,
+ * of the last stormgpu_map call on ctx, which stay on the device (a call that failed leaves none:
+ * STORMGPU_ESTATE); order (host) holds n int32,
  * *n_placed receives how many are placed. */
 int stormgpu_genome_map_greedy(stormgpu_ctx *ctx, int32_t uniqueness_threshold, int32_t *order,
                                int64_t *n_placed);
